@@ -367,6 +367,17 @@ cudaError_t matmul_few_sliced(cudaStream_t stream, const Mat& w, const void* pac
 bool matmul_few_experts_supported(const Mat& w, const Mat* up, uint32_t n_rows, uint32_t n_experts, uint32_t n_tokens);
 cudaError_t matmul_few_experts(cudaStream_t stream, const Mat& w, const Mat* up, uint32_t n_rows, uint32_t n_experts, const void* packed,
                                const uint32_t* offsets, const uint32_t* entries, float* y, uint32_t n_tokens, uint32_t n_entries);
+// Products of a few rows with f32 operands (kernels_matmul_exact.cu): up to four Q4_0 matrices that
+// share the rows, with the rows' RMSNorm when given, in one launch; gate and up of a SwiGLU; the
+// experts of a grouped batch. `matmul` and `matmul_experts` hand over to these when their shape allows
+// (BOBCAT_NO_EXACT_MATMUL=1 keeps them on the tile kernels).
+bool matmul_exact_supported(const Mat& w, uint32_t n_tokens);
+cudaError_t matmul_exact(cudaStream_t stream, const Mat* const* ws, float* const* ys, const uint32_t* strides, int n, const float* x, Norm norm,
+                         uint32_t n_tokens, int32_t store);
+cudaError_t matmul_exact_swiglu(cudaStream_t stream, const Mat& gate, const Mat& up, const float* x, Norm norm, float* y, uint32_t n_tokens);
+bool matmul_exact_experts_supported(const Mat& w, const Mat* up, uint32_t n_rows, uint32_t n_tokens);
+cudaError_t matmul_exact_experts(cudaStream_t stream, const Mat& w, const Mat* up, uint32_t n_rows, uint32_t n_experts, const float* x, bool gather,
+                                 const uint32_t* offsets, const uint32_t* entries, uint32_t n_used, float* y, uint32_t n_tokens);
 // Nonzero once a bounded wait inside the tensor-core prefill kernel gave up (1: producers on a free
 // stage, 2: epilogue on the accumulator, 3: token copy on a free stage, 4: MMA thread on a full stage).
 int matmul_error_flag();

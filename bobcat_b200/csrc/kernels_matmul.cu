@@ -237,6 +237,10 @@ cudaError_t matmul(cudaStream_t stream, const Mat& w, const float* x, float* y, 
         if (e != cudaSuccess) return e;
         return matmul_umma(stream, w, pack, y, n_tokens, y_stride, store);
     }
+    if (matmul_exact_supported(w, n_tokens) && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
+        const Mat* ws[1] = {&w};
+        return matmul_exact(stream, ws, &y, &y_stride, 1, x, Norm{}, n_tokens, store);
+    }
     MatmulParams p{w, x, y, n_tokens, y_stride, store};
     dim3 grid((n_tokens + kTileTokens - 1) / kTileTokens, (w.n_rows + kTileRows - 1) / kTileRows);
     matmul_simt_kernel<<<grid, kThreads, 0, stream>>>(p);

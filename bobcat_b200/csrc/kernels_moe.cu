@@ -447,6 +447,8 @@ cudaError_t matmul_experts(cudaStream_t stream, const Mat& w, const Mat* up, uin
     if (n_tokens == 0) return cudaSuccess;
     if (scratch && matmul_experts_umma_supported(w, up, n_tokens))
         return matmul_experts_umma(stream, w, up, n_rows, n_experts, x, gather, offsets, entries, n_used, y, n_tokens, scratch);
+    if (matmul_exact_experts_supported(w, up, n_rows, n_tokens) && (reinterpret_cast<uintptr_t>(x) & 15) == 0)
+        return matmul_exact_experts(stream, w, up, n_rows, n_experts, x, gather, offsets, entries, n_used, y, n_tokens);
     GroupedParams p{w, up ? *up : w, up != nullptr, x, gather, offsets, entries, y, n_rows, n_used};
     // Any one expert can receive up to n_tokens entries (a token picks an expert at most once).
     dim3 grid((n_tokens + 63) / 64, (n_rows + 63) / 64, n_experts);

@@ -175,6 +175,12 @@ struct Recorder {
     // ffn = silu(gate x^) * (up x^) over the batch, x^ the normalised rows.
     void normed_swiglu(const float* x, const float* norm_weight, uint32_t n, const k::Mat& gate, const k::Mat& up, float* y) {
         if (!tensor_products() || !k::matmul_umma_swiglu_supported(gate, up, n, min_tensor_rows)) {
+            // A few rows with f32 operands: the normalisation and both matrices in one launch.
+            if (k::matmul_exact_supported(gate, n) && k::matmul_exact_supported(up, n) && gate.n_rows == up.n_rows && gate.n_cols == up.n_cols) {
+                run("matmul_swiglu", gate.n_rows, gate.n_cols, 2 * gate.bytes(), 1,
+                    [&] { return k::matmul_exact_swiglu(stream, gate, up, x, norm(norm_weight), y, n); });
+                return;
+            }
             // The up projection's store combines with the gate projection already in the buffer.
             normed_matmuls(x, norm_weight, n, {{&gate, y, BC_STORE_OVERWRITE}, {&up, y, BC_STORE_SWIGLU}});
             return;
@@ -221,6 +227,26 @@ struct Recorder {
         for (const Product& q : products) {
             fused = fused && tensor_products() && k::matmul_umma_supported(*q.w, n, min_tensor_rows);
             bytes = std::max(bytes, (size_t)k::matmul_scratch_bytes(*q.w, n));
+        }
+        // A few rows with f32 operands: the normalisation and all the products in one launch.
+        bool exact = !fused && products.size() <= 4;
+        for (const Product& q : products) exact = exact && q.store == BC_STORE_OVERWRITE && k::matmul_exact_supported(*q.w, n) && q.w->n_cols == cols;
+        if (exact) {
+            const k::Mat* ws[4];
+            float* ys[4];
+            uint32_t strides[4], rows = 0;
+            uint64_t bytes_read = 0;
+            int count = 0;
+            for (const Product& q : products) {
+                ws[count] = q.w;
+                ys[count] = q.y;
+                strides[count++] = q.w->n_rows;
+                rows += q.w->n_rows;
+                bytes_read += q.w->bytes();
+            }
+            run("matmul", rows, cols, bytes_read, 1,
+                [&] { return k::matmul_exact(stream, ws, ys, strides, count, x, norm(norm_weight), n, BC_STORE_OVERWRITE); });
+            return;
         }
         if (!fused) {
             run("rms_norm", n, cols, 0, 1, [&] { return k::rms_norm(stream, x, norm_weight, s.normed, cols, n, hp.norm_eps); });

@@ -463,7 +463,9 @@ bc_status bc_seq_prefill(bc_seq* s, const uint32_t* tokens, size_t n_tokens, flo
         auto encode_start = Clock::now();
         Recorder r(*s);
         size_t layer_stride = (size_t)s->trace_rows * n_embd;
-        r.batch(pos, count, last, traced || (final_norm && last), layer_stride);
+        const bool traces = traced || (final_norm && last);
+        if (count == 1 && !traces) r.step(pos, last, false);  // a lone token is a decode step
+        else r.batch(pos, count, last, traces, layer_stride);
         encode += since(encode_start);
         if (r.status != BC_OK) {
             cudaStreamSynchronize(stream);
