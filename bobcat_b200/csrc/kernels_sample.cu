@@ -7,10 +7,9 @@
 // top-p cut, the min-p floor, the draw). Walking a sorted list until a running sum crosses a
 // target is a selection problem: it needs the key at which the sum crosses, not the order of
 // everything else. Logits map to 32-bit keys that sort the same way (descending logit = ascending
-// key), and a key is found eight bits at a time: a histogram of the summed weight per value of the
-// next eight bits (over the candidates that match the bits decided so far), a walk over its 256
-// buckets to the one where the running sum crosses, four rounds. So every step is a few passes
-// over the logits by one CTA:
+// key), and a key is found four bits at a time: the summed weight per value of the next four bits
+// (over the candidates that match the bits decided so far), a walk over the 16 sums to the one
+// where the running sum crosses, eight rounds:
 //   top-k   - the key of the k-th largest logit (weights 1),
 //   top-p   - the key where the softmax at temperature one, summed from the largest logit down,
 //             reaches top_p,
@@ -20,8 +19,13 @@
 // Where the reference's unstable sort breaks ties between equal logits arbitrarily at a cut, every
 // logit equal to the cut value is kept here. The uniform draw comes from the caller (the
 // reference draws it from fastrand, whose stream is the host's business), so the kernel is a
-// function of its inputs; its histogram sums are taken in whatever order the threads arrive, so a
-// draw that lands within rounding of a boundary between two tokens may fall either way.
+// function of its inputs. All sums are taken in a fixed order.
+//
+// What bounds it: the chain of rounds. A cluster of eight CTAs holds the logits in its shared memory (8 192
+// or 18 992 per CTA at the vocabularies in use), so a round reads nothing from global memory; a thread keeps its 16 sums in
+// registers (selects and adds, no atomics: most logits share the first bits of their keys, and a
+// histogram by shared-memory float atomics spent its time on that contention, in one CTA 587 us per draw at 65 536
+// logits with top-k and top-p); the CTAs exchange 16 floats each through distributed shared memory.
 
 #include <cfloat>
 
@@ -54,102 +58,159 @@ struct SampleParams {
     uint32_t* readback;
 };
 
+constexpr uint32_t kCtas = 8, kWarps = kSampleThreads / 32;
+constexpr int kDigits = 16;
+
 struct Shared {
-    float hist[256];
-    float reduce[32];
-    uint32_t reduce_index[32];
-    uint32_t counts[kSampleThreads / 32];
-    uint32_t prefix;   // key bits decided so far
-    float below;       // weight of keys below the decided prefix
-    float scalar;
-    uint32_t word;
+    float warps[kWarps][kDigits];     // the warps' sums of a round
+    float mine[2][kDigits];           // this CTA's, read by the cluster; the parity alternates between exchanges
+    float all[kCtas][kDigits];        // every CTA's
+    uint32_t counts[kWarps];
 };
 
-__device__ float block_max(float v, Shared& sh) {
-    v = warp_max(v);
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) sh.reduce[threadIdx.x >> 5] = v;
-    __syncthreads();
-    float m = sh.reduce[0];
-    for (int w = 1; w < kSampleThreads / 32; ++w) m = fmaxf(m, sh.reduce[w]);
-    return m;
+__device__ __forceinline__ void cluster_sync() { asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory"); }
+__device__ __forceinline__ float remote_float(const float* p, uint32_t rank) {
+    uint32_t at;
+    float v;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(at) : "memory");
+    return v;
 }
 
-__device__ float block_total(float v, Shared& sh) {
-    v = warp_sum(v);
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) sh.reduce[threadIdx.x >> 5] = v;
-    __syncthreads();
-    float total = 0.f;
-    for (int w = 0; w < kSampleThreads / 32; ++w) total += sh.reduce[w];
-    return total;
-}
+// The CTA's share of the logits and the exchange with the other CTAs.
+struct Slice {
+    const float* v;     // shared memory, or the logits themselves when a share does not fit there
+    uint32_t count;     // logits of this CTA
+    uint32_t parity;    // of the next exchange
+    Shared& sh;
+
+    // sh.mine[parity] of every CTA into sh.all. Whoever writes sh.mine again does so with the
+    // other parity, and the exchange after that orders it behind this one's reads.
+    __device__ void exchange(int n) {
+        cluster_sync();
+        for (int i = threadIdx.x; i < (int)kCtas * n; i += kSampleThreads) sh.all[i / n][i % n] = remote_float(&sh.mine[parity][i % n], i / n);
+        __syncthreads();
+        parity ^= 1;
+    }
+    // The sums over the CTAs, in rank order, into sh.all[0].
+    __device__ void exchange_sums() {
+        cluster_sync();
+        if (threadIdx.x < kDigits) {
+            float x = 0.f;
+#pragma unroll
+            for (uint32_t r = 0; r < kCtas; ++r) x += remote_float(&sh.mine[parity][threadIdx.x], r);
+            sh.all[0][threadIdx.x] = x;
+        }
+        __syncthreads();
+        parity ^= 1;
+    }
+    __device__ float total(float x, bool largest) {
+        x = largest ? warp_max(x) : warp_sum(x);
+        __syncthreads();
+        if ((threadIdx.x & 31) == 0) sh.warps[threadIdx.x >> 5][0] = x;
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            x = sh.warps[threadIdx.x][0];
+            x = largest ? warp_max(x) : warp_sum(x);
+            if (threadIdx.x == 0) sh.mine[parity][0] = x;
+        }
+        exchange(1);
+        float t = sh.all[0][0];
+        for (uint32_t r = 1; r < kCtas; ++r) t = largest ? fmaxf(t, sh.all[r][0]) : t + sh.all[r][0];
+        return t;
+    }
+};
 
 // The smallest key K among the candidates (keys <= limit) at which the weight summed over keys
 // <= K passes `target` (exceeds it, or reaches it when `inclusive`). `weight(logit)` gives a
-// candidate's weight. Returns K; sh.below then holds the weight of the candidates with smaller keys.
+// candidate's weight. Returns K; `below` then holds the weight of the candidates with smaller keys.
 // When the target lies beyond the total (rounding), the largest candidate key is returned.
 template <typename W>
-__device__ uint32_t select_key(const SampleParams& p, uint32_t limit, float target, bool inclusive, W weight, Shared& sh) {
-    if (threadIdx.x == 0) {
-        sh.prefix = 0;
-        sh.below = 0.f;
-    }
-    for (int shift = 24; shift >= 0; shift -= 8) {
-        for (int b = threadIdx.x; b < 256; b += kSampleThreads) sh.hist[b] = 0.f;
-        __syncthreads();
-        const uint32_t prefix = sh.prefix;
-        for (uint32_t i = threadIdx.x; i < p.n; i += kSampleThreads) {
-            const float v = p.logits[i];
+__device__ uint32_t select_key(Slice& slice, uint32_t limit, float target, bool inclusive, W weight, float& below) {
+    Shared& sh = slice.sh;
+    uint32_t prefix = 0;
+    below = 0.f;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int shift = 28; shift >= 0; shift -= 4) {
+        float sums[kDigits];
+#pragma unroll
+        for (int d = 0; d < kDigits; ++d) sums[d] = 0.f;
+        for (uint32_t i = threadIdx.x; i < slice.count; i += kSampleThreads) {
+            const float v = slice.v[i];
             const uint32_t key = descending_key(v);
-            if (key > limit) continue;
-            if (shift < 24 && (key >> (shift + 8)) != prefix) continue;
-            atomicAdd(&sh.hist[(key >> shift) & 255u], weight(v));
+            if (key > limit || (shift < 28 && (key >> (shift + 4)) != prefix)) continue;
+            const uint32_t digit = (key >> shift) & 15u;
+            const float w = weight(v);
+#pragma unroll
+            for (int d = 0; d < kDigits; ++d) sums[d] += digit == (uint32_t)d ? w : 0.f;
         }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            float running = sh.below;
-            int chosen = -1, last_filled = -1;
-            for (int b = 0; b < 256; ++b) {
-                const float h = sh.hist[b];
-                if (h <= 0.f) continue;
-                last_filled = b;
-                const float with = running + h;
-                if (inclusive ? with >= target : with > target) {
-                    chosen = b;
-                    break;
-                }
-                running = with;
+        // A warp's 16 sums by halving: after the step of `half`, a lane keeps half as many digits.
+        // Lanes 2 d and 2 d + 1 end up with digit d.
+#pragma unroll
+        for (int half = 8, bit = 16; half >= 1; half >>= 1, bit >>= 1) {
+#pragma unroll
+            for (int d = 0; d < half; ++d) {
+                const bool high = lane & bit;
+                const float give = high ? sums[d] : sums[d + half];
+                const float got = __shfl_xor_sync(0xffffffffu, give, bit);
+                sums[d] = (high ? sums[d + half] : sums[d]) + got;
             }
-            if (chosen < 0) {
-                // Past the end: settle on the last filled bucket, with everything before it below.
-                chosen = last_filled < 0 ? 0 : last_filled;
-                running = sh.below;
-                for (int b = 0; b < chosen; ++b) running += sh.hist[b];
-            }
-            sh.below = running;
-            sh.prefix = (prefix << 8) | (uint32_t)chosen;
         }
+        sums[0] += __shfl_xor_sync(0xffffffffu, sums[0], 1);
         __syncthreads();
+        if ((lane & 1) == 0) sh.warps[warp][lane >> 1] = sums[0];
+        __syncthreads();
+        if (threadIdx.x < kDigits) {
+            float x = 0.f;
+            for (uint32_t w = 0; w < kWarps; ++w) x += sh.warps[w][threadIdx.x];
+            sh.mine[slice.parity][threadIdx.x] = x;
+        }
+        slice.exchange_sums();
+        // Every thread walks the same 16 sums.
+        float running = below, before_last = below;
+        int chosen = -1, last_filled = 0;
+#pragma unroll 1
+        for (int d = 0; d < kDigits; ++d) {
+            const float h = sh.all[0][d];
+            if (h <= 0.f) continue;
+            last_filled = d;
+            before_last = running;
+            const float with = running + h;
+            if (inclusive ? with >= target : with > target) {
+                chosen = d;
+                break;
+            }
+            running = with;
+        }
+        if (chosen < 0) {
+            // Past the end: settle on the last filled digit, with everything before it below.
+            chosen = last_filled;
+            running = before_last;
+        }
+        below = running;
+        prefix = (prefix << 4) | (uint32_t)chosen;
     }
-    return sh.prefix;
+    return prefix;
 }
 
-__global__ void __launch_bounds__(kSampleThreads) sample_kernel(SampleParams p) {
+__global__ void __launch_bounds__(kSampleThreads) sample_kernel(SampleParams p, uint32_t share, int in_shared) {
+    extern __shared__ float held[];
     __shared__ Shared sh;
     pdl_launch_dependents();
     pdl_wait();
     const Sampling s = p.settings;
-    const int tid = threadIdx.x;
+    const uint32_t tid = threadIdx.x, rank = blockIdx.x;
+    const uint32_t begin = min(p.n, rank * share), count = min(p.n - begin, share);
+    float* logits = p.logits + begin;
 
-    // Repetition penalty: each distinct token among the last 64 takes it once (sampler.rs:47-63).
+    // Repetition penalty: each distinct token among the last 64 takes it once (sampler.rs:47-63), from the CTA that holds its logit.
     if (fabsf(s.repeat_penalty - 1.0f) > FLT_EPSILON && p.n_recent) {
         const uint32_t window = min(p.n_recent, kRepeatLastN);
         const uint32_t* recent = p.recent + (p.n_recent - window);
-        if ((uint32_t)tid < window) {
+        if (tid < window) {
             const uint32_t token = recent[tid];
-            bool first = token < p.n;
-            for (int j = 0; j < tid && first; ++j) first = recent[j] != token;
+            bool first = token >= begin && token < begin + count;
+            for (uint32_t j = 0; j < tid && first; ++j) first = recent[j] != token;
             if (first) {
                 const float logit = p.logits[token];
                 p.logits[token] = logit > 0.f ? logit / s.repeat_penalty : logit * s.repeat_penalty;
@@ -157,46 +218,53 @@ __global__ void __launch_bounds__(kSampleThreads) sample_kernel(SampleParams p) 
         }
         __syncthreads();
     }
+    Slice slice{in_shared ? held : logits, count, 0, sh};
 
     // The largest logit and its lowest index.
     float best = -INFINITY;
     uint32_t best_index = 0xffffffffu;
-    for (uint32_t i = tid; i < p.n; i += kSampleThreads) {
-        const float v = p.logits[i];
+    for (uint32_t i = tid; i < count; i += kSampleThreads) {
+        const float v = logits[i];
+        if (in_shared) held[i] = v;  // read back by the same thread, and by others after the barriers below
         if (v > best || best_index == 0xffffffffu) {
             best = v;
-            best_index = i;
+            best_index = begin + i;
         }
     }
-    const float top = block_max(best, sh);
+    const float top = slice.total(best, true);
     if (s.temperature <= 0.f) {
         // Greedy: the first maximum (sampler.rs:70-76).
         uint32_t candidate = best == top ? best_index : 0xffffffffu;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) candidate = min(candidate, __shfl_xor_sync(0xffffffffu, candidate, o));
+        candidate = __reduce_min_sync(0xffffffffu, candidate);
+        if ((tid & 31) == 0) sh.counts[tid >> 5] = candidate;
         __syncthreads();
-        if ((tid & 31) == 0) sh.reduce_index[tid >> 5] = candidate;
-        __syncthreads();
-        if (tid == 0) {
+        if (tid < 32) {
+            candidate = __reduce_min_sync(0xffffffffu, sh.counts[tid]);
+            if (tid == 0) sh.mine[slice.parity][0] = __uint_as_float(candidate);
+        }
+        slice.exchange(1);
+        if (rank == 0 && tid == 0) {
             uint32_t index = 0xffffffffu;
-            for (int w = 0; w < kSampleThreads / 32; ++w) index = min(index, sh.reduce_index[w]);
+            for (uint32_t r = 0; r < kCtas; ++r) index = min(index, __float_as_uint(sh.all[r][0]));
             *p.out = index;
             if (p.readback) *p.readback = index;
         }
+        cluster_sync();  // no CTA leaves while another reads its sums
         return;
     }
 
     uint32_t limit = 0xffffffffu;  // candidates are the logits whose key is <= limit
-    if (s.top_k > 0 && s.top_k < p.n) limit = select_key(p, limit, (float)s.top_k - 0.5f, false, [](float) { return 1.0f; }, sh);
+    float below;
+    if (s.top_k > 0 && s.top_k < p.n) limit = select_key(slice, limit, (float)s.top_k - 0.5f, false, [](float) { return 1.0f; }, below);
     auto unit_softmax = [top](float v) { return expf(v - top); };
     if (s.top_p < 1.0f) {
         float mine = 0.f;
-        for (uint32_t i = tid; i < p.n; i += kSampleThreads) {
-            const float v = p.logits[i];
+        for (uint32_t i = tid; i < count; i += kSampleThreads) {
+            const float v = slice.v[i];
             if (descending_key(v) <= limit) mine += unit_softmax(v);
         }
-        const float total = block_total(mine, sh);
-        limit = select_key(p, limit, s.top_p * total, true, unit_softmax, sh);
+        const float total = slice.total(mine, false);
+        limit = select_key(slice, limit, s.top_p * total, true, unit_softmax, below);
     }
     if (s.min_p > 0.f) {
         // p >= p_first * min_p, with p proportional to exp(logit - top) (sampler.rs:98-99).
@@ -208,61 +276,72 @@ __global__ void __launch_bounds__(kSampleThreads) sample_kernel(SampleParams p) 
     const float inv_t = 1.0f / s.temperature;
     auto tempered = [top, inv_t](float v) { return expf((v - top) * inv_t); };
     float mine = 0.f;
-    for (uint32_t i = tid; i < p.n; i += kSampleThreads) {
-        const float v = p.logits[i];
+    for (uint32_t i = tid; i < count; i += kSampleThreads) {
+        const float v = slice.v[i];
         if (descending_key(v) <= limit) mine += tempered(v);
     }
-    const float total = block_total(mine, sh);
+    const float total = slice.total(mine, false);
     const float target = p.uniform * total;
-    const uint32_t picked_key = select_key(p, limit, target, false, tempered, sh);
+    const uint32_t picked_key = select_key(slice, limit, target, false, tempered, below);
 
-    // Equal logits share the key: the draw's remainder picks among them by index.
-    const uint32_t per_thread = (p.n + kSampleThreads - 1) / kSampleThreads;
-    const uint32_t first = tid * per_thread, last = min(p.n, first + per_thread);
+    // Equal logits share the key: the draw's remainder picks among them by index. A thread looks at
+    // neighbouring logits, so ties are counted in the order of their indexes.
+    const uint32_t per_thread = (count + kSampleThreads - 1) / kSampleThreads;
+    const uint32_t first = min(count, tid * per_thread), last = min(count, first + per_thread);
     uint32_t ties = 0;
     float tie_weight = 0.f;
     for (uint32_t i = first; i < last; ++i) {
-        const float v = p.logits[i];
+        const float v = slice.v[i];
         if (descending_key(v) == picked_key) {
             ++ties;
             tie_weight = tempered(v);
         }
     }
-    // Exclusive scan of the per-thread tie counts.
     uint32_t inclusive_scan = ties;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         uint32_t other = __shfl_up_sync(0xffffffffu, inclusive_scan, o);
         if ((tid & 31) >= o) inclusive_scan += other;
     }
-    __syncthreads();
     if ((tid & 31) == 31) sh.counts[tid >> 5] = inclusive_scan;
-    if (tid == 0) sh.scalar = 0.f;
+    tie_weight = warp_max(tie_weight);  // the same value from every thread that has one
+    if ((tid & 31) == 0) sh.warps[tid >> 5][0] = tie_weight;
     __syncthreads();
-    uint32_t before = inclusive_scan - ties;
-    for (int w = 0; w < (tid >> 5); ++w) before += sh.counts[w];
+    uint32_t before = inclusive_scan - ties, in_cta = 0;
+    for (uint32_t w = 0; w < (tid >> 5); ++w) before += sh.counts[w];
+    if (tid == 0) {
+        float w = 0.f;
+        for (uint32_t i = 0; i < kWarps; ++i) in_cta += sh.counts[i], w = fmaxf(w, sh.warps[i][0]);
+        sh.mine[slice.parity][0] = __uint_as_float(in_cta);
+        sh.mine[slice.parity][1] = w;
+    }
+    slice.exchange(2);
     uint32_t all_ties = 0;
-    for (int w = 0; w < kSampleThreads / 32; ++w) all_ties += sh.counts[w];
-    if (ties) sh.scalar = tie_weight;  // the same value from every thread that has one
-    __syncthreads();
-    const float w = sh.scalar;
+    float w = 0.f;
+    for (uint32_t r = 0; r < kCtas; ++r) {
+        const uint32_t there = __float_as_uint(sh.all[r][0]);
+        if (r < rank) before += there;
+        all_ties += there;
+        w = fmaxf(w, sh.all[r][1]);
+    }
     uint32_t wanted = 0;
     if (w > 0.f && all_ties > 1) {
-        const float remainder = fmaxf(target - sh.below, 0.f);
+        const float remainder = fmaxf(target - below, 0.f);
         wanted = min((uint32_t)(remainder / w), all_ties - 1);
     }
     if (ties && wanted >= before && wanted < before + ties) {
         uint32_t seen = before;
         for (uint32_t i = first; i < last; ++i) {
-            if (descending_key(p.logits[i]) != picked_key) continue;
+            if (descending_key(slice.v[i]) != picked_key) continue;
             if (seen == wanted) {
-                *p.out = i;
-                if (p.readback) *p.readback = i;
+                *p.out = begin + i;
+                if (p.readback) *p.readback = begin + i;
                 break;
             }
             ++seen;
         }
     }
+    cluster_sync();
 }
 
 }  // namespace
@@ -270,8 +349,25 @@ __global__ void __launch_bounds__(kSampleThreads) sample_kernel(SampleParams p) 
 cudaError_t sample(cudaStream_t stream, float* logits, uint32_t n, const uint32_t* recent, uint32_t n_recent, const Sampling& settings,
                    float uniform, uint32_t* out, uint32_t* readback) {
     SampleParams p{logits, n, recent, n_recent, settings, uniform, out, readback};
-    void* args[] = {&p};
-    return launch_kernel((const void*)sample_kernel, dim3(1), dim3(kSampleThreads), 0, stream, args);
+    const uint32_t share = (n + kCtas - 1) / kCtas;
+    constexpr size_t most = 200 * 1024;  // beside the kernel's static shared memory
+    const size_t bytes = (size_t)share * 4 <= most ? (size_t)share * 4 : 0;
+    cudaError_t e = ensure_dynamic_smem((const void*)sample_kernel, bytes);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(kCtas);
+    config.blockDim = dim3(kSampleThreads);
+    config.dynamicSmemBytes = bytes;
+    config.stream = stream;
+    cudaLaunchAttribute attributes[2];
+    attributes[0].id = cudaLaunchAttributeClusterDimension;
+    attributes[0].val.clusterDim.x = kCtas;
+    attributes[0].val.clusterDim.y = attributes[0].val.clusterDim.z = 1;
+    attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attributes[1].val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = attributes;
+    config.numAttrs = pdl_enabled() ? 2 : 1;
+    return cudaLaunchKernelEx(&config, sample_kernel, p, share, bytes ? 1 : 0);
 }
 
 }  // namespace k
