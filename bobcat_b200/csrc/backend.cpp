@@ -3,6 +3,7 @@
 
 #include "backend.h"
 
+#include <atomic>
 #include <cstdarg>
 #include <cstring>
 #include <initializer_list>
@@ -37,13 +38,46 @@ bc_status check_range(const bc_backend* backend, const bc_buffer* buffer, size_t
     return BC_OK;
 }
 
-// A kernel whose bounded wait ran out leaves a flag rather than hanging the device. Reading a flag
+namespace {
+
+// Per device: one word of mapped host memory per kernel file with bounded waits, for the life of the process.
+constexpr int kWaitWords = 4, kMaxDevices = 64;
+std::atomic<volatile int*> g_wait_words[kMaxDevices];
+
+bc_status set_wait_words(int device) {
+    static std::mutex mutex;
+    if (device >= kMaxDevices) return BC_OK;  // waits that run out go unreported there
+    std::lock_guard<std::mutex> lock(mutex);
+    if (g_wait_words[device].load()) return BC_OK;
+    int* words = nullptr;
+    BC_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&words), kWaitWords * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
+    for (int i = 0; i < kWaitWords; ++i) words[i] = 0;
+    BC_CUDA(k::matvec_wait_word(words));
+    BC_CUDA(k::matmul_wait_word(words + 1));
+    BC_CUDA(k::matmul_few_wait_word(words + 2));
+    BC_CUDA(k::peer_wait_word(words + 3));
+    g_wait_words[device].store(words);
+    return BC_OK;
+}
+
+}  // namespace
+
+// A kernel whose bounded wait ran out leaves a code rather than hanging the device. Reading a code
 // clears it, so one failure is reported once and later healthy work is not blamed for it.
 bc_status kernel_wait_status() {
-    if (int flag = k::matvec_error_flag()) return fail(BC_ERR_EXECUTION, "a decode kernel gave up waiting for its weight stream or its input (code %d)", flag);
-    if (int flag = k::matmul_error_flag()) return fail(BC_ERR_EXECUTION, "a prefill kernel gave up waiting on its pipeline (code %d)", flag);
-    if (int flag = k::matmul_few_error_flag()) return fail(BC_ERR_EXECUTION, "a few-token product gave up waiting for its weights (code %d)", flag);
-    if (int flag = k::peer_error_flag()) return fail(BC_ERR_EXECUTION, "a sum over ranks gave up waiting for rank %d", flag - 1);
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess || device >= kMaxDevices) return BC_OK;
+    volatile int* words = g_wait_words[device].load();
+    if (!words) return BC_OK;
+    auto take = [&](int i) {
+        const int code = words[i];
+        if (code) words[i] = 0;
+        return code;
+    };
+    if (int code = take(0)) return fail(BC_ERR_EXECUTION, "a decode kernel gave up waiting for its weight stream or its input (code %d)", code);
+    if (int code = take(1)) return fail(BC_ERR_EXECUTION, "a prefill kernel gave up waiting on its pipeline (code %d)", code);
+    if (int code = take(2)) return fail(BC_ERR_EXECUTION, "a few-token product gave up waiting for its weights (code %d)", code);
+    if (int code = take(3)) return fail(BC_ERR_EXECUTION, "a sum over ranks gave up waiting for rank %d", code - 1);
     return BC_OK;
 }
 
@@ -143,6 +177,7 @@ bc_status bc_backend_open(int32_t device, void* stream, bc_backend** out) {
     std::unique_ptr<bc_backend> b(new bc_backend());
     b->device = device;
     BC_TRY(b->activate());
+    BC_TRY(set_wait_words(device));
     if (stream) {
         b->stream = static_cast<cudaStream_t>(stream);
     } else {

@@ -92,9 +92,12 @@ cudaError_t matvec_swiglu_mma(cudaStream_t stream, const Mat& gate, const Mat& u
 cudaError_t matvec_conv_mma(cudaStream_t stream, const Mat& in_proj, const float* x, Norm norm, const float* taps, float* history,
                             float* out, uint32_t n_embd, uint32_t kernel);
 cudaError_t matvec_mma_prepare(uint32_t widest_cols);
-// Nonzero once a bounded wait inside a kernel gave up (1: a ring slot never freed, 2: a chunk never
-// arrived). Reading clears it.
-int matvec_error_flag();
+// Bounded waits. A kernel whose wait ran out stores a code into a word of host memory that the device
+// can write (one word per kernel file, handed over once per device by these functions, which set the
+// file's pointer on the current device), so the host learns of it with a plain read after it has waited for
+// the stream: reading device flags back cost four copies, 40 us, at the end of every call.
+// Codes of the decode kernels: 2, a chunk never arrived.
+cudaError_t matvec_wait_word(int* word);
 // Raise the shared-memory limit of every matvec kernel for input vectors of up to `widest_cols`.
 cudaError_t matvec_prepare(uint32_t widest_cols);
 cudaError_t matvec(cudaStream_t stream, const MatvecSegment* segments, int n_segments, const float* x, Norm norm,
@@ -138,6 +141,8 @@ cudaError_t rope_table(cudaStream_t stream, float2* table, uint32_t n_positions,
 cudaError_t rope_store(cudaStream_t stream, const RopeStore& p, Pos pos);
 // One thread: *counter += 1.
 cudaError_t advance(cudaStream_t stream, uint32_t* counter);
+// One thread: *counter = seed[0], tokens[seed[0]] = seed[1]; `seed` may lie in host-mapped memory.
+cudaError_t seed_step(cudaStream_t stream, const uint32_t* seed, uint32_t* counter, uint32_t* tokens);
 // argmax for a replayed decode: pos = *counter (after adding 1 to it when `advance`), then
 // tokens[pos + offset] = argmax(x) and, when `ring` is non-null, ring[pos % ring_slots] too.
 cudaError_t argmax_step(cudaStream_t stream, const float* x, uint32_t n, uint32_t* counter, bool advance, uint32_t* tokens,
@@ -196,8 +201,8 @@ struct PeerBuffers {
 };
 inline uint64_t peer_buffer_bytes(uint32_t world) { return (uint64_t)2 * world * kPeerSlotFloats * 4 + 2 * world * 4 + 64; }
 cudaError_t peer_all_reduce_add(cudaStream_t stream, const PeerBuffers& peers, const float* partial, float* y, uint32_t count);
-// Nonzero once a rank's flag did not arrive within the wait's limit (1 + that rank). Reading clears it.
-int peer_error_flag();
+// Code of the sum over ranks: 1 + the rank whose flag did not arrive.
+cudaError_t peer_wait_word(int* word);
 
 // ---- sampling (kernels_sample.cu): Sampler::sample of crates/bobcat-cli/src/sampler.rs:45-112.
 struct Sampling {
@@ -353,8 +358,7 @@ cudaError_t matmul_umma_swiglu(cudaStream_t stream, const Mat& gate, const Mat& 
 // matmul_umma_several, matmul_umma_swiglu and matmul_experts_umma hand over to these whenever the
 // shape allows (BOBCAT_NO_FEW_MATMUL=1 keeps them on the tcgen05 kernel).
 bool matmul_few_supported(const Mat& w, uint32_t n_tokens);
-// Nonzero once a warp of that kernel gave up waiting for its weights.
-int matmul_few_error_flag();
+cudaError_t matmul_few_wait_word(int* word);
 cudaError_t matmul_few(cudaStream_t stream, const Mat* const* ws, float* const* ys, const uint32_t* strides, int n, const void* packed,
                        uint32_t n_tokens, int32_t store);
 cudaError_t matmul_few_swiglu(cudaStream_t stream, const Mat& gate, const Mat& up, const void* packed, float* y, uint32_t n_tokens, uint32_t y_stride,
@@ -378,9 +382,9 @@ cudaError_t matmul_exact_swiglu(cudaStream_t stream, const Mat& gate, const Mat&
 bool matmul_exact_experts_supported(const Mat& w, const Mat* up, uint32_t n_rows, uint32_t n_tokens);
 cudaError_t matmul_exact_experts(cudaStream_t stream, const Mat& w, const Mat* up, uint32_t n_rows, uint32_t n_experts, const float* x, bool gather,
                                  const uint32_t* offsets, const uint32_t* entries, uint32_t n_used, float* y, uint32_t n_tokens);
-// Nonzero once a bounded wait inside the tensor-core prefill kernel gave up (1: producers on a free
-// stage, 2: epilogue on the accumulator, 3: token copy on a free stage, 4: MMA thread on a full stage).
-int matmul_error_flag();
+// Codes of the tensor-core prefill kernel: 1: producers on a free stage, 2: epilogue on the
+// accumulator, 3: token copy on a free stage, 4: MMA thread on a full stage.
+cudaError_t matmul_wait_word(int* word);
 
 }  // namespace k
 }  // namespace bc

@@ -30,7 +30,7 @@ namespace {
 constexpr int kPeerThreads = 1024;
 constexpr uint32_t kPeerSpinLimit = 1u << 21;  // polls of a local flag, each followed by a short sleep
 
-__device__ int g_peer_error;
+__device__ int* g_wait_word;  // where a wait that ran out leaves its code (kernels.h), null until set
 
 __global__ void __launch_bounds__(kPeerThreads) peer_all_reduce_add_kernel(PeerBuffers peers, const float* __restrict__ partial,
                                                                             float* __restrict__ y, uint32_t count) {
@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(kPeerThreads) peer_all_reduce_add_kernel(PeerB
             }
             __nanosleep(40);
         }
-        if (!seen) atomicExch(&g_peer_error, 1 + tid);
+        if (!seen && g_wait_word) *reinterpret_cast<volatile int*>(g_wait_word) = 1 + tid;
     }
     __syncthreads();
     // Step 4: the slots in rank order.
@@ -109,15 +109,7 @@ cudaError_t peer_all_reduce_add(cudaStream_t stream, const PeerBuffers& peers, c
     return launch_kernel((const void*)peer_all_reduce_add_kernel, dim3(1), dim3(kPeerThreads), 0, stream, args);
 }
 
-int peer_error_flag() {
-    int flag = 0;
-    cudaMemcpyFromSymbol(&flag, g_peer_error, sizeof flag);
-    if (flag) {
-        const int zero = 0;
-        cudaMemcpyToSymbol(g_peer_error, &zero, sizeof zero);
-    }
-    return flag;
-}
+cudaError_t peer_wait_word(int* word) { return cudaMemcpyToSymbol(g_wait_word, &word, sizeof word); }
 
 }  // namespace k
 }  // namespace bc

@@ -108,7 +108,7 @@ constexpr int kSlotBytes = 8 * 576;                          // a warp's slot: u
 constexpr uint32_t kMaxTokenBytes = 128 * 1024;              // packed tokens a CTA keeps in shared memory
 constexpr uint32_t kSpinLimit = 1u << 22;                    // bounded waits: give up rather than hang
 
-__device__ int g_few_error;
+__device__ int* g_wait_word;  // where a wait that ran out leaves its code (kernels.h), null until set
 
 // Pairs [first, last) of one tile against NT groups of 8 tokens. acc[j]: rows g and g + 8 x tokens
 // 8j + 2t, + 1 in the m16n8 accumulator layout. The weights come through the warp's
@@ -180,7 +180,8 @@ struct Worker {
         uint32_t pending = size0, after = size1;
         while (pending > 0) {
             const uint32_t from = slot + (taken & 1) * kSlotStep;
-            if (!async::mbar_wait(bar + (taken & 1) * 8, (taken >> 1) & 1, kSpinLimit, &g_few_error)) g_few_error = 1;  // and carry on: the group's barriers still need this warp
+            int dead = 0;
+            if (!async::mbar_wait(bar + (taken & 1) * 8, (taken >> 1) & 1, kSpinLimit, &dead) && g_wait_word) *reinterpret_cast<volatile int*>(g_wait_word) = 1;  // and carry on: the group's barriers still need this warp
             ++taken;
 #pragma unroll 2
             for (uint32_t i = 0; i < pending; ++i) {
@@ -484,15 +485,7 @@ cudaError_t launch_few(cudaStream_t stream, FewParams p, uint32_t most_jobs, uin
 
 }  // namespace
 
-int matmul_few_error_flag() {
-    int flag = 0;
-    cudaMemcpyFromSymbol(&flag, g_few_error, sizeof flag);
-    if (flag) {
-        const int zero = 0;
-        cudaMemcpyToSymbol(g_few_error, &zero, sizeof zero);
-    }
-    return flag;
-}
+cudaError_t matmul_few_wait_word(int* word) { return cudaMemcpyToSymbol(g_wait_word, &word, sizeof word); }
 
 bool matmul_few_supported(const Mat& w, uint32_t n_tokens) {
     return !few_disabled() && w.format == BC_Q4_0 && w.tiles != nullptr && n_tokens > 0 && n_tokens <= kMaxFewTokens && w.n_cols % 64 == 0 && w.n_cols > 0 &&

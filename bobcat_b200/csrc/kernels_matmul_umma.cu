@@ -86,7 +86,7 @@ struct Shape {
     static constexpr size_t kSmemBytes = kStages * (kStageA + kStageB) + kRawBytes + (2 * kStages + 1) * 8 + 16;
 };
 
-__device__ int g_matmul_error;
+__device__ int* g_wait_word;  // where a wait that ran out leaves its code (kernels.h), null until set
 
 struct UmmaParams {
     const uint4* quants[2];   // split layout: [n_rows][n_blocks] 16-byte groups (the second matrix only when DUAL == 2)
@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(256) pack_grouped_kernel(const float* __restri
 
 __device__ __forceinline__ void give_up(volatile int* dead, int code) {
     *dead = 1;
-    atomicCAS(&g_matmul_error, 0, code);
+    if (g_wait_word) *reinterpret_cast<volatile int*>(g_wait_word) = code;
 }
 
 template <int DUAL>
@@ -998,15 +998,7 @@ cudaError_t matmul_experts_umma(cudaStream_t stream, const Mat& w, const Mat* up
     return cudaGetLastError();
 }
 
-int matmul_error_flag() {
-    int flag = 0;
-    cudaMemcpyFromSymbol(&flag, g_matmul_error, sizeof flag);
-    if (flag) {
-        const int zero = 0;
-        cudaMemcpyToSymbol(g_matmul_error, &zero, sizeof zero);
-    }
-    return flag;
-}
+cudaError_t matmul_wait_word(int* word) { return cudaMemcpyToSymbol(g_wait_word, &word, sizeof word); }
 
 }  // namespace k
 }  // namespace bc

@@ -58,7 +58,7 @@ constexpr int kBlockBytes = 288;                 // 16 rows x 18 bytes
 constexpr int kStageBytes = kChunkBlocks * kBlockBytes;
 constexpr uint32_t kSpinLimit = 1u << 22;        // bounded waits: give up rather than hang
 
-__device__ int g_error_flag;
+__device__ int* g_wait_word;  // where a wait that ran out leaves its code (kernels.h), null until set
 
 // ---- mbarrier and bulk-copy wrappers (shared::cta addresses as 32-bit integers)
 
@@ -388,7 +388,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) matvec_mma_kernel(Params
             // A wait that runs out marks the launch failed; the warp then skips its remaining chunks
             // but still meets its group at every barrier, so nothing is left waiting on it.
             if (!dead && !mbar_wait(smem_u32(&full_bar[stage]), use & 1)) {
-                atomicExch(&g_error_flag, 2);
+                if (g_wait_word) *reinterpret_cast<volatile int*>(g_wait_word) = 2;
                 dead = true;
             }
             if (dead) continue;
@@ -605,15 +605,7 @@ cudaError_t matvec_mma_prepare(uint32_t widest_cols) {
     return cudaSuccess;
 }
 
-int matvec_error_flag() {
-    int flag = 0;
-    cudaMemcpyFromSymbol(&flag, g_error_flag, sizeof flag);
-    if (flag) {
-        const int zero = 0;
-        cudaMemcpyToSymbol(g_error_flag, &zero, sizeof zero);
-    }
-    return flag;
-}
+cudaError_t matvec_wait_word(int* word) { return cudaMemcpyToSymbol(g_wait_word, &word, sizeof word); }
 
 cudaError_t matvec_mma(cudaStream_t stream, const MatvecSegment* segments, int n_segments, const float* x, Norm norm, bool accumulate) {
     Params p{};

@@ -439,6 +439,14 @@ __global__ void advance_kernel(uint32_t* counter) {
     *counter += 1;
 }
 
+__global__ void seed_step_kernel(const volatile uint32_t* seed, uint32_t* counter, uint32_t* tokens) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const uint32_t pos = seed[0];
+    *counter = pos;
+    tokens[pos] = seed[1];
+}
+
 }  // namespace
 
 cudaError_t repack_q4_0(cudaStream_t stream, const uint8_t* raw, uint64_t n_blocks, void* quants, __half* scales) {
@@ -553,6 +561,10 @@ cudaError_t add_floats(cudaStream_t stream, float* y, const float* x, uint64_t n
 cudaError_t advance(cudaStream_t stream, uint32_t* counter) {
     void* args[] = {&counter};
     return launch_kernel((const void*)advance_kernel, dim3(1), dim3(1), 0, stream, args);
+}
+
+cudaError_t seed_step(cudaStream_t stream, const uint32_t* seed, uint32_t* counter, uint32_t* tokens) {
+    return launch_dependent(seed_step_kernel, dim3(1), dim3(1), 0, stream, static_cast<const volatile uint32_t*>(seed), counter, tokens);
 }
 
 cudaError_t rope_table(cudaStream_t stream, float2* table, uint32_t n_positions, uint32_t n_rot, float theta) {

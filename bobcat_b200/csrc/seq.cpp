@@ -71,26 +71,33 @@ bool replay_enabled(const bc_seq* s) {
     return s->use_graphs && !s->backend->profiling && s->backend->stream != nullptr && s->backend->stream != cudaStreamLegacy;
 }
 
-// Capture one generated step into a graph. The generate variant picks tokens[pos] from the logits,
-// then runs the forward pass at pos; the stream variant runs the forward pass at pos, then picks
-// tokens[pos + 1] and mirrors it into the host-mapped ring at slot pos % kGenerateInFlight. Both
-// start by adding one to s->step_pos, so the host seeds it with the first position minus one.
-bc_status capture_step(bc_seq* s, bool stream_variant) {
+// The kinds of step that are captured into a graph.
+enum StepKind { kStepOnly = 0, kStepLogits = 1, kGenerate = 2, kStream = 3 };
+
+// Capture one step into a graph. The generate kind picks tokens[pos] from the logits, then runs the
+// forward pass at pos; the stream kind runs the forward pass at pos, then picks tokens[pos + 1] and
+// mirrors it into the host-mapped ring at slot pos % kGenerateInFlight. Both start by adding one to
+// s->step_pos, so the host seeds it with the first position minus one. The step kinds take the
+// position and its token from s->step_seed and run the forward pass there, with or without logits.
+bc_status capture_step(bc_seq* s, StepKind kind) {
     cudaStream_t stream = s->backend->stream;
     const uint32_t n_vocab = s->hp.n_vocab;
     uint64_t before = s->launches;
     BC_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
     Recorder r(*s);
     r.replayed = true;
-    if (stream_variant) {
+    if (kind == kStream) {
         r.run("advance", 1, 1, 0, 1, [&] { return k::advance(stream, s->step_pos); });
         r.step(0, true, false);
         r.run("argmax", 1, n_vocab, 0, 1,
               [&] { return k::argmax_step(stream, s->logits, n_vocab, s->step_pos, false, s->tokens, 1, s->readback, kGenerateInFlight); });
-    } else {
+    } else if (kind == kGenerate) {
         r.run("argmax", 1, n_vocab, 0, 1,
               [&] { return k::argmax_step(stream, s->logits, n_vocab, s->step_pos, true, s->tokens, 0, nullptr, 1); });
         r.step(0, true, false);
+    } else {
+        r.run("seed_step", 1, 1, 0, 1, [&] { return k::seed_step(stream, s->step_seed, s->step_pos, s->tokens); });
+        r.step(0, kind == kStepLogits, false);
     }
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamEndCapture(stream, &graph);
@@ -105,19 +112,22 @@ bc_status capture_step(bc_seq* s, bool stream_variant) {
     e = cudaGraphInstantiate(&exec, graph, 0);
     cudaGraphDestroy(graph);
     if (e != cudaSuccess) return cuda_fail(e, "cudaGraphInstantiate");
-    if (stream_variant) {
+    if (kind == kStream) {
         s->stream_graph = exec;
         s->stream_graph_kernels = kernels;
-    } else {
+    } else if (kind == kGenerate) {
         s->generate_graph = exec;
         s->generate_graph_kernels = kernels;
+    } else {
+        s->step_graph[kind] = exec;
+        s->step_graph_kernels[kind] = kernels;
     }
     return BC_OK;
 }
 
 // Make sure the wanted graph exists and seed the device position for a run that starts at `first`.
 bc_status prepare_replay(bc_seq* s, bool stream_variant, uint32_t first) {
-    if (stream_variant ? !s->stream_graph : !s->generate_graph) BC_TRY(capture_step(s, stream_variant));
+    if (stream_variant ? !s->stream_graph : !s->generate_graph) BC_TRY(capture_step(s, stream_variant ? kStream : kGenerate));
     s->host_pos = first - 1;  // first >= 1: generation needs a prompt
     BC_CUDA(cudaMemcpyAsync(s->step_pos, &s->host_pos, 4, cudaMemcpyHostToDevice, s->backend->stream));
     return BC_OK;
@@ -198,6 +208,11 @@ void bc_seq::release() {
     trace_routes = nullptr;
     if (readback) cudaFreeHost(readback);
     readback = nullptr;
+    step_seed = nullptr;
+    for (cudaGraphExec_t& g : step_graph) {
+        if (g) cudaGraphExecDestroy(g);
+        g = nullptr;
+    }
     if (generate_graph) cudaGraphExecDestroy(generate_graph);
     if (stream_graph) cudaGraphExecDestroy(stream_graph);
     generate_graph = stream_graph = nullptr;
@@ -340,8 +355,9 @@ bc_status seq_new(bc_model* model, bc_backend* backend, bc_comm* tp, uint32_t n_
     }
     if (hp.n_attention_layers && !qwen) BC_CUDA(k::rope_table(backend->stream, s->rope_table, n_ctx, hp.n_rot, hp.rope_theta));
     BC_TRY(ensure_trace_rows(s.get(), 1));
-    e = cudaHostAlloc((void**)&s->readback, sizeof(uint32_t) * kGenerateInFlight, cudaHostAllocMapped);
+    e = cudaHostAlloc((void**)&s->readback, sizeof(uint32_t) * (kGenerateInFlight + 2), cudaHostAllocMapped);
     if (e != cudaSuccess) return fail(BC_ERR_ALLOCATION, "cannot allocate the token readback: %s", cudaGetErrorString(e));
+    s->step_seed = s->readback + kGenerateInFlight;
     for (int i = 0; i < kGenerateInFlight; ++i) BC_CUDA(cudaEventCreateWithFlags(&s->slot_done[i], cudaEventDisableTiming));
     BC_CUDA(cudaEventCreate(&s->timing_start));
     BC_CUDA(cudaEventCreate(&s->timing_end));
@@ -403,11 +419,25 @@ bc_status step_impl(bc_seq* s, uint32_t token, float* logits, size_t logits_len,
     BC_TRY(s->backend->activate());
     cudaStream_t stream = s->backend->stream;
 
-    BC_CUDA(cudaMemcpyAsync(s->tokens + pos, &token, 4, cudaMemcpyHostToDevice, stream));
+    // A sequence that keeps stepping replays the step: one launch call and no token copy. Its first two
+    // steps are launched kernel by kernel, which costs less than a capture that would serve only them.
+    const bool want_logits = logits != nullptr || device_logits;
+    const StepKind kind = want_logits ? kStepLogits : kStepOnly;
+    const bool replay = !trace && replay_enabled(s) && (s->step_graph[kind] || ++s->steps_taken[kind] > 2);
+    if (replay && !s->step_graph[kind]) BC_TRY(capture_step(s, kind));
+
+    if (!replay) BC_CUDA(cudaMemcpyAsync(s->tokens + pos, &token, 4, cudaMemcpyHostToDevice, stream));
     auto encode_start = Clock::now();
     BC_TRY(timing_begin(s));
     Recorder r(*s);
-    r.step(pos, logits != nullptr || device_logits, trace != nullptr);
+    if (replay) {
+        s->step_seed[0] = pos;  // the last replay has been waited for
+        s->step_seed[1] = token;
+        BC_CUDA(cudaGraphLaunch(s->step_graph[kind], stream));
+        s->launches += s->step_graph_kernels[kind];
+    } else {
+        r.step(pos, want_logits, trace != nullptr);
+    }
     double encode = since(encode_start);
     double gpu = 0;
     bc_status finish = timing_end(s, &gpu);
@@ -839,6 +869,10 @@ bc_status bc_seq_set_skip(bc_seq* s, const char* name, uint32_t n_rows, uint32_t
     if (s->generate_graph) cudaGraphExecDestroy(s->generate_graph);
     if (s->stream_graph) cudaGraphExecDestroy(s->stream_graph);
     s->generate_graph = s->stream_graph = nullptr;
+    for (cudaGraphExec_t& g : s->step_graph) {
+        if (g) cudaGraphExecDestroy(g);
+        g = nullptr;
+    }
     return BC_OK;
 }
 

@@ -105,6 +105,12 @@ struct bc_seq {
     cudaGraphExec_t generate_graph = nullptr; // argmax -> tokens[pos], forward pass at pos
     cudaGraphExec_t stream_graph = nullptr;   // forward pass at pos, argmax -> tokens[pos + 1] and the readback ring
     uint64_t generate_graph_kernels = 0, stream_graph_kernels = 0;  // kernels per replay, for the launch count
+    // A single step replayed: (position, token) from host-mapped memory, forward pass there, without [0]
+    // or with [1] logits. Captured when a sequence steps the same way a third time.
+    cudaGraphExec_t step_graph[2] = {};
+    uint64_t step_graph_kernels[2] = {};
+    uint32_t steps_taken[2] = {};
+    uint32_t* step_seed = nullptr;            // host-mapped: the position and the token of a replayed step
     uint32_t host_pos = 0;                    // staging for the seed of step_pos
     // Timing diagnostics (bc_seq_set_skip): launches of this name (and shape, when nonzero) are left out.
     std::string skip_name;
