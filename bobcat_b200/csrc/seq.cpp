@@ -234,6 +234,23 @@ bc_prefix::~bc_prefix() {
     cudaFree(tail);
 }
 
+SpareState::~SpareState() {
+    if (!block) return;
+    cudaSetDevice(device);
+    cudaFree(block);
+}
+
+bc_checkpoint::~bc_checkpoint() {
+    if (!device_state) return;
+    {
+        std::lock_guard<std::mutex> lock(spare->mutex);
+        if (!spare->block) std::swap(spare->block, device_state);
+    }
+    if (!device_state) return;
+    cudaSetDevice(spare->device);
+    cudaFree(device_state);
+}
+
 void release_seq(bc_seq* seq) { seq->release(); }
 
 namespace {
@@ -667,10 +684,10 @@ bc_status bc_seq_reset(bc_seq* s) {
     // needs no clearing, because attention reads only the positions a sequence has written.
     if (s->conv_floats) BC_CUDA(cudaMemsetAsync(s->conv_state, 0, s->conv_floats * 4, s->backend->stream));
     if (s->delta_floats) BC_CUDA(cudaMemsetAsync(s->delta_state, 0, s->delta_floats * 4, s->backend->stream));
-    BC_CUDA(cudaStreamSynchronize(s->backend->stream));
     // A sequence that started from a cached prefix shares the prefix's pages; a new sequence
     // writes from position zero again, so it takes pages of its own back first.
     if (s->k_pages && s->shared_positions) {
+        BC_CUDA(cudaStreamSynchronize(s->backend->stream));  // remapping pages needs the stream idle
         const PageGeometry& g = s->k_pages->geometry();
         for (uint32_t slot = 0; slot < g.n_layers * g.pages_per_layer(); ++slot) {
             BC_TRY(s->k_pages->make_private(slot));
@@ -690,13 +707,30 @@ bc_status bc_seq_checkpoint(bc_seq* s, bc_checkpoint** out) {
     c->owner = s;
     c->resets = s->resets;
     c->n_past = s->n_past;
-    c->conv_state.resize(s->conv_floats);
-    c->logits.resize(s->hp.n_vocab);
+    c->conv_floats = s->conv_floats;
+    c->delta_floats = s->delta_floats;
+    c->n_vocab = s->hp.n_vocab;
+    const size_t total = c->conv_floats + c->delta_floats + c->n_vocab;
     cudaStream_t stream = s->backend->stream;
-    if (s->conv_floats) BC_CUDA(cudaMemcpyAsync(c->conv_state.data(), s->conv_state, s->conv_floats * 4, cudaMemcpyDeviceToHost, stream));
-    c->delta_state.resize(s->delta_floats);
-    if (s->delta_floats) BC_CUDA(cudaMemcpyAsync(c->delta_state.data(), s->delta_state, s->delta_floats * 4, cudaMemcpyDeviceToHost, stream));
-    BC_CUDA(cudaMemcpyAsync(c->logits.data(), s->logits, c->logits.size() * 4, cudaMemcpyDeviceToHost, stream));
+    if (!s->spare_checkpoint) {
+        s->spare_checkpoint = std::make_shared<SpareState>();
+        s->spare_checkpoint->device = s->backend->device;
+    }
+    c->spare = s->spare_checkpoint;
+    {
+        std::lock_guard<std::mutex> lock(c->spare->mutex);
+        std::swap(c->device_state, c->spare->block);  // the sequence's stream orders its earlier reads before the copies below
+    }
+    if (!c->device_state && cudaMalloc(&c->device_state, total * 4) != cudaSuccess) {
+        cudaGetLastError();
+        c->device_state = nullptr;
+        c->host_state.resize(total);
+    }
+    float* at = c->device_state ? c->device_state : c->host_state.data();
+    for (auto [src, n] : {std::pair<const float*, size_t>{s->conv_state, c->conv_floats}, {s->delta_state, c->delta_floats}, {s->logits, c->n_vocab}}) {
+        if (n) BC_CUDA(cudaMemcpyAsync(at, src, n * 4, cudaMemcpyDefault, stream));
+        at += n;
+    }
     BC_CUDA(cudaStreamSynchronize(stream));
     *out = c.release();
     return BC_OK;
@@ -709,14 +743,18 @@ bc_status bc_seq_restore(bc_seq* s, const bc_checkpoint* c) {
     if (c->owner != s) return fail(BC_ERR_ARGUMENT, "the checkpoint belongs to another sequence");
     if (c->resets != s->resets) return fail(BC_ERR_ARGUMENT, "the checkpoint predates a reset");
     if (c->n_past < s->shared_positions) return fail(BC_ERR_ARGUMENT, "the checkpoint lies inside the shared prefix of %u positions", s->shared_positions);
-    if (c->conv_state.size() != s->conv_floats || c->delta_state.size() != s->delta_floats || c->logits.size() != s->hp.n_vocab || c->n_past > s->n_ctx)
+    if (c->conv_floats != s->conv_floats || c->delta_floats != s->delta_floats || c->n_vocab != s->hp.n_vocab || c->n_past > s->n_ctx)
         return fail(BC_ERR_ARGUMENT, "the checkpoint comes from a different model or context");
     BC_TRY(s->backend->activate());
     cudaStream_t stream = s->backend->stream;
-    if (s->conv_floats) BC_CUDA(cudaMemcpyAsync(s->conv_state, c->conv_state.data(), s->conv_floats * 4, cudaMemcpyHostToDevice, stream));
-    if (s->delta_floats) BC_CUDA(cudaMemcpyAsync(s->delta_state, c->delta_state.data(), s->delta_floats * 4, cudaMemcpyHostToDevice, stream));
-    BC_CUDA(cudaMemcpyAsync(s->logits, c->logits.data(), c->logits.size() * 4, cudaMemcpyHostToDevice, stream));
-    BC_CUDA(cudaStreamSynchronize(stream));
+    const float* at = c->device_state ? c->device_state : c->host_state.data();
+    for (auto [dst, n] : {std::pair<float*, size_t>{s->conv_state, c->conv_floats}, {s->delta_state, c->delta_floats}, {s->logits, c->n_vocab}}) {
+        if (n) BC_CUDA(cudaMemcpyAsync(dst, at, n * 4, cudaMemcpyDefault, stream));
+        at += n;
+    }
+    // Copies on the device are ordered before whatever the sequence runs next; host memory must not
+    // change under a copy.
+    if (!c->device_state) BC_CUDA(cudaStreamSynchronize(stream));
     s->n_past = c->n_past;
     return BC_OK;
 }
@@ -832,7 +870,6 @@ bc_status bc_seq_prefix_load(bc_seq* s, const bc_prefix* p) {
     if (s->conv_floats) BC_CUDA(cudaMemcpyAsync(s->conv_state, p->state, s->conv_floats * 4, cudaMemcpyDeviceToDevice, stream));
     if (s->delta_floats) BC_CUDA(cudaMemcpyAsync(s->delta_state, p->state + s->conv_floats, s->delta_floats * 4, cudaMemcpyDeviceToDevice, stream));
     BC_CUDA(cudaMemcpyAsync(s->logits, p->state + s->conv_floats + s->delta_floats, (size_t)hp.n_vocab * 4, cudaMemcpyDeviceToDevice, stream));
-    BC_CUDA(cudaStreamSynchronize(stream));
     s->shared_positions = first_copied;
     s->n_past = p->n_past;
     return BC_OK;

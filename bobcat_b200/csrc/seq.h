@@ -4,6 +4,7 @@
 
 #include <chrono>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -37,13 +38,30 @@ struct bc_prefix {
     ~bc_prefix();
 };
 
+// The device memory of a freed checkpoint, kept for the next one of the same sequence (a conversation
+// frees one and takes one at every turn): at most one block, shared by the sequence and its
+// checkpoints and given back with the last of them.
+struct SpareState {
+    std::mutex mutex;
+    float* block = nullptr;
+    int device = 0;
+    ~SpareState();
+};
+
+// The recurrent state at a position: [conv history | DeltaNet state | logits], on the device (9B shape:
+// 53 MB, which took longer to bring back from host memory than three decode steps take), or in host
+// memory when the device has no room.
 struct bc_checkpoint {
     const bc_seq* owner = nullptr;
     uint64_t resets = 0;
     uint32_t n_past = 0;
-    std::vector<float> conv_state;   // LFM2 conv history, or Qwen conv history of every DeltaNet layer
-    std::vector<float> delta_state;  // Qwen DeltaNet state matrices
-    std::vector<float> logits;
+    size_t conv_floats = 0;          // LFM2 conv history, or Qwen conv history of every DeltaNet layer
+    size_t delta_floats = 0;         // Qwen DeltaNet state matrices
+    size_t n_vocab = 0;
+    float* device_state = nullptr;
+    std::vector<float> host_state;
+    std::shared_ptr<SpareState> spare;
+    ~bc_checkpoint();
 };
 
 struct bc_comm;
@@ -73,6 +91,7 @@ struct bc_seq {
     // caches are paged (then k_cache / v_cache are the bases of the paged ranges below).
     uint32_t kv_stride = 0;
     std::unique_ptr<bc::PagedCache> k_pages, v_pages;
+    std::shared_ptr<SpareState> spare_checkpoint;
     uint32_t shared_positions = 0;  // positions [0, shared_positions) lie in pages shared with a prefix
     float *k = nullptr, *v = nullptr, *conv_state = nullptr, *hidden = nullptr, *normed = nullptr, *bcx = nullptr;
     float *conv_out = nullptr, *q = nullptr, *attn = nullptr, *scores = nullptr, *ffn = nullptr, *logits = nullptr;
