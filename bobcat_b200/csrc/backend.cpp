@@ -41,7 +41,7 @@ bc_status check_range(const bc_backend* backend, const bc_buffer* buffer, size_t
 namespace {
 
 // Per device: one word of mapped host memory per kernel file with bounded waits, for the life of the process.
-constexpr int kWaitWords = 4, kMaxDevices = 64;
+constexpr int kWaitWords = 5, kMaxDevices = 64;
 std::atomic<volatile int*> g_wait_words[kMaxDevices];
 
 bc_status set_wait_words(int device) {
@@ -56,6 +56,7 @@ bc_status set_wait_words(int device) {
     BC_CUDA(k::matmul_wait_word(words + 1));
     BC_CUDA(k::matmul_few_wait_word(words + 2));
     BC_CUDA(k::peer_wait_word(words + 3));
+    BC_CUDA(k::matmul_half_wait_word(words + 4));
     g_wait_words[device].store(words);
     return BC_OK;
 }
@@ -76,6 +77,7 @@ bc_status kernel_wait_status() {
     };
     if (int code = take(0)) return fail(BC_ERR_EXECUTION, "a decode kernel gave up waiting for its weight stream or its input (code %d)", code);
     if (int code = take(1)) return fail(BC_ERR_EXECUTION, "a prefill kernel gave up waiting on its pipeline (code %d)", code);
+    if (int code = take(4)) return fail(BC_ERR_EXECUTION, "a prefill kernel gave up waiting on its pipeline (code %d)", code);
     if (int code = take(2)) return fail(BC_ERR_EXECUTION, "a few-token product gave up waiting for its weights (code %d)", code);
     if (int code = take(3)) return fail(BC_ERR_EXECUTION, "a sum over ranks gave up waiting for rank %d", code - 1);
     return BC_OK;
@@ -150,6 +152,23 @@ bc_status matrix_view(bc_backend* b, bc_buffer* buffer, size_t offset, int32_t f
     return BC_OK;
 }
 
+// Expand an uploaded matrix for products of many tokens, once. Without room the other kernels serve.
+bc_status expand_for_many_tokens(bc_backend* b, bc_buffer* buffer) {
+    if (buffer->half_tiles_tried) return BC_OK;
+    buffer->half_tiles_tried = true;
+    k::Mat& m = buffer->matrix;
+    const uint64_t bytes = k::half_tiles_bytes(m.n_rows, m.n_cols);
+    if (m.format != BC_Q4_0 || !k::half_tiles_supported(m.n_cols) || !k::half_tiles_fit(bytes)) return BC_OK;
+    if (cudaMalloc(&buffer->half_tiles, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        buffer->half_tiles = nullptr;
+        return BC_OK;
+    }
+    m.half_tiles = buffer->half_tiles;
+    BC_CUDA(k::expand_half_tiles(b->stream, m.data, m.scales, m.n_rows, m.n_cols, buffer->half_tiles));
+    return BC_OK;
+}
+
 // The vectorised kernels read activations 16 bytes at a time: views of activation vectors must
 // start on a 16-byte boundary (cudaMalloc bases are 256-byte aligned, so only the offset matters).
 // Checked before any launch, because a misaligned vector load is a device fault, not a status code.
@@ -201,7 +220,8 @@ void bc_backend_close(bc_backend* b) {
     // Buffers that outlive their backend are orphaned; their frees become no-ops on the pointer.
     for (bc_buffer* buffer : b->buffers) {
         cudaFree(buffer->ptr);
-        buffer->ptr = nullptr;
+        cudaFree(buffer->half_tiles);
+        buffer->ptr = buffer->half_tiles = nullptr;
         buffer->backend = nullptr;
     }
     if (b->pack) cudaFree(b->pack);
@@ -241,6 +261,7 @@ void bc_buffer_free(bc_buffer* buffer) {
         cudaStreamSynchronize(buffer->backend->stream);
         buffer->backend->buffers.erase(buffer);
         cudaFree(buffer->ptr);
+        cudaFree(buffer->half_tiles);
     }
     delete buffer;
 }
@@ -506,6 +527,10 @@ bc_status bc_op_matmul(bc_backend* b, int32_t format, bc_buffer* weights, size_t
     if (store < BC_STORE_OVERWRITE || store > BC_STORE_SWIGLU) return fail(BC_ERR_ARGUMENT, "unknown store mode %d", store);
     k::Mat w;
     BC_TRY(matrix_view(b, weights, w_off, format, n_rows, n_cols, "matmul", &w));
+    if (n_tokens >= k::kMinHalfTokens) {
+        BC_TRY(expand_for_many_tokens(b, weights));
+        BC_TRY(matrix_view(b, weights, w_off, format, n_rows, n_cols, "matmul", &w));
+    }
     BC_TRY(check_range(b, x, x_off, (size_t)n_tokens * n_cols * 4, "matmul"));
     BC_TRY(check_range(b, y, y_off, (size_t)n_tokens * n_rows * 4, "matmul"));
     BC_TRY(check_aligned("matmul", {x_off, y_off}));

@@ -24,6 +24,10 @@ struct bc_buffer {
     // Set by bc_matrix_upload: the matrix this buffer holds in the device layout.
     bool is_matrix = false;
     bc::k::Mat matrix;
+    // The matrix expanded for products of many tokens, made by the first such product (most uploaded
+    // matrices, expert stacks among them, never meet one), unless the device had no room then.
+    void* half_tiles = nullptr;
+    bool half_tiles_tried = false;
 };
 
 // Token slots in host-mapped memory that argmax launches write and the CPU reads once the

@@ -25,6 +25,9 @@ struct Mat {
     // Q4_0 only, optional: the same values in the 16-row tile layout the tensor-core decode kernel
     // streams (see kernels_matvec_mma.cu). Null when the matrix has no such copy.
     const void* tiles = nullptr;
+    // Q4_0 only, optional: the values expanded to fp16 in 128-row operand tiles of the tensor cores
+    // (kernels_matmul_half.cu), for products of many tokens.
+    const void* half_tiles = nullptr;
     uint32_t n_rows = 0, n_cols = 0;
     // Rows [first, first + rows) of this matrix.
     Mat rows(uint32_t first, uint32_t count) const;
@@ -353,6 +356,24 @@ bool matmul_umma_swiglu_supported(const Mat& gate, const Mat& up, uint32_t n_tok
 // is not touched.
 cudaError_t matmul_umma_swiglu(cudaStream_t stream, const Mat& gate, const Mat& up, const void* packed, float* y, uint32_t n_tokens,
                                uint32_t y_stride, void* packed_out = nullptr);
+// The same products from expanded weights (kernels_matmul_half.cu), for batches of kMinHalfTokens and more
+// of matrices that carry half_tiles; the functions above hand over to them (BOBCAT_NO_HALF_MATMUL=1: no
+// matrix gets half_tiles).
+constexpr uint32_t kMinHalfTokens = 33;
+cudaError_t matmul_half_wait_word(int* word);
+uint64_t half_tiles_bytes(uint32_t n_rows, uint32_t n_cols);
+bool half_tiles_supported(uint32_t n_cols);
+// Whether the current device has room for `bytes` of expanded weights: they may take at most half of
+// the memory that is free, the rest belongs to caches.
+bool half_tiles_fit(uint64_t bytes);
+cudaError_t expand_half_tiles(cudaStream_t stream, const void* quants, const __half* scales, uint32_t n_rows, uint32_t n_cols, void* tiles);
+bool matmul_half_supported(const Mat& w, uint32_t n_tokens);
+// Parts K is split into (1: none); with more, y takes `split` arrays of [n_tokens][n_rows] partial products.
+uint32_t matmul_half_split(const Mat& w, uint32_t n_tokens);
+cudaError_t matmul_half(cudaStream_t stream, const Mat* const* ws, float* const* ys, int n, const void* packed, uint32_t n_tokens, uint32_t y_stride,
+                        int32_t store, uint32_t split);
+cudaError_t matmul_half_swiglu(cudaStream_t stream, const Mat& gate, const Mat& up, const void* packed, float* y, uint32_t n_tokens, uint32_t y_stride,
+                               void* packed_out);
 // The same products for at most 32 tokens (kernels_matmul_few.cu): the matrices' decode tiles against
 // the packed inputs on warp-level MMAs, one launch, no split of K left open. matmul_umma,
 // matmul_umma_several, matmul_umma_swiglu and matmul_experts_umma hand over to these whenever the

@@ -1,0 +1,436 @@
+// The prefill contraction for more than a few tokens: Y[t][r] (store) sum_c W[r][c] X[t][c] on tcgen05
+// from weights that were expanded to fp16 once, when the model was uploaded.
+//
+// Arithmetic: that of kernels_matmul_umma.cu, operand for operand. Weights are (q - 8) * d rounded to fp16
+// once (dequant_word, at upload instead of on every launch), inputs are rounded to fp16, products
+// accumulate in f32 (the reference's Q4_0 prefill kernel, crates/bobcat-metal/src/matmul.metal:249-470).
+//
+// Why expanded weights. The kernel that dequantises on the way into shared memory is bound by that
+// conversion: its tensor cores wait for operands half of the time (2.6B shape, 512 tokens: 410 TFLOP/s). A
+// weight takes 2 bytes here instead of 18/32, which a device with 180 GB has room for (4.9 GB at 2.6B), and
+// reading them costs 0.75 ms per pass at the HBM rate, less than the multiply of 100 tokens and more. When
+// the expanded copy does not fit the device, Mat::half_tiles is null and the dequantising kernel serves.
+//
+// Shape. Persistent CTAs of ten warps, one per SM: a loader thread, an MMA thread, eight epilogue warps.
+// A tile is 128 weight rows x up to 256 tokens (or 128 rows of both matrices of a SwiGLU x up to 128
+// tokens, two accumulators). K advances 64 columns per stage through a four-stage ring; both operands
+// arrive by bulk copies of contiguous memory (the weight tile is stored as the 16 KB image the MMA reads,
+// the tokens come packed, kernels_matmul_umma.cu's pack kernels), so no thread touches an operand. Tensor
+// memory holds two accumulators of 256 columns: a tile's epilogue runs under the next tile's main
+// loop. Measured apart on this device: one tcgen05.mma M128 N256 K16 per 128 cycles (2.19 PFLOP/s), full rate
+// down to N = 128, with or without swizzle; bulk copies out of L2 above 15 TB/s.
+//
+// Matrices with few tiles split K; the partial products go to scratch and are added in index order by
+// the next normalisation or by reduce_kernel. Every wait is bounded, as in kernels_matmul_umma.cu.
+
+#include <cstdlib>
+
+#include "async_utils.cuh"
+#include "device_utils.cuh"
+#include "kernels.h"
+#include "../../include/bobcat_cuda.h"
+
+namespace bc {
+namespace k {
+
+namespace {
+
+using namespace async;
+
+constexpr uint32_t kRows = 128, kChunkK = 64, kCores = kChunkK / 8;
+constexpr uint32_t kATile = kRows * kChunkK * 2;       // 16 KB: [8-row group][core along K][row][16 bytes]
+constexpr uint32_t kGroupBytes = 8 * kChunkK * 2, kCoreBytes = 128;
+constexpr uint32_t kStages = 4, kStageBytes = 48 * 1024;
+constexpr uint32_t kEpilogueWarps = 8, kThreads = (2 + kEpilogueWarps) * 32;
+constexpr uint32_t kTmemColumns = 512, kAccColumns = 256;
+constexpr uint32_t kSpinLimit = 1u << 22;
+constexpr uint32_t kTurnBytes = 1152;                  // per epilogue warp: a 32 x 16 block turned into operand layout
+constexpr size_t kSmemBytes = kStages * kStageBytes + kEpilogueWarps * kTurnBytes + 1024;
+constexpr uint32_t kMaxSplit = 8;
+
+__device__ int* g_wait_word;  // where a wait that ran out leaves its code (kernels.h), null until set
+
+struct HalfParams {
+    // Up to four matrices that read the same inputs: row tiles [first_tile[i], first_tile[i + 1]) are
+    // matrix i's. Dual: tiles[0] = gate, tiles[1] = up, one matrix of outputs.
+    const __half* tiles[4];
+    float* y[4];
+    uint32_t first_tile[5], rows[4], stride[4];
+    int n_matrices;
+    const __half* packed;      // [n_chunks][token_groups][8 cores][8 tokens][8 halves]
+    uint32_t n_chunks, n_tokens, token_groups;
+    uint32_t tile_tokens, token_tiles, split, n_tiles;  // n_tiles = row tiles x split x token tiles
+    int store;
+    __half* packed_out;        // dual: the result as the packed operand of the product that consumes it
+};
+
+struct Tile {
+    uint32_t row_tile, part, tok0, n;      // n: the MMA's N, a multiple of 16
+    uint32_t chunk0, chunks;
+};
+
+__device__ __forceinline__ Tile tile_at(const HalfParams& p, uint32_t i) {
+    Tile t;
+    const uint32_t token_tile = i % p.token_tiles, rest = i / p.token_tiles;
+    t.part = rest % p.split;
+    t.row_tile = rest / p.split;
+    t.tok0 = token_tile * p.tile_tokens;
+    const uint32_t left = p.n_tokens - t.tok0;
+    t.n = left >= p.tile_tokens ? p.tile_tokens : (left + 15u) & ~15u;
+    const uint32_t per = (p.n_chunks + p.split - 1) / p.split;
+    t.chunk0 = min(t.part * per, p.n_chunks);
+    t.chunks = min(per, p.n_chunks - t.chunk0);
+    return t;
+}
+
+__device__ __forceinline__ void give_up(volatile int* dead, int code) {
+    *dead = 1;
+    if (g_wait_word) *reinterpret_cast<volatile int*>(g_wait_word) = code;
+}
+
+template <int DUAL>
+__global__ void __launch_bounds__(kThreads, 1) matmul_half_kernel(const __grid_constant__ HalfParams p) {
+    extern __shared__ __align__(1024) uint8_t smem[];
+    uint8_t* turns = smem + kStages * kStageBytes;
+    __shared__ __align__(8) uint64_t bars[2 * kStages + 4];
+    __shared__ uint32_t tmem_slot;
+    __shared__ volatile int dead_flag;
+    volatile int* dead = &dead_flag;
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t full0 = smem_u32(bars), empty0 = full0 + kStages * 8, acc_full0 = empty0 + kStages * 8, acc_empty0 = acc_full0 + 16;
+    const uint32_t ring = smem_u32(smem);
+    // The next launch may set itself up; it waits for this one before it touches its outputs.
+    pdl_launch_dependents();
+    if (tid == 0) {
+        for (uint32_t s = 0; s < kStages; ++s) {
+            mbar_init(full0 + 8 * s, 1);   // the loader's arrive.expect_tx
+            mbar_init(empty0 + 8 * s, 1);  // the MMA thread's commit
+        }
+        for (uint32_t a = 0; a < 2; ++a) {
+            mbar_init(acc_full0 + 8 * a, 1);
+            mbar_init(acc_empty0 + 8 * a, kEpilogueWarps);
+        }
+        dead_flag = 0;
+        mbar_init_fence();
+    }
+    if (warp == 1) tmem_alloc(smem_u32(&tmem_slot), kTmemColumns);
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    const uint32_t tmem = tmem_slot;
+
+    if (warp == 0) {
+        // ---- loader. The weights are nobody's output: the first tile's weight copies go out before the
+        // wait for the preceding launch, the tokens' follow it.
+        if (lane == 0) {
+            uint32_t stage = 0, phase = 1;
+            bool waited = false;
+            for (uint32_t i = blockIdx.x; i < p.n_tiles; i += gridDim.x) {
+                const Tile t = tile_at(p, i);
+                int m = 0;
+                if (DUAL == 1)
+                    while (m + 1 < p.n_matrices && t.row_tile >= p.first_tile[m + 1]) ++m;
+                const uint64_t at = ((uint64_t)(t.row_tile - (DUAL == 1 ? p.first_tile[m] : 0)) * p.n_chunks + t.chunk0) * (kATile / 2);
+                const __half* a = p.tiles[m] + at;
+                const __half* a2 = DUAL == 2 ? p.tiles[1] + at : nullptr;
+                const __half* b = p.packed + ((uint64_t)t.chunk0 * p.token_groups + t.tok0 / 8) * (8 * kChunkK);
+                const uint32_t b_bytes = t.n * kChunkK * 2;
+                auto weights = [&](uint32_t c, uint32_t s) {
+                    mbar_arrive_expect(full0 + 8 * s, DUAL * kATile + b_bytes);
+                    bulk_load(ring + s * kStageBytes, a + (uint64_t)c * (kATile / 2), kATile, full0 + 8 * s);
+                    if (DUAL == 2) bulk_load(ring + s * kStageBytes + kATile, a2 + (uint64_t)c * (kATile / 2), kATile, full0 + 8 * s);
+                };
+                auto tokens = [&](uint32_t c, uint32_t s) {
+                    bulk_load(ring + s * kStageBytes + DUAL * kATile, b + (uint64_t)c * p.token_groups * (8 * kChunkK), b_bytes, full0 + 8 * s);
+                };
+                uint32_t c = 0;
+                if (!waited) {
+                    const uint32_t first = t.chunks < kStages ? t.chunks : kStages;  // free stages: nothing to wait for
+                    for (; c < first; ++c) weights(c, c);
+                    pdl_wait();
+                    waited = true;
+                    for (uint32_t s = 0; s < first; ++s) tokens(s, s);
+                    stage = first % kStages;
+                    phase = first == kStages ? 0 : 1;
+                }
+                for (; c < t.chunks; ++c) {
+                    if (!mbar_wait(empty0 + 8 * stage, phase, kSpinLimit, dead)) {
+                        give_up(dead, 3);
+                        break;
+                    }
+                    weights(c, stage);
+                    tokens(c, stage);
+                    if (++stage == kStages) stage = 0, phase ^= 1;
+                }
+                if (*dead) break;
+            }
+        }
+    } else if (warp == 1) {
+        // ---- the tensor core
+        if (lane == 0) {
+            uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 1;
+            const uint64_t desc0 = umma_desc(ring, kCoreBytes, kGroupBytes);
+            bool alive = true;
+            for (uint32_t i = blockIdx.x; i < p.n_tiles && alive; i += gridDim.x) {
+                const Tile t = tile_at(p, i);
+                const uint32_t idesc = umma_idesc_f16(kRows, t.n);
+                if (!mbar_wait(acc_empty0 + 8 * acc, acc_phase, kSpinLimit, dead)) {
+                    give_up(dead, 1);
+                    break;
+                }
+                tc_fence_after_sync();
+                for (uint32_t c = 0; c < t.chunks; ++c) {
+                    if (!mbar_wait(full0 + 8 * stage, phase, kSpinLimit, dead)) {
+                        give_up(dead, 4);
+                        alive = false;
+                        break;
+                    }
+                    tc_fence_after_sync();
+                    const uint64_t a_desc = desc0 + ((stage * kStageBytes) >> 4), b_desc = a_desc + ((DUAL * kATile) >> 4);
+#pragma unroll
+                    for (uint32_t m = 0; m < (uint32_t)DUAL; ++m)
+#pragma unroll
+                        for (uint32_t j = 0; j < kChunkK / 16; ++j)
+                            umma_f16(tmem + acc * kAccColumns + m * (kAccColumns / 2), a_desc + ((m * kATile + j * 2 * kCoreBytes) >> 4),
+                                     b_desc + ((j * 2 * kCoreBytes) >> 4), idesc, (c | j) != 0);
+                    umma_commit(empty0 + 8 * stage);
+                    if (++stage == kStages) stage = 0, phase ^= 1;
+                }
+                if (alive) umma_commit(acc_full0 + 8 * acc);
+                if (++acc == 2) acc = 0, acc_phase ^= 1;
+            }
+        }
+    } else {
+        // ---- epilogue: a warp reads lanes 32 * (warp % 4).. of tensor memory and every other 16 columns
+        const uint32_t ew = warp - 2, quarter = warp & 3, half = ew >> 2;
+        uint32_t acc = 0, acc_phase = 0;
+        pdl_wait();  // y, the partial products and the packed output are other launches' to read or write until now
+        for (uint32_t i = blockIdx.x; i < p.n_tiles; i += gridDim.x) {
+            const Tile t = tile_at(p, i);
+            int m = 0;
+            if (DUAL == 1)
+                while (m + 1 < p.n_matrices && t.row_tile >= p.first_tile[m + 1]) ++m;
+            const uint32_t rows = p.rows[m], stride = p.stride[m];
+            const uint32_t row0 = (t.row_tile - (DUAL == 1 ? p.first_tile[m] : 0)) * kRows, out_row = row0 + quarter * 32 + lane;
+            float* out = p.y[m] + (p.split > 1 ? (uint64_t)t.part * p.n_tokens * stride : 0);
+            const bool ok = lane != 0 || mbar_wait(acc_full0 + 8 * acc, acc_phase, kSpinLimit, dead);
+            if (!__all_sync(0xffffffffu, ok)) {
+                if (lane == 0) give_up(dead, 2);
+                break;
+            }
+            tc_fence_after_sync();
+            const uint32_t from = tmem + ((quarter * 32) << 16) + acc * kAccColumns, units = t.n / 16;
+            for (uint32_t u = half; u < units; u += 2) {
+                float v[16];
+                __syncwarp();
+                tmem_load_16(from + u * 16, v);
+                if (DUAL == 2) {
+                    float up[16];
+                    tmem_load_16(from + kAccColumns / 2 + u * 16, up);
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) v[j] = v[j] / (1.f + expf(-v[j])) * up[j];
+                }
+                if (DUAL == 2 && p.packed_out) {
+                    // The warp's 32 rows are one block of 32 columns of the consuming product, its 16
+                    // tokens two groups of 8. The values turn through shared memory into 16-byte
+                    // core-matrix rows (17 rows of 16 bytes per core matrix keep both sides free of
+                    // bank conflicts); a lane stores two, 8 lanes to a 128-byte line.
+                    if (row0 + quarter * 32 < rows) {
+                        __half* turn = reinterpret_cast<__half*>(turns + ew * kTurnBytes);
+                        const uint32_t core = (lane & 15) >> 2, e = lane & 3;
+                        const uint32_t at = (lane >> 4) * 4 + (e & 1) * 2 + (e >> 1);
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) turn[(core * 17 + j) * 8 + at] = __float2half_rn(v[j]);
+                        __syncwarp();
+                        const uint32_t tr = lane & 7, mm = lane >> 3;
+                        const uint32_t chunk = (row0 >> 6) + (quarter >> 1), jj = (quarter & 1) * 4 + mm;
+#pragma unroll
+                        for (uint32_t it = 0; it < 2; ++it) {
+                            const uint4 row16 = *reinterpret_cast<const uint4*>(turn + (mm * 17 + it * 8 + tr) * 8);
+                            const uint32_t tg = ((t.tok0 + u * 16) >> 3) + it;
+                            reinterpret_cast<uint4*>(p.packed_out)[(((uint64_t)chunk * p.token_groups + tg) * kCores + jj) * 8 + tr] = row16;
+                        }
+                    }
+                    continue;
+                }
+                if (out_row < rows) {
+                    const uint32_t tok = t.tok0 + u * 16, live = p.n_tokens > tok ? p.n_tokens - tok : 0;
+                    float* to = out + (uint64_t)tok * stride + out_row;
+                    float old[16];
+                    if (DUAL == 1 && p.store != BC_STORE_OVERWRITE) {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) old[j] = (uint32_t)j < live ? __ldcg(to + (uint64_t)j * stride) : 0.f;
+                    }
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {
+                        if ((uint32_t)j < live) {
+                            float r = t.chunks ? v[j] : 0.f;
+                            if (DUAL == 1 && p.store == BC_STORE_ACCUMULATE) r += old[j];
+                            else if (DUAL == 1 && p.store == BC_STORE_SWIGLU) r = old[j] / (1.f + expf(-old[j])) * r;
+                            to[(uint64_t)j * stride] = r;
+                        }
+                    }
+                }
+            }
+            // The accumulator is read: the MMA thread may overwrite it.
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(acc_empty0 + 8 * acc);
+            if (++acc == 2) acc = 0, acc_phase ^= 1;
+        }
+    }
+
+    tc_fence_before_sync();
+    __syncthreads();
+    if (*dead) __nanosleep(100000);  // let copies and instructions still in flight land before the CTA goes
+    if (warp == 1) {
+        __syncwarp();
+        tc_fence_after_sync();
+        tmem_dealloc(tmem, kTmemColumns);
+    }
+}
+
+// Split layout -> expanded operand tiles: one thread per 16 bytes (eight weights of one row).
+__global__ void expand_tiles_kernel(const uint4* __restrict__ quants, const __half* __restrict__ scales, uint32_t n_rows, uint32_t n_blocks,
+                                    uint4* __restrict__ tiles, uint64_t total) {
+    const uint64_t o = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (o >= total) return;
+    const uint32_t in_tile = o % (kATile / 16), row_in_group = in_tile & 7, core = (in_tile >> 3) & (kCores - 1), group = in_tile >> 6;
+    const uint64_t tile = o / (kATile / 16);
+    const uint32_t n_chunks = n_blocks / 2, chunk = tile % n_chunks, row = (uint32_t)(tile / n_chunks) * kRows + group * 8 + row_in_group;
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (row < n_rows) {
+        const uint64_t block = (uint64_t)row * n_blocks + chunk * 2 + (core >> 2);
+        const uint4 q = quants[block];
+        const uint32_t w = (core & 3) == 0 ? q.x : (core & 3) == 1 ? q.y : (core & 3) == 2 ? q.z : q.w;
+        v = dequant_word(w, __half2half2(scales[block]));
+    }
+    tiles[o] = v;
+}
+
+struct Tiling {
+    uint32_t tile_tokens, split;
+};
+
+// The tiling with the smallest modelled time, in cycles: waves of tiles over the SMs, each chunk of 64
+// columns bound by the MMA (2 cycles per token and matrix, no less than a tile of 96 tokens costs) or by the
+// SM's share of L2 (fitted: 75 bytes per cycle), an exposed prologue and last epilogue, and a split's extra pass.
+Tiling choose_tiling(uint32_t row_tiles, uint32_t n_chunks, uint32_t n_tokens, int dual, bool may_split) {
+    const uint32_t sms = (uint32_t)sm_count(), widest = dual == 2 ? 128 : 256;
+    Tiling best{widest, 1};
+    double best_cost = 1e30;
+    const uint32_t fewest = (n_tokens + widest - 1) / widest;
+    for (uint32_t token_tiles = fewest; token_tiles <= fewest + 6; ++token_tiles) {
+        const uint32_t width = ((n_tokens + token_tiles - 1) / token_tiles + 15u) & ~15u;
+        if (width < 48 && token_tiles > fewest) break;
+        const uint32_t needed = (n_tokens + width - 1) / width;
+        for (uint32_t split = 1; split <= (may_split && dual == 1 ? kMaxSplit : 1u); ++split) {
+            if (split > 1 && n_chunks / split < 4) break;
+            const uint32_t tiles = row_tiles * needed * split, waves = (tiles + sms - 1) / sms;
+            const double mma = (width < 96 ? 192.0 : 2.0 * width) * dual, load = (16384.0 * dual + 128.0 * width) / 75.0;
+            double cost = waves * ((n_chunks + split - 1) / split) * (mma > load ? mma : load) + 3000.0 + 12.0 * width;
+            if (split > 1) cost += 1500.0 + (double)split * n_tokens * row_tiles * kRows * 4 * 2 / 4000.0;
+            if (cost < best_cost) best_cost = cost, best = Tiling{width, split};
+        }
+    }
+    return best;
+}
+
+bool half_disabled() {
+    static const bool off = [] {
+        const char* v = std::getenv("BOBCAT_NO_HALF_MATMUL");
+        return v && v[0] == '1';
+    }();
+    return off;
+}
+
+template <int DUAL>
+cudaError_t launch_half(cudaStream_t stream, HalfParams& p, Tiling tiling) {
+    p.tile_tokens = tiling.tile_tokens;
+    p.token_tiles = (p.n_tokens + tiling.tile_tokens - 1) / tiling.tile_tokens;
+    p.split = tiling.split;
+    p.n_tiles = p.first_tile[p.n_matrices] * p.split * p.token_tiles;
+    if (p.n_tiles == 0) return cudaSuccess;
+    const void* kernel = (const void*)matmul_half_kernel<DUAL>;
+    cudaError_t e = ensure_dynamic_smem(kernel, kSmemBytes);
+    if (e != cudaSuccess) return e;
+    const uint32_t sms = (uint32_t)sm_count();
+    void* args[] = {&p};
+    return launch_kernel(kernel, dim3(p.n_tiles < sms ? p.n_tiles : sms), dim3(kThreads), kSmemBytes, stream, args);
+}
+
+uint32_t row_tiles_of(const Mat& w) { return (w.n_rows + kRows - 1) / kRows; }
+
+void common(HalfParams& p, const Mat& w, const void* packed, uint32_t n_tokens, int store) {
+    p.packed = static_cast<const __half*>(packed);
+    p.n_chunks = w.n_cols / kChunkK;
+    p.n_tokens = n_tokens;
+    p.token_groups = ((n_tokens + 15u) & ~15u) / 8;
+    p.store = store;
+}
+
+}  // namespace
+
+cudaError_t matmul_half_wait_word(int* word) { return cudaMemcpyToSymbol(g_wait_word, &word, sizeof word); }
+
+uint64_t half_tiles_bytes(uint32_t n_rows, uint32_t n_cols) { return (uint64_t)((n_rows + kRows - 1) / kRows) * (n_cols / kChunkK) * kATile; }
+
+bool half_tiles_supported(uint32_t n_cols) { return !half_disabled() && n_cols % kChunkK == 0 && n_cols > 0; }
+
+bool half_tiles_fit(uint64_t bytes) {
+    size_t free_bytes = 0, total_bytes = 0;
+    return cudaMemGetInfo(&free_bytes, &total_bytes) == cudaSuccess && bytes <= free_bytes / 2;
+}
+
+cudaError_t expand_half_tiles(cudaStream_t stream, const void* quants, const __half* scales, uint32_t n_rows, uint32_t n_cols, void* tiles) {
+    const uint64_t total = half_tiles_bytes(n_rows, n_cols) / 16;
+    if (total == 0) return cudaSuccess;
+    expand_tiles_kernel<<<(unsigned)((total + 255) / 256), 256, 0, stream>>>(static_cast<const uint4*>(quants), scales, n_rows, n_cols / 32,
+                                                                          static_cast<uint4*>(tiles), total);
+    return cudaGetLastError();
+}
+
+bool matmul_half_supported(const Mat& w, uint32_t n_tokens) { return w.half_tiles != nullptr && n_tokens >= kMinHalfTokens && !half_disabled(); }
+
+uint32_t matmul_half_split(const Mat& w, uint32_t n_tokens) {
+    return choose_tiling(row_tiles_of(w), w.n_cols / kChunkK, n_tokens, 1, w.n_rows % 4 == 0).split;
+}
+
+cudaError_t matmul_half(cudaStream_t stream, const Mat* const* ws, float* const* ys, int n, const void* packed, uint32_t n_tokens, uint32_t y_stride,
+                        int32_t store, uint32_t split) {
+    if (n < 1 || n > 4) return cudaErrorInvalidValue;
+    HalfParams p{};
+    common(p, *ws[0], packed, n_tokens, store);
+    p.n_matrices = n;
+    for (int i = 0; i < n; ++i) {
+        if (ws[i]->n_cols != ws[0]->n_cols || !ws[i]->half_tiles) return cudaErrorInvalidValue;
+        p.tiles[i] = static_cast<const __half*>(ws[i]->half_tiles);
+        p.y[i] = ys[i];
+        p.rows[i] = ws[i]->n_rows;
+        p.stride[i] = n == 1 ? y_stride : ws[i]->n_rows;
+        p.first_tile[i + 1] = p.first_tile[i] + row_tiles_of(*ws[i]);
+    }
+    Tiling tiling = choose_tiling(p.first_tile[n], p.n_chunks, n_tokens, 1, split > 1);
+    if (split > 1 && tiling.split != split) return cudaErrorInvalidValue;  // the caller sized the partial products by matmul_half_split
+    return launch_half<1>(stream, p, tiling);
+}
+
+cudaError_t matmul_half_swiglu(cudaStream_t stream, const Mat& gate, const Mat& up, const void* packed, float* y, uint32_t n_tokens, uint32_t y_stride,
+                               void* packed_out) {
+    if (gate.n_rows != up.n_rows || gate.n_cols != up.n_cols || !gate.half_tiles || !up.half_tiles || (packed_out && gate.n_rows % kChunkK != 0))
+        return cudaErrorInvalidValue;
+    HalfParams p{};
+    common(p, gate, packed, n_tokens, BC_STORE_OVERWRITE);
+    p.n_matrices = 1;
+    p.tiles[0] = static_cast<const __half*>(gate.half_tiles);
+    p.tiles[1] = static_cast<const __half*>(up.half_tiles);
+    p.y[0] = y;
+    p.rows[0] = gate.n_rows;
+    p.stride[0] = y_stride;
+    p.first_tile[1] = row_tiles_of(gate);
+    p.packed_out = static_cast<__half*>(packed_out);
+    return launch_half<2>(stream, p, choose_tiling(p.first_tile[1], p.n_chunks, n_tokens, 2, false));
+}
+
+}  // namespace k
+}  // namespace bc

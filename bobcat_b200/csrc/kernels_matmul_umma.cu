@@ -734,7 +734,7 @@ uint64_t matmul_pack_bytes(uint32_t n_tokens, uint32_t n_cols) { return (uint64_
 
 uint64_t matmul_partial_bytes(const Mat& w, uint32_t n_tokens) {
     if (const uint32_t slices = matmul_few_slices(w, n_tokens)) return (uint64_t)slices * n_tokens * w.n_rows * 4;
-    uint32_t split = choose_tiling(w.n_rows, w.n_cols, n_tokens, w.n_rows, 1, true).split;
+    const uint32_t split = matmul_half_supported(w, n_tokens) ? matmul_half_split(w, n_tokens) : choose_tiling(w.n_rows, w.n_cols, n_tokens, w.n_rows, 1, true).split;
     return split > 1 ? (uint64_t)split * n_tokens * w.n_rows * 4 : 0;
 }
 
@@ -746,6 +746,7 @@ uint64_t matmul_scratch_bytes(const Mat& w, uint32_t n_tokens) {
 int matmul_umma_launches(const Mat& w, uint32_t n_tokens) {
     if (matmul_few_supported(w, n_tokens)) return 2;
     if (matmul_few_slices(w, n_tokens)) return 3;
+    if (matmul_half_supported(w, n_tokens)) return matmul_half_split(w, n_tokens) > 1 ? 3 : 2;
     return choose_tiling(w.n_rows, w.n_cols, n_tokens, w.n_rows, 1, true).split > 1 ? 3 : 2;
 }
 
@@ -807,14 +808,22 @@ cudaError_t matmul_umma(cudaStream_t stream, const Mat& w, const void* scratch, 
         return launch_dependent(reduce_kernel, dim3((unsigned)((quads + 255) / 256)), dim3(256), 0, stream, static_cast<const float*>(partial), y, w.n_rows,
                                 n_tokens, y_stride, slices, (int)store);
     }
-    cudaError_t err = ensure_dynamic_smem(reinterpret_cast<const void*>(&matmul_umma_kernel<1>), Shape<1>::kSmemBytes);
-    if (err != cudaSuccess) return err;
+    const bool half = matmul_half_supported(w, n_tokens);
+    cudaError_t err = cudaSuccess;
+    if (!half && (err = ensure_dynamic_smem(reinterpret_cast<const void*>(&matmul_umma_kernel<1>), Shape<1>::kSmemBytes)) != cudaSuccess) return err;
     // The split must match matmul_scratch_bytes, which sized the scratch for a dense output.
-    const Tiling tiling = choose_tiling(w.n_rows, w.n_cols, n_tokens, y_stride, 1, y_stride == w.n_rows);
+    const Tiling tiling = half ? Tiling{0, y_stride == w.n_rows ? matmul_half_split(w, n_tokens) : 1}
+                               : choose_tiling(w.n_rows, w.n_cols, n_tokens, y_stride, 1, y_stride == w.n_rows);
     const uint32_t split = tiling.split;
     float* partial = partial_at ? partial_at
                                 : reinterpret_cast<float*>(static_cast<char*>(const_cast<void*>(scratch)) +
                                                            ((matmul_pack_bytes(n_tokens, w.n_cols) + 255) & ~255ull));
+    if (half) {
+        const Mat* ws[1] = {&w};
+        float* to = split > 1 ? partial : y;
+        if ((err = matmul_half(stream, ws, &to, 1, scratch, n_tokens, split > 1 ? w.n_rows : y_stride, split > 1 ? (int32_t)BC_STORE_OVERWRITE : store, split)) != cudaSuccess)
+            return err;
+    }
     UmmaParams p{};
     p.quants[0] = static_cast<const uint4*>(w.data);
     p.scales[0] = w.scales;
@@ -829,8 +838,8 @@ cudaError_t matmul_umma(cudaStream_t stream, const Mat& w, const void* scratch, 
     p.split = split;
     p.tile_tokens = tiling.tile_tokens;
     p.store = split > 1 ? BC_STORE_OVERWRITE : store;
-    dim3 grid((n_tokens + tiling.tile_tokens - 1) / tiling.tile_tokens, (w.n_rows + kRows - 1) / kRows, split);
-    {
+    if (!half) {
+        dim3 grid((n_tokens + tiling.tile_tokens - 1) / tiling.tile_tokens, (w.n_rows + kRows - 1) / kRows, split);
         void* args[] = {&p};
         cudaError_t launched = launch_kernel(reinterpret_cast<const void*>(&matmul_umma_kernel<1>), grid, dim3(Shape<1>::kThreads), Shape<1>::kSmemBytes, stream, args);
         if (launched != cudaSuccess) return launched;
@@ -856,6 +865,9 @@ cudaError_t matmul_umma_several(cudaStream_t stream, const Mat* const* ws, float
         for (int i = 0; i < n; ++i) strides[i] = ws[i]->n_rows;
         return matmul_few(stream, ws, ys, strides, n, packed, n_tokens, BC_STORE_OVERWRITE);
     }
+    bool half = true;
+    for (int i = 0; i < n; ++i) half = half && matmul_half_supported(*ws[i], n_tokens) && ws[i]->n_cols == ws[0]->n_cols;
+    if (half) return matmul_half(stream, ws, ys, n, packed, n_tokens, ws[0]->n_rows, BC_STORE_OVERWRITE, 1);
     cudaError_t err = ensure_dynamic_smem(reinterpret_cast<const void*>(&matmul_umma_kernel<1>), Shape<1>::kSmemBytes);
     if (err != cudaSuccess) return err;
     uint32_t total_rows = 0, tiles = 0;
@@ -907,6 +919,8 @@ cudaError_t matmul_umma_swiglu(cudaStream_t stream, const Mat& gate, const Mat& 
     if (n_tokens == 0 || gate.n_rows == 0) return cudaSuccess;
     if (matmul_few_supported(gate, n_tokens) && matmul_few_supported(up, n_tokens))
         return matmul_few_swiglu(stream, gate, up, packed, y, n_tokens, y_stride, packed_out);
+    if (matmul_half_supported(gate, n_tokens) && matmul_half_supported(up, n_tokens))
+        return matmul_half_swiglu(stream, gate, up, packed, y, n_tokens, y_stride, packed_out);
     cudaError_t err = ensure_dynamic_smem(reinterpret_cast<const void*>(&matmul_umma_kernel<2>), Shape<2>::kSmemBytes);
     if (err != cudaSuccess) return err;
     UmmaParams p{};

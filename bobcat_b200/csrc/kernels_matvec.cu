@@ -281,6 +281,7 @@ Mat Mat::rows(uint32_t first, uint32_t count) const {
         m.data = static_cast<const uint4*>(data) + first * nb;
         m.scales = scales + first * nb;
         // Tiles hold 16 rows each, so only a tile-aligned row range keeps its tile copy.
+        m.half_tiles = (half_tiles && first % 128 == 0) ? static_cast<const uint8_t*>(half_tiles) + (uint64_t)(first / 128) * (n_cols / 64) * 16384 : nullptr;
         m.tiles = (tiles && first % 16 == 0) ? static_cast<const uint8_t*>(tiles) + (uint64_t)(first / 16) * nb * 288 : nullptr;
     } else if (format == BC_F16) {
         m.data = static_cast<const __half*>(data) + (uint64_t)first * n_cols;

@@ -285,6 +285,7 @@ uint64_t device_bytes(const HostMatrix& hm) {
 bc::DeviceModel::~DeviceModel() {
     if (arena || !extra.empty()) cudaSetDevice(device);
     if (arena) cudaFree(arena);
+    if (half_arena) cudaFree(half_arena);
     for (void* p : extra) cudaFree(p);
 }
 
@@ -409,6 +410,31 @@ bc_status bc_model::device_model(bc_backend* backend, std::shared_ptr<DeviceMode
         BC_TRY(upload_vector(S.a, &D.a));
         BC_TRY(upload_vector(S.ssm_norm, &D.ssm_norm));
         BC_TRY(upload_vector(S.expert_bias, &D.expert_bias));
+    }
+    // The expanded copies of the dense matrices (an expert's matrices meet a few tokens at a time).
+    std::vector<k::Mat*> dense;
+    uint64_t half_bytes = 0;
+    for (size_t il = 0; il < layers.size(); ++il) {
+        DeviceLayer& D = dm->layers[il];
+        for (k::Mat* m : {&D.q, &D.k, &D.v, &D.output, &D.in_proj, &D.out_proj, &D.qkv, &D.z, &D.beta, &D.alpha, &D.ssm_out, &D.gate, &D.up, &D.down}) {
+            if (layers[il].moe && (m == &D.gate || m == &D.up || m == &D.down)) continue;
+            if (!m->data || m->format != BC_Q4_0 || !k::half_tiles_supported(m->n_cols)) continue;
+            dense.push_back(m);
+            half_bytes += k::half_tiles_bytes(m->n_rows, m->n_cols);
+        }
+    }
+    if (half_bytes && k::half_tiles_fit(half_bytes)) {
+        if (cudaMalloc(&dm->half_arena, half_bytes) != cudaSuccess) {
+            cudaGetLastError();
+            dm->half_arena = nullptr;
+        } else {
+            char* at = static_cast<char*>(dm->half_arena);
+            for (k::Mat* m : dense) {
+                BC_CUDA(k::expand_half_tiles(backend->stream, m->data, m->scales, m->n_rows, m->n_cols, at));
+                m->half_tiles = at;
+                at += k::half_tiles_bytes(m->n_rows, m->n_cols);
+            }
+        }
     }
     BC_CUDA(cudaStreamSynchronize(backend->stream));
     on_device[backend->device] = dm;

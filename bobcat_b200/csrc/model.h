@@ -55,6 +55,7 @@ struct DeviceModel {
     int device = 0;
     void* arena = nullptr;
     size_t arena_bytes = 0;
+    void* half_arena = nullptr;  // the dense Q4_0 matrices expanded for products of many tokens; null when they do not fit
     std::vector<DeviceLayer> layers;
     k::Mat token_embd, output;
     const float* output_norm = nullptr;

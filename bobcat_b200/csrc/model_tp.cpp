@@ -81,6 +81,13 @@ struct Uploader {
                 mat->tiles = tiles;
                 BC_CUDA(k::repack_tiles(stream, dst, mat->scales, n_rows, n_cols, tiles));
             }
+            const uint64_t half_bytes = k::half_tiles_bytes(n_rows, n_cols);
+            if (k::half_tiles_supported(n_cols) && k::half_tiles_fit(half_bytes)) {
+                char* half_tiles = nullptr;
+                BC_TRY(device_alloc(half_bytes, &half_tiles));
+                BC_CUDA(k::expand_half_tiles(stream, dst, mat->scales, n_rows, n_cols, half_tiles));
+                mat->half_tiles = half_tiles;
+            }
             BC_CUDA(cudaStreamSynchronize(stream));
             return BC_OK;
         }
