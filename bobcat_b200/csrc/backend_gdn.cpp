@@ -64,6 +64,16 @@ bc_status bc_op_gdn_recurrence(bc_backend* b, bc_buffer* qkv, size_t qkv_off, bc
     BC_TRY(check_range(b, decay, decay_off, (size_t)n_tokens * n_v_heads * 4, "gdn_recurrence"));
     BC_TRY(check_range(b, state, state_off, (size_t)n_v_heads * k_dim * v_dim * 4, "gdn_recurrence"));
     BC_TRY(check_range(b, out, out_off, (size_t)n_tokens * n_v_heads * v_dim * 4, "gdn_recurrence"));
+    const auto address = [](const bc_buffer* buffer, size_t offset) { return reinterpret_cast<uintptr_t>(buffer->ptr) + offset; };
+    const bool aligned = ((address(qkv, qkv_off) | address(state, state_off) | address(out, out_off)) & 15) == 0;
+    if (!normalize && aligned && k::gdn_chunk_supported(n_v_heads, k_dim, v_dim, n_tokens)) {
+        void* scratch = nullptr;
+        BC_TRY(b->pack_scratch(k::gdn_chunk_scratch_bytes(n_v_heads, n_tokens), &scratch));
+        return b->run("gdn_recurrence", n_tokens, n_v_heads * v_dim, (uint64_t)n_v_heads * k_dim * v_dim * 8, 2, [&] {
+            return k::gdn_chunk(b->stream, at<const float>(qkv, qkv_off), at<const float>(beta, beta_off), at<const float>(decay, decay_off),
+                                at<float>(state, state_off), at<float>(out, out_off), scratch, n_k_heads, n_v_heads, k_dim, v_dim, n_tokens);
+        });
+    }
     return b->run("gdn_recurrence", n_tokens, n_v_heads * v_dim, (uint64_t)n_v_heads * k_dim * v_dim * 8, 1, [&] {
         return k::gdn_recurrence(b->stream, at<const float>(qkv, qkv_off), at<const float>(beta, beta_off), at<const float>(decay, decay_off),
                                  at<float>(state, state_off), at<float>(out, out_off), n_k_heads, n_v_heads, k_dim, v_dim, n_tokens, normalize != 0);

@@ -256,6 +256,12 @@ cudaError_t gdn_gates(cudaStream_t stream, float* beta, float* alpha, const floa
 // The gated delta rule over n_tokens; state [n_v_heads][k_dim][v_dim]; `normalize` L2-normalises q and k.
 cudaError_t gdn_recurrence(cudaStream_t stream, const float* qkv, const float* beta, const float* decay, float* state, float* out,
                            uint32_t n_k_heads, uint32_t n_v_heads, uint32_t k_dim, uint32_t v_dim, uint32_t n_tokens, bool normalize);
+// The same rule for a batch in chunks of 64 tokens (kernels_gdn_chunk.cu, two launches): q and k already
+// normalised, 16-byte aligned pointers, `scratch` of gdn_chunk_scratch_bytes.
+bool gdn_chunk_supported(uint32_t n_v_heads, uint32_t k_dim, uint32_t v_dim, uint32_t n_tokens);
+uint64_t gdn_chunk_scratch_bytes(uint32_t n_v_heads, uint32_t n_tokens);
+cudaError_t gdn_chunk(cudaStream_t stream, const float* qkv, const float* beta, const float* decay, float* state, float* out, void* scratch,
+                      uint32_t n_k_heads, uint32_t n_v_heads, uint32_t k_dim, uint32_t v_dim, uint32_t n_tokens);
 // The q and k heads of qkv ([n_tokens][2 * n_k_heads * k_dim + n_v_heads * v_dim]) L2-normalised in
 // place, q also times 1 / sqrt(k_dim): what gdn_recurrence does per token with `normalize`, done
 // for the whole batch at once, so the recurrence can run without it.

@@ -559,7 +559,15 @@ struct Recorder {
         uint64_t state_bytes = (uint64_t)hp.n_v_heads * hp.k_head_dim * hp.v_head_dim * 4 * 2;
         run("gdn_qk_norm", n * 2 * hp.n_k_heads, hp.k_head_dim, 0, 1,
             [&] { return k::gdn_qk_norm(stream, s.gdn_conv_out, hp.n_k_heads, hp.n_v_heads, hp.k_head_dim, hp.v_head_dim, n); });
-        run("gdn_recurrence", n, value_dim(), state_bytes, 1, [&] {
+        if (k::gdn_chunk_supported(hp.n_v_heads, hp.k_head_dim, hp.v_head_dim, n)) {
+            // No packed input is alive between the projections and the output projection.
+            void* scratch = nullptr;
+            if (status == BC_OK) status = s.backend->pack_scratch(k::gdn_chunk_scratch_bytes(hp.n_v_heads, n), &scratch);
+            run("gdn_recurrence", n, value_dim(), state_bytes, 2, [&] {
+                return k::gdn_chunk(stream, s.gdn_conv_out, s.gdn_beta, s.gdn_alpha, state, s.gdn_out, scratch, hp.n_k_heads, hp.n_v_heads, hp.k_head_dim,
+                                    hp.v_head_dim, n);
+            });
+        } else run("gdn_recurrence", n, value_dim(), state_bytes, 1, [&] {
             return k::gdn_recurrence(stream, s.gdn_conv_out, s.gdn_beta, s.gdn_alpha, state, s.gdn_out, hp.n_k_heads, hp.n_v_heads, hp.k_head_dim,
                                      hp.v_head_dim, n, false);
         });
