@@ -37,7 +37,7 @@ struct bc_batch {
     uint64_t launches = 0;
 
     ~bc_batch() {
-        if (backend) {
+        if (backend && !seqs.empty() && seqs[0]->backend) {  // a closed backend has detached its sequences
             cudaSetDevice(backend->device);
             cudaStreamSynchronize(backend->stream);
         }

@@ -383,22 +383,16 @@ cudaError_t matmul_half_swiglu(cudaStream_t stream, const Mat& gate, const Mat& 
 // The same products for at most 32 tokens (kernels_matmul_few.cu): the matrices' decode tiles against
 // the packed inputs on warp-level MMAs, one launch, no split of K left open. matmul_umma,
 // matmul_umma_several, matmul_umma_swiglu and matmul_experts_umma hand over to these whenever the
-// shape allows (BOBCAT_NO_FEW_MATMUL=1 keeps them on the tcgen05 kernel).
+// shape allows (BOBCAT_NO_FEW_MATMUL=1 keeps them on the tcgen05 kernels).
 bool matmul_few_supported(const Mat& w, uint32_t n_tokens);
-cudaError_t matmul_few_wait_word(int* word);
 cudaError_t matmul_few(cudaStream_t stream, const Mat* const* ws, float* const* ys, const uint32_t* strides, int n, const void* packed,
                        uint32_t n_tokens, int32_t store);
 cudaError_t matmul_few_swiglu(cudaStream_t stream, const Mat& gate, const Mat& up, const void* packed, float* y, uint32_t n_tokens, uint32_t y_stride,
                               void* packed_out);
-// A matrix too wide for matmul_few (more packed tokens than a CTA keeps): the number of slices of
-// K it is cut into (0: not this kernel's), and the product as that many arrays of
-// [n_tokens][w.n_rows] partial sums, to be added in index order.
-uint32_t matmul_few_slices(const Mat& w, uint32_t n_tokens);
-cudaError_t matmul_few_sliced(cudaStream_t stream, const Mat& w, const void* packed, float* partial, uint32_t n_tokens);
-bool matmul_few_experts_supported(const Mat& w, const Mat* up, uint32_t n_rows, uint32_t n_experts, uint32_t n_tokens);
+bool matmul_few_experts_supported(const Mat& w, const Mat* up, uint32_t n_rows, uint32_t n_experts, uint32_t n_tokens, uint32_t n_used);
 cudaError_t matmul_few_experts(cudaStream_t stream, const Mat& w, const Mat* up, uint32_t n_rows, uint32_t n_experts, const void* packed,
                                const uint32_t* offsets, const uint32_t* entries, float* y, uint32_t n_tokens, uint32_t n_entries);
-// Products of a few rows with f32 operands (kernels_matmul_exact.cu): up to four Q4_0 matrices that
+// Products of a few rows with f32 operands (the same file): up to four Q4_0 matrices that
 // share the rows, with the rows' RMSNorm when given, in one launch; gate and up of a SwiGLU; the
 // experts of a grouped batch. `matmul` and `matmul_experts` hand over to these when their shape allows
 // (BOBCAT_NO_EXACT_MATMUL=1 keeps them on the tile kernels).
