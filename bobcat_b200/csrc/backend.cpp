@@ -512,7 +512,7 @@ bc_status bc_op_short_conv(bc_backend* b, bc_buffer* bcx, size_t bcx_off, bc_buf
     BC_TRY(check_range(b, taps, taps_off, (size_t)n_embd * kernel * 4, "short_conv"));
     BC_TRY(check_range(b, history, hist_off, (size_t)n_embd * (kernel - 1) * 4, "short_conv"));
     BC_TRY(check_range(b, out, out_off, (size_t)n_tokens * n_embd * 4, "short_conv"));
-    return b->run("short_conv", n_tokens, n_embd, 0, 2, [&] {
+    return b->run("short_conv", n_tokens, n_embd, 0, 1, [&] {
         return k::short_conv(b->stream, reinterpret_cast<const float*>(at(bcx, bcx_off)), reinterpret_cast<const float*>(at(taps, taps_off)),
                              reinterpret_cast<float*>(at(history, hist_off)), reinterpret_cast<float*>(at(out, out_off)), n_embd, kernel,
                              n_tokens);

@@ -140,6 +140,20 @@ struct RopeStore {
     const float2* table = nullptr;
 };
 // (cos, sin) of every rotation pair at positions [0, n_positions), the values rope_store computes.
+// A batch's queries and keys, normalised and rotated, and its keys and values in the caches, in one launch.
+struct RopeBatch {
+    const float* q;   // [token][q_stride], heads q_head_stride apart
+    float* q_dst;     // [token][q_dst_stride], heads q_dst_head_stride apart; may be q
+    const float *k, *v;  // [token][n_kv_heads * head_dim]
+    void* k_dst;      // cache row of the first token
+    __half* v_dst;    // the same of the values, or null when they are in the cache already
+    const float *q_norm, *k_norm;
+    uint32_t n_heads, n_kv_heads, head_dim, q_stride, q_head_stride, q_dst_stride, q_dst_head_stride, n_rot, first_pos, n_tokens;
+    float theta, eps;
+    bool kv_half;
+    const float2* rope_table;  // [position][n_rot / 2] (cos, sin), or null to compute them
+};
+cudaError_t rope_store_batch(cudaStream_t stream, const RopeBatch& p);
 cudaError_t rope_table(cudaStream_t stream, float2* table, uint32_t n_positions, uint32_t n_rot, float theta);
 cudaError_t rope_store(cudaStream_t stream, const RopeStore& p, Pos pos);
 // One thread: *counter += 1.
@@ -249,7 +263,9 @@ cudaError_t advance_seqs(cudaStream_t stream, uint32_t* pos, uint32_t n_seqs);
 // DeltaNet causal convolution with SiLU over [n_tokens][conv_dim]; history [conv_dim][kernel - 1].
 cudaError_t gdn_conv(cudaStream_t stream, const float* x, const float* taps, float* history, float* out, uint32_t conv_dim,
                      uint32_t kernel, uint32_t n_tokens);
-int gdn_conv_launches(uint32_t n_tokens);
+// gdn_conv over q heads, k heads and v heads, then the L2 norms of q and k (q also times 1 / sqrt(k_dim)), and gdn_gates, in one launch.
+cudaError_t gdn_conv_gates(cudaStream_t stream, const float* x, const float* taps, float* history, float* out, float* beta, float* alpha, const float* a,
+                           const float* dt_bias, uint32_t n_k_heads, uint32_t n_v_heads, uint32_t k_dim, uint32_t v_dim, uint32_t kernel, uint32_t n_tokens);
 // In place: beta = sigmoid(beta); alpha = exp(a * softplus(alpha + dt_bias)).
 cudaError_t gdn_gates(cudaStream_t stream, float* beta, float* alpha, const float* a, const float* dt_bias, uint32_t n_v_heads,
                       uint32_t n_tokens);
@@ -262,10 +278,6 @@ bool gdn_chunk_supported(uint32_t n_v_heads, uint32_t k_dim, uint32_t v_dim, uin
 uint64_t gdn_chunk_scratch_bytes(uint32_t n_v_heads, uint32_t n_tokens);
 cudaError_t gdn_chunk(cudaStream_t stream, const float* qkv, const float* beta, const float* decay, float* state, float* out, void* scratch,
                       uint32_t n_k_heads, uint32_t n_v_heads, uint32_t k_dim, uint32_t v_dim, uint32_t n_tokens);
-// The q and k heads of qkv ([n_tokens][2 * n_k_heads * k_dim + n_v_heads * v_dim]) L2-normalised in
-// place, q also times 1 / sqrt(k_dim): what gdn_recurrence does per token with `normalize`, done
-// for the whole batch at once, so the recurrence can run without it.
-cudaError_t gdn_qk_norm(cudaStream_t stream, float* qkv, uint32_t n_k_heads, uint32_t n_v_heads, uint32_t k_dim, uint32_t v_dim, uint32_t n_tokens);
 // One token through the whole mixer after its projections (conv with history shift, gates, L2
 // norms, delta rule, gated norm) in one launch; gdn_step_supported says whether the shape fits.
 bool gdn_step_supported(uint32_t n_k_heads, uint32_t n_v_heads, uint32_t k_dim, uint32_t v_dim, uint32_t kernel);
@@ -275,6 +287,10 @@ cudaError_t gdn_step(cudaStream_t stream, const float* qkv, const float* taps, f
 // x = RMSNorm(x) * weight * silu(z) per row of v_dim.
 cudaError_t gdn_gated_norm(cudaStream_t stream, float* x, const float* z, const float* weight, uint32_t v_dim, uint32_t n_rows,
                            float eps);
+// The same over n_heads rows a token, as the packed fp16 input of a product (x keeps its values).
+bool gdn_gated_norm_pack_supported(uint32_t v_dim);
+cudaError_t gdn_gated_norm_pack(cudaStream_t stream, const float* x, const float* z, const float* weight, uint32_t v_dim, uint32_t n_heads, uint32_t n_tokens,
+                                float eps, void* packed);
 // out *= sigmoid(gate), the gate read from the interleaved [q | gate] projection.
 cudaError_t attention_gate(cudaStream_t stream, float* out, const float* q_gate, uint32_t n_heads, uint32_t head_dim, uint32_t n_tokens);
 
@@ -339,6 +355,8 @@ struct Deferred {
 };
 // Bytes of partial products matmul_umma writes for this shape (zero when it does not split K).
 uint64_t matmul_partial_bytes(const Mat& w, uint32_t n_tokens);
+// matmul_pack of x times the sigmoid of its gates (attention_gate), heads of a multiple of 32 elements.
+cudaError_t matmul_pack_gated(cudaStream_t stream, const float* x, const float* q_gate, uint32_t head_dim, uint32_t n_tokens, uint32_t n_cols, void* packed);
 // With `add` (for this x: n_tokens rows of n_cols), x += the deferred partial products first, so
 // the sum a split-K product into the residual stream left open costs no launch of its own.
 cudaError_t matmul_pack_norm(cudaStream_t stream, float* x, Norm norm, uint32_t n_tokens, uint32_t n_cols, void* packed,

@@ -15,87 +15,23 @@ namespace k {
 
 namespace {
 
-constexpr uint32_t kConvSerialTokens = 4;  // up to this many tokens one launch walks them serially
-
-// One thread per (token, channel). x and out are [n_tokens][conv_dim]; taps are [conv_dim][K],
-// oldest first; history is [conv_dim][K - 1] raw inputs, oldest first. The sum starts from the
-// newest tap's term and adds the earlier inputs oldest first (qwen35.rs:449-461), from the batch or,
-// for its first tokens, from the history, so any split into batches gives the same bits. K <= 8.
-// The history is only read here; gdn_conv_history_kernel rewrites it afterwards.
-__global__ void __launch_bounds__(256) gdn_conv_kernel(const float* __restrict__ x, const float* __restrict__ taps,
-                                                       const float* __restrict__ history, float* __restrict__ out, uint32_t conv_dim,
-                                                       uint32_t kernel, uint32_t n_tokens) {
-    pdl_launch_dependents();
-    pdl_wait();
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= conv_dim) return;
-    const uint32_t H = kernel - 1;
-    float tap[8];
-    for (uint32_t i = 0; i < kernel; ++i) tap[i] = taps[(uint64_t)c * kernel + i];
-    for (uint32_t t = blockIdx.y; t < n_tokens; t += gridDim.y) {
-        float sum = tap[H] * x[(uint64_t)t * conv_dim + c];
-        for (uint32_t i = 0; i < H; ++i) {
-            int64_t src = (int64_t)t - (int64_t)H + i;  // tap i meets the input of token t - H + i
-            float past = src >= 0 ? x[(uint64_t)src * conv_dim + c] : history[(uint64_t)c * H + (uint32_t)(src + (int64_t)H)];
-            sum += tap[i] * past;
-        }
-        out[(uint64_t)t * conv_dim + c] = sum / (1.f + expf(-sum));
-    }
-}
-
-// The history after the batch: slot i holds the input of token n_tokens - H + i, or an older slot
-// when the batch is shorter than the history. One thread per channel.
-__global__ void gdn_conv_history_kernel(const float* __restrict__ x, float* __restrict__ history, uint32_t conv_dim, uint32_t kernel,
-                                        uint32_t n_tokens) {
-    pdl_launch_dependents();
-    pdl_wait();
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= conv_dim) return;
-    const uint32_t H = kernel - 1;
-    float next[7];
-    for (uint32_t i = 0; i < H; ++i) {
-        int64_t src = (int64_t)n_tokens - (int64_t)H + i;
-        next[i] = src >= 0 ? x[(uint64_t)src * conv_dim + c] : history[(uint64_t)c * H + (uint32_t)(src + (int64_t)H)];
-    }
-    for (uint32_t i = 0; i < H; ++i) history[(uint64_t)c * H + i] = next[i];
-}
-
-// The same for a few tokens (a decode step): one thread per channel walks the tokens and
-// updates the history itself, so one launch does it all. Same order of additions, same bits.
-__global__ void gdn_conv_serial_kernel(const float* __restrict__ x, const float* __restrict__ taps, float* __restrict__ history,
-                                       float* __restrict__ out, uint32_t conv_dim, uint32_t kernel, uint32_t n_tokens) {
-    pdl_launch_dependents();
-    pdl_wait();
-    uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= conv_dim) return;
-    const uint32_t H = kernel - 1;
-    float tap[8], past[7];
-    for (uint32_t i = 0; i < kernel; ++i) tap[i] = taps[(uint64_t)c * kernel + i];
-    for (uint32_t i = 0; i < H; ++i) past[i] = history[(uint64_t)c * H + i];
-    for (uint32_t t = 0; t < n_tokens; ++t) {
-        float input = x[(uint64_t)t * conv_dim + c];
-        float sum = tap[H] * input;
-        for (uint32_t i = 0; i < H; ++i) sum += tap[i] * past[i];
-        out[(uint64_t)t * conv_dim + c] = sum / (1.f + expf(-sum));
-        for (uint32_t i = 0; i + 1 < H; ++i) past[i] = past[i + 1];
-        past[H - 1] = input;
-    }
-    for (uint32_t i = 0; i < H; ++i) history[(uint64_t)c * H + i] = past[i];
-}
-
 // beta = sigmoid(beta); decay = exp(a * softplus(alpha + dt_bias)), softplus(x) = x above 20
 // (qwen35.rs:479-481, :776-778). In place over [n_tokens][n_v_heads]; alpha receives the decay.
+__device__ __forceinline__ void gate_pair(float* __restrict__ beta, float* __restrict__ alpha, const float* __restrict__ a,
+                                          const float* __restrict__ dt_bias, uint32_t n_v_heads, uint32_t i) {
+    const uint32_t head = i % n_v_heads;
+    beta[i] = 1.f / (1.f + expf(-beta[i]));
+    const float v = alpha[i] + dt_bias[head];
+    const float sp = v > 20.f ? v : log1pf(expf(v));
+    alpha[i] = expf(a[head] * sp);
+}
+
 __global__ void gdn_gates_kernel(float* __restrict__ beta, float* __restrict__ alpha, const float* __restrict__ a,
                                  const float* __restrict__ dt_bias, uint32_t n_v_heads, uint32_t n) {
     pdl_launch_dependents();
     pdl_wait();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    uint32_t head = i % n_v_heads;
-    beta[i] = 1.f / (1.f + expf(-beta[i]));
-    float v = alpha[i] + dt_bias[head];
-    float sp = v > 20.f ? v : log1pf(expf(v));
-    alpha[i] = expf(a[head] * sp);
+    if (i < n) gate_pair(beta, alpha, a, dt_bias, n_v_heads, i);
 }
 
 struct RecurrenceParams {
@@ -120,25 +56,100 @@ __device__ __forceinline__ float l2_factor(const float (&x)[PER]) {
     return 1.0f / sqrtf(sum + 1e-6f);
 }
 
-// The q and k heads of a batch normalised in place, q also scaled by 1 / sqrt(k_dim): one warp
-// per (token, q or k, key head). Run before the recurrence so that its token loop does not carry
-// the reductions.
-template <int KDIM>
-__global__ void __launch_bounds__(256) gdn_qk_norm_kernel(float* __restrict__ qkv, uint32_t n_k_heads, uint32_t conv_dim, uint32_t n_tokens) {
-    constexpr int PER = KDIM / 32;
+// The causal convolution with SiLU over a batch. x and out are [n_tokens][conv_dim]; taps are [conv_dim][kernel],
+// oldest first; history is [conv_dim][kernel - 1] raw inputs, oldest first. The sum starts from the newest tap's term
+// and adds the earlier inputs oldest first (qwen35.rs:449-461), from the batch or, for its first tokens, from the
+// history, so any split into batches gives the same bits. kernel <= K.
+//
+// A warp takes 32 * PER neighbouring channels of R tokens, a lane channels e * 32 + lane, with the window of inputs in
+// registers. With `n_norm` the first n_norm groups of channels are q heads, then k heads: their outputs are also
+// L2-normalised here (q scaled by 1 / sqrt(head size)), which is why a warp holds a whole head. CTAs past the
+// convolution's compute the gates. Only the first run of tokens reads the history (R >= K - 1); its threads
+// rewrite it. Bound by L2 traffic and latency: 512 tokens of 8192 channels took 44 us for the convolution (a thread per
+// element that read its inputs `kernel` times), 4.1 for the norms, 2.4 for the history and 2.0 for the gates in four
+// launches, now 14.9 in one; 64 tokens of 6144 channels 13.7, now 8.4.
+struct ConvParams {
+    const float *x, *taps;
+    float *history, *out;
+    uint32_t conv_dim, kernel, n_tokens, n_norm, conv_ctas;
+    float *beta, *alpha;  // gates: with n_gates
+    const float *a, *dt_bias;
+    uint32_t n_v_heads, n_gates;
+};
+
+template <int PER, int K, int R>
+__global__ void __launch_bounds__(256) gdn_conv_kernel(const __grid_constant__ ConvParams p) {
+    static_assert(R >= K - 1, "only the first run may read the history");
     pdl_launch_dependents();
+    if (blockIdx.x >= p.conv_ctas) {
+        pdl_wait();
+        const uint32_t i = (blockIdx.x - p.conv_ctas) * blockDim.x + threadIdx.x;
+        if (i < p.n_gates) gate_pair(p.beta, p.alpha, p.a, p.dt_bias, p.n_v_heads, i);
+        return;
+    }
+    const uint32_t lane = threadIdx.x & 31, n_groups = (p.conv_dim + 32 * PER - 1) / (32 * PER), skip = K - p.kernel;
+    const uint64_t item = (uint64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    const uint32_t group = (uint32_t)(item % n_groups), t0 = (uint32_t)(item / n_groups) * R;
+    if (t0 >= p.n_tokens) return;
+    const uint32_t c0 = group * 32 * PER + lane;
+    float tap[PER][K], window[PER][K - 1 + R];  // inputs of tokens t0 - (K - 1) .. t0 + R - 1
+#pragma unroll
+    for (int e = 0; e < PER; ++e) {
+        const uint32_t c = c0 + e * 32;
+#pragma unroll
+        for (int i = 0; i < K; ++i) tap[e][i] = i >= (int)skip && c < p.conv_dim ? p.taps[(uint64_t)c * p.kernel + i - skip] : 0.f;
+    }
     pdl_wait();
-    const uint32_t lane = threadIdx.x & 31, item = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
-    if (item >= n_tokens * 2 * n_k_heads) return;
-    const uint32_t t = item / (2 * n_k_heads), which = (item / n_k_heads) & 1, head = item % n_k_heads;
-    float* x = qkv + (uint64_t)t * conv_dim + (uint64_t)which * n_k_heads * KDIM + head * KDIM;
-    float v[PER];
 #pragma unroll
-    for (int e = 0; e < PER; ++e) v[e] = x[e * 32 + lane];
-    const float factor = l2_factor<PER>(v);
-    const float scale = which == 0 ? (1.0f / sqrtf((float)KDIM)) * factor : factor;
+    for (int i = 0; i < K - 1 + R; ++i) {
+        const int64_t src = (int64_t)t0 - (K - 1) + i;
 #pragma unroll
-    for (int e = 0; e < PER; ++e) x[e * 32 + lane] = v[e] * scale;
+        for (int e = 0; e < PER; ++e) {
+            const uint32_t c = c0 + e * 32;
+            window[e][i] = 0.f;
+            if (c >= p.conv_dim || i < (int)skip) continue;
+            if (src < 0) window[e][i] = p.history[(uint64_t)c * (p.kernel - 1) + i - skip];
+            else if (src < (int64_t)p.n_tokens) window[e][i] = p.x[(uint64_t)src * p.conv_dim + c];
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        if (t0 + r >= p.n_tokens) break;
+        float v[PER];
+#pragma unroll
+        for (int e = 0; e < PER; ++e) {
+            float sum = tap[e][K - 1] * window[e][K - 1 + r];
+#pragma unroll
+            for (int i = 0; i < K - 1; ++i)
+                if (i >= (int)skip) sum += tap[e][i] * window[e][i + r];
+            v[e] = sum / (1.f + expf(-sum));
+        }
+        if (group < p.n_norm) {
+            float factor = l2_factor<PER>(v);
+            if (group < p.n_norm / 2) factor = (1.0f / sqrtf((float)(32 * PER))) * factor;
+#pragma unroll
+            for (int e = 0; e < PER; ++e) v[e] *= factor;
+        }
+#pragma unroll
+        for (int e = 0; e < PER; ++e)
+            if (c0 + e * 32 < p.conv_dim) p.out[(uint64_t)(t0 + r) * p.conv_dim + c0 + e * 32] = v[e];
+    }
+    if (t0 != 0) return;
+    // The history after the batch: slot i holds the input of token n_tokens - (kernel - 1) + i, or an older slot when the
+    // batch is shorter than the history.
+#pragma unroll
+    for (int e = 0; e < PER; ++e) {
+        const uint32_t c = c0 + e * 32;
+        if (c >= p.conv_dim) continue;
+#pragma unroll
+        for (int i = 0; i < K - 1; ++i) {
+            if (i < (int)skip) continue;
+            // Slots are rewritten oldest first, so an older slot that moves down is still there to be read.
+            const int64_t src = (int64_t)p.n_tokens - (K - 1) + i;
+            const float next = src >= 0 ? p.x[(uint64_t)src * p.conv_dim + c] : p.history[(uint64_t)c * (p.kernel - 1) + src + (K - 1) - skip];
+            p.history[(uint64_t)c * (p.kernel - 1) + i - skip] = next;
+        }
+    }
 }
 
 // The delta rule over a run of tokens. One warp (a CTA of its own) per 8 state columns of a value
@@ -274,13 +285,14 @@ __global__ void __launch_bounds__(32 * kRecurrenceWarps) gdn_recurrence_kernel(R
 }
 
 // One warp per (token, value head): x = RMSNorm(x) * weight * silu(z) (qwen35.rs:508-513).
-__global__ void gdn_gated_norm_kernel(float* __restrict__ x, const float* __restrict__ z, const float* __restrict__ weight,
-                                      uint32_t v_dim, float eps) {
+__global__ void __launch_bounds__(256) gdn_gated_norm_kernel(float* __restrict__ x, const float* __restrict__ z, const float* __restrict__ weight,
+                                                             uint32_t v_dim, uint32_t n_rows, float eps) {
     pdl_launch_dependents();
     pdl_wait();
-    const int lane = threadIdx.x;
-    float* row = x + (uint64_t)blockIdx.x * v_dim;
-    const float* gate = z + (uint64_t)blockIdx.x * v_dim;
+    const uint32_t lane = threadIdx.x & 31, index = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (index >= n_rows) return;
+    float* row = x + (uint64_t)index * v_dim;
+    const float* gate = z + (uint64_t)index * v_dim;
     float sumsq = 0.f;
     for (uint32_t d = lane; d < v_dim; d += 32) sumsq += row[d] * row[d];
     sumsq = warp_sum(sumsq);
@@ -289,6 +301,40 @@ __global__ void gdn_gated_norm_kernel(float* __restrict__ x, const float* __rest
         float g = gate[d];
         row[d] = weight[d] * (row[d] * scale) * (g / (1.f + expf(-g)));
     }
+}
+
+// The same with the result as the fp16 operand of the product that follows (kernels_matmul_umma.cu's pack_kernel), rows up to
+// the next multiple of 16 tokens zero. LANES = v_dim / 8 lanes share a row, each with one 16-byte output. Bound by L2
+// traffic: 512 tokens of 32 heads of 128 took 17.0 us with one warp per CTA and 3.8 for the packing, now 5.9; 64
+// tokens of 16 heads 4.2 + 2.1, now 4.2.
+template <int LANES>
+__global__ void __launch_bounds__(256) gdn_gated_norm_pack_kernel(const float* __restrict__ x, const float* __restrict__ z, const float* __restrict__ weight,
+                                                                  __half* __restrict__ packed, uint32_t n_heads, uint32_t n_tokens, uint32_t token_groups,
+                                                                  float eps) {
+    constexpr uint32_t kDim = LANES * 8;
+    pdl_launch_dependents();
+    const uint32_t i = threadIdx.x % LANES, index = blockIdx.x * (256 / LANES) + threadIdx.x / LANES;
+    const uint32_t token = index / n_heads, head = index % n_heads;
+    const uint32_t d = (i >> 3) * 64 + ((i >> 2) & 1) * 32 + 4 * (i & 3);  // elements d .. d + 3 and d + 16 .. d + 19 of the head
+    const float4 wl = __ldg(reinterpret_cast<const float4*>(weight + d)), wh = __ldg(reinterpret_cast<const float4*>(weight + d + 16));
+    pdl_wait();
+    float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo, gl = lo, gh = lo;
+    if (token < n_tokens) {
+        const uint64_t at = ((uint64_t)token * n_heads + head) * kDim + d;
+        lo = *reinterpret_cast<const float4*>(x + at), hi = *reinterpret_cast<const float4*>(x + at + 16);
+        gl = *reinterpret_cast<const float4*>(z + at), gh = *reinterpret_cast<const float4*>(z + at + 16);
+    }
+    float sumsq = (lo.x * lo.x + lo.y * lo.y + lo.z * lo.z + lo.w * lo.w) + (hi.x * hi.x + hi.y * hi.y + hi.z * hi.z + hi.w * hi.w);
+#pragma unroll
+    for (int o = 1; o < LANES; o <<= 1) sumsq += __shfl_xor_sync(0xffffffffu, sumsq, o);
+    const float scale = rsqrtf(sumsq / (float)kDim + eps);
+    auto value = [&](float v, float w, float g) { return w * (v * scale) * (g / (1.f + expf(-g))); };
+    const __half2 p0 = __floats2half2_rn(value(lo.x, wl.x, gl.x), value(lo.z, wl.z, gl.z)), p1 = __floats2half2_rn(value(lo.y, wl.y, gl.y), value(lo.w, wl.w, gl.w));
+    const __half2 p2 = __floats2half2_rn(value(hi.x, wh.x, gh.x), value(hi.z, wh.z, gh.z)), p3 = __floats2half2_rn(value(hi.y, wh.y, gh.y), value(hi.w, wh.w, gh.w));
+    if (token < token_groups * 8)
+        *reinterpret_cast<uint4*>(packed + packed_operand_index(token, head * kDim + d, token_groups)) =
+            make_uint4(*reinterpret_cast<const uint32_t*>(&p0), *reinterpret_cast<const uint32_t*>(&p1), *reinterpret_cast<const uint32_t*>(&p2),
+                       *reinterpret_cast<const uint32_t*>(&p3));
 }
 
 // ---- One token through a whole DeltaNet mixer in one launch (decode): the causal convolution
@@ -453,22 +499,37 @@ __global__ void attention_gate_kernel(float* __restrict__ out, const float* __re
 
 }  // namespace
 
-int gdn_conv_launches(uint32_t n_tokens) { return n_tokens <= kConvSerialTokens ? 1 : 2; }
+template <int PER>
+cudaError_t launch_conv(cudaStream_t stream, ConvParams& p) {
+    // Runs of 8 tokens read 1.4 times what they must, runs of 4 1.75 times: the short ones while the long ones would leave
+    // fewer than 16 warps to an SM.
+    const uint32_t groups = (p.conv_dim + 32 * PER - 1) / (32 * PER);
+    const bool brief = p.kernel <= 4 && (uint64_t)groups * ((p.n_tokens + 7) / 8) < (uint64_t)sm_count() * 16;
+    const uint32_t run = brief ? 4 : 8;
+    p.conv_ctas = (uint32_t)(((uint64_t)groups * ((p.n_tokens + run - 1) / run) + 7) / 8);
+    void* args[] = {&p};
+    const void* kernel = p.kernel > 4 ? (const void*)gdn_conv_kernel<PER, 8, 8> : brief ? (const void*)gdn_conv_kernel<PER, 4, 4> : (const void*)gdn_conv_kernel<PER, 4, 8>;
+    return launch_kernel(kernel, dim3(p.conv_ctas + (p.n_gates + 255) / 256), dim3(256), 0, stream, args);
+}
 
 cudaError_t gdn_conv(cudaStream_t stream, const float* x, const float* taps, float* history, float* out, uint32_t conv_dim,
                      uint32_t kernel, uint32_t n_tokens) {
     if (n_tokens == 0) return cudaSuccess;
-    if (n_tokens <= kConvSerialTokens) {
-        void* args[] = {&x, &taps, &history, &out, &conv_dim, &kernel, &n_tokens};
-        return launch_kernel((const void*)gdn_conv_serial_kernel, dim3((conv_dim + 127) / 128), dim3(128), 0, stream, args);
+    ConvParams p{x, taps, history, out, conv_dim, kernel, n_tokens, 0, 0, nullptr, nullptr, nullptr, nullptr, 1, 0};
+    return launch_conv<4>(stream, p);
+}
+
+cudaError_t gdn_conv_gates(cudaStream_t stream, const float* x, const float* taps, float* history, float* out, float* beta, float* alpha, const float* a,
+                           const float* dt_bias, uint32_t n_k_heads, uint32_t n_v_heads, uint32_t k_dim, uint32_t v_dim, uint32_t kernel, uint32_t n_tokens) {
+    if (n_tokens == 0) return cudaSuccess;
+    ConvParams p{x, taps, history, out, 2 * n_k_heads * k_dim + n_v_heads * v_dim, kernel, n_tokens, 2 * n_k_heads, 0, beta, alpha, a, dt_bias, n_v_heads,
+                 n_v_heads * n_tokens};
+    switch (k_dim) {
+        case 32: return launch_conv<1>(stream, p);
+        case 64: return launch_conv<2>(stream, p);
+        case 96: return launch_conv<3>(stream, p);
+        default: return launch_conv<4>(stream, p);
     }
-    const float* read_history = history;
-    void* args[] = {&x, &taps, &read_history, &out, &conv_dim, &kernel, &n_tokens};
-    cudaError_t e = launch_kernel((const void*)gdn_conv_kernel, dim3((conv_dim + 255) / 256, n_tokens < 65535u ? n_tokens : 65535u), dim3(256), 0,
-                                  stream, args);
-    if (e != cudaSuccess) return e;
-    void* history_args[] = {&x, &history, &conv_dim, &kernel, &n_tokens};
-    return launch_kernel((const void*)gdn_conv_history_kernel, dim3((conv_dim + 127) / 128), dim3(128), 0, stream, history_args);
 }
 
 cudaError_t gdn_gates(cudaStream_t stream, float* beta, float* alpha, const float* a, const float* dt_bias, uint32_t n_v_heads,
@@ -489,16 +550,6 @@ cudaError_t gdn_recurrence(cudaStream_t stream, const float* qkv, const float* b
                        : k_dim == 96 ? (const void*)gdn_recurrence_kernel<96> : (const void*)gdn_recurrence_kernel<128>;
     const uint32_t units = n_v_heads * ((v_dim + 7) / 8);
     return launch_kernel(kernel, dim3((units + kRecurrenceWarps - 1) / kRecurrenceWarps), dim3(32 * kRecurrenceWarps), 0, stream, args);
-}
-
-cudaError_t gdn_qk_norm(cudaStream_t stream, float* qkv, uint32_t n_k_heads, uint32_t n_v_heads, uint32_t k_dim, uint32_t v_dim, uint32_t n_tokens) {
-    if (n_tokens == 0) return cudaSuccess;
-    uint32_t conv_dim = 2 * n_k_heads * k_dim + n_v_heads * v_dim;
-    const uint32_t items = n_tokens * 2 * n_k_heads;
-    void* args[] = {&qkv, &n_k_heads, &conv_dim, &n_tokens};
-    const void* kernel = k_dim == 32 ? (const void*)gdn_qk_norm_kernel<32> : k_dim == 64 ? (const void*)gdn_qk_norm_kernel<64>
-                       : k_dim == 96 ? (const void*)gdn_qk_norm_kernel<96> : (const void*)gdn_qk_norm_kernel<128>;
-    return launch_kernel(kernel, dim3((items + 7) / 8), dim3(256), 0, stream, args);
 }
 
 bool gdn_step_supported(uint32_t n_k_heads, uint32_t n_v_heads, uint32_t k_dim, uint32_t v_dim, uint32_t kernel) {
@@ -522,8 +573,22 @@ cudaError_t gdn_step(cudaStream_t stream, const float* qkv, const float* taps, f
 cudaError_t gdn_gated_norm(cudaStream_t stream, float* x, const float* z, const float* weight, uint32_t v_dim, uint32_t n_rows,
                            float eps) {
     if (n_rows == 0) return cudaSuccess;
-    void* args[] = {&x, &z, &weight, &v_dim, &eps};
-    return launch_kernel((const void*)gdn_gated_norm_kernel, dim3(n_rows), dim3(32), 0, stream, args);
+    void* args[] = {&x, &z, &weight, &v_dim, &n_rows, &eps};
+    return launch_kernel((const void*)gdn_gated_norm_kernel, dim3((n_rows + 7) / 8), dim3(256), 0, stream, args);
+}
+
+bool gdn_gated_norm_pack_supported(uint32_t v_dim) { return v_dim == 64 || v_dim == 128 || v_dim == 256; }
+
+cudaError_t gdn_gated_norm_pack(cudaStream_t stream, const float* x, const float* z, const float* weight, uint32_t v_dim, uint32_t n_heads, uint32_t n_tokens,
+                                float eps, void* packed) {
+    if (n_tokens == 0) return cudaSuccess;
+    if (!gdn_gated_norm_pack_supported(v_dim)) return cudaErrorInvalidValue;
+    uint32_t token_groups = ((n_tokens + 15u) & ~15u) / 8;
+    const uint32_t lanes = v_dim / 8, rows = token_groups * 8 * n_heads, per_cta = 256 / lanes;
+    void* args[] = {&x, &z, &weight, &packed, &n_heads, &n_tokens, &token_groups, &eps};
+    const void* kernel = lanes == 8 ? (const void*)gdn_gated_norm_pack_kernel<8> : lanes == 16 ? (const void*)gdn_gated_norm_pack_kernel<16>
+                                                                                              : (const void*)gdn_gated_norm_pack_kernel<32>;
+    return launch_kernel(kernel, dim3((rows + per_cta - 1) / per_cta), dim3(256), 0, stream, args);
 }
 
 cudaError_t attention_gate(cudaStream_t stream, float* out, const float* q_gate, uint32_t n_heads, uint32_t head_dim, uint32_t n_tokens) {

@@ -119,9 +119,11 @@ struct UmmaParams {
 };
 
 // X [n_tokens][n_cols] f32 -> fp16 operand layout, zero rows up to the padded token count. One
-// thread writes one core-matrix row (16 bytes): 8 halves of one token.
+// thread writes one core-matrix row (16 bytes): 8 halves of one token. GATED: the values are first multiplied by the
+// sigmoid of their gates (the arithmetic of attention_gate_kernel), which lie in q_gate[token][head][head_dim + d].
+template <bool GATED>
 __global__ void __launch_bounds__(256) pack_kernel(const float* __restrict__ x, __half* __restrict__ packed, uint32_t n_tokens,
-                                                   uint32_t n_cols, uint32_t token_groups, uint64_t total) {
+                                                   uint32_t n_cols, uint32_t token_groups, uint64_t total, const float* __restrict__ q_gate, uint32_t head_dim) {
     pdl_launch_dependents();  // the product that reads this packing may set itself up meanwhile
     pdl_wait();
     uint64_t o = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;  // index of the 16-byte output
@@ -134,6 +136,13 @@ __global__ void __launch_bounds__(256) pack_kernel(const float* __restrict__ x, 
     if (token < n_tokens) {
         const float* src = x + (uint64_t)token * n_cols + chunk * kChunkK + (j >> 2) * 32 + 4 * (j & 3);
         float4 lo = *reinterpret_cast<const float4*>(src), hi = *reinterpret_cast<const float4*>(src + 16);
+        if (GATED) {
+            const uint32_t col = chunk * kChunkK + (j >> 2) * 32 + 4 * (j & 3);
+            const float* gates = q_gate + 2 * (uint64_t)token * n_cols + (uint64_t)(col / head_dim) * 2 * head_dim + head_dim + col % head_dim;
+            const float4 gl = *reinterpret_cast<const float4*>(gates), gh = *reinterpret_cast<const float4*>(gates + 16);
+            lo.x *= 1.f / (1.f + expf(-gl.x)); lo.y *= 1.f / (1.f + expf(-gl.y)); lo.z *= 1.f / (1.f + expf(-gl.z)); lo.w *= 1.f / (1.f + expf(-gl.w));
+            hi.x *= 1.f / (1.f + expf(-gh.x)); hi.y *= 1.f / (1.f + expf(-gh.y)); hi.z *= 1.f / (1.f + expf(-gh.z)); hi.w *= 1.f / (1.f + expf(-gh.w));
+        }
         __half2 a = __floats2half2_rn(lo.x, lo.z), b = __floats2half2_rn(lo.y, lo.w);
         __half2 c = __floats2half2_rn(hi.x, hi.z), d = __floats2half2_rn(hi.y, hi.w);
         out.x = *reinterpret_cast<uint32_t*>(&a);
@@ -145,112 +154,69 @@ __global__ void __launch_bounds__(256) pack_kernel(const float* __restrict__ x, 
 }
 
 // RMSNorm and packing in one pass: packed = fp16(weight * (x * scale)), scale = 1 / sqrt(mean x^2 + eps)
-// per token, the arithmetic of rms_norm_kernel followed by pack_kernel. A CTA serves a group of 8
-// tokens: a warp per token sums its squares, then the CTA writes the group's kilobyte of its share
-// of the chunks (blockIdx.y of gridDim.y; each share repeats the cheap sums, which keeps the grid
-// wide). Rows past the batch are zero.
-__global__ void __launch_bounds__(256) pack_norm_kernel(const float* __restrict__ x, const float* __restrict__ weight, float eps,
-                                                        __half* __restrict__ packed, uint32_t n_tokens, uint32_t n_cols, uint32_t token_groups) {
-    __shared__ float scales[8];
+// per token, the arithmetic of rms_norm_kernel followed by pack_kernel; rows past the batch are zero. With ADD
+// the rows still lack a split-K launch's partial products: they first take the `split` partial rows in index
+// order (like reduce_kernel) and x keeps the sums.
+//
+// Bound by latency at a few tokens and by L2 traffic at many. A CTA per token reads its row once, all loads of a thread
+// in flight together, into shared memory, from where the first warp sums the squares (one warp, so that the order of
+// the sum is that of a warp per row) and all write their part of the operand. The forms before it (8 tokens per CTA with 4 or
+// 8 CTAs repeating the sums; 4 tokens per CTA with the partial sums) read rows twice: 512 tokens of 4096 took 13.0 us
+// plain and 19.0 us with four partial sums, now 8.2 and 10.7; 64 tokens of 2048 with a reduce_kernel before it 7.0, now 6.1.
+template <bool ADD>
+__global__ void __launch_bounds__(256) pack_norm_kernel(float* __restrict__ x, const float* __restrict__ weight, float eps, __half* __restrict__ packed,
+                                                        uint32_t n_tokens, uint32_t n_cols, uint32_t token_groups, const float* __restrict__ partial,
+                                                        uint32_t split) {
+    extern __shared__ float4 norm_row[];
+    __shared__ float shared_scale;
     pdl_launch_dependents();
+    const uint32_t token = blockIdx.x, tid = threadIdx.x, quads = n_cols / 4;
     pdl_wait();
-    const uint32_t tg = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    {
-        const uint32_t token = tg * 8 + warp;
-        float sumsq = 0.f;
-        if (token < n_tokens) {
-            const float4* row = reinterpret_cast<const float4*>(x + (uint64_t)token * n_cols);
-            for (uint32_t i = lane; i < n_cols / 4; i += 32) {
-                float4 v = row[i];
-                sumsq += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
-            }
-        }
-        sumsq = warp_sum(sumsq);
-        if (lane == 0) scales[warp] = rsqrtf(sumsq / (float)n_cols + eps);
+    uint4* out = reinterpret_cast<uint4*>(packed) + (token & 7);
+    auto place = [&](uint32_t i) { return (((uint64_t)(i >> 3) * token_groups + (token >> 3)) * kCores + (i & 7)) * 8; };
+    if (token >= n_tokens) {
+        for (uint32_t i = tid; i < n_cols / 8; i += 256) out[place(i)] = make_uint4(0, 0, 0, 0);
+        return;
     }
-    __syncthreads();
-    const uint32_t tr = tid & 7, j = (tid >> 3) & (kCores - 1), sub = tid / (8 * kCores);  // 256 / 64 = 4 chunks per pass
-    const uint32_t token = tg * 8 + tr, n_chunks = n_cols / kChunkK;
-    const float scale = scales[tr];
-    for (uint32_t chunk = blockIdx.y * (256 / (8 * kCores)) + sub; chunk < n_chunks; chunk += gridDim.y * (256 / (8 * kCores))) {
-        uint4 out = make_uint4(0, 0, 0, 0);
-        if (token < n_tokens) {
-            const uint32_t col = chunk * kChunkK + (j >> 2) * 32 + 4 * (j & 3);
-            const float* src = x + (uint64_t)token * n_cols + col;
-            float4 lo = *reinterpret_cast<const float4*>(src), hi = *reinterpret_cast<const float4*>(src + 16);
-            const float4 wl = __ldg(reinterpret_cast<const float4*>(weight + col)), wh = __ldg(reinterpret_cast<const float4*>(weight + col + 16));
-            lo.x = wl.x * (lo.x * scale); lo.y = wl.y * (lo.y * scale); lo.z = wl.z * (lo.z * scale); lo.w = wl.w * (lo.w * scale);
-            hi.x = wh.x * (hi.x * scale); hi.y = wh.y * (hi.y * scale); hi.z = wh.z * (hi.z * scale); hi.w = wh.w * (hi.w * scale);
-            __half2 a = __floats2half2_rn(lo.x, lo.z), b = __floats2half2_rn(lo.y, lo.w);
-            __half2 c = __floats2half2_rn(hi.x, hi.z), d = __floats2half2_rn(hi.y, hi.w);
-            out.x = *reinterpret_cast<uint32_t*>(&a);
-            out.y = *reinterpret_cast<uint32_t*>(&b);
-            out.z = *reinterpret_cast<uint32_t*>(&c);
-            out.w = *reinterpret_cast<uint32_t*>(&d);
-        }
-        reinterpret_cast<uint4*>(packed)[(((uint64_t)chunk * token_groups + tg) * kCores + j) * 8 + tr] = out;
-    }
-}
-
-// pack_norm_kernel for a batch whose rows still lack the sum of a split-K launch's partial
-// products: a token's row first takes the `split` partial rows in index order (like
-// reduce_kernel) and x keeps the sums. One CTA of 16 warps per 4 tokens (half a token group, so
-// the grid is twice as wide), four warps to a token: a row is summed and written by exactly one
-// CTA, which then packs its 4 tokens (64 of a group's 128 bytes per core-matrix row).
-__global__ void __launch_bounds__(512) pack_norm_add_kernel(float* __restrict__ x, const float* __restrict__ weight, float eps,
-                                                            __half* __restrict__ packed, uint32_t n_tokens, uint32_t n_cols, uint32_t token_groups,
-                                                            const float* __restrict__ partial, uint32_t split) {
-    __shared__ float sums[4][4];
-    __shared__ float scales[4];
-    pdl_launch_dependents();
-    pdl_wait();
-    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, token0 = blockIdx.x * 4;
-    {
-        const uint32_t token = token0 + (warp >> 2), cols4 = n_cols / 4;
-        float sumsq = 0.f;
-        if (token < n_tokens) {
-            float4* row = reinterpret_cast<float4*>(x + (uint64_t)token * n_cols);
-            const uint64_t total4 = (uint64_t)n_tokens * cols4;
-            const float4* part = reinterpret_cast<const float4*>(partial) + (uint64_t)token * cols4;
+    float4* row = reinterpret_cast<float4*>(x) + (uint64_t)token * quads;
+    const float4* part = reinterpret_cast<const float4*>(partial) + (uint64_t)token * quads;
+    const uint64_t total = (uint64_t)n_tokens * quads;
 #pragma unroll 4
-            for (uint32_t i = (warp & 3) * 32 + lane; i < cols4; i += 128) {
-                float4 sum = __ldcg(part + i);
-                for (uint32_t sp = 1; sp < split; ++sp) {
-                    const float4 o = __ldcg(part + sp * total4 + i);
-                    sum.x += o.x; sum.y += o.y; sum.z += o.z; sum.w += o.w;
-                }
-                float4 v = row[i];
-                v.x += sum.x; v.y += sum.y; v.z += sum.z; v.w += sum.w;
-                row[i] = v;
-                sumsq += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+    for (uint32_t i = tid; i < quads; i += 256) {
+        float4 v = __ldcg(row + i);
+        if (ADD) {
+            float4 sum = __ldcg(part + i);
+            for (uint32_t sp = 1; sp < split; ++sp) {
+                const float4 o = __ldcg(part + sp * total + i);
+                sum.x += o.x; sum.y += o.y; sum.z += o.z; sum.w += o.w;
             }
+            v.x += sum.x; v.y += sum.y; v.z += sum.z; v.w += sum.w;
+            row[i] = v;
         }
-        sumsq = warp_sum(sumsq);
-        if (lane == 0) sums[warp >> 2][warp & 3] = sumsq;
+        norm_row[i] = v;
     }
     __syncthreads();
-    if (tid < 4) scales[tid] = rsqrtf(((sums[tid][0] + sums[tid][1]) + (sums[tid][2] + sums[tid][3])) / (float)n_cols + eps);
-    __syncthreads();
-    const uint32_t tr = tid & 3, j = (tid >> 2) & (kCores - 1), sub = tid / (4 * kCores);  // 512 / 32 = 16 chunks per pass
-    const uint32_t token = token0 + tr, n_chunks = n_cols / kChunkK, tg = token0 >> 3, in_group = (token0 & 4) + tr;
-    const float scale = scales[tr];
-    for (uint32_t chunk = sub; chunk < n_chunks; chunk += 512 / (4 * kCores)) {
-        uint4 out = make_uint4(0, 0, 0, 0);
-        if (token < n_tokens) {
-            const uint32_t col = chunk * kChunkK + (j >> 2) * 32 + 4 * (j & 3);
-            const float* src = x + (uint64_t)token * n_cols + col;
-            float4 lo = *reinterpret_cast<const float4*>(src), hi = *reinterpret_cast<const float4*>(src + 16);
-            const float4 wl = __ldg(reinterpret_cast<const float4*>(weight + col)), wh = __ldg(reinterpret_cast<const float4*>(weight + col + 16));
-            lo.x = wl.x * (lo.x * scale); lo.y = wl.y * (lo.y * scale); lo.z = wl.z * (lo.z * scale); lo.w = wl.w * (lo.w * scale);
-            hi.x = wh.x * (hi.x * scale); hi.y = wh.y * (hi.y * scale); hi.z = wh.z * (hi.z * scale); hi.w = wh.w * (hi.w * scale);
-            __half2 a = __floats2half2_rn(lo.x, lo.z), b = __floats2half2_rn(lo.y, lo.w);
-            __half2 c = __floats2half2_rn(hi.x, hi.z), d = __floats2half2_rn(hi.y, hi.w);
-            out.x = *reinterpret_cast<uint32_t*>(&a);
-            out.y = *reinterpret_cast<uint32_t*>(&b);
-            out.z = *reinterpret_cast<uint32_t*>(&c);
-            out.w = *reinterpret_cast<uint32_t*>(&d);
+    if (tid < 32) {
+        float sumsq = 0.f;
+#pragma unroll 4
+        for (uint32_t i = tid; i < quads; i += 32) {
+            float4 v = norm_row[i];
+            sumsq += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
         }
-        reinterpret_cast<uint4*>(packed)[(((uint64_t)chunk * token_groups + tg) * kCores + j) * 8 + in_group] = out;
+        sumsq = warp_sum(sumsq);
+        if (tid == 0) shared_scale = rsqrtf(sumsq / (float)n_cols + eps);
+    }
+    __syncthreads();
+    const float scale = shared_scale;
+#pragma unroll 2
+    for (uint32_t i = tid; i < n_cols / 8; i += 256) {  // a 16-byte output: four columns and the four that are 16 further
+        const uint32_t quad = (i >> 3) * (kChunkK / 4) + ((i >> 2) & 1) * 8 + (i & 3);
+        const float4 l = norm_row[quad], u = norm_row[quad + 4];
+        const float4 a = __ldg(reinterpret_cast<const float4*>(weight) + quad), b = __ldg(reinterpret_cast<const float4*>(weight) + quad + 4);
+        const __half2 p0 = __floats2half2_rn(a.x * (l.x * scale), a.z * (l.z * scale)), p1 = __floats2half2_rn(a.y * (l.y * scale), a.w * (l.w * scale));
+        const __half2 p2 = __floats2half2_rn(b.x * (u.x * scale), b.z * (u.z * scale)), p3 = __floats2half2_rn(b.y * (u.y * scale), b.w * (u.w * scale));
+        out[place(i)] = make_uint4(*reinterpret_cast<const uint32_t*>(&p0), *reinterpret_cast<const uint32_t*>(&p1), *reinterpret_cast<const uint32_t*>(&p2),
+                                   *reinterpret_cast<const uint32_t*>(&p3));
     }
 }
 
@@ -757,8 +723,16 @@ cudaError_t matmul_pack(cudaStream_t stream, const float* x, uint32_t n_tokens, 
     uint32_t token_groups = ((n_tokens + 15u) & ~15u) / 8;
     uint64_t total = (uint64_t)(n_cols / kChunkK) * token_groups * (8 * kCores);
     if (total == 0) return cudaSuccess;
-    return launch_dependent(pack_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, stream, x, static_cast<__half*>(packed), n_tokens, n_cols,
-                            token_groups, total);
+    return launch_dependent(pack_kernel<false>, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, stream, x, static_cast<__half*>(packed), n_tokens, n_cols,
+                            token_groups, total, static_cast<const float*>(nullptr), 1u);
+}
+
+cudaError_t matmul_pack_gated(cudaStream_t stream, const float* x, const float* q_gate, uint32_t head_dim, uint32_t n_tokens, uint32_t n_cols, void* packed) {
+    uint32_t token_groups = ((n_tokens + 15u) & ~15u) / 8;
+    uint64_t total = (uint64_t)(n_cols / kChunkK) * token_groups * (8 * kCores);
+    if (total == 0) return cudaSuccess;
+    return launch_dependent(pack_kernel<true>, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, stream, x, static_cast<__half*>(packed), n_tokens, n_cols,
+                            token_groups, total, q_gate, head_dim);
 }
 
 cudaError_t matmul_pack_norm(cudaStream_t stream, float* x, Norm norm, uint32_t n_tokens, uint32_t n_cols, void* packed, const Deferred* add) {
@@ -766,13 +740,14 @@ cudaError_t matmul_pack_norm(cudaStream_t stream, float* x, Norm norm, uint32_t 
     if (token_groups == 0 || n_cols == 0) return cudaSuccess;
     const bool adding = add && add->partial;
     if (adding && (add->n_tokens != n_tokens || add->n_rows != n_cols || n_cols % 4 != 0)) return cudaErrorInvalidValue;
-    const uint32_t shares = token_groups >= 256 ? 1 : token_groups >= 64 ? 4 : 8;
-    if (adding) {
-        return launch_dependent(pack_norm_add_kernel, dim3(token_groups * 2), dim3(512), 0, stream, x, norm.weight, norm.eps, static_cast<__half*>(packed),
-                                n_tokens, n_cols, token_groups, add->partial, add->split);
-    }
-    return launch_dependent(pack_norm_kernel, dim3(token_groups, shares), dim3(256), 0, stream, static_cast<const float*>(x), norm.weight, norm.eps,
-                            static_cast<__half*>(packed), n_tokens, n_cols, token_groups);
+    const size_t smem = (size_t)n_cols * 4;
+    auto launch = [&](auto kernel) {
+        cudaError_t e = ensure_dynamic_smem((const void*)kernel, smem);
+        if (e != cudaSuccess) return e;
+        return launch_dependent(kernel, dim3(token_groups * 8), dim3(256), smem, stream, x, norm.weight, norm.eps, static_cast<__half*>(packed), n_tokens, n_cols,
+                                token_groups, adding ? add->partial : static_cast<const float*>(nullptr), adding ? add->split : 0u);
+    };
+    return adding ? launch(pack_norm_kernel<true>) : launch(pack_norm_kernel<false>);
 }
 
 cudaError_t matmul_reduce(cudaStream_t stream, const Deferred& d, float* y) {

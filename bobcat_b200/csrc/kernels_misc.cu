@@ -201,68 +201,103 @@ __global__ void norm_rope_kernel(NormRopeParams p) {
 // The gated short convolution over a batch (crates/bobcat/src/lfm2.rs:456-475): bx = B * X, the
 // taps over bx of this token and the kernel - 1 before it (from the batch, or from the history for
 // the first tokens), times C. bcx is [n_tokens][3 n_embd], out is [n_tokens][n_embd], history is
-// [kernel - 1][n_embd], oldest first. kernel <= 9. One thread per (token, channel); the sum runs in
-// the order of the token-by-token recurrence, so batches of any split give the same bits. The
-// history is only read here; short_conv_history_kernel rewrites it afterwards.
-__device__ __forceinline__ float short_conv_token(const float* __restrict__ bcx, const float* __restrict__ taps,
-                                                  const float* __restrict__ history, uint32_t n_embd, uint32_t kernel, uint32_t t, uint32_t ch) {
-    const float* row = bcx + (uint64_t)t * 3 * n_embd;
-    const float b = row[ch], c = row[n_embd + ch], x = row[2 * n_embd + ch];
-    float sum = taps[(uint64_t)ch * kernel + kernel - 1] * (b * x);
-    // Tap kk meets the product of token t - (kernel - 1) + kk.
-    for (uint32_t kk = 0; kk + 1 < kernel; ++kk) {
-        int64_t src = (int64_t)t - (int64_t)(kernel - 1) + kk;
-        float past;
-        if (src >= 0) {
-            const float* r = bcx + (uint64_t)src * 3 * n_embd;
-            past = r[ch] * r[2 * n_embd + ch];
-        } else {
-            past = history[(uint64_t)(src + (int64_t)(kernel - 1)) * n_embd + ch];
-        }
-        sum += taps[(uint64_t)ch * kernel + kk] * past;
-    }
-    return c * sum;
-}
-
-// With `packed`, the results go out as the fp16 operand of the product that consumes them
-// (rows up to the next multiple of 16 tokens zero) instead of as f32 rows.
-__global__ void __launch_bounds__(256) short_conv_kernel(const float* __restrict__ bcx, const float* __restrict__ taps,
-                                                         const float* __restrict__ history, float* __restrict__ out, __half* __restrict__ packed,
-                                                         uint32_t n_embd, uint32_t kernel, uint32_t n_tokens) {
+// [kernel - 1][n_embd], oldest first. kernel <= K. The sum runs in the order of the token-by-token
+// recurrence, so batches of any split give the same bits. With `packed`, the results go out as the fp16 operand
+// of the product that consumes them (rows up to the next multiple of 16 tokens zero) instead of as f32 rows.
+//
+// Bound by L2 traffic. A thread takes V neighbouring channels (four when they can be loaded at once) of R tokens and
+// keeps the window of products in registers, so B and X are read 1 + (K - 1) / R times; one thread per element, which
+// reads them K times, took 9.1 us at 512 tokens of 2048 channels and 1.9 more for the history in a second launch, now
+// 5.2 together. Only the first run of tokens reads the history (R >= K - 1), and the same threads rewrite it.
+template <int K, int V>
+__global__ void __launch_bounds__(128) short_conv_kernel(const float* __restrict__ bcx, const float* __restrict__ taps, float* history,
+                                                         float* __restrict__ out, __half* __restrict__ packed, uint32_t n_embd, uint32_t kernel,
+                                                         uint32_t n_tokens) {
+    constexpr int R = K <= 4 ? 4 : 8;
+    static_assert(R >= K - 1, "only the first run may read the history");
     pdl_launch_dependents();  // the output projection that reads the packed results may set itself up meanwhile
-    pdl_wait();
-    const uint32_t ch = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t ch = (blockIdx.x * blockDim.x + threadIdx.x) * V, skip = K - kernel;  // taps and window are aligned to the newest
     if (ch >= n_embd) return;
-    if (packed) {
-        const uint32_t padded = (n_tokens + 15u) & ~15u;
-        for (uint32_t t = blockIdx.y; t < padded; t += gridDim.y) {
-            const float v = t < n_tokens ? short_conv_token(bcx, taps, history, n_embd, kernel, t, ch) : 0.f;
-            packed[packed_operand_index(t, ch, padded / 8)] = __float2half_rn(v);
-        }
-        return;
-    }
-    for (uint32_t t = blockIdx.y; t < n_tokens; t += gridDim.y) out[(uint64_t)t * n_embd + ch] = short_conv_token(bcx, taps, history, n_embd, kernel, t, ch);
-}
-
-// The history after the batch: slot kk holds the product of token n_tokens - (kernel - 1) + kk, or
-// an older slot when the batch is shorter than the history. One thread per channel.
-__global__ void short_conv_history_kernel(const float* __restrict__ bcx, float* __restrict__ history, uint32_t n_embd, uint32_t kernel,
-                                          uint32_t n_tokens) {
-    pdl_launch_dependents();
+    float tap[K][V];
+#pragma unroll
+    for (int kk = 0; kk < K; ++kk)
+#pragma unroll
+        for (int v = 0; v < V; ++v) tap[kk][v] = kk >= (int)skip ? taps[(uint64_t)(ch + v) * kernel + kk - skip] : 0.f;
     pdl_wait();
-    const uint32_t ch = blockIdx.x * blockDim.x + threadIdx.x;
-    if (ch >= n_embd) return;
-    float next[8];
-    for (uint32_t kk = 0; kk + 1 < kernel; ++kk) {
-        int64_t src = (int64_t)n_tokens - (int64_t)(kernel - 1) + kk;
-        if (src >= 0) {
-            const float* r = bcx + (uint64_t)src * 3 * n_embd;
-            next[kk] = r[ch] * r[2 * n_embd + ch];
+    auto load = [&](const float* at, float (&to)[V]) {
+        if (V == 4) {
+            const float4 f = *reinterpret_cast<const float4*>(at);
+            to[0] = f.x, to[1 % V] = f.y, to[2 % V] = f.z, to[3 % V] = f.w;
         } else {
-            next[kk] = history[(uint64_t)(src + (int64_t)(kernel - 1)) * n_embd + ch];
+            to[0] = *at;
+        }
+    };
+    auto products = [&](uint32_t t, float (&to)[V]) {
+        float b[V], x[V];
+        load(bcx + (uint64_t)t * 3 * n_embd + ch, b);
+        load(bcx + (uint64_t)t * 3 * n_embd + 2 * n_embd + ch, x);
+#pragma unroll
+        for (int v = 0; v < V; ++v) to[v] = b[v] * x[v];
+    };
+    const uint32_t rows = packed ? (n_tokens + 15u) & ~15u : n_tokens;
+    for (uint32_t run = blockIdx.y; (uint64_t)run * R < rows; run += gridDim.y) {
+        const uint32_t t0 = run * R;
+        float window[K - 1][V], bx[R][V], c[R][V];
+#pragma unroll
+        for (int kk = 0; kk < K - 1; ++kk) {
+#pragma unroll
+            for (int v = 0; v < V; ++v) window[kk][v] = 0.f;
+            if (kk < (int)skip) continue;
+            const int64_t src = (int64_t)t0 - (K - 1) + kk;
+            if (t0 == 0) load(history + (uint64_t)(kk - skip) * n_embd + ch, window[kk]);
+            else if (src < (int64_t)n_tokens) products((uint32_t)src, window[kk]);
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+#pragma unroll
+            for (int v = 0; v < V; ++v) bx[r][v] = c[r][v] = 0.f;
+            if (t0 + r < n_tokens) {
+                products(t0 + r, bx[r]);
+                load(bcx + (uint64_t)(t0 + r) * 3 * n_embd + n_embd + ch, c[r]);
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            float y[V];
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+                float sum = tap[K - 1][v] * bx[r][v];
+#pragma unroll
+                for (int kk = 0; kk < K - 1; ++kk)
+                    if (kk >= (int)skip) sum += tap[kk][v] * (r + kk < K - 1 ? window[r + kk < K - 1 ? r + kk : 0][v] : bx[r + kk >= K - 1 ? r + kk - (K - 1) : 0][v]);
+                y[v] = c[r][v] * sum;
+            }
+            if (t0 + r >= rows) break;
+            if (packed) {  // four neighbouring columns are 8 bytes in the order 0, 2, 1, 3
+                const __half2 p0 = __floats2half2_rn(y[0], y[2 % V]), p1 = __floats2half2_rn(y[1 % V], y[3 % V]);
+                *reinterpret_cast<uint2*>(packed + packed_operand_index(t0 + r, ch, rows / 8)) =
+                    make_uint2(*reinterpret_cast<const uint32_t*>(&p0), *reinterpret_cast<const uint32_t*>(&p1));
+            } else if (V == 4) {
+                *reinterpret_cast<float4*>(out + (uint64_t)(t0 + r) * n_embd + ch) = make_float4(y[0], y[1 % V], y[2 % V], y[3 % V]);
+            } else {
+                out[(uint64_t)(t0 + r) * n_embd + ch] = y[0];
+            }
+        }
+        if (t0 != 0) continue;
+        // The history after the batch: slot kk holds the product of token n_tokens - (kernel - 1) + kk, or an older
+        // slot when the batch is shorter than the history.
+#pragma unroll
+        for (int kk = 0; kk < K - 1; ++kk) {
+            if (kk < (int)skip) continue;
+            const int64_t src = (int64_t)n_tokens - (K - 1) + kk;
+            float next[V];
+            // Slots are rewritten oldest first, so an older slot that moves down is still there to be read.
+            if (src >= 0) products((uint32_t)src, next);
+            else load(history + (uint64_t)(src + K - 1 - skip) * n_embd + ch, next);
+#pragma unroll
+            for (int v = 0; v < V; ++v) history[(uint64_t)(kk - skip) * n_embd + ch + v] = next[v];
         }
     }
-    for (uint32_t kk = 0; kk + 1 < kernel; ++kk) history[(uint64_t)kk * n_embd + ch] = next[kk];
 }
 
 // One CTA of 1024 threads scans the vocabulary; ties go to the lowest index.
@@ -414,6 +449,85 @@ __global__ void rope_store_kernel(RopeStore p, Pos pos_ref) {
     }
 }
 
+// The batch form: norm and rotation of q and k, and the K and V rows into the caches. A CTA serves a token (with gridDim.y
+// CTAs to a token when there are few), a warp a head at a time; the token's cosines and sines, the costly part, are
+// computed once per CTA (or read from the table), where a launch each for q, k and v with a warp per head computed them
+// per element: 24.5 us together at 512 tokens of 32 + 8 + 8 heads of 64, now 8.7. Same arithmetic as norm_rope_kernel.
+constexpr int kRopeWarps = 8;
+
+__global__ void __launch_bounds__(32 * kRopeWarps) rope_store_batch_kernel(RopeBatch p) {
+    __shared__ float head_values[kRopeWarps][256];
+    __shared__ float2 rot[128];
+    pdl_launch_dependents();
+    const uint32_t token = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t half_rot = p.n_rot / 2, pos = p.first_pos + token;
+    if (tid < half_rot) {
+        if (p.rope_table) {
+            rot[tid] = p.rope_table[(uint64_t)pos * half_rot + tid];
+        } else {
+            const float inv_freq = 1.0f / powf(p.theta, (float)(2 * tid) / (float)p.n_rot);
+            float sn, cs;
+            sincosf((float)pos * inv_freq, &sn, &cs);
+            rot[tid] = make_float2(cs, sn);
+        }
+    }
+    __syncthreads();
+    pdl_wait();
+    const uint32_t hd = p.head_dim, kv_dim = p.n_kv_heads * hd, heads = p.n_heads + p.n_kv_heads + (p.v_dst ? p.n_kv_heads : 0);
+    float* values = head_values[warp];
+    const int per_lane = hd / 32;
+    for (uint32_t item = blockIdx.y * kRopeWarps + warp; item < heads; item += gridDim.y * kRopeWarps) {
+        const bool is_q = item < p.n_heads, is_v = item >= p.n_heads + p.n_kv_heads;
+        const uint32_t head = is_q ? item : is_v ? item - p.n_heads - p.n_kv_heads : item - p.n_heads;
+        const float* src = is_q ? p.q + (uint64_t)token * p.q_stride + (uint64_t)head * p.q_head_stride
+                                : (is_v ? p.v : p.k) + (uint64_t)token * kv_dim + (uint64_t)head * hd;
+        const uint64_t at = (uint64_t)token * kv_dim + (uint64_t)head * hd;
+        float v[8];
+        float sumsq = 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            v[j] = 0.f;
+            if (j < per_lane) {
+                v[j] = src[lane + 32 * j];
+                sumsq += v[j] * v[j];
+            }
+        }
+        if (is_v) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                if (j < per_lane) p.v_dst[at + lane + 32 * j] = __float2half_rn(v[j]);
+            continue;
+        }
+        sumsq = warp_sum(sumsq);
+        const float scale = rsqrtf(sumsq / (float)hd + p.eps);
+        const float* weight = is_q ? p.q_norm : p.k_norm;
+        __syncwarp();  // the previous head's values are read
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            if (j < per_lane) {
+                v[j] = weight[lane + 32 * j] * (v[j] * scale);
+                values[lane + 32 * j] = v[j];
+            }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            if (j >= per_lane) continue;
+            const uint32_t e = lane + 32 * j;
+            float result = v[j];
+            if (e < p.n_rot) {
+                const uint32_t i = e < half_rot ? e : e - half_rot;
+                const float a = values[i], b = values[i + half_rot];
+                const float2 cs = rot[i];
+                result = e < half_rot ? a * cs.x - b * cs.y : b * cs.x + a * cs.y;
+            }
+            if (is_q) p.q_dst[(uint64_t)token * p.q_dst_stride + (uint64_t)head * p.q_dst_head_stride + e] = result;
+            else if (p.kv_half) static_cast<__half*>(p.k_dst)[at + e] = __float2half_rn(result);
+            else static_cast<float*>(p.k_dst)[at + e] = result;
+        }
+    }
+}
+
 __global__ void rope_table_kernel(float2* table, uint32_t n_positions, uint32_t n_rot, float theta) {
     const uint32_t half_rot = n_rot / 2;
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -532,11 +646,17 @@ cudaError_t short_conv(cudaStream_t stream, const float* bcx, const float* taps,
                        uint32_t kernel, uint32_t n_tokens, void* packed) {
     if (n_tokens == 0) return cudaSuccess;
     if (packed && n_embd % 64 != 0) return cudaErrorInvalidValue;
+    if (kernel < 2 || kernel > 9) return cudaErrorInvalidValue;
     const uint32_t rows = packed ? ((n_tokens + 15u) & ~15u) : n_tokens;
-    cudaError_t e = launch_dependent(short_conv_kernel, dim3(blocks_for(n_embd, 256), rows < 65535u ? rows : 65535u), dim3(256), 0, stream, bcx, taps,
-                                     static_cast<const float*>(history), out, static_cast<__half*>(packed), n_embd, kernel, n_tokens);
-    if (e != cudaSuccess) return e;
-    return launch_dependent(short_conv_history_kernel, dim3(blocks_for(n_embd, 128)), dim3(128), 0, stream, bcx, history, n_embd, kernel, n_tokens);
+    const bool wide = n_embd % 4 == 0 && ((uintptr_t)bcx | (uintptr_t)history | (uintptr_t)out) % 16 == 0;
+    if (packed && !wide) return cudaErrorInvalidValue;
+    auto launch = [&](auto conv, uint32_t per_thread, uint32_t run) {
+        const uint32_t runs = (rows + run - 1) / run;
+        return launch_dependent(conv, dim3((n_embd / per_thread + 127) / 128, runs < 65535u ? runs : 65535u), dim3(128), 0, stream, bcx, taps, history, out,
+                                static_cast<__half*>(packed), n_embd, kernel, n_tokens);
+    };
+    if (kernel <= 4) return wide ? launch(short_conv_kernel<4, 4>, 4, 4) : launch(short_conv_kernel<4, 1>, 1, 4);
+    return wide ? launch(short_conv_kernel<9, 4>, 4, 8) : launch(short_conv_kernel<9, 1>, 1, 8);
 }
 
 cudaError_t argmax(cudaStream_t stream, const float* x, uint32_t n, uint32_t* out, uint32_t* readback) {
@@ -572,6 +692,16 @@ cudaError_t rope_table(cudaStream_t stream, float2* table, uint32_t n_positions,
     if (items == 0) return cudaSuccess;
     rope_table_kernel<<<(unsigned)((items + 255) / 256), 256, 0, stream>>>(table, n_positions, n_rot, theta);
     return cudaGetLastError();
+}
+
+cudaError_t rope_store_batch(cudaStream_t stream, const RopeBatch& p) {
+    if (p.n_tokens == 0) return cudaSuccess;
+    const uint32_t heads = p.n_heads + p.n_kv_heads + (p.v_dst ? p.n_kv_heads : 0);
+    uint32_t parts = (uint32_t)(2 * sm_count()) / p.n_tokens, most = (heads + kRopeWarps - 1) / kRopeWarps;
+    parts = parts < 1 ? 1 : parts > most ? most : parts;  // about two CTAs per SM at least, no CTA without a head per warp
+    RopeBatch params = p;
+    void* args[] = {&params};
+    return launch_kernel((const void*)rope_store_batch_kernel, dim3(p.n_tokens, parts), dim3(32 * kRopeWarps), 0, stream, args);
 }
 
 cudaError_t rope_store(cudaStream_t stream, const RopeStore& p, Pos pos) {

@@ -139,9 +139,7 @@ struct Recorder {
         const uint64_t partial_bytes = k::matmul_partial_bytes(w, n);
         if (status == BC_OK && partial_bytes) status = s.backend->partial_scratch(partial_bytes, &partial);
         k::Deferred left{};
-        // The normalisation that would take the sum runs one CTA per 4 tokens: with few rows the
-        // separate, wide sum is quicker.
-        const bool may_defer = store == BC_STORE_ACCUMULATE && n >= 128;
+        const bool may_defer = store == BC_STORE_ACCUMULATE;
         run("matmul", w.n_rows, w.n_cols, w.bytes(), 1, [&] {
             return k::matmul_umma(stream, w, packed, y, n, w.n_rows, store, static_cast<float*>(partial), may_defer ? &left : nullptr);
         });
@@ -213,11 +211,14 @@ struct Recorder {
         pack_normed(hidden, norm_weight, n, cols, in_pack);
         run("matmul_swiglu", gate.n_rows, gate.n_cols, 2 * gate.bytes(), 1,
             [&] { return k::matmul_umma_swiglu(stream, gate, up, in_pack, nullptr, n, gate.n_rows, scratch); });
-        product_of_packed(down, scratch, s.tp ? s.partial : hidden, n, s.tp ? BC_STORE_OVERWRITE : BC_STORE_ACCUMULATE);
-        if (s.tp) {
-            s.launches += 1;
-            run_status([&] { return comm_all_reduce_add(s.tp, s.partial, hidden, (size_t)n * down.n_rows); });
-        }
+        product_of_packed_reduced(down, scratch, hidden, n);
+    }
+    // y += w x of packed rows, summed over the ranks of a tensor-parallel group.
+    void product_of_packed_reduced(const k::Mat& w, const void* packed, float* y, uint32_t n) {
+        product_of_packed(w, packed, s.tp ? s.partial : y, n, s.tp ? BC_STORE_OVERWRITE : BC_STORE_ACCUMULATE);
+        if (!s.tp) return;
+        s.launches += 1;
+        run_status([&] { return comm_all_reduce_add(s.tp, s.partial, y, (size_t)n * w.n_rows); });
     }
 
     void normed_matmuls(const float* x, const float* norm_weight, uint32_t n, std::initializer_list<Product> products) {
@@ -293,20 +294,19 @@ struct Recorder {
         matvec(D.out_proj, s.conv_out, s.hidden, k::Norm{}, true);
     }
 
+    // Norm and rotation of a batch's q and k, and its K and V rows into the caches.
+    void rotate_batch(const DeviceLayer& D, size_t slot, uint32_t pos, uint32_t n, float* q_dst, uint32_t q_stride, uint32_t q_head_stride, uint32_t q_dst_stride,
+                      uint32_t q_dst_head_stride) {
+        const k::RopeBatch rb{s.q, q_dst, s.k, s.v, cache_at(s.k_cache, slot), s.kv_half ? static_cast<__half*>(cache_at(s.v_cache, slot)) : nullptr,
+                              D.q_norm, D.k_norm, hp.n_heads, hp.n_kv_heads, hp.head_dim, q_stride, q_head_stride, q_dst_stride, q_dst_head_stride, hp.n_rot,
+                              pos, n, hp.rope_theta, hp.norm_eps, s.kv_half, hp.architecture == BC_ARCH_QWEN35 ? nullptr : s.rope_table};
+        run("norm_rope", (hp.n_heads + hp.n_kv_heads) * n, hp.head_dim, 0, 1, [&] { return k::rope_store_batch(stream, rb); });
+    }
+
     // Norm and rotation of q and k, cache stores, attention over positions [0, pos + n).
     void rotate_and_attend(const DeviceLayer& D, uint32_t cache_index, uint32_t pos, uint32_t n, uint32_t q_stride, uint32_t q_head_stride) {
         size_t slot = layer_base(cache_index) + (size_t)pos * kv_dim();
-        run("norm_rope", hp.n_heads * n, hp.head_dim, 0, 1, [&] {
-            return k::norm_rope(stream, s.q, s.q, false, D.q_norm, hp.n_heads, hp.head_dim, q_head_stride, hp.n_rot, pos, n, q_stride, q_stride,
-                                hp.rope_theta, hp.norm_eps);
-        });
-        run("norm_rope", hp.n_kv_heads * n, hp.head_dim, 0, 1, [&] {
-            return k::norm_rope(stream, s.k, cache_at(s.k_cache, slot), s.kv_half, D.k_norm, hp.n_kv_heads, hp.head_dim, hp.head_dim, hp.n_rot,
-                                pos, n, (uint32_t)kv_dim(), (uint32_t)kv_dim(), hp.rope_theta, hp.norm_eps);
-        });
-        if (s.kv_half)
-            run("convert_half", 1, n * (uint32_t)kv_dim(), 0, 1,
-                [&] { return k::convert_half(stream, s.v, static_cast<__half*>(cache_at(s.v_cache, slot)), (uint64_t)n * kv_dim()); });
+        rotate_batch(D, slot, pos, n, s.q, q_stride, q_head_stride, q_stride, q_head_stride);
         k::AttentionShape shape{hp.n_heads, hp.n_kv_heads, hp.head_dim, pos, n, s.n_ctx, q_stride, q_head_stride};
         int kernels = k::attention_launches(s.kv_half, shape);
         uint64_t kv_bytes = (uint64_t)(pos + n) * kv_dim() * kv_element_bytes() * 2;
@@ -511,11 +511,11 @@ struct Recorder {
                     // The convolution writes the packed input of the output projection itself.
                     void* pack = nullptr;
                     if (status == BC_OK) status = s.backend->pack_scratch(k::matmul_pack_bytes(n, n_embd), &pack);
-                    run("short_conv", n, n_embd, 0, 2,
+                    run("short_conv", n, n_embd, 0, 1,
                         [&] { return k::short_conv(stream, s.bcx, D.taps, history, nullptr, n_embd, hp.conv_kernel, n, pack); });
                     product_of_packed(D.out_proj, pack, s.hidden, n, BC_STORE_ACCUMULATE);
                 } else {
-                    run("short_conv", n, n_embd, 0, 2,
+                    run("short_conv", n, n_embd, 0, 1,
                         [&] { return k::short_conv(stream, s.bcx, D.taps, history, s.conv_out, n_embd, hp.conv_kernel, n); });
                     matmul(D.out_proj, s.conv_out, s.hidden, n, BC_STORE_ACCUMULATE);
                 }
@@ -554,11 +554,11 @@ struct Recorder {
             });
             return;
         }
-        run("gdn_conv", n, conv_dim(), 0, k::gdn_conv_launches(n), [&] { return k::gdn_conv(stream, s.gdn_qkv, D.conv1d, history, s.gdn_conv_out, conv_dim(), K, n); });
-        run("gdn_gates", n, hp.n_v_heads, 0, 1, [&] { return k::gdn_gates(stream, s.gdn_beta, s.gdn_alpha, D.a, D.dt_bias, hp.n_v_heads, n); });
+        run("gdn_conv", n, conv_dim(), 0, 1, [&] {
+            return k::gdn_conv_gates(stream, s.gdn_qkv, D.conv1d, history, s.gdn_conv_out, s.gdn_beta, s.gdn_alpha, D.a, D.dt_bias, hp.n_k_heads, hp.n_v_heads,
+                                     hp.k_head_dim, hp.v_head_dim, K, n);
+        });
         uint64_t state_bytes = (uint64_t)hp.n_v_heads * hp.k_head_dim * hp.v_head_dim * 4 * 2;
-        run("gdn_qk_norm", n * 2 * hp.n_k_heads, hp.k_head_dim, 0, 1,
-            [&] { return k::gdn_qk_norm(stream, s.gdn_conv_out, hp.n_k_heads, hp.n_v_heads, hp.k_head_dim, hp.v_head_dim, n); });
         if (k::gdn_chunk_supported(hp.n_v_heads, hp.k_head_dim, hp.v_head_dim, n)) {
             // No packed input is alive between the projections and the output projection.
             void* scratch = nullptr;
@@ -571,8 +571,26 @@ struct Recorder {
             return k::gdn_recurrence(stream, s.gdn_conv_out, s.gdn_beta, s.gdn_alpha, state, s.gdn_out, hp.n_k_heads, hp.n_v_heads, hp.k_head_dim,
                                      hp.v_head_dim, n, false);
         });
+        if (n > 1) return;  // qwen_delta_project normalises on the way into the output projection
         run("gdn_gated_norm", n * hp.n_v_heads, hp.v_head_dim, 0, 1,
             [&] { return k::gdn_gated_norm(stream, s.gdn_out, s.gdn_z, D.ssm_norm, hp.v_head_dim, n * hp.n_v_heads, hp.norm_eps); });
+    }
+
+    // The gated norm of the rule's outputs and the output projection of a batch. The norm writes the packed input of the
+    // projection where that runs on the tensor cores.
+    void qwen_delta_project(const DeviceLayer& D, uint32_t n) {
+        if (tensor_products() && k::matmul_umma_supported(D.ssm_out, n, min_tensor_rows) && k::gdn_gated_norm_pack_supported(hp.v_head_dim)) {
+            void* pack = nullptr;
+            if (status == BC_OK) status = s.backend->pack_scratch(k::matmul_pack_bytes(n, D.ssm_out.n_cols), &pack);
+            run("gdn_gated_norm", n * hp.n_v_heads, hp.v_head_dim, 0, 1, [&] {
+                return k::gdn_gated_norm_pack(stream, s.gdn_out, s.gdn_z, D.ssm_norm, hp.v_head_dim, hp.n_v_heads, n, hp.norm_eps, pack);
+            });
+            product_of_packed_reduced(D.ssm_out, pack, s.hidden, n);
+            return;
+        }
+        run("gdn_gated_norm", n * hp.n_v_heads, hp.v_head_dim, 0, 1,
+            [&] { return k::gdn_gated_norm(stream, s.gdn_out, s.gdn_z, D.ssm_norm, hp.v_head_dim, n * hp.n_v_heads, hp.norm_eps); });
+        matmul_reduced(D.ssm_out, s.gdn_out, s.hidden, n);
     }
 
     // qwen35_metal.rs:1038-1134
@@ -622,30 +640,29 @@ struct Recorder {
                                {{&D.q, s.q, BC_STORE_OVERWRITE}, {&D.k, s.k, BC_STORE_OVERWRITE}, {&D.v, value_target(S.cache_index, pos), BC_STORE_OVERWRITE}});
                 size_t slot = layer_base(S.cache_index) + (size_t)pos * kv_dim();
                 // The rotated queries go to their own compact rows; the gates stay in the projection.
-                run("norm_rope", hp.n_heads * n, hp.head_dim, 0, 1, [&] {
-                    return k::norm_rope(stream, s.q, s.q_rot, false, D.q_norm, hp.n_heads, hp.head_dim, 2 * hp.head_dim, hp.n_rot, pos, n, 2 * q_dim,
-                                        q_dim, hp.rope_theta, hp.norm_eps);
-                });
-                run("norm_rope", hp.n_kv_heads * n, hp.head_dim, 0, 1, [&] {
-                    return k::norm_rope(stream, s.k, cache_at(s.k_cache, slot), s.kv_half, D.k_norm, hp.n_kv_heads, hp.head_dim, hp.head_dim,
-                                        hp.n_rot, pos, n, (uint32_t)kv_dim(), (uint32_t)kv_dim(), hp.rope_theta, hp.norm_eps);
-                });
-                if (s.kv_half)
-                    run("convert_half", 1, n * (uint32_t)kv_dim(), 0, 1,
-                        [&] { return k::convert_half(stream, s.v, static_cast<__half*>(cache_at(s.v_cache, slot)), (uint64_t)n * kv_dim()); });
+                rotate_batch(D, slot, pos, n, s.q_rot, 2 * q_dim, 2 * hp.head_dim, q_dim, hp.head_dim);
                 k::AttentionShape shape{hp.n_heads, hp.n_kv_heads, hp.head_dim, pos, n, s.n_ctx, q_dim, hp.head_dim};
                 run("attention", n, pos + n, (uint64_t)(pos + n) * kv_dim() * kv_element_bytes() * 2, k::attention_launches(s.kv_half, shape), [&] {
                     return k::attention(stream, s.q_rot, cache_at(s.k_cache, layer_base(S.cache_index)), cache_at(s.v_cache, layer_base(S.cache_index)),
                                         s.kv_half, s.scores, s.attn, shape);
                 });
-                run("attention_gate", n, q_dim, 0, 1, [&] { return k::attention_gate(stream, s.attn, s.q, hp.n_heads, hp.head_dim, n); });
-                matmul_reduced(D.output, s.attn, s.hidden, n);
+                if (tensor_products() && k::matmul_umma_supported(D.output, n, min_tensor_rows) && hp.head_dim % 32 == 0) {
+                    // The gates on the way into the packed input of the output projection.
+                    void* pack = nullptr;
+                    if (status == BC_OK) status = s.backend->pack_scratch(k::matmul_pack_bytes(n, q_dim), &pack);
+                    run("attention_gate", n, q_dim, 0, 1, [&] { return k::matmul_pack_gated(stream, s.attn, s.q, hp.head_dim, n, q_dim, pack); });
+                    product_of_packed_reduced(D.output, pack, s.hidden, n);
+                } else {
+                    run("attention_gate", n, q_dim, 0, 1, [&] { return k::attention_gate(stream, s.attn, s.q, hp.n_heads, hp.head_dim, n); });
+                    matmul_reduced(D.output, s.attn, s.hidden, n);
+                }
             } else {
                 normed_matmuls(s.hidden, D.attn_norm, n,
                                {{&D.qkv, s.gdn_qkv, BC_STORE_OVERWRITE}, {&D.z, s.gdn_z, BC_STORE_OVERWRITE}, {&D.beta, s.gdn_beta, BC_STORE_OVERWRITE},
                                 {&D.alpha, s.gdn_alpha, BC_STORE_OVERWRITE}});
                 qwen_delta_tail(D, S.cache_index, n);
-                matmul_reduced(D.ssm_out, s.gdn_out, s.hidden, n);
+                if (n > 1) qwen_delta_project(D, n);
+                else matmul_reduced(D.ssm_out, s.gdn_out, s.hidden, n);
             }
             normed_ffn(s.hidden, D.ffn_norm, n, D.gate, D.up, D.down);
             if (traced) copy(s.hidden, s.trace_layers + il * trace_stride, (uint64_t)n * n_embd);
