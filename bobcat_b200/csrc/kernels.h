@@ -75,6 +75,12 @@ int sm_count();
 // Repack GGUF Q4_0 bytes (18-byte blocks) already on the device into the split layout.
 cudaError_t repack_q4_0(cudaStream_t stream, const uint8_t* raw, uint64_t n_blocks, void* quants, __half* scales);
 
+// Products of a large f32 matrix with one row (normalised first when `norm` says so) or with up to sixteen (kernels_stream_f32.cu).
+bool stream_f32_supported(const Mat& w, const float* x);
+cudaError_t stream_f32(cudaStream_t stream, const Mat& w, const float* x, Norm norm, float* y);
+bool stream_f32_rows_supported(const Mat& w, const float* x, uint32_t n_tokens);
+cudaError_t stream_f32_rows(cudaStream_t stream, const Mat& w, const float* x, float* y, uint32_t n_tokens, uint32_t y_stride);
+
 // The tile layout of a Q4_0 matrix: its size, whether this width has one, and the conversion from
 // the split layout (both already on the device).
 uint64_t tiles_bytes(uint32_t n_rows, uint32_t n_cols);

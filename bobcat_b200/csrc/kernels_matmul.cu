@@ -114,8 +114,8 @@ __global__ void __launch_bounds__(kThreads) matmul_simt_kernel(MatmulParams p) {
     }
 }
 
-// An f32 matrix against at most 32 rows of X (the logits of a pass over several sequences: the
-// output matrix is the model's largest and is kept in f32): Y[t][r] = sum_c W[r][c] X[t][c], f32
+// An f32 matrix against 17 to 32 rows of X, or fewer where they do not fit beside the ring of
+// kernels_stream_f32.cu: Y[t][r] = sum_c W[r][c] X[t][c], f32
 // throughout, every sum one chain of fused multiply-adds over the columns in order. The tile kernel
 // above spends a pass over a 65536 x 2048 matrix mostly on loads of single elements (0.97 ms for 32
 // rows). Here a CTA is ONE warp with 64 weight rows to itself: 1024 such warps spread evenly over
@@ -224,6 +224,7 @@ __global__ void __launch_bounds__(kFewThreads) matmul_f32_few_kernel(const float
 cudaError_t matmul(cudaStream_t stream, const Mat& w, const float* x, float* y, uint32_t n_tokens, uint32_t y_stride,
                    int32_t store, void* pack) {
     if (n_tokens == 0 || w.n_rows == 0) return cudaSuccess;
+    if (store == BC_STORE_OVERWRITE && stream_f32_rows_supported(w, x, n_tokens)) return stream_f32_rows(stream, w, x, y, n_tokens, y_stride);
     if (w.format == BC_F32 && n_tokens <= 32 && store == BC_STORE_OVERWRITE && w.n_cols % 32 == 0 && w.n_cols > 0 &&
         ((reinterpret_cast<uintptr_t>(w.data) | reinterpret_cast<uintptr_t>(x)) & 15) == 0) {
         constexpr size_t bytes = few_smem_bytes<32, 2>();

@@ -322,6 +322,7 @@ cudaError_t matvec(cudaStream_t stream, const MatvecSegment* segments, int n_seg
     bool tiled = segments[0].w.format == BC_Q4_0;
     for (int i = 0; i < n_segments; ++i) tiled = tiled && segments[i].w.tiles != nullptr;
     if (tiled) return matvec_mma(stream, segments, n_segments, x, norm, accumulate);
+    if (n_segments == 1 && !accumulate && stream_f32_supported(segments[0].w, x)) return stream_f32(stream, segments[0].w, x, norm, segments[0].y);
     Params p{};
     p.n_segments = n_segments;
     for (int i = 0; i < n_segments; ++i) {
