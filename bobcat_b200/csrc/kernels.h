@@ -189,6 +189,7 @@ struct AttentionShape {
     uint32_t n_heads, n_kv_heads, head_dim, first_pos, n_queries, n_ctx;
     uint32_t q_stride, q_head_stride;
     const uint32_t* pos_ptr = nullptr;  // when set, first_pos is *pos_ptr + first_pos and the grid covers n_ctx
+    uint64_t scratch_floats = 0;  // what the scratch holds; 0: attention_scratch_floats of this shape
 };
 uint64_t attention_scratch_floats(uint32_t n_heads, uint32_t head_dim, uint32_t n_ctx, uint32_t n_queries);
 cudaError_t attention(cudaStream_t stream, const float* q, const void* k_cache, const void* v_cache, bool kv_half,
@@ -204,7 +205,8 @@ cudaError_t attention_step(cudaStream_t stream, const RopeStore& r, float* scrat
 // The tensor-core prefill kernel (kernels_attention_flash.cu): heads of 64 elements, f16 cache, at
 // least 32 queries, positions known at launch. `attention` picks it when it applies.
 bool attention_flash_supported(bool kv_half, const AttentionShape& shape);
-cudaError_t attention_flash(cudaStream_t stream, const float* q, const void* k_cache, const void* v_cache, float* out,
+int attention_flash_launches(const AttentionShape& s);
+cudaError_t attention_flash(cudaStream_t stream, const float* q, const void* k_cache, const void* v_cache, float* scratch, float* out,
                             const AttentionShape& shape);
 
 // argmax over n floats, ties to the lowest index. `out` is a device word; `readback` (nullable) is

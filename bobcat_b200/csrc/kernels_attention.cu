@@ -517,7 +517,7 @@ uint64_t attention_scratch_floats(uint32_t n_heads, uint32_t head_dim, uint32_t 
 }
 
 int attention_launches(bool kv_half, const AttentionShape& s) {
-    if (attention_flash_supported(kv_half, s)) return 1;
+    if (attention_flash_supported(kv_half, s)) return attention_flash_launches(s);
     return 2 * (int)((s.n_queries + kQueryBatch - 1) / kQueryBatch);
 }
 
@@ -527,7 +527,7 @@ cudaError_t attention(cudaStream_t stream, const float* q, const void* k_cache, 
     // The tensor-core kernel reads q and out 8 bytes and the caches 16 bytes at a time; views that
     // do not start on those boundaries take the chunk kernels, whose loads are scalar.
     const bool flash_aligned = ((uintptr_t)q | (uintptr_t)out) % 8 == 0 && ((uintptr_t)k_cache | (uintptr_t)v_cache) % 16 == 0;
-    if (flash_aligned && attention_flash_supported(kv_half, s)) return attention_flash(stream, q, k_cache, v_cache, out, s);
+    if (flash_aligned && attention_flash_supported(kv_half, s)) return attention_flash(stream, q, k_cache, v_cache, scratch, out, s);
     const uint32_t group = s.n_heads / s.n_kv_heads;
     const uint32_t chunk = s.n_queries <= (uint32_t)kDecodeQueries ? decode_chunk(s.n_ctx) : (uint32_t)kChunk;
     const uint32_t max_chunks = (s.n_ctx + chunk - 1) / chunk;

@@ -1,7 +1,6 @@
-// Prefill attention for heads of 64, 128 or 256 elements over an f16 cache: one CTA per (64
-// queries, head), 64-key tiles, online softmax, the two products on tensor cores. Counterpart of
-// attention_flash (crates/bobcat-metal/src/attention.metal:290-480), which the reference uses for
-// head_dim == 64 and at least 32 queries (backend.rs:2185-2225); the wider heads (Qwen3.5's
+// Prefill attention for heads of 64, 128 or 256 elements over an f16 cache: 64-key tiles, online softmax, the two
+// products on tensor cores. Counterpart of attention_flash (crates/bobcat-metal/src/attention.metal:290-480), which
+// the reference uses for head_dim == 64 and at least 32 queries (backend.rs:2185-2225); the wider heads (Qwen3.5's
 // attention layers have 256 elements) take the same path here instead of the chunk kernels.
 //
 // Arithmetic. Keys and values are the cache's fp16 values, exactly. The scaled query and the
@@ -10,12 +9,24 @@
 // an f32 evaluation only by summation order. The row maximum, exponentials (expf) and row sums are
 // f32, as in the chunk kernels.
 //
-// A warp owns 16 queries. Scores S = Q K^T come from mma.m16n8k16 with the query fragments held in
+// Work. A CTA of eight warps takes 128 rows of one KV head (four warps and 64 rows for heads of 64), a row being a query of one of the heads that share it (the
+// heads of a query are neighbouring rows), so a tile of keys is fetched once for all of them. The keys are
+// also cut, into `splits` neighbouring parts of a CTA's tiles, where that fills the device: 64 queries of eight heads are four CTAs
+// otherwise. Each part leaves its unnormalised sums with its maximum and sum of exponentials, and a second launch joins them.
+//
+// A warp owns 16 rows. Scores S = Q K^T come from mma.m16n8k16 with the query fragments held in
 // registers (heads of 64; wider heads re-read them from the staged queries at every step, their
 // registers hold the output instead) and key fragments read with ldmatrix from the staged tile; the accumulator layout of S
 // is the A-fragment layout of the second product, so probabilities go from registers straight into
-// P V, whose value fragments are ldmatrix.trans reads of the staged tile.
+// P V, whose value fragments are ldmatrix.trans reads of the staged tile. Keys and values have a buffer each: the values of a
+// tile arrive under its scores, the next keys under its P V. Bound by the multiplies (one per 8 cycles and
+// scheduler) for wide heads, by the exponentials' instructions for heads of 64.
+//
+// Measured: 64 queries of 8 heads of 256 behind 0 to 2000 positions 110 us before (four warps, loads and multiplies in
+// turn, a CTA per head), 39 with the join; 512 queries of 16 heads behind 4500 positions 500 us, 284; 512 queries
+// of 32 heads of 64 from position 0 33 us, 29.
 
+#include "async_utils.cuh"
 #include "device_utils.cuh"
 #include "kernels.h"
 
@@ -24,14 +35,18 @@ namespace k {
 
 namespace {
 
-constexpr int kQueries = 64;   // queries per CTA: 4 warps x 16
 constexpr int kKeys = 64;      // keys per tile
-constexpr int kFlashThreads = 128;
+// Rows per CTA, 16 to a warp. Heads of 64 take small CTAs, four to an SM (their registers allow it): more, finer work.
+template <int HD>
+constexpr int flash_rows() { return HD == 64 ? 64 : 128; }
+template <int HD>
+constexpr int flash_threads() { return 2 * flash_rows<HD>(); }
+constexpr uint32_t kMaxSplits = 32;
 // Halves per staged row: 16 bytes more than the head, so the 8 rows of an ldmatrix fall in distinct banks.
 template <int HD>
 constexpr int flash_pitch() { return HD + 8; }
 template <int HD>
-constexpr size_t flash_smem_bytes() { return (size_t)(2 * kQueries + 2 * kKeys) * flash_pitch<HD>() * 2; }
+constexpr size_t flash_smem_bytes() { return (size_t)(2 * flash_rows<HD>() + 2 * kKeys) * flash_pitch<HD>() * 2; }
 
 struct FlashParams {
     const float* q;
@@ -39,6 +54,8 @@ struct FlashParams {
     const __half* v_cache;
     float* out;
     uint32_t n_heads, n_kv_heads, first_pos, n_queries, q_stride, q_head_stride;
+    uint32_t splits;
+    float* parts;      // splits > 1: [split][query][head][HD] unnormalised sums, then [split][query][head] (maximum, sum)
 };
 
 __device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) {
@@ -64,50 +81,69 @@ __device__ __forceinline__ void split_half2(float x, float y, uint32_t& hi, uint
 }
 
 template <int HD>
-__global__ void __launch_bounds__(kFlashThreads) attention_flash_kernel(FlashParams p) {
-    constexpr int kHead = HD, kPitch = flash_pitch<HD>();
+__global__ void __launch_bounds__(flash_threads<HD>(), HD == 64 ? 4 : 1) attention_flash_kernel(const __grid_constant__ FlashParams p) {
+    constexpr int kRows = flash_rows<HD>(), kFlashThreads = flash_threads<HD>(), kHead = HD, kPitch = flash_pitch<HD>();
     constexpr bool kQueriesInRegisters = HD == 64;
     extern __shared__ __align__(16) uint8_t flash_smem[];
     __half (*q_hi)[kPitch] = reinterpret_cast<__half (*)[kPitch]>(flash_smem);
-    __half (*q_lo)[kPitch] = q_hi + kQueries;
-    __half (*k_tile)[kPitch] = q_lo + kQueries;
+    __half (*q_lo)[kPitch] = q_hi + kRows;
+    __half (*k_tile)[kPitch] = q_lo + kRows;
     __half (*v_tile)[kPitch] = k_tile + kKeys;
 
     pdl_launch_dependents();
     pdl_wait();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
-    const uint32_t q0 = blockIdx.x * kQueries, head = blockIdx.y;
-    const uint32_t kv_head = head / (p.n_heads / p.n_kv_heads);
+    const uint32_t group = p.n_heads / p.n_kv_heads, n_rows = p.n_queries * group;
+    const uint32_t row0 = (gridDim.x - 1 - blockIdx.x) * kRows, kv_head = blockIdx.y;  // the last queries see most keys: first
     const uint32_t kv_dim = p.n_kv_heads * kHead;
     const uint32_t kv_len = p.first_pos + p.n_queries;  // cache rows that exist
     const float scale = 1.0f / sqrtf((float)kHead);
 
+    // Key tiles up to the position of the CTA's last query, and this CTA's part of them.
+    const uint32_t last_query = (min(row0 + kRows, n_rows) - 1) / group;
+    const uint32_t all_tiles = (p.first_pos + last_query) / kKeys + 1, per_split = (all_tiles + p.splits - 1) / p.splits;
+    const uint32_t first_tile = blockIdx.z * per_split, end_tile = min(first_tile + per_split, all_tiles);
+
+    const __half* kc = p.k_cache + (uint64_t)kv_head * kHead;
+    const __half* vc = p.v_cache + (uint64_t)kv_head * kHead;
+    // Rows past the cache's end repeat its last one: their scores are masked.
+    auto bring = [&](const __half* from, __half (*to)[kPitch], uint32_t tile) {
+#pragma unroll
+        for (int n = 0; n < kKeys * (kHead / 8) / kFlashThreads; ++n) {
+            const int i = tid + n * kFlashThreads, row = i / (kHead / 8), piece = i % (kHead / 8);
+            const uint32_t key = min(tile * kKeys + row, kv_len - 1);
+            async::cp_async_16((uint32_t)__cvta_generic_to_shared(&to[row][8 * piece]), from + (uint64_t)key * kv_dim + 8 * piece);
+        }
+        async::cp_async_commit();
+    };
+    if (first_tile < end_tile) bring(kc, k_tile, first_tile);
+
     // Stage the scaled queries as hi + lo halves; rows past the batch are zero.
-    for (int i = tid; i < kQueries * (kHead / 2); i += kFlashThreads) {
-        int row = i / (kHead / 2), pair = i % (kHead / 2);
+    for (int i = tid; i < kRows * (kHead / 2); i += kFlashThreads) {
+        const int row = i / (kHead / 2), pair = i % (kHead / 2);
         float2 v = make_float2(0.f, 0.f);
-        if (q0 + row < p.n_queries) {
-            const float* src = p.q + (uint64_t)(q0 + row) * p.q_stride + (uint64_t)head * p.q_head_stride + 2 * pair;
-            v = *reinterpret_cast<const float2*>(src);
+        if (row0 + row < n_rows) {
+            const uint32_t query = (row0 + row) / group, head = kv_head * group + (row0 + row) % group;
+            v = *reinterpret_cast<const float2*>(p.q + (uint64_t)query * p.q_stride + (uint64_t)head * p.q_head_stride + 2 * pair);
         }
         uint32_t hi, lo;
         split_half2(v.x * scale, v.y * scale, hi, lo);
         *reinterpret_cast<uint32_t*>(&q_hi[row][2 * pair]) = hi;
         *reinterpret_cast<uint32_t*>(&q_lo[row][2 * pair]) = lo;
     }
-    __syncthreads();
 
     // Query fragments: k-steps of 16 elements, hi and lo.
     constexpr int kHeld = kQueriesInRegisters ? kHead / 16 : 1;
     uint32_t qa_hi[kHeld][4], qa_lo[kHeld][4];
+    const int m = lane >> 3, r = lane & 7;
     auto query_fragments = [&](int ks, uint32_t (&hi)[4], uint32_t (&lo)[4]) {
-        const int m = lane >> 3, r = lane & 7;
         const int row = warp * 16 + (m & 1) * 8 + r, col = ks * 16 + (m >> 1) * 8;
         ldmatrix_x4(hi, (uint32_t)__cvta_generic_to_shared(&q_hi[row][col]));
         ldmatrix_x4(lo, (uint32_t)__cvta_generic_to_shared(&q_lo[row][col]));
     };
     if (kQueriesInRegisters) {
+        __syncthreads();
 #pragma unroll
         for (int ks = 0; ks < kHeld; ++ks) query_fragments(ks, qa_hi[ks], qa_lo[ks]);
     }
@@ -119,144 +155,210 @@ __global__ void __launch_bounds__(kFlashThreads) attention_flash_kernel(FlashPar
         for (int i = 0; i < 4; ++i) o[n][i] = 0.f;
     float row_max[2] = {-INFINITY, -INFINITY}, row_sum[2] = {0.f, 0.f};
 
-    // The position of this thread's two rows (g and g + 8 of the warp's 16 queries).
-    const uint32_t pos_a = p.first_pos + q0 + warp * 16 + g, pos_b = pos_a + 8;
-    // Keys up to the position of the CTA's last query.
-    const uint32_t last_query = min(q0 + kQueries, p.n_queries) - 1;
-    const uint32_t n_tiles = (p.first_pos + last_query) / kKeys + 1;
+    // This thread's two rows, g and g + 8 of the warp's 16, and their positions.
+    const uint32_t row_a = row0 + warp * 16 + g, row_b = row_a + 8;
+    const uint32_t pos_a = p.first_pos + row_a / group, pos_b = p.first_pos + row_b / group;
     // A warp whose queries all lie before a tile has nothing to add from it.
-    const uint32_t warp_last_pos = p.first_pos + q0 + warp * 16 + 15;
+    const uint32_t warp_first_pos = p.first_pos + (row0 + warp * 16) / group, warp_last_pos = p.first_pos + (row0 + warp * 16 + 15) / group;
 
-    const __half* kc = p.k_cache + (uint64_t)kv_head * kHead;
-    const __half* vc = p.v_cache + (uint64_t)kv_head * kHead;
-
-    for (uint32_t tile = 0; tile < n_tiles; ++tile) {
+    for (uint32_t tile = first_tile; tile < end_tile; ++tile) {
         const uint32_t key0 = tile * kKeys;
-        __syncthreads();  // the previous tile has been read
-        for (int i = tid; i < kKeys * (kHead / 8); i += kFlashThreads) {
-            int row = i / (kHead / 8), piece = i % (kHead / 8);
-            uint4 kv = make_uint4(0, 0, 0, 0), vv = kv;
-            if (key0 + row < kv_len) {
-                kv = *reinterpret_cast<const uint4*>(kc + (uint64_t)(key0 + row) * kv_dim + 8 * piece);
-                vv = *reinterpret_cast<const uint4*>(vc + (uint64_t)(key0 + row) * kv_dim + 8 * piece);
-            }
-            *reinterpret_cast<uint4*>(&k_tile[row][8 * piece]) = kv;
-            *reinterpret_cast<uint4*>(&v_tile[row][8 * piece]) = vv;
-        }
-        __syncthreads();
-        if (key0 > warp_last_pos) continue;  // warp-uniform
+        const bool skip = key0 > warp_last_pos;  // warp-uniform
+        async::cp_async_wait<0>();
+        __syncthreads();  // the keys are there, the previous values have been read
+        bring(vc, v_tile, tile);
 
-        // S = Q K^T: 8 tiles of 8 keys.
+        // S = Q K^T: 8 tiles of 8 keys. Four accumulators take their hi products, then their lo ones: a product does not wait
+        // for the one before it.
         float s[8][4];
+        if (!skip) {
 #pragma unroll
-        for (int n = 0; n < 8; ++n)
+            for (int n = 0; n < 8; ++n)
 #pragma unroll
-            for (int i = 0; i < 4; ++i) s[n][i] = 0.f;
-        {
-            const int m = lane >> 3, r = lane & 7;
+                for (int i = 0; i < 4; ++i) s[n][i] = 0.f;
 #pragma unroll
             for (int ks = 0; ks < kHead / 16; ++ks) {
                 if (!kQueriesInRegisters) query_fragments(ks, qa_hi[0], qa_lo[0]);
                 const uint32_t (&a_hi)[4] = qa_hi[kQueriesInRegisters ? ks : 0];
                 const uint32_t (&a_lo)[4] = qa_lo[kQueriesInRegisters ? ks : 0];
 #pragma unroll
-                for (int np = 0; np < 4; ++np) {  // pairs of key tiles
-                    uint32_t b[4];
-                    ldmatrix_x4(b, (uint32_t)__cvta_generic_to_shared(&k_tile[np * 16 + (m >> 1) * 8 + r][ks * 16 + (m & 1) * 8]));
-                    mma_f16(s[2 * np], a_hi, b[0], b[1]);
-                    mma_f16(s[2 * np], a_lo, b[0], b[1]);
-                    mma_f16(s[2 * np + 1], a_hi, b[2], b[3]);
-                    mma_f16(s[2 * np + 1], a_lo, b[2], b[3]);
+                for (int np = 0; np < 4; np += 2) {  // two pairs of key tiles
+                    uint32_t b[2][4];
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+                        ldmatrix_x4(b[h], (uint32_t)__cvta_generic_to_shared(&k_tile[(np + h) * 16 + (m >> 1) * 8 + r][ks * 16 + (m & 1) * 8]));
+#pragma unroll
+                    for (int n = 0; n < 4; ++n) mma_f16(s[2 * np + n], a_hi, b[n >> 1][(n & 1) * 2], b[n >> 1][(n & 1) * 2 + 1]);
+#pragma unroll
+                    for (int n = 0; n < 4; ++n) mma_f16(s[2 * np + n], a_lo, b[n >> 1][(n & 1) * 2], b[n >> 1][(n & 1) * 2 + 1]);
                 }
             }
-        }
-        // Causal mask (only tiles that reach past a query's position need it).
-        if (key0 + kKeys - 1 > p.first_pos + q0 + warp * 16) {
+            // Causal mask (only tiles that reach past a query's position need it).
+            if (key0 + kKeys - 1 > warp_first_pos) {
+#pragma unroll
+                for (int n = 0; n < 8; ++n) {
+                    const uint32_t key = key0 + n * 8 + 2 * t;
+                    if (key > pos_a) s[n][0] = -INFINITY;
+                    if (key + 1 > pos_a) s[n][1] = -INFINITY;
+                    if (key > pos_b) s[n][2] = -INFINITY;
+                    if (key + 1 > pos_b) s[n][3] = -INFINITY;
+                }
+            }
+            // Online softmax. A row that has seen no key yet (a part of the keys may lie past it) keeps a maximum of
+            // minus infinity and sums of zero.
+            float tile_max[2] = {-INFINITY, -INFINITY};
 #pragma unroll
             for (int n = 0; n < 8; ++n) {
-                const uint32_t key = key0 + n * 8 + 2 * t;
-                if (key > pos_a) s[n][0] = -INFINITY;
-                if (key + 1 > pos_a) s[n][1] = -INFINITY;
-                if (key > pos_b) s[n][2] = -INFINITY;
-                if (key + 1 > pos_b) s[n][3] = -INFINITY;
+                tile_max[0] = fmaxf(tile_max[0], fmaxf(s[n][0], s[n][1]));
+                tile_max[1] = fmaxf(tile_max[1], fmaxf(s[n][2], s[n][3]));
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                tile_max[h] = fmaxf(tile_max[h], __shfl_xor_sync(0xffffffffu, tile_max[h], 1));
+                tile_max[h] = fmaxf(tile_max[h], __shfl_xor_sync(0xffffffffu, tile_max[h], 2));
+            }
+            float correction[2], top[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const float m_new = fmaxf(row_max[h], tile_max[h]);
+                top[h] = m_new == -INFINITY ? 0.f : m_new;
+                correction[h] = expf(row_max[h] - top[h]);  // exp(-inf) = 0 on the first keys
+                row_max[h] = m_new;
+            }
+            float tile_sum[2] = {0.f, 0.f};
+#pragma unroll
+            for (int n = 0; n < 8; ++n) {
+                s[n][0] = expf(s[n][0] - top[0]);
+                s[n][1] = expf(s[n][1] - top[0]);
+                s[n][2] = expf(s[n][2] - top[1]);
+                s[n][3] = expf(s[n][3] - top[1]);
+                tile_sum[0] += s[n][0] + s[n][1];
+                tile_sum[1] += s[n][2] + s[n][3];
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                tile_sum[h] += __shfl_xor_sync(0xffffffffu, tile_sum[h], 1);
+                tile_sum[h] += __shfl_xor_sync(0xffffffffu, tile_sum[h], 2);
+                row_sum[h] = row_sum[h] * correction[h] + tile_sum[h];
+            }
+#pragma unroll
+            for (int n = 0; n < kHead / 8; ++n) {
+                o[n][0] *= correction[0];
+                o[n][1] *= correction[0];
+                o[n][2] *= correction[1];
+                o[n][3] *= correction[1];
             }
         }
-        // Online softmax. Key 0 is visible to every query, so after the first tile the maxima are finite.
-        float tile_max[2] = {-INFINITY, -INFINITY};
-#pragma unroll
-        for (int n = 0; n < 8; ++n) {
-            tile_max[0] = fmaxf(tile_max[0], fmaxf(s[n][0], s[n][1]));
-            tile_max[1] = fmaxf(tile_max[1], fmaxf(s[n][2], s[n][3]));
-        }
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            tile_max[h] = fmaxf(tile_max[h], __shfl_xor_sync(0xffffffffu, tile_max[h], 1));
-            tile_max[h] = fmaxf(tile_max[h], __shfl_xor_sync(0xffffffffu, tile_max[h], 2));
-        }
-        float correction[2];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            float m_new = fmaxf(row_max[h], tile_max[h]);
-            correction[h] = expf(row_max[h] - m_new);  // exp(-inf) = 0 on the first tile
-            row_max[h] = m_new;
-        }
-        float tile_sum[2] = {0.f, 0.f};
-#pragma unroll
-        for (int n = 0; n < 8; ++n) {
-            s[n][0] = expf(s[n][0] - row_max[0]);
-            s[n][1] = expf(s[n][1] - row_max[0]);
-            s[n][2] = expf(s[n][2] - row_max[1]);
-            s[n][3] = expf(s[n][3] - row_max[1]);
-            tile_sum[0] += s[n][0] + s[n][1];
-            tile_sum[1] += s[n][2] + s[n][3];
-        }
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            tile_sum[h] += __shfl_xor_sync(0xffffffffu, tile_sum[h], 1);
-            tile_sum[h] += __shfl_xor_sync(0xffffffffu, tile_sum[h], 2);
-            row_sum[h] = row_sum[h] * correction[h] + tile_sum[h];
-        }
-#pragma unroll
-        for (int n = 0; n < kHead / 8; ++n) {
-            o[n][0] *= correction[0];
-            o[n][1] *= correction[0];
-            o[n][2] *= correction[1];
-            o[n][3] *= correction[1];
-        }
-        // O += P V: 4 k-steps of 16 keys; the scores' accumulator layout is the A-fragment layout.
-        {
-            const int m = lane >> 3, r = lane & 7;
-#pragma unroll
-            for (int kk = 0; kk < 4; ++kk) {
-                uint32_t pa_hi[4], pa_lo[4];
-                split_half2(s[2 * kk][0], s[2 * kk][1], pa_hi[0], pa_lo[0]);
-                split_half2(s[2 * kk][2], s[2 * kk][3], pa_hi[1], pa_lo[1]);
-                split_half2(s[2 * kk + 1][0], s[2 * kk + 1][1], pa_hi[2], pa_lo[2]);
-                split_half2(s[2 * kk + 1][2], s[2 * kk + 1][3], pa_hi[3], pa_lo[3]);
-#pragma unroll
-                for (int np = 0; np < kHead / 16; ++np) {  // pairs of 8-element output tiles
-                    uint32_t b[4];
-                    ldmatrix_x4_trans(b, (uint32_t)__cvta_generic_to_shared(&v_tile[kk * 16 + (m & 1) * 8 + r][np * 16 + (m >> 1) * 8]));
-                    mma_f16(o[2 * np], pa_hi, b[0], b[1]);
-                    mma_f16(o[2 * np], pa_lo, b[0], b[1]);
-                    mma_f16(o[2 * np + 1], pa_hi, b[2], b[3]);
-                    mma_f16(o[2 * np + 1], pa_lo, b[2], b[3]);
-                }
-            }
-        }
-    }
+        async::cp_async_wait<0>();
+        __syncthreads();  // the values are there, the keys have been read
+        if (tile + 1 < end_tile) bring(kc, k_tile, tile + 1);
+        if (skip) continue;
 
-    // Normalise and store: row g holds columns 2t, 2t + 1 of each 8-element tile.
-    const uint32_t query_a = q0 + warp * 16 + g, query_b = query_a + 8;
-    const float inv_a = 1.f / row_sum[0], inv_b = 1.f / row_sum[1];
+        // O += P V: 4 k-steps of 16 keys; the scores' accumulator layout is the A-fragment layout.
 #pragma unroll
-    for (int n = 0; n < kHead / 8; ++n) {
-        const uint32_t col = head * kHead + n * 8 + 2 * t;
-        if (query_a < p.n_queries)
-            *reinterpret_cast<float2*>(p.out + (uint64_t)query_a * p.n_heads * kHead + col) = make_float2(o[n][0] * inv_a, o[n][1] * inv_a);
-        if (query_b < p.n_queries)
-            *reinterpret_cast<float2*>(p.out + (uint64_t)query_b * p.n_heads * kHead + col) = make_float2(o[n][2] * inv_b, o[n][3] * inv_b);
+        for (int kk = 0; kk < 4; ++kk) {
+            uint32_t pa_hi[4], pa_lo[4];
+            split_half2(s[2 * kk][0], s[2 * kk][1], pa_hi[0], pa_lo[0]);
+            split_half2(s[2 * kk][2], s[2 * kk][3], pa_hi[1], pa_lo[1]);
+            split_half2(s[2 * kk + 1][0], s[2 * kk + 1][1], pa_hi[2], pa_lo[2]);
+            split_half2(s[2 * kk + 1][2], s[2 * kk + 1][3], pa_hi[3], pa_lo[3]);
+#pragma unroll
+            for (int np = 0; np < kHead / 16; np += 2) {  // two pairs of 8-element output tiles
+                uint32_t b[2][4];
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    ldmatrix_x4_trans(b[h], (uint32_t)__cvta_generic_to_shared(&v_tile[kk * 16 + (m & 1) * 8 + r][(np + h) * 16 + (m >> 1) * 8]));
+#pragma unroll
+                for (int n = 0; n < 4; ++n) mma_f16(o[2 * np + n], pa_hi, b[n >> 1][(n & 1) * 2], b[n >> 1][(n & 1) * 2 + 1]);
+#pragma unroll
+                for (int n = 0; n < 4; ++n) mma_f16(o[2 * np + n], pa_lo, b[n >> 1][(n & 1) * 2], b[n >> 1][(n & 1) * 2 + 1]);
+            }
+        }
     }
+    async::cp_async_wait<0>();
+
+    // Normalise and store: row g holds columns 2t, 2t + 1 of each 8-element tile. A part of the keys leaves its sums as they are.
+    const bool whole = p.splits == 1;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const uint32_t row = h ? row_b : row_a;
+        if (row >= n_rows) continue;
+        const uint64_t at = (uint64_t)(row / group) * p.n_heads + kv_head * group + row % group, total = (uint64_t)p.n_queries * p.n_heads;
+        if (!whole) {
+            if (t == 0)
+                *reinterpret_cast<float2*>(p.parts + p.splits * total * kHead + (blockIdx.z * total + at) * 2) = make_float2(row_max[h], row_sum[h]);
+            if (row_max[h] == -INFINITY) continue;  // joins with a weight of zero, unread
+        }
+        const float factor = whole ? 1.f / row_sum[h] : 1.f;
+        float* out = (whole ? p.out + at * kHead : p.parts + (blockIdx.z * total + at) * kHead) + 2 * t;
+#pragma unroll
+        for (int n = 0; n < kHead / 8; ++n) *reinterpret_cast<float2*>(out + n * 8) = make_float2(o[n][2 * h] * factor, o[n][2 * h + 1] * factor);
+    }
+}
+
+// Joins the parts of the keys, a warp per (query, head).
+template <int HD>
+__global__ void __launch_bounds__(256) attention_join_kernel(const float* __restrict__ parts, float* __restrict__ out, uint32_t splits, uint32_t total) {
+    constexpr int kQuads = HD / 64;  // pairs of elements a lane holds
+    pdl_launch_dependents();
+    pdl_wait();
+    const uint32_t lane = threadIdx.x & 31, at = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (at >= total) return;
+    float2 ms = make_float2(-INFINITY, 0.f);
+    if (lane < splits) ms = __ldcg(reinterpret_cast<const float2*>(parts + (uint64_t)splits * total * HD + ((uint64_t)lane * total + at) * 2));
+    const float top = warp_max(ms.x), weight = ms.x == -INFINITY ? 0.f : expf(ms.x - top);
+    const float inverse = 1.f / warp_sum(weight * ms.y);
+    float2 sum[kQuads];
+#pragma unroll
+    for (int i = 0; i < kQuads; ++i) sum[i] = make_float2(0.f, 0.f);
+#pragma unroll 4
+    for (uint32_t z = 0; z < splits; ++z) {
+        const float w = __shfl_sync(0xffffffffu, weight, z);
+        if (w == 0.f) continue;
+        const float2* from = reinterpret_cast<const float2*>(parts + ((uint64_t)z * total + at) * HD) + lane;
+#pragma unroll
+        for (int i = 0; i < kQuads; ++i) {
+            const float2 v = __ldcg(from + i * 32);
+            sum[i].x += w * v.x;
+            sum[i].y += w * v.y;
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < kQuads; ++i) reinterpret_cast<float2*>(out + (uint64_t)at * HD)[lane + i * 32] = make_float2(sum[i].x * inverse, sum[i].y * inverse);
+}
+
+// Parts of the keys: the fewest modelled time. A tile takes 3.6 us (heads of 64, up to four CTAs to an SM) to 7.1 (heads of 256), a CTA 6 us around them, a
+// part's sums are written and read once at L2 rates, the joining launch costs 4 us. The sums must fit the scratch the caller
+// has (attention_scratch_floats), and a head's rows of (maximum, sum) a warp.
+uint32_t choose_splits(const AttentionShape& s) {
+    const uint32_t rows = s.head_dim == 64 ? flash_rows<64>() : flash_rows<256>(), units = (s.n_queries * (s.n_heads / s.n_kv_heads) + rows - 1) / rows * s.n_kv_heads;
+    const uint32_t tiles = (s.first_pos + s.n_queries - 1) / kKeys + 1, slots = (uint32_t)sm_count() * (s.head_dim == 64 ? 4 : 1);
+    const uint64_t floats = s.scratch_floats ? s.scratch_floats : attention_scratch_floats(s.n_heads, s.head_dim, s.n_ctx, s.n_queries);
+    const uint64_t room = floats / ((uint64_t)s.n_queries * s.n_heads * (s.head_dim + 2));
+    uint32_t most = tiles < kMaxSplits ? tiles : kMaxSplits, best = 1;
+    if (room < most) most = room > 0 ? (uint32_t)room : 1;
+    float least = 0.f;
+    const float tile_us = 2.5f + s.head_dim * 0.018f, part_us = (float)s.n_queries * s.n_heads * s.head_dim * 8e-6f / 8.f;
+    for (uint32_t splits = 1; splits <= most; ++splits) {
+        const uint32_t waves = (units * splits + slots - 1) / slots, per = (tiles + splits - 1) / splits;
+        const float us = waves * (per * tile_us + 6.f) + (splits > 1 ? 4.f + splits * part_us : 0.f);
+        if (splits == 1 || us < least) {
+            best = splits;
+            least = us;
+        }
+    }
+    return best;
+}
+
+template <int HD>
+cudaError_t launch_flash(cudaStream_t stream, const FlashParams& p) {
+    const uint32_t group = p.n_heads / p.n_kv_heads, total = p.n_queries * p.n_heads;
+    cudaError_t e = ensure_dynamic_smem((const void*)attention_flash_kernel<HD>, flash_smem_bytes<HD>());
+    if (e != cudaSuccess) return e;
+    e = launch_dependent(attention_flash_kernel<HD>, dim3((p.n_queries * group + flash_rows<HD>() - 1) / flash_rows<HD>(), p.n_kv_heads, p.splits), dim3(flash_threads<HD>()),
+                         flash_smem_bytes<HD>(), stream, p);
+    if (e != cudaSuccess || p.splits == 1) return e;
+    return launch_dependent(attention_join_kernel<HD>, dim3((total + 7) / 8), dim3(256), 0, stream, static_cast<const float*>(p.parts), p.out, p.splits, total);
 }
 
 }  // namespace
@@ -266,22 +368,17 @@ bool attention_flash_supported(bool kv_half, const AttentionShape& s) {
            s.n_kv_heads > 0 && s.n_heads % s.n_kv_heads == 0 && s.q_stride % 2 == 0 && s.q_head_stride % 2 == 0;
 }
 
-cudaError_t attention_flash(cudaStream_t stream, const float* q, const void* k_cache, const void* v_cache, float* out,
+int attention_flash_launches(const AttentionShape& s) { return choose_splits(s) > 1 ? 2 : 1; }
+
+cudaError_t attention_flash(cudaStream_t stream, const float* q, const void* k_cache, const void* v_cache, float* scratch, float* out,
                             const AttentionShape& s) {
-    FlashParams p{q, static_cast<const __half*>(k_cache), static_cast<const __half*>(v_cache), out, s.n_heads, s.n_kv_heads,
-                  s.first_pos, s.n_queries, s.q_stride, s.q_head_stride};
-    dim3 grid((s.n_queries + kQueries - 1) / kQueries, s.n_heads);
-    cudaError_t e;
+    const uint32_t splits = (uintptr_t)scratch % 8 == 0 ? choose_splits(s) : 1;
+    const FlashParams p{q, static_cast<const __half*>(k_cache), static_cast<const __half*>(v_cache), out, s.n_heads, s.n_kv_heads,
+                        s.first_pos, s.n_queries, s.q_stride, s.q_head_stride, splits, scratch};
     switch (s.head_dim) {
-        case 64:
-            if ((e = ensure_dynamic_smem((const void*)attention_flash_kernel<64>, flash_smem_bytes<64>())) != cudaSuccess) return e;
-            return launch_dependent(attention_flash_kernel<64>, grid, dim3(kFlashThreads), flash_smem_bytes<64>(), stream, p);
-        case 128:
-            if ((e = ensure_dynamic_smem((const void*)attention_flash_kernel<128>, flash_smem_bytes<128>())) != cudaSuccess) return e;
-            return launch_dependent(attention_flash_kernel<128>, grid, dim3(kFlashThreads), flash_smem_bytes<128>(), stream, p);
-        default:
-            if ((e = ensure_dynamic_smem((const void*)attention_flash_kernel<256>, flash_smem_bytes<256>())) != cudaSuccess) return e;
-            return launch_dependent(attention_flash_kernel<256>, grid, dim3(kFlashThreads), flash_smem_bytes<256>(), stream, p);
+        case 64: return launch_flash<64>(stream, p);
+        case 128: return launch_flash<128>(stream, p);
+        default: return launch_flash<256>(stream, p);
     }
 }
 

@@ -307,7 +307,7 @@ struct Recorder {
     void rotate_and_attend(const DeviceLayer& D, uint32_t cache_index, uint32_t pos, uint32_t n, uint32_t q_stride, uint32_t q_head_stride) {
         size_t slot = layer_base(cache_index) + (size_t)pos * kv_dim();
         rotate_batch(D, slot, pos, n, s.q, q_stride, q_head_stride, q_stride, q_head_stride);
-        k::AttentionShape shape{hp.n_heads, hp.n_kv_heads, hp.head_dim, pos, n, s.n_ctx, q_stride, q_head_stride};
+        k::AttentionShape shape{hp.n_heads, hp.n_kv_heads, hp.head_dim, pos, n, s.n_ctx, q_stride, q_head_stride, nullptr, s.scratch_floats};
         int kernels = k::attention_launches(s.kv_half, shape);
         uint64_t kv_bytes = (uint64_t)(pos + n) * kv_dim() * kv_element_bytes() * 2;
         run("attention", n, pos + n, kv_bytes, kernels, [&] {
@@ -641,7 +641,7 @@ struct Recorder {
                 size_t slot = layer_base(S.cache_index) + (size_t)pos * kv_dim();
                 // The rotated queries go to their own compact rows; the gates stay in the projection.
                 rotate_batch(D, slot, pos, n, s.q_rot, 2 * q_dim, 2 * hp.head_dim, q_dim, hp.head_dim);
-                k::AttentionShape shape{hp.n_heads, hp.n_kv_heads, hp.head_dim, pos, n, s.n_ctx, q_dim, hp.head_dim};
+                k::AttentionShape shape{hp.n_heads, hp.n_kv_heads, hp.head_dim, pos, n, s.n_ctx, q_dim, hp.head_dim, nullptr, s.scratch_floats};
                 run("attention", n, pos + n, (uint64_t)(pos + n) * kv_dim() * kv_element_bytes() * 2, k::attention_launches(s.kv_half, shape), [&] {
                     return k::attention(stream, s.q_rot, cache_at(s.k_cache, layer_base(S.cache_index)), cache_at(s.v_cache, layer_base(S.cache_index)),
                                         s.kv_half, s.scores, s.attn, shape);
