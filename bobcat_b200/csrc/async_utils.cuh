@@ -125,6 +125,33 @@ __device__ __forceinline__ void tmem_load_16(uint32_t taddr, float (&v)[16]) {
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// The load alone; tmem_load_wait completes every one that was started before it. Its arguments are the two arrays, which
+// nothing may read before.
+__device__ __forceinline__ void tmem_load_16_start(uint32_t taddr, float (&v)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]), "=f"(v[8]), "=f"(v[9]),
+          "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15])
+        : "r"(taddr)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_load_wait(float (&v)[16], float (&w)[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]), "+f"(v[6]), "+f"(v[7]), "+f"(v[8]), "+f"(v[9]),
+                   "+f"(v[10]), "+f"(v[11]), "+f"(v[12]), "+f"(v[13]), "+f"(v[14]), "+f"(v[15]),
+                   "+f"(w[0]), "+f"(w[1]), "+f"(w[2]), "+f"(w[3])
+                 :
+                 : "memory");
+    asm volatile("" : "+f"(w[4]), "+f"(w[5]), "+f"(w[6]), "+f"(w[7]), "+f"(w[8]), "+f"(w[9]), "+f"(w[10]), "+f"(w[11]), "+f"(w[12]),
+                      "+f"(w[13]), "+f"(w[14]), "+f"(w[15]) : : "memory");
+}
+// One lane of a converged warp, always the same one.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t mine;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(mine));
+    return mine != 0;
+}
+
 }  // namespace async
 }  // namespace k
 }  // namespace bc

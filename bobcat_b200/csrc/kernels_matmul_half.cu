@@ -88,6 +88,59 @@ __device__ __forceinline__ void give_up(volatile int* dead, int code) {
     if (g_wait_word) *reinterpret_cast<volatile int*>(g_wait_word) = code;
 }
 
+// The epilogue of a plain product: a warp's 32 rows, every other unit of 16 tokens, two units in flight. Bound by
+// instructions while it asked for every value what to do with it: 8 us for 128 rows x 256 tokens, which nothing
+// hides when a CTA has one tile; 512 tokens of 6144 x 2048 19.0 us with it, 14.1 now (with the MMA warp's change).
+__device__ __forceinline__ void store_tile(uint32_t from, uint32_t half, uint32_t units, const Tile& t, float* out, uint32_t stride, uint32_t out_row,
+                                           uint32_t rows, uint32_t n_tokens, int store) {
+    const bool stores = out_row < rows;
+    auto put = [&](uint32_t u, float (&v)[16]) {
+        const uint32_t tok = t.tok0 + u * 16;
+        if (!stores || tok >= n_tokens) return;
+        if (t.chunks == 0) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] = 0.f;
+        }
+        const uint32_t live = n_tokens - tok;
+        float* to = out + (uint64_t)tok * stride + out_row;
+        if (store == BC_STORE_OVERWRITE && live >= 16) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j, to += stride) *to = v[j];
+            return;
+        }
+        if (store == BC_STORE_OVERWRITE) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j, to += stride)
+                if ((uint32_t)j < live) *to = v[j];
+            return;
+        }
+        float old[16];
+        float* at = to;
+#pragma unroll
+        for (int j = 0; j < 16; ++j, at += stride) old[j] = (uint32_t)j < live ? __ldcg(at) : 0.f;
+        if (store == BC_STORE_ACCUMULATE) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] += old[j];
+        } else {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] = old[j] / (1.f + expf(-old[j])) * v[j];
+        }
+#pragma unroll
+        for (int j = 0; j < 16; ++j, to += stride)
+            if ((uint32_t)j < live) *to = v[j];
+    };
+    for (uint32_t u = half; u < units; u += 4) {
+        float v[16], w[16];
+        const bool second = u + 2 < units;  // the same for the whole warp
+        __syncwarp();
+        tmem_load_16_start(from + u * 16, v);
+        if (second) tmem_load_16_start(from + (u + 2) * 16, w);
+        tmem_load_wait(v, w);
+        put(u, v);
+        if (second) put(u + 2, w);
+    }
+}
+
 template <int DUAL>
 __global__ void __launch_bounds__(kThreads, 1) matmul_half_kernel(const __grid_constant__ HalfParams p) {
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -166,27 +219,29 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_half_kernel(const __grid_c
             }
         }
     } else if (warp == 1) {
-        // ---- the tensor core
-        if (lane == 0) {
-            uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 1;
-            const uint64_t desc0 = umma_desc(ring, kCoreBytes, kGroupBytes);
-            bool alive = true;
-            for (uint32_t i = blockIdx.x; i < p.n_tiles && alive; i += gridDim.x) {
-                const Tile t = tile_at(p, i);
-                const uint32_t idesc = umma_idesc_f16(kRows, t.n);
-                if (!mbar_wait(acc_empty0 + 8 * acc, acc_phase, kSpinLimit, dead)) {
-                    give_up(dead, 1);
+        // ---- the tensor core. The whole warp walks the chunks and one lane issues: values the warp shares stay in uniform
+        // registers, where the instruction wants its descriptors (a loop inside one lane moved them there for every
+        // multiply: 510 cycles per chunk whatever its width, the multiplies of 256 tokens).
+        uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 1;
+        const uint64_t desc0 = umma_desc(ring, kCoreBytes, kGroupBytes);
+        bool alive = true;
+        for (uint32_t i = blockIdx.x; i < p.n_tiles && alive; i += gridDim.x) {
+            const Tile t = tile_at(p, i);
+            const uint32_t idesc = umma_idesc_f16(kRows, t.n);
+            if (!__all_sync(0xffffffffu, mbar_wait(acc_empty0 + 8 * acc, acc_phase, kSpinLimit, dead))) {
+                if (lane == 0) give_up(dead, 1);
+                break;
+            }
+            tc_fence_after_sync();
+            for (uint32_t c = 0; c < t.chunks; ++c) {
+                if (!__all_sync(0xffffffffu, mbar_wait(full0 + 8 * stage, phase, kSpinLimit, dead))) {
+                    if (lane == 0) give_up(dead, 4);
+                    alive = false;
                     break;
                 }
                 tc_fence_after_sync();
-                for (uint32_t c = 0; c < t.chunks; ++c) {
-                    if (!mbar_wait(full0 + 8 * stage, phase, kSpinLimit, dead)) {
-                        give_up(dead, 4);
-                        alive = false;
-                        break;
-                    }
-                    tc_fence_after_sync();
-                    const uint64_t a_desc = desc0 + ((stage * kStageBytes) >> 4), b_desc = a_desc + ((DUAL * kATile) >> 4);
+                const uint64_t a_desc = desc0 + ((stage * kStageBytes) >> 4), b_desc = a_desc + ((DUAL * kATile) >> 4);
+                if (elect_one()) {
 #pragma unroll
                     for (uint32_t m = 0; m < (uint32_t)DUAL; ++m)
 #pragma unroll
@@ -194,11 +249,11 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_half_kernel(const __grid_c
                             umma_f16(tmem + acc * kAccColumns + m * (kAccColumns / 2), a_desc + ((m * kATile + j * 2 * kCoreBytes) >> 4),
                                      b_desc + ((j * 2 * kCoreBytes) >> 4), idesc, (c | j) != 0);
                     umma_commit(empty0 + 8 * stage);
-                    if (++stage == kStages) stage = 0, phase ^= 1;
                 }
-                if (alive) umma_commit(acc_full0 + 8 * acc);
-                if (++acc == 2) acc = 0, acc_phase ^= 1;
+                if (++stage == kStages) stage = 0, phase ^= 1;
             }
+            if (alive && elect_one()) umma_commit(acc_full0 + 8 * acc);
+            if (++acc == 2) acc = 0, acc_phase ^= 1;
         }
     } else {
         // ---- epilogue: a warp reads lanes 32 * (warp % 4).. of tensor memory and every other 16 columns
@@ -220,55 +275,43 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_half_kernel(const __grid_c
             }
             tc_fence_after_sync();
             const uint32_t from = tmem + ((quarter * 32) << 16) + acc * kAccColumns, units = t.n / 16;
-            for (uint32_t u = half; u < units; u += 2) {
-                float v[16];
-                __syncwarp();
-                tmem_load_16(from + u * 16, v);
-                if (DUAL == 2) {
-                    float up[16];
-                    tmem_load_16(from + kAccColumns / 2 + u * 16, up);
+            if (DUAL == 1) {
+                store_tile(from, half, units, t, out, stride, out_row, rows, p.n_tokens, p.store);
+            } else {
+                for (uint32_t u = half; u < units; u += 2) {
+                    float v[16], up[16];
+                    __syncwarp();
+                    tmem_load_16_start(from + u * 16, v);
+                    tmem_load_16_start(from + kAccColumns / 2 + u * 16, up);
+                    tmem_load_wait(v, up);
 #pragma unroll
                     for (int j = 0; j < 16; ++j) v[j] = v[j] / (1.f + expf(-v[j])) * up[j];
-                }
-                if (DUAL == 2 && p.packed_out) {
-                    // The warp's 32 rows are one block of 32 columns of the consuming product, its 16
-                    // tokens two groups of 8. The values turn through shared memory into 16-byte
-                    // core-matrix rows (17 rows of 16 bytes per core matrix keep both sides free of
-                    // bank conflicts); a lane stores two, 8 lanes to a 128-byte line.
-                    if (row0 + quarter * 32 < rows) {
-                        __half* turn = reinterpret_cast<__half*>(turns + ew * kTurnBytes);
-                        const uint32_t core = (lane & 15) >> 2, e = lane & 3;
-                        const uint32_t at = (lane >> 4) * 4 + (e & 1) * 2 + (e >> 1);
+                    if (p.packed_out) {
+                        // The warp's 32 rows are one block of 32 columns of the consuming product, its 16
+                        // tokens two groups of 8. The values turn through shared memory into 16-byte
+                        // core-matrix rows (17 rows of 16 bytes per core matrix keep both sides free of
+                        // bank conflicts); a lane stores two, 8 lanes to a 128-byte line.
+                        if (row0 + quarter * 32 < rows) {
+                            __half* turn = reinterpret_cast<__half*>(turns + ew * kTurnBytes);
+                            const uint32_t core = (lane & 15) >> 2, e = lane & 3;
+                            const uint32_t at = (lane >> 4) * 4 + (e & 1) * 2 + (e >> 1);
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) turn[(core * 17 + j) * 8 + at] = __float2half_rn(v[j]);
-                        __syncwarp();
-                        const uint32_t tr = lane & 7, mm = lane >> 3;
-                        const uint32_t chunk = (row0 >> 6) + (quarter >> 1), jj = (quarter & 1) * 4 + mm;
+                            for (int j = 0; j < 16; ++j) turn[(core * 17 + j) * 8 + at] = __float2half_rn(v[j]);
+                            __syncwarp();
+                            const uint32_t tr = lane & 7, mm = lane >> 3;
+                            const uint32_t chunk = (row0 >> 6) + (quarter >> 1), jj = (quarter & 1) * 4 + mm;
 #pragma unroll
-                        for (uint32_t it = 0; it < 2; ++it) {
-                            const uint4 row16 = *reinterpret_cast<const uint4*>(turn + (mm * 17 + it * 8 + tr) * 8);
-                            const uint32_t tg = ((t.tok0 + u * 16) >> 3) + it;
-                            reinterpret_cast<uint4*>(p.packed_out)[(((uint64_t)chunk * p.token_groups + tg) * kCores + jj) * 8 + tr] = row16;
+                            for (uint32_t it = 0; it < 2; ++it) {
+                                const uint4 row16 = *reinterpret_cast<const uint4*>(turn + (mm * 17 + it * 8 + tr) * 8);
+                                const uint32_t tg = ((t.tok0 + u * 16) >> 3) + it;
+                                reinterpret_cast<uint4*>(p.packed_out)[(((uint64_t)chunk * p.token_groups + tg) * kCores + jj) * 8 + tr] = row16;
+                            }
                         }
-                    }
-                    continue;
-                }
-                if (out_row < rows) {
-                    const uint32_t tok = t.tok0 + u * 16, live = p.n_tokens > tok ? p.n_tokens - tok : 0;
-                    float* to = out + (uint64_t)tok * stride + out_row;
-                    float old[16];
-                    if (DUAL == 1 && p.store != BC_STORE_OVERWRITE) {
+                    } else if (out_row < rows) {
+                        float* to = out + (uint64_t)(t.tok0 + u * 16) * stride + out_row;
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) old[j] = (uint32_t)j < live ? __ldcg(to + (uint64_t)j * stride) : 0.f;
-                    }
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        if ((uint32_t)j < live) {
-                            float r = t.chunks ? v[j] : 0.f;
-                            if (DUAL == 1 && p.store == BC_STORE_ACCUMULATE) r += old[j];
-                            else if (DUAL == 1 && p.store == BC_STORE_SWIGLU) r = old[j] / (1.f + expf(-old[j])) * r;
-                            to[(uint64_t)j * stride] = r;
-                        }
+                        for (int j = 0; j < 16; ++j, to += stride)
+                            if (t.tok0 + u * 16 + j < p.n_tokens) *to = v[j];
                     }
                 }
             }
@@ -312,25 +355,29 @@ struct Tiling {
     uint32_t tile_tokens, split;
 };
 
-// The tiling with the smallest modelled time, in cycles: waves of tiles over the SMs, each chunk of 64
-// columns bound by the MMA (2 cycles per token and matrix, no less than a tile of 96 tokens costs) or by the
-// SM's share of L2 (fitted: 75 bytes per cycle), an exposed prologue and last epilogue, and a split's extra pass.
+// The tiling with the smallest modelled time, in us, fitted to 33 to 512 tokens of matrices of 2048 to 10752 rows and columns:
+// waves of tiles over the SMs, each chunk of 64 columns bound by the MMA (2 cycles per token and matrix at 1.4 GHz),
+// by the SM's share of L2 or by the ring's round trip; a start and a last epilogue that nothing hides; a split's partial
+// products, written and read once; never less than the weights' time from HBM.
 Tiling choose_tiling(uint32_t row_tiles, uint32_t n_chunks, uint32_t n_tokens, int dual, bool may_split) {
     const uint32_t sms = (uint32_t)sm_count(), widest = dual == 2 ? 128 : 256;
     Tiling best{widest, 1};
-    double best_cost = 1e30;
+    double best_us = 1e30;
     const uint32_t fewest = (n_tokens + widest - 1) / widest;
     for (uint32_t token_tiles = fewest; token_tiles <= fewest + 6; ++token_tiles) {
         const uint32_t width = ((n_tokens + token_tiles - 1) / token_tiles + 15u) & ~15u;
         if (width < 48 && token_tiles > fewest) break;
         const uint32_t needed = (n_tokens + width - 1) / width;
+        const double mma = 2.0 * width * dual / 1400.0, load = (16384.0 * dual + 128.0 * width) / (dual == 2 ? 105e3 : 125e3);
+        const double chunk = mma > load ? (mma > 0.25 ? mma : 0.25) : (load > 0.25 ? load : 0.25);
         for (uint32_t split = 1; split <= (may_split && dual == 1 ? kMaxSplit : 1u); ++split) {
             if (split > 1 && n_chunks / split < 4) break;
             const uint32_t tiles = row_tiles * needed * split, waves = (tiles + sms - 1) / sms;
-            const double mma = (width < 96 ? 192.0 : 2.0 * width) * dual, load = (16384.0 * dual + 128.0 * width) / 75.0;
-            double cost = waves * ((n_chunks + split - 1) / split) * (mma > load ? mma : load) + 3000.0 + 12.0 * width;
-            if (split > 1) cost += 1500.0 + (double)split * n_tokens * row_tiles * kRows * 4 * 2 / 4000.0;
-            if (cost < best_cost) best_cost = cost, best = Tiling{width, split};
+            double us = waves * ((n_chunks + split - 1) / split) * chunk;
+            const double hbm = (double)row_tiles * dual * n_chunks * kATile / 6.2e6;
+            us = (us > hbm ? us : hbm) + 2.8 + 0.0095 * width * dual;
+            if (split > 1) us += 1.0 + (double)split * n_tokens * row_tiles * kRows * 4 / 8e6;
+            if (us < best_us) best_us = us, best = Tiling{width, split};
         }
     }
     return best;
