@@ -12,8 +12,8 @@
 // the expanded copy does not fit the device, Mat::half_tiles is null and the dequantising kernel serves.
 //
 // Shape. Persistent CTAs of ten warps, one per SM: a loader thread, an MMA thread, eight epilogue warps.
-// A tile is 128 weight rows x up to 256 tokens (or 128 rows of both matrices of a SwiGLU x up to 128
-// tokens, two accumulators). K advances 64 columns per stage through a four-stage ring; both operands
+// A tile is 128 weight rows x up to 256 tokens (of a SwiGLU 64 rows of either matrix, or 128 of both x up to 128 tokens).
+// K advances 64 columns per stage through a ring of 192 KB, four to eight stages; both operands
 // arrive by bulk copies of contiguous memory (the weight tile is stored as the 16 KB image the MMA reads,
 // the tokens come packed, kernels_matmul_umma.cu's pack kernels), so no thread touches an operand. Tensor
 // memory holds two accumulators of 256 columns: a tile's epilogue runs under the next tile's main
@@ -40,15 +40,21 @@ using namespace async;
 constexpr uint32_t kRows = 128, kChunkK = 64, kCores = kChunkK / 8;
 constexpr uint32_t kATile = kRows * kChunkK * 2;       // 16 KB: [8-row group][core along K][row][16 bytes]
 constexpr uint32_t kGroupBytes = 8 * kChunkK * 2, kCoreBytes = 128;
-constexpr uint32_t kStages = 4, kStageBytes = 48 * 1024;
+constexpr uint32_t kMaxStages = 8, kRingBytes = 192 * 1024;  // a stage: a tile's weights and its tokens
 constexpr uint32_t kEpilogueWarps = 8, kThreads = (2 + kEpilogueWarps) * 32;
 constexpr uint32_t kTmemColumns = 512, kAccColumns = 256;
 constexpr uint32_t kSpinLimit = 1u << 22;
-constexpr uint32_t kTurnBytes = 1152;                  // per epilogue warp: a 32 x 16 block turned into operand layout
-constexpr size_t kSmemBytes = kStages * kStageBytes + kEpilogueWarps * kTurnBytes + 1024;
+constexpr uint32_t kTurnBytes = 640;                   // per epilogue warp: a 32 x 8 block turned into operand layout
+constexpr uint32_t kSwapBytes = 2 * 2 * 8 * 32 * 4;    // per pair of epilogue warps: 8 columns of 32 rows each way, twice
+constexpr size_t kSmemBytes = kRingBytes + kEpilogueWarps * kTurnBytes + kEpilogueWarps / 2 * kSwapBytes + 1024;
 constexpr uint32_t kMaxSplit = 8;
 
 __device__ int* g_wait_word;  // where a wait that ran out leaves its code (kernels.h), null until set
+
+// What a tile of 128 accumulator rows is: rows of one matrix; 128 rows of both matrices of a SwiGLU (two accumulators, up to
+// 128 tokens); or 64 rows of either (one accumulator, up to 256 tokens: more, finer tiles from the same bytes).
+enum Kind { kPlain = 1, kWhole = 2, kHalves = 3 };
+constexpr uint32_t a_bytes(int kind) { return kind == kWhole ? 2 * kATile : kATile; }
 
 struct HalfParams {
     // Up to four matrices that read the same inputs: row tiles [first_tile[i], first_tile[i + 1]) are
@@ -59,6 +65,7 @@ struct HalfParams {
     int n_matrices;
     const __half* packed;      // [n_chunks][token_groups][8 cores][8 tokens][8 halves]
     uint32_t n_chunks, n_tokens, token_groups;
+    uint32_t stages, stage_bytes;
     uint32_t tile_tokens, token_tiles, split, n_tiles;  // n_tiles = row tiles x split x token tiles
     int store;
     __half* packed_out;        // dual: the result as the packed operand of the product that consumes it
@@ -141,21 +148,40 @@ __device__ __forceinline__ void store_tile(uint32_t from, uint32_t half, uint32_
     }
 }
 
-template <int DUAL>
+// A warp's 32 rows x 8 tokens as fp16 operand of the consuming product, of which the rows are a block of 32 columns and the tokens a
+// group. The values turn through shared memory into 16-byte core-matrix rows (9 rows of 16 bytes per core matrix
+// keep both sides free of bank conflicts); a lane stores one, 8 lanes to a 128-byte line.
+__device__ __forceinline__ void put_group(const float* v, uint8_t* turn_bytes, const HalfParams& p, uint32_t row0, uint32_t block, uint32_t tok, uint32_t lane) {
+    __half* turn = reinterpret_cast<__half*>(turn_bytes);
+    const uint32_t core = (lane & 15) >> 2, e = lane & 3;
+    const uint32_t at = (lane >> 4) * 4 + (e & 1) * 2 + (e >> 1);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) turn[(core * 9 + j) * 8 + at] = __float2half_rn(v[j]);
+    __syncwarp();
+    const uint32_t tr = lane & 7, mm = lane >> 3;
+    const uint4 row16 = *reinterpret_cast<const uint4*>(turn + (mm * 9 + tr) * 8);
+    const uint32_t chunk = (row0 >> 6) + (block >> 1), jj = (block & 1) * 4 + mm;
+    reinterpret_cast<uint4*>(p.packed_out)[(((uint64_t)chunk * p.token_groups + (tok >> 3)) * kCores + jj) * 8 + tr] = row16;
+}
+
+template <int KIND>
 __global__ void __launch_bounds__(kThreads, 1) matmul_half_kernel(const __grid_constant__ HalfParams p) {
+    constexpr bool kDual = KIND != kPlain;
+    constexpr uint32_t kABytes = a_bytes(KIND);
     extern __shared__ __align__(1024) uint8_t smem[];
-    uint8_t* turns = smem + kStages * kStageBytes;
-    __shared__ __align__(8) uint64_t bars[2 * kStages + 4];
+    uint8_t* turns = smem + kRingBytes;
+    const uint32_t n_stages = p.stages, stage_bytes = p.stage_bytes;
+    __shared__ __align__(8) uint64_t bars[2 * kMaxStages + 4];
     __shared__ uint32_t tmem_slot;
     __shared__ volatile int dead_flag;
     volatile int* dead = &dead_flag;
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t full0 = smem_u32(bars), empty0 = full0 + kStages * 8, acc_full0 = empty0 + kStages * 8, acc_empty0 = acc_full0 + 16;
+    const uint32_t full0 = smem_u32(bars), empty0 = full0 + kMaxStages * 8, acc_full0 = empty0 + kMaxStages * 8, acc_empty0 = acc_full0 + 16;
     const uint32_t ring = smem_u32(smem);
     // The next launch may set itself up; it waits for this one before it touches its outputs.
     pdl_launch_dependents();
     if (tid == 0) {
-        for (uint32_t s = 0; s < kStages; ++s) {
+        for (uint32_t s = 0; s < n_stages; ++s) {
             mbar_init(full0 + 8 * s, 1);   // the loader's arrive.expect_tx
             mbar_init(empty0 + 8 * s, 1);  // the MMA thread's commit
         }
@@ -181,30 +207,32 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_half_kernel(const __grid_c
             for (uint32_t i = blockIdx.x; i < p.n_tiles; i += gridDim.x) {
                 const Tile t = tile_at(p, i);
                 int m = 0;
-                if (DUAL == 1)
+                if (!kDual)
                     while (m + 1 < p.n_matrices && t.row_tile >= p.first_tile[m + 1]) ++m;
-                const uint64_t at = ((uint64_t)(t.row_tile - (DUAL == 1 ? p.first_tile[m] : 0)) * p.n_chunks + t.chunk0) * (kATile / 2);
+                const uint64_t at = KIND == kHalves ? ((uint64_t)(t.row_tile / 2) * p.n_chunks * 2 + (t.row_tile & 1)) * (kATile / 4)  // half of a 128-row tile
+                                                    : ((uint64_t)(t.row_tile - (kDual ? 0 : p.first_tile[m])) * p.n_chunks + t.chunk0) * (kATile / 2);
                 const __half* a = p.tiles[m] + at;
-                const __half* a2 = DUAL == 2 ? p.tiles[1] + at : nullptr;
+                const __half* a2 = kDual ? p.tiles[1] + at : nullptr;
                 const __half* b = p.packed + ((uint64_t)t.chunk0 * p.token_groups + t.tok0 / 8) * (8 * kChunkK);
                 const uint32_t b_bytes = t.n * kChunkK * 2;
                 auto weights = [&](uint32_t c, uint32_t s) {
-                    mbar_arrive_expect(full0 + 8 * s, DUAL * kATile + b_bytes);
-                    bulk_load(ring + s * kStageBytes, a + (uint64_t)c * (kATile / 2), kATile, full0 + 8 * s);
-                    if (DUAL == 2) bulk_load(ring + s * kStageBytes + kATile, a2 + (uint64_t)c * (kATile / 2), kATile, full0 + 8 * s);
+                    constexpr uint32_t kEach = kDual ? kABytes / 2 : kABytes;
+                    mbar_arrive_expect(full0 + 8 * s, kABytes + b_bytes);
+                    bulk_load(ring + s * stage_bytes, a + (uint64_t)c * (kATile / 2), kEach, full0 + 8 * s);
+                    if (kDual) bulk_load(ring + s * stage_bytes + kEach, a2 + (uint64_t)c * (kATile / 2), kEach, full0 + 8 * s);
                 };
                 auto tokens = [&](uint32_t c, uint32_t s) {
-                    bulk_load(ring + s * kStageBytes + DUAL * kATile, b + (uint64_t)c * p.token_groups * (8 * kChunkK), b_bytes, full0 + 8 * s);
+                    bulk_load(ring + s * stage_bytes + kABytes, b + (uint64_t)c * p.token_groups * (8 * kChunkK), b_bytes, full0 + 8 * s);
                 };
                 uint32_t c = 0;
                 if (!waited) {
-                    const uint32_t first = t.chunks < kStages ? t.chunks : kStages;  // free stages: nothing to wait for
+                    const uint32_t first = t.chunks < n_stages ? t.chunks : n_stages;  // free stages: nothing to wait for
                     for (; c < first; ++c) weights(c, c);
                     pdl_wait();
                     waited = true;
                     for (uint32_t s = 0; s < first; ++s) tokens(s, s);
-                    stage = first % kStages;
-                    phase = first == kStages ? 0 : 1;
+                    stage = first % n_stages;
+                    phase = first == n_stages ? 0 : 1;
                 }
                 for (; c < t.chunks; ++c) {
                     if (!mbar_wait(empty0 + 8 * stage, phase, kSpinLimit, dead)) {
@@ -213,7 +241,7 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_half_kernel(const __grid_c
                     }
                     weights(c, stage);
                     tokens(c, stage);
-                    if (++stage == kStages) stage = 0, phase ^= 1;
+                    if (++stage == n_stages) stage = 0, phase ^= 1;
                 }
                 if (*dead) break;
             }
@@ -240,17 +268,17 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_half_kernel(const __grid_c
                     break;
                 }
                 tc_fence_after_sync();
-                const uint64_t a_desc = desc0 + ((stage * kStageBytes) >> 4), b_desc = a_desc + ((DUAL * kATile) >> 4);
+                const uint64_t a_desc = desc0 + ((stage * stage_bytes) >> 4), b_desc = a_desc + (kABytes >> 4);
                 if (elect_one()) {
 #pragma unroll
-                    for (uint32_t m = 0; m < (uint32_t)DUAL; ++m)
+                    for (uint32_t m = 0; m < (KIND == kWhole ? 2u : 1u); ++m)
 #pragma unroll
                         for (uint32_t j = 0; j < kChunkK / 16; ++j)
                             umma_f16(tmem + acc * kAccColumns + m * (kAccColumns / 2), a_desc + ((m * kATile + j * 2 * kCoreBytes) >> 4),
                                      b_desc + ((j * 2 * kCoreBytes) >> 4), idesc, (c | j) != 0);
                     umma_commit(empty0 + 8 * stage);
                 }
-                if (++stage == kStages) stage = 0, phase ^= 1;
+                if (++stage == n_stages) stage = 0, phase ^= 1;
             }
             if (alive && elect_one()) umma_commit(acc_full0 + 8 * acc);
             if (++acc == 2) acc = 0, acc_phase ^= 1;
@@ -263,21 +291,20 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_half_kernel(const __grid_c
         for (uint32_t i = blockIdx.x; i < p.n_tiles; i += gridDim.x) {
             const Tile t = tile_at(p, i);
             int m = 0;
-            if (DUAL == 1)
+            if (!kDual)
                 while (m + 1 < p.n_matrices && t.row_tile >= p.first_tile[m + 1]) ++m;
             const uint32_t rows = p.rows[m], stride = p.stride[m];
-            const uint32_t row0 = (t.row_tile - (DUAL == 1 ? p.first_tile[m] : 0)) * kRows, out_row = row0 + quarter * 32 + lane;
+            const uint32_t row0 = KIND == kHalves ? t.row_tile * (kRows / 2) : (t.row_tile - (kDual ? 0 : p.first_tile[m])) * kRows;
+            const uint32_t block = KIND == kHalves ? quarter & 1 : quarter, out_row = row0 + block * 32 + lane;  // the warp's 32 rows of the tile
             float* out = p.y[m] + (p.split > 1 ? (uint64_t)t.part * p.n_tokens * stride : 0);
             const bool ok = lane != 0 || mbar_wait(acc_full0 + 8 * acc, acc_phase, kSpinLimit, dead);
-            if (!__all_sync(0xffffffffu, ok)) {
-                if (lane == 0) give_up(dead, 2);
-                break;
-            }
+            // A wait that ran out voids the results; the warp walks on (further waits end at once), because others meet it below.
+            if (!__all_sync(0xffffffffu, ok) && lane == 0) give_up(dead, 2);
             tc_fence_after_sync();
             const uint32_t from = tmem + ((quarter * 32) << 16) + acc * kAccColumns, units = t.n / 16;
-            if (DUAL == 1) {
+            if (KIND == kPlain) {
                 store_tile(from, half, units, t, out, stride, out_row, rows, p.n_tokens, p.store);
-            } else {
+            } else if (KIND == kWhole) {
                 for (uint32_t u = half; u < units; u += 2) {
                     float v[16], up[16];
                     __syncwarp();
@@ -286,32 +313,53 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_half_kernel(const __grid_c
                     tmem_load_wait(v, up);
 #pragma unroll
                     for (int j = 0; j < 16; ++j) v[j] = v[j] / (1.f + expf(-v[j])) * up[j];
+                    const uint32_t tok = t.tok0 + u * 16;
                     if (p.packed_out) {
-                        // The warp's 32 rows are one block of 32 columns of the consuming product, its 16
-                        // tokens two groups of 8. The values turn through shared memory into 16-byte
-                        // core-matrix rows (17 rows of 16 bytes per core matrix keep both sides free of
-                        // bank conflicts); a lane stores two, 8 lanes to a 128-byte line.
-                        if (row0 + quarter * 32 < rows) {
-                            __half* turn = reinterpret_cast<__half*>(turns + ew * kTurnBytes);
-                            const uint32_t core = (lane & 15) >> 2, e = lane & 3;
-                            const uint32_t at = (lane >> 4) * 4 + (e & 1) * 2 + (e >> 1);
-#pragma unroll
-                            for (int j = 0; j < 16; ++j) turn[(core * 17 + j) * 8 + at] = __float2half_rn(v[j]);
+                        if (row0 + block * 32 < rows) {
+                            put_group(v, turns + ew * kTurnBytes, p, row0, block, tok, lane);
                             __syncwarp();
-                            const uint32_t tr = lane & 7, mm = lane >> 3;
-                            const uint32_t chunk = (row0 >> 6) + (quarter >> 1), jj = (quarter & 1) * 4 + mm;
-#pragma unroll
-                            for (uint32_t it = 0; it < 2; ++it) {
-                                const uint4 row16 = *reinterpret_cast<const uint4*>(turn + (mm * 17 + it * 8 + tr) * 8);
-                                const uint32_t tg = ((t.tok0 + u * 16) >> 3) + it;
-                                reinterpret_cast<uint4*>(p.packed_out)[(((uint64_t)chunk * p.token_groups + tg) * kCores + jj) * 8 + tr] = row16;
-                            }
+                            put_group(v + 8, turns + ew * kTurnBytes, p, row0, block, tok + 8, lane);
                         }
                     } else if (out_row < rows) {
-                        float* to = out + (uint64_t)(t.tok0 + u * 16) * stride + out_row;
+                        float* to = out + (uint64_t)tok * stride + out_row;
 #pragma unroll
                         for (int j = 0; j < 16; ++j, to += stride)
-                            if (t.tok0 + u * 16 + j < p.n_tokens) *to = v[j];
+                            if (tok + j < p.n_tokens) *to = v[j];
+                    }
+                }
+            } else {
+                // Lanes 0 to 63 of the accumulator are rows of gate, the other 64 the same rows of up. Of 16 tokens the warp
+                // that reads the gates takes the first 8 and the warp that reads the same rows of up the others; they
+                // swap what the other one needs. Two buffers in turn: whoever is at the next barrier has read this one.
+                const bool has_gate = quarter < 2;
+                const uint32_t pair = half * 2 + (quarter & 1);
+                float* swap = reinterpret_cast<float*>(turns + kEpilogueWarps * kTurnBytes + pair * kSwapBytes);
+                for (uint32_t u = half; u < units; u += 2) {
+                    float v[16];
+                    __syncwarp();
+                    tmem_load_16(from + u * 16, v);
+                    float* buffer = swap + ((u >> 1) & 1) * (2 * 8 * 32);
+                    float mine[8], other[8];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        mine[j] = has_gate ? v[j] : v[8 + j];
+                        buffer[(has_gate ? 8 + j : j) * 32 + lane] = has_gate ? v[8 + j] : v[j];
+                    }
+                    asm volatile("bar.sync %0, 64;" ::"r"(1 + pair) : "memory");
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        other[j] = buffer[(has_gate ? j : 8 + j) * 32 + lane];
+                        const float g = has_gate ? mine[j] : other[j], up = has_gate ? other[j] : mine[j];
+                        mine[j] = g / (1.f + expf(-g)) * up;
+                    }
+                    const uint32_t tok = t.tok0 + u * 16 + (has_gate ? 0 : 8);
+                    if (p.packed_out) {
+                        if (row0 + block * 32 < rows) put_group(mine, turns + ew * kTurnBytes, p, row0, block, tok, lane);
+                    } else if (out_row < rows) {
+                        float* to = out + (uint64_t)tok * stride + out_row;
+#pragma unroll
+                        for (int j = 0; j < 8; ++j, to += stride)
+                            if (tok + j < p.n_tokens) *to = mine[j];
                     }
                 }
             }
@@ -353,31 +401,35 @@ __global__ void expand_tiles_kernel(const uint4* __restrict__ quants, const __ha
 
 struct Tiling {
     uint32_t tile_tokens, split;
+    int kind;
 };
 
 // The tiling with the smallest modelled time, in us, fitted to 33 to 512 tokens of matrices of 2048 to 10752 rows and columns:
 // waves of tiles over the SMs, each chunk of 64 columns bound by the MMA (2 cycles per token and matrix at 1.4 GHz),
 // by the SM's share of L2 or by the ring's round trip; a start and a last epilogue that nothing hides; a split's partial
 // products, written and read once; never less than the weights' time from HBM.
-Tiling choose_tiling(uint32_t row_tiles, uint32_t n_chunks, uint32_t n_tokens, int dual, bool may_split) {
-    const uint32_t sms = (uint32_t)sm_count(), widest = dual == 2 ? 128 : 256;
-    Tiling best{widest, 1};
+Tiling choose_tiling(uint32_t rows, uint32_t n_chunks, uint32_t n_tokens, bool dual, bool may_split) {
+    const uint32_t sms = (uint32_t)sm_count();
+    Tiling best{};
     double best_us = 1e30;
-    const uint32_t fewest = (n_tokens + widest - 1) / widest;
-    for (uint32_t token_tiles = fewest; token_tiles <= fewest + 6; ++token_tiles) {
-        const uint32_t width = ((n_tokens + token_tiles - 1) / token_tiles + 15u) & ~15u;
-        if (width < 48 && token_tiles > fewest) break;
-        const uint32_t needed = (n_tokens + width - 1) / width;
-        const double mma = 2.0 * width * dual / 1400.0, load = (16384.0 * dual + 128.0 * width) / (dual == 2 ? 105e3 : 125e3);
-        const double chunk = mma > load ? (mma > 0.25 ? mma : 0.25) : (load > 0.25 ? load : 0.25);
-        for (uint32_t split = 1; split <= (may_split && dual == 1 ? kMaxSplit : 1u); ++split) {
-            if (split > 1 && n_chunks / split < 4) break;
-            const uint32_t tiles = row_tiles * needed * split, waves = (tiles + sms - 1) / sms;
-            double us = waves * ((n_chunks + split - 1) / split) * chunk;
-            const double hbm = (double)row_tiles * dual * n_chunks * kATile / 6.2e6;
-            us = (us > hbm ? us : hbm) + 2.8 + 0.0095 * width * dual;
-            if (split > 1) us += 1.0 + (double)split * n_tokens * row_tiles * kRows * 4 / 8e6;
-            if (us < best_us) best_us = us, best = Tiling{width, split};
+    for (int kind = dual ? kWhole : kPlain; kind <= (dual ? kHalves : kPlain); ++kind) {
+        const uint32_t row_tiles = kind == kHalves ? (rows + kRows / 2 - 1) / (kRows / 2) : (rows + kRows - 1) / kRows;
+        const uint32_t widest = kind == kWhole ? 128 : 256, fewest = (n_tokens + widest - 1) / widest;
+        for (uint32_t token_tiles = fewest; token_tiles <= fewest + 6; ++token_tiles) {
+            const uint32_t width = ((n_tokens + token_tiles - 1) / token_tiles + 15u) & ~15u;
+            if (width < 48 && token_tiles > fewest) break;
+            const uint32_t needed = (n_tokens + width - 1) / width;
+            const double mma = 2.0 * width * (kind == kWhole ? 2 : 1) / 1400.0, load = (a_bytes(kind) + 128.0 * width) / (kind == kPlain ? 125e3 : kind == kHalves ? 115e3 : 105e3);
+            const double trip = kind == kHalves ? 0.285 : 0.25, bound = mma > load ? mma : load, chunk = bound > trip ? bound : trip;
+            for (uint32_t split = 1; split <= (may_split && !dual ? kMaxSplit : 1u); ++split) {
+                if (split > 1 && n_chunks / split < 4) break;
+                const uint32_t tiles = row_tiles * needed * split, waves = (tiles + sms - 1) / sms;
+                double us = waves * ((n_chunks + split - 1) / split) * chunk;
+                const double hbm = (double)row_tiles * n_chunks * a_bytes(kind) / 6.2e6;
+                us = (us > hbm ? us : hbm) + 2.8 + 0.0095 * width * (dual ? 2 : 1) + (kind == kWhole ? 2.0 : 0.0);
+                if (split > 1) us += 1.0 + (double)split * n_tokens * rows * 4 / 8e6;
+                if (us < best_us) best_us = us, best = Tiling{width, split, kind};
+            }
         }
     }
     return best;
@@ -391,19 +443,29 @@ bool half_disabled() {
     return off;
 }
 
-template <int DUAL>
+template <int KIND>
+cudaError_t launch_kind(cudaStream_t stream, HalfParams& p) {
+    p.stage_bytes = a_bytes(KIND) + p.tile_tokens * kChunkK * 2;
+    p.stages = kRingBytes / p.stage_bytes < kMaxStages ? kRingBytes / p.stage_bytes : kMaxStages;
+    const void* kernel = (const void*)matmul_half_kernel<KIND>;
+    cudaError_t e = ensure_dynamic_smem(kernel, kSmemBytes);
+    if (e != cudaSuccess) return e;
+    const uint32_t sms = (uint32_t)sm_count();
+    void* args[] = {&p};
+    return launch_kernel(kernel, dim3(p.n_tiles < sms ? p.n_tiles : sms), dim3(kThreads), kSmemBytes, stream, args);
+}
+
 cudaError_t launch_half(cudaStream_t stream, HalfParams& p, Tiling tiling) {
     p.tile_tokens = tiling.tile_tokens;
     p.token_tiles = (p.n_tokens + tiling.tile_tokens - 1) / tiling.tile_tokens;
     p.split = tiling.split;
     p.n_tiles = p.first_tile[p.n_matrices] * p.split * p.token_tiles;
     if (p.n_tiles == 0) return cudaSuccess;
-    const void* kernel = (const void*)matmul_half_kernel<DUAL>;
-    cudaError_t e = ensure_dynamic_smem(kernel, kSmemBytes);
-    if (e != cudaSuccess) return e;
-    const uint32_t sms = (uint32_t)sm_count();
-    void* args[] = {&p};
-    return launch_kernel(kernel, dim3(p.n_tiles < sms ? p.n_tiles : sms), dim3(kThreads), kSmemBytes, stream, args);
+    switch (tiling.kind) {
+        case kPlain: return launch_kind<kPlain>(stream, p);
+        case kWhole: return launch_kind<kWhole>(stream, p);
+        default: return launch_kind<kHalves>(stream, p);
+    }
 }
 
 uint32_t row_tiles_of(const Mat& w) { return (w.n_rows + kRows - 1) / kRows; }
@@ -440,7 +502,7 @@ cudaError_t expand_half_tiles(cudaStream_t stream, const void* quants, const __h
 bool matmul_half_supported(const Mat& w, uint32_t n_tokens) { return w.half_tiles != nullptr && n_tokens >= kMinHalfTokens && !half_disabled(); }
 
 uint32_t matmul_half_split(const Mat& w, uint32_t n_tokens) {
-    return choose_tiling(row_tiles_of(w), w.n_cols / kChunkK, n_tokens, 1, w.n_rows % 4 == 0).split;
+    return choose_tiling(w.n_rows, w.n_cols / kChunkK, n_tokens, false, w.n_rows % 4 == 0).split;
 }
 
 cudaError_t matmul_half(cudaStream_t stream, const Mat* const* ws, float* const* ys, int n, const void* packed, uint32_t n_tokens, uint32_t y_stride,
@@ -457,9 +519,9 @@ cudaError_t matmul_half(cudaStream_t stream, const Mat* const* ws, float* const*
         p.stride[i] = n == 1 ? y_stride : ws[i]->n_rows;
         p.first_tile[i + 1] = p.first_tile[i] + row_tiles_of(*ws[i]);
     }
-    Tiling tiling = choose_tiling(p.first_tile[n], p.n_chunks, n_tokens, 1, split > 1);
+    Tiling tiling = choose_tiling(n == 1 ? ws[0]->n_rows : p.first_tile[n] * kRows, p.n_chunks, n_tokens, false, split > 1);
     if (split > 1 && tiling.split != split) return cudaErrorInvalidValue;  // the caller sized the partial products by matmul_half_split
-    return launch_half<1>(stream, p, tiling);
+    return launch_half(stream, p, tiling);
 }
 
 cudaError_t matmul_half_swiglu(cudaStream_t stream, const Mat& gate, const Mat& up, const void* packed, float* y, uint32_t n_tokens, uint32_t y_stride,
@@ -474,9 +536,10 @@ cudaError_t matmul_half_swiglu(cudaStream_t stream, const Mat& gate, const Mat& 
     p.y[0] = y;
     p.rows[0] = gate.n_rows;
     p.stride[0] = y_stride;
-    p.first_tile[1] = row_tiles_of(gate);
+    const Tiling tiling = choose_tiling(gate.n_rows, p.n_chunks, n_tokens, true, false);
+    p.first_tile[1] = tiling.kind == kHalves ? (gate.n_rows + kRows / 2 - 1) / (kRows / 2) : row_tiles_of(gate);
     p.packed_out = static_cast<__half*>(packed_out);
-    return launch_half<2>(stream, p, choose_tiling(p.first_tile[1], p.n_chunks, n_tokens, 2, false));
+    return launch_half(stream, p, tiling);
 }
 
 }  // namespace k
