@@ -162,11 +162,12 @@ __global__ void __launch_bounds__(256) pack_kernel(const float* __restrict__ x, 
 // in flight together, into shared memory, from where the first warp sums the squares (one warp, so that the order of
 // the sum is that of a warp per row) and all write their part of the operand. The forms before it (8 tokens per CTA with 4 or
 // 8 CTAs repeating the sums; 4 tokens per CTA with the partial sums) read rows twice: 512 tokens of 4096 took 13.0 us
-// plain and 19.0 us with four partial sums, now 8.2 and 10.7; 64 tokens of 2048 with a reduce_kernel before it 7.0, now 6.1.
+// plain and 19.0 us with four partial sums, now 8.2 and 10.7; 64 tokens of 2048 with a reduce_kernel before it 7.0, now 4.9.
 template <bool ADD>
 __global__ void __launch_bounds__(256) pack_norm_kernel(float* __restrict__ x, const float* __restrict__ weight, float eps, __half* __restrict__ packed,
                                                         uint32_t n_tokens, uint32_t n_cols, uint32_t token_groups, const float* __restrict__ partial,
                                                         uint32_t split) {
+    constexpr uint32_t kMostParts = 8;
     extern __shared__ float4 norm_row[];
     __shared__ float shared_scale;
     pdl_launch_dependents();
@@ -181,14 +182,20 @@ __global__ void __launch_bounds__(256) pack_norm_kernel(float* __restrict__ x, c
     float4* row = reinterpret_cast<float4*>(x) + (uint64_t)token * quads;
     const float4* part = reinterpret_cast<const float4*>(partial) + (uint64_t)token * quads;
     const uint64_t total = (uint64_t)n_tokens * quads;
-#pragma unroll 4
+#pragma unroll ADD ? 1 : 4
     for (uint32_t i = tid; i < quads; i += 256) {
         float4 v = __ldcg(row + i);
         if (ADD) {
             float4 sum = __ldcg(part + i);
-            for (uint32_t sp = 1; sp < split; ++sp) {
-                const float4 o = __ldcg(part + sp * total + i);
-                sum.x += o.x; sum.y += o.y; sum.z += o.z; sum.w += o.w;
+            float4 o[kMostParts - 1];  // all of them on their way before the first is added
+#pragma unroll
+            for (uint32_t sp = 1; sp < kMostParts; ++sp) o[sp - 1] = sp < split ? __ldcg(part + sp * total + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (uint32_t sp = 1; sp < kMostParts; ++sp)
+                if (sp < split) sum.x += o[sp - 1].x, sum.y += o[sp - 1].y, sum.z += o[sp - 1].z, sum.w += o[sp - 1].w;
+            for (uint32_t sp = kMostParts; sp < split; ++sp) {
+                const float4 more = __ldcg(part + sp * total + i);
+                sum.x += more.x; sum.y += more.y; sum.z += more.z; sum.w += more.w;
             }
             v.x += sum.x; v.y += sum.y; v.z += sum.z; v.w += sum.w;
             row[i] = v;

@@ -32,75 +32,181 @@ struct RouteParams {
     const float* router;       // [n_experts][n_cols] f32
     const float* bias;
     uint32_t* route;
-    uint32_t n_cols, n_experts, n_used;
+    uint32_t n_cols, n_experts, n_used, n_tokens;
 };
 
 constexpr int kRouteThreads = 1024;
 constexpr int kRouteWarps = kRouteThreads / 32;
+constexpr uint32_t kRouteCluster = 8;  // CTAs that share a token when there are few
+constexpr int kRouteTokens = 2, kRouteExperts = 4;  // with many tokens: tokens of a CTA, experts of a warp
 
-// One CTA per token, a warp per expert. The token's norm and the router's dot products accumulate
-// in f64, as the scalar reference does (scalar.rs:240-249, :292-304), so the scores - and with them
-// the picked expert ids - do not depend on the order a parallel sum happens to take. Each lane
-// keeps four independent sums so the f64 adds do not wait on one another.
-__global__ void __launch_bounds__(kRouteThreads) moe_route_kernel(RouteParams p) {
-    extern __shared__ float xs[];  // the normalised token
-    __shared__ double reduce[kRouteWarps];
-    __shared__ float scores[kMaxExperts];
+// The token's norm and the router's dot products accumulate in f64, as the scalar reference does (scalar.rs:240-249,
+// :292-304), so the scores - and with them the picked expert ids - do not depend on the order a parallel sum happens to
+// take.
+//
+// Bound by f64 arithmetic (measured: about six operations per cycle and SM) when tokens are many, by one SM's share of it and of
+// L2 when they are few: a CTA per token took 11 us for one token and 20.5 for 256 (32 experts of 2048). Few tokens: a
+// cluster of eight CTAs shares a token's experts, several warps to an expert, the weights on their way before the wait
+// for the preceding launch; the scores meet in the first CTA, which picks: 7.5 us. Many: TOKENS of them to a CTA and
+// EXPERTS experts to a warp, so that a weight is converted and an input read from shared memory once for several products:
+// 18.7 us (one expert and four tokens to a warp: 38).
+template <int TOKENS, int EXPERTS, typename X>
+__global__ void __launch_bounds__(kRouteThreads) moe_route_kernel(const __grid_constant__ RouteParams p, uint32_t ranks, uint32_t warps_per_expert) {
+    constexpr int kHeld = EXPERTS > 1 ? 1 : 2;  // 16-byte loads in flight per lane and expert
+    extern __shared__ __align__(16) uint8_t route_smem[];
+    X* xs = reinterpret_cast<X*>(route_smem);  // [TOKENS][n_cols], normalised
+    __shared__ double reduce[EXPERTS * TOKENS][kRouteWarps];
+    __shared__ float scores[TOKENS][kMaxExperts];
     pdl_launch_dependents();
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n_cols = p.n_cols;
+    const uint32_t rank = blockIdx.x % ranks, token0 = blockIdx.x / ranks * TOKENS, here = min((uint32_t)TOKENS, p.n_tokens - token0);
+    const uint32_t groups = kRouteWarps / warps_per_expert, group = warp / warps_per_expert, member = warp % warps_per_expert;
+    const bool wide = (n_cols & 3u) == 0 && (reinterpret_cast<uintptr_t>(p.router) & 15u) == 0;
+    // A warp's share of a row: quads member * 32 + lane, then every warps_per_expert * 32.
+    const uint32_t quads = n_cols / 4, stride = warps_per_expert * 32, first = member * 32 + lane;
+    float4 held[EXPERTS][kHeld];
+    auto load = [&](uint32_t local, uint32_t at) {
+#pragma unroll
+        for (int m = 0; m < EXPERTS; ++m) {
+            const uint32_t e = rank + ranks * (local + m);
+            const float4* row = reinterpret_cast<const float4*>(p.router + (uint64_t)e * n_cols);
+#pragma unroll
+            for (int k = 0; k < kHeld; ++k) held[m][k] = e < p.n_experts && at + k * stride < quads ? __ldg(row + at + k * stride) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    };
+    if (wide) load(EXPERTS * group, first);
+    if (ranks > 1) asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");  // this CTA runs: its shared memory may be written
     pdl_wait();
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint32_t token = blockIdx.x, n_cols = p.n_cols;
-    const float* x = p.x + (uint64_t)token * n_cols;
+
     if (p.norm_weight) {
-        double sumsq = 0.0;
-        for (uint32_t c = tid; c < n_cols; c += kRouteThreads) sumsq += (double)x[c] * (double)x[c];
-        sumsq = warp_sum_f64(sumsq);
-        if (lane == 0) reduce[warp] = sumsq;
+#pragma unroll
+        for (int t = 0; t < TOKENS; ++t) {
+            double sumsq = 0.0;
+            if ((uint32_t)t < here) {
+                const float* x = p.x + (uint64_t)(token0 + t) * n_cols;
+                for (uint32_t c = tid; c < n_cols; c += kRouteThreads) sumsq += (double)x[c] * (double)x[c];
+            }
+            sumsq = warp_sum_f64(sumsq);
+            if (lane == 0) reduce[t][warp] = sumsq;
+        }
         __syncthreads();
-        double total = 0.0;
-        for (int w = 0; w < kRouteWarps; ++w) total += reduce[w];
-        float scale = (float)(1.0 / sqrt(total / (double)n_cols + (double)p.eps));
-        float* normed = p.normed + (uint64_t)token * n_cols;
+    }
+#pragma unroll
+    for (int t = 0; t < TOKENS; ++t) {
+        if ((uint32_t)t >= here) {
+            for (uint32_t c = tid; c < n_cols; c += kRouteThreads) xs[t * n_cols + c] = (X)0;
+            continue;
+        }
+        const float* x = p.x + (uint64_t)(token0 + t) * n_cols;
+        if (!p.norm_weight) {
+            for (uint32_t c = tid; c < n_cols; c += kRouteThreads) xs[t * n_cols + c] = (X)x[c];
+            continue;
+        }
+        const double total = warp_sum_f64(reduce[t][lane]);
+        const float scale = (float)(1.0 / sqrt(total / (double)n_cols + (double)p.eps));
+        float* normed = p.normed + (uint64_t)(token0 + t) * n_cols;
         for (uint32_t c = tid; c < n_cols; c += kRouteThreads) {
-            float v = p.norm_weight[c] * (x[c] * scale);
-            xs[c] = v;
-            normed[c] = v;
+            const float v = p.norm_weight[c] * (x[c] * scale);
+            xs[t * n_cols + c] = (X)v;
+            if (rank == 0) normed[c] = v;
         }
+    }
+    __syncthreads();
+
+    if (ranks > 1) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    // Every warp takes part in every pass (the sums of a pass meet at a barrier).
+    const uint32_t mine_count = (p.n_experts + ranks - 1 - rank) / ranks, passes = (mine_count + groups * EXPERTS - 1) / (groups * EXPERTS);
+    for (uint32_t pass = 0; pass < passes; ++pass) {
+        const uint32_t local = (pass * groups + group) * EXPERTS;
+        double sum[EXPERTS][TOKENS];
+#pragma unroll
+        for (int m = 0; m < EXPERTS; ++m)
+#pragma unroll
+            for (int t = 0; t < TOKENS; ++t) sum[m][t] = 0.0;
+        if (wide) {
+            if (pass > 0) load(local, first);
+            for (uint32_t at = first; at < quads;) {
+                float4 w[EXPERTS][kHeld];
+#pragma unroll
+                for (int m = 0; m < EXPERTS; ++m)
+#pragma unroll
+                    for (int k = 0; k < kHeld; ++k) w[m][k] = held[m][k];
+                const uint32_t now = at;
+                at += kHeld * stride;
+                if (at < quads) load(local, at);
+#pragma unroll
+                for (int k = 0; k < kHeld; ++k) {
+                    const uint32_t quad = now + k * stride;
+                    if (quad >= quads) break;
+                    double v[TOKENS][4];
+#pragma unroll
+                    for (int t = 0; t < TOKENS; ++t)
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) v[t][i] = (double)xs[t * n_cols + quad * 4 + i];
+#pragma unroll
+                    for (int m = 0; m < EXPERTS; ++m) {
+                        const double w0 = w[m][k].x, w1 = w[m][k].y, w2 = w[m][k].z, w3 = w[m][k].w;
+#pragma unroll
+                        for (int t = 0; t < TOKENS; ++t) sum[m][t] += (w0 * v[t][0] + w1 * v[t][1]) + (w2 * v[t][2] + w3 * v[t][3]);
+                    }
+                }
+            }
+        } else {
+#pragma unroll
+            for (int m = 0; m < EXPERTS; ++m) {
+                const uint32_t e = rank + ranks * (local + m);
+                if (e >= p.n_experts) break;
+                for (uint32_t c = first; c < n_cols; c += stride) {
+                    const double w = p.router[(uint64_t)e * n_cols + c];
+#pragma unroll
+                    for (int t = 0; t < TOKENS; ++t) sum[m][t] += w * (double)xs[t * n_cols + c];
+                }
+            }
+        }
+#pragma unroll
+        for (int m = 0; m < EXPERTS; ++m)
+#pragma unroll
+            for (int t = 0; t < TOKENS; ++t) sum[m][t] = warp_sum_f64(sum[m][t]);
+        if (warps_per_expert > 1) {
+            __syncthreads();  // the sums of the pass before are read
+            if (lane == 0) {
+#pragma unroll
+                for (int m = 0; m < EXPERTS; ++m)
+#pragma unroll
+                    for (int t = 0; t < TOKENS; ++t) reduce[m * TOKENS + t][warp] = sum[m][t];
+            }
+            __syncthreads();
+        }
+        if (member != 0 || lane != 0) continue;
+#pragma unroll
+        for (int m = 0; m < EXPERTS; ++m) {
+            const uint32_t e = rank + ranks * (local + m);
+            if (e >= p.n_experts) break;
+#pragma unroll
+            for (int t = 0; t < TOKENS; ++t) {
+                double total = warps_per_expert > 1 ? 0.0 : sum[m][t];
+                if (warps_per_expert > 1)
+                    for (uint32_t w = 0; w < warps_per_expert; ++w) total += reduce[m * TOKENS + t][warp + w];
+                const float score = 1.0f / (1.0f + expf(-(float)total));
+                if (rank == 0) {
+                    scores[t][e] = score;
+                } else {
+                    uint32_t at;
+                    asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(at) : "r"((uint32_t)__cvta_generic_to_shared(&scores[t][e])));
+                    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(at), "f"(score) : "memory");
+                }
+            }
+        }
+    }
+    if (ranks > 1) {
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+        if (rank != 0) return;
     } else {
-        for (uint32_t c = tid; c < n_cols; c += kRouteThreads) xs[c] = x[c];
+        __syncthreads();
     }
-    __syncthreads();
-    for (uint32_t e = warp; e < p.n_experts; e += kRouteWarps) {
-        const float* row = p.router + (uint64_t)e * n_cols;
-        double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-        uint32_t c = 0;
-        if ((n_cols & 3u) == 0 && (reinterpret_cast<uintptr_t>(row) & 15u) == 0) {
-            // Four 16-byte loads in flight per lane and trip, so a row costs a few round trips to L2, not one per element.
-            const float4* row4 = reinterpret_cast<const float4*>(row);
-            const float4* x4 = reinterpret_cast<const float4*>(xs);
-            const uint32_t n4 = n_cols / 4;
-            uint32_t i = lane;
-            for (; i + 96 < n4; i += 128) {
-                const float4 a = __ldg(row4 + i), b = __ldg(row4 + i + 32), cc = __ldg(row4 + i + 64), d = __ldg(row4 + i + 96);
-                const float4 xa = x4[i], xb = x4[i + 32], xc = x4[i + 64], xd = x4[i + 96];
-                s0 += (double)a.x * xa.x + (double)a.y * xa.y + (double)a.z * xa.z + (double)a.w * xa.w;
-                s1 += (double)b.x * xb.x + (double)b.y * xb.y + (double)b.z * xb.z + (double)b.w * xb.w;
-                s2 += (double)cc.x * xc.x + (double)cc.y * xc.y + (double)cc.z * xc.z + (double)cc.w * xc.w;
-                s3 += (double)d.x * xd.x + (double)d.y * xd.y + (double)d.z * xd.z + (double)d.w * xd.w;
-            }
-            for (; i < n4; i += 32) {
-                const float4 a = __ldg(row4 + i);
-                const float4 xa = x4[i];
-                s0 += (double)a.x * xa.x + (double)a.y * xa.y + (double)a.z * xa.z + (double)a.w * xa.w;
-            }
-            c = n_cols;
-        }
-        for (c += lane; c < n_cols; c += 32) s0 += (double)row[c] * (double)xs[c];
-        double sum = warp_sum_f64((s0 + s1) + (s2 + s3));
-        if (lane == 0) scores[e] = 1.0f / (1.0f + expf(-(float)sum));
-    }
-    __syncthreads();
-    if (warp == 0) {
+    if (warp < here) {
+        const float* mine = scores[warp];
         // Top n_used by repeated argmax of score + bias, ties to the lower id; the weights are the
         // unbiased scores over their f32 sum plus 1e-6 (lfm2.rs:698-708). Lane l looks after experts
         // l, l + 32, l + 64, l + 96; a round is a lane-local scan and a warp-wide compare.
@@ -109,7 +215,7 @@ __global__ void __launch_bounds__(kRouteThreads) moe_route_kernel(RouteParams p)
 #pragma unroll
         for (int k = 0; k < kMaxExperts / 32; ++k) {
             const uint32_t e = lane + 32 * k;
-            value[k] = e < p.n_experts ? scores[e] + p.bias[e] : 0.f;
+            value[k] = e < p.n_experts ? mine[e] + p.bias[e] : 0.f;
             taken[k] = e >= p.n_experts;
         }
         uint32_t picked = 0;   // lane i < n_used ends up holding the i-th pick
@@ -136,7 +242,7 @@ __global__ void __launch_bounds__(kRouteThreads) moe_route_kernel(RouteParams p)
 #pragma unroll
             for (int k = 0; k < kMaxExperts / 32; ++k)
                 if (best == lane + 32 * k) taken[k] = true;
-            const float score = scores[best];
+            const float score = mine[best];
             sum += score;  // in pick order, as the scalar code adds them
             if (lane == i) {
                 picked = best;
@@ -144,7 +250,7 @@ __global__ void __launch_bounds__(kRouteThreads) moe_route_kernel(RouteParams p)
             }
         }
         const float norm = sum + 1e-6f;
-        uint32_t* route = p.route + (uint64_t)token * 2 * p.n_used;
+        uint32_t* route = p.route + (uint64_t)(token0 + warp) * 2 * p.n_used;
         if (lane < p.n_used) {
             route[lane] = picked;
             route[p.n_used + lane] = __float_as_uint(picked_score / norm);
@@ -386,12 +492,43 @@ cudaError_t launch_experts(Kernel kernel, dim3 grid, size_t smem, cudaStream_t s
 cudaError_t moe_route(cudaStream_t stream, const float* x, Norm norm, float* normed, const float* router, const float* bias,
                       uint32_t* route, uint32_t n_cols, uint32_t n_experts, uint32_t n_used, uint32_t n_tokens) {
     if (n_tokens == 0) return cudaSuccess;
-    RouteParams p{x, norm.weight, norm.eps, normed, router, bias, route, n_cols, n_experts, n_used};
-    size_t smem = (size_t)n_cols * 4;
-    cudaError_t e = ensure_dynamic_smem((const void*)moe_route_kernel, smem);
-    if (e != cudaSuccess) return e;
-    void* args[] = {&p};
-    return launch_kernel((const void*)moe_route_kernel, dim3(n_tokens), dim3(kRouteThreads), smem, stream, args);
+    const RouteParams p{x, norm.weight, norm.eps, normed, router, bias, route, n_cols, n_experts, n_used, n_tokens};
+    // A cluster per token until they fill the device; rows too wide for f64 in shared memory stay f32 there.
+    const bool few = n_tokens * kRouteCluster <= (uint32_t)sm_count();
+    const bool wide = (size_t)n_cols * 8 * (few ? 1 : kRouteTokens) <= 200 * 1024;
+    const uint32_t ranks = few ? kRouteCluster : 1, tokens = few || !wide ? 1 : kRouteTokens;
+    uint32_t per = 1;  // warps per expert, or per group of them
+    const uint32_t units = (n_experts + ranks - 1) / ranks, groups = tokens > 1 ? (units + kRouteExperts - 1) / kRouteExperts : units;
+    while (per < (uint32_t)kRouteWarps && per * 2 * groups <= (uint32_t)kRouteWarps) per *= 2;
+    const bool f64 = (size_t)n_cols * 8 * tokens <= 200 * 1024;
+    const size_t smem = (size_t)n_cols * (f64 ? 8 : 4) * tokens;
+    auto launch = [&](auto kernel) {
+        cudaError_t e = ensure_dynamic_smem((const void*)kernel, smem);
+        if (e != cudaSuccess) return e;
+        cudaLaunchConfig_t config = {};
+        config.gridDim = dim3(ranks * ((n_tokens + tokens - 1) / tokens));
+        config.blockDim = dim3(kRouteThreads);
+        config.dynamicSmemBytes = smem;
+        config.stream = stream;
+        cudaLaunchAttribute attributes[2];
+        int n = 0;
+        if (ranks > 1) {
+            attributes[n].id = cudaLaunchAttributeClusterDimension;
+            attributes[n].val.clusterDim.x = ranks;
+            attributes[n].val.clusterDim.y = attributes[n].val.clusterDim.z = 1;
+            ++n;
+        }
+        if (pdl_enabled()) {
+            attributes[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            attributes[n].val.programmaticStreamSerializationAllowed = 1;
+            ++n;
+        }
+        config.attrs = attributes;
+        config.numAttrs = n;
+        return cudaLaunchKernelEx(&config, kernel, p, ranks, per);
+    };
+    if (tokens > 1) return launch(moe_route_kernel<kRouteTokens, kRouteExperts, double>);
+    return f64 ? launch(moe_route_kernel<1, 1, double>) : launch(moe_route_kernel<1, 1, float>);
 }
 
 cudaError_t moe_group(cudaStream_t stream, const uint32_t* route, uint32_t* offsets, uint32_t* entries, uint32_t n_experts,
