@@ -359,57 +359,95 @@ struct StepParams {
     float eps;
 };
 
-// The convolution of one channel for one token, and the history shift (same order of additions as gdn_conv).
-__device__ __forceinline__ float conv_step(const StepParams& p, uint32_t channel) {
+constexpr int kStepParts = 4;   // threads that share a state column, each holding a quarter of its rows, when a CTA serves a key head
+constexpr uint32_t kStepRanks = 4;  // CTAs that share a key head where its columns allow it
+
+// The convolution of one channel for one token (same order of additions as gdn_conv) and the shifted history, which the
+// caller stores when nobody reads the old one any more.
+struct ConvStep {
+    float value, next[7];
+};
+__device__ __forceinline__ ConvStep conv_step(const StepParams& p, uint32_t channel) {
     const uint32_t H = p.kernel - 1;
     const float* tap = p.taps + (uint64_t)channel * p.kernel;
-    float* hist = p.history + (uint64_t)channel * H;
+    const float* hist = p.history + (uint64_t)channel * H;
     const float input = p.qkv[channel];
-    float sum = tap[H] * input;
-    float past[7];
-    for (uint32_t i = 0; i < H; ++i) {
-        past[i] = hist[i];
-        sum += tap[i] * past[i];
+    float past[7], taps[8];
+#pragma unroll
+    for (uint32_t i = 0; i < 7; ++i) {
+        past[i] = i < H ? hist[i] : 0.f;
+        taps[i] = i < H ? tap[i] : 0.f;
     }
-    for (uint32_t i = 0; i + 1 < H; ++i) hist[i] = past[i + 1];
-    hist[H - 1] = input;
-    return sum / (1.f + expf(-sum));
+    float sum = tap[H] * input;
+    ConvStep c;
+#pragma unroll
+    for (uint32_t i = 0; i < 7; ++i) {
+        if (i < H) sum += taps[i] * past[i];
+        c.next[i] = i + 1 < H && i < 6 ? past[i < 6 ? i + 1 : 6] : input;
+    }
+    c.value = sum / (1.f + expf(-sum));
+    return c;
+}
+__device__ __forceinline__ void keep_history(const StepParams& p, uint32_t channel, const ConvStep& c) {
+    const uint32_t H = p.kernel - 1;
+    float* hist = p.history + (uint64_t)channel * H;
+#pragma unroll
+    for (uint32_t i = 0; i < 7; ++i)
+        if (i < H) hist[i] = c.next[i];
 }
 
-constexpr int kStepParts = 4;  // threads that share a state column, each holding a quarter of its rows
-
-template <int KDIM>
-__global__ void __launch_bounds__(1024) gdn_step_kernel(StepParams p) {
-    // Thread (part, m, j): rows [part * KDIM / 4, (part + 1) * KDIM / 4) of column j of the state of
-    // value head key_head + m * n_k_heads. The quarter column is loaded into registers first of
-    // all, so that read overlaps the convolution; the quarters' partial dot products meet in shared memory.
-    constexpr int kRows = KDIM / kStepParts;
+// ROWS rows of a state column to a thread, up to COLUMNS columns to a CTA. `ranks` CTAs (a cluster) share the columns of a key head's value heads: the state
+// is 4 MB of traffic, which one CTA per key head (16 of them) moved in 11.6 us; with four it is on 64 SMs, is asked for
+// in L2 before the wait for the preceding launch, and takes 7.4 us. Every CTA convolves q and k for itself; the first
+// one stores their history when all have read it. A value head's sum of squares meets through distributed shared memory.
+template <int KDIM, int ROWS, int COLUMNS>
+__global__ void __launch_bounds__(1024) gdn_step_kernel(const __grid_constant__ StepParams p, uint32_t ranks) {
+    // Thread (part, column): rows [part * ROWS, (part + 1) * ROWS) of a column of the state of value head
+    // key_head + m * n_k_heads. The rows are loaded into registers first of all, so that read overlaps the convolution;
+    // the parts' partial dot products meet in shared memory.
+    constexpr int kParts = KDIM / ROWS;
     __shared__ __align__(16) float qs[KDIM], ks[KDIM];
     __shared__ float scratch[96];
-    __shared__ float r_part[kStepParts][256], o_part[kStepParts][256], o_full[256];
+    __shared__ float r_part[kParts][COLUMNS], o_part[kParts][COLUMNS], v_full[COLUMNS];
+    __shared__ float head_squares;  // of this CTA's columns, where a value head spans several CTAs
     pdl_launch_dependents();
-    pdl_wait();
-    const uint32_t key_head = blockIdx.x, tid = threadIdx.x, vd = p.v_dim;
+    const uint32_t rank = blockIdx.x % ranks, key_head = blockIdx.x / ranks, tid = threadIdx.x, vd = p.v_dim;
     const uint32_t lane = tid & 31, warp = tid >> 5;
-    const uint32_t key_dim = p.n_k_heads * KDIM, ratio = p.n_v_heads / p.n_k_heads;
-    const uint32_t column_id = tid % (ratio * vd), part = tid / (ratio * vd);  // blockDim.x == kStepParts * ratio * v_dim
-    const uint32_t m = column_id / vd, j = column_id % vd, head = key_head + m * p.n_k_heads;
-    float* column = p.state + (uint64_t)head * KDIM * vd + (uint64_t)(part * kRows) * vd + j;
-    float S[kRows];
+    const uint32_t key_dim = p.n_k_heads * KDIM, columns = p.n_v_heads / p.n_k_heads * vd / ranks;
+    const uint32_t column_id = tid % columns, part = tid / columns;  // blockDim.x == kParts * columns
+    const uint32_t m = (rank * columns + column_id) / vd, j = (rank * columns + column_id) % vd, head = key_head + m * p.n_k_heads;
+    float* column = p.state + (uint64_t)head * KDIM * vd + (uint64_t)(part * ROWS) * vd + j;
+    if (lane == 0) {  // a warp's 32 columns of a row are a line (a hint: what is in flight is still seen)
 #pragma unroll
-    for (int i = 0; i < kRows; ++i) S[i] = column[(uint64_t)i * vd];
-    // q and k of this key head: threads below KDIM convolve one channel of each.
-    float qv = 0.f, kv = 0.f;
-    if (tid < KDIM) {
-        qv = conv_step(p, key_head * KDIM + tid);
-        kv = conv_step(p, key_dim + key_head * KDIM + tid);
+        for (int i = 0; i < ROWS; ++i) asm volatile("prefetch.global.L2 [%0];" ::"l"(column + (uint64_t)i * vd));
     }
+    pdl_wait();
+    float S[ROWS];
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) S[i] = column[(uint64_t)i * vd];
+    // q and k of this key head: threads below KDIM convolve one channel of each. The column's element of v: part 0.
+    ConvStep qc{}, kc{}, vc{};
+    if (tid < KDIM) {
+        qc = conv_step(p, key_head * KDIM + tid);
+        kc = conv_step(p, key_dim + key_head * KDIM + tid);
+    }
+    if (part == 0) {
+        vc = conv_step(p, 2 * key_dim + head * vd + j);
+        keep_history(p, 2 * key_dim + head * vd + j, vc);
+        v_full[column_id] = vc.value;  // where every part can read it
+    }
+    const float qv = qc.value, kv = kc.value;
     // l2_normalize (qwen35.rs:762-768): f32 sum of squares, x *= scale / sqrt(sum + 1e-6).
-    float q2 = warp_sum(qv * qv), k2 = warp_sum(kv * kv);
+    const float q2 = warp_sum(qv * qv), k2 = warp_sum(kv * kv);
     if (lane == 0) {
         scratch[warp] = q2;
         scratch[32 + warp] = k2;
     }
+    // beta = sigmoid(beta); decay = exp(a * softplus(alpha + dt_bias)), softplus(x) = x above 20.
+    const float braw = p.beta[head], araw = p.alpha[head] + p.dt_bias[head];
+    const float beta = 1.f / (1.f + expf(-braw));
+    const float decay = expf(p.a[head] * (araw > 20.f ? araw : log1pf(expf(araw))));
+    const float gate = part == 0 ? p.z[head * vd + j] : 0.f, norm_weight = part == 0 ? p.norm_weight[j] : 0.f;
     __syncthreads();
     if (tid < KDIM) {
         float qsum = 0.f, ksum = 0.f;
@@ -420,19 +458,12 @@ __global__ void __launch_bounds__(1024) gdn_step_kernel(StepParams p) {
         qs[tid] = qv * ((1.0f / sqrtf((float)KDIM)) / sqrtf(qsum + 1e-6f));
         ks[tid] = kv * (1.0f / sqrtf(ksum + 1e-6f));
     }
-    // The column's element of v (convolved once, by the part-0 thread) and the head's gates.
-    float v = 0.f;
-    if (part == 0) v = conv_step(p, 2 * key_dim + head * vd + j);
-    // beta = sigmoid(beta); decay = exp(a * softplus(alpha + dt_bias)), softplus(x) = x above 20.
-    const float braw = p.beta[head], araw = p.alpha[head] + p.dt_bias[head];
-    const float beta = 1.f / (1.f + expf(-braw));
-    const float decay = expf(p.a[head] * (araw > 20.f ? araw : log1pf(expf(araw))));
     __syncthreads();
-    const float4* k4 = reinterpret_cast<const float4*>(ks + part * kRows);
-    const float4* q4 = reinterpret_cast<const float4*>(qs + part * kRows);
+    const float4* k4 = reinterpret_cast<const float4*>(ks + part * ROWS);
+    const float4* q4 = reinterpret_cast<const float4*>(qs + part * ROWS);
     float r0 = 0.f, r1 = 0.f;
 #pragma unroll
-    for (int i = 0; i < kRows / 4; ++i) {
+    for (int i = 0; i < ROWS / 4; ++i) {
         const float4 kk = k4[i];
         S[4 * i] *= decay;
         S[4 * i + 1] *= decay;
@@ -442,15 +473,14 @@ __global__ void __launch_bounds__(1024) gdn_step_kernel(StepParams p) {
         r1 += S[4 * i + 1] * kk.y + S[4 * i + 3] * kk.w;
     }
     r_part[part][column_id] = r0 + r1;
-    if (part == 0) o_full[column_id] = v;  // parks v where every part can read it
     __syncthreads();
     float r = 0.f;
 #pragma unroll
-    for (int q = 0; q < kStepParts; ++q) r += r_part[q][column_id];  // every part adds them in the same order
-    const float delta = (o_full[column_id] - r) * beta;
+    for (int q = 0; q < kParts; ++q) r += r_part[q][column_id];  // every part adds them in the same order
+    const float delta = (v_full[column_id] - r) * beta;
     float o0 = 0.f, o1 = 0.f;
 #pragma unroll
-    for (int i = 0; i < kRows / 4; ++i) {
+    for (int i = 0; i < ROWS / 4; ++i) {
         const float4 kk = k4[i], qq = q4[i];
         S[4 * i] += kk.x * delta;
         S[4 * i + 1] += kk.y * delta;
@@ -459,28 +489,50 @@ __global__ void __launch_bounds__(1024) gdn_step_kernel(StepParams p) {
         o0 += S[4 * i] * qq.x + S[4 * i + 2] * qq.z;
         o1 += S[4 * i + 1] * qq.y + S[4 * i + 3] * qq.w;
     }
-#pragma unroll
-    for (int i = 0; i < kRows; ++i) column[(uint64_t)i * vd] = S[i];
     o_part[part][column_id] = o0 + o1;
     __syncthreads();
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) column[(uint64_t)i * vd] = S[i];
     // Gated RMSNorm over each value head's v_dim outputs, by the part-0 threads (v_dim is a multiple
     // of 32, so a warp belongs to one head): out = weight * (o * scale) * silu(z).
     float o = 0.f;
     if (part == 0) {
 #pragma unroll
-        for (int q = 0; q < kStepParts; ++q) o += o_part[q][column_id];
+        for (int q = 0; q < kParts; ++q) o += o_part[q][column_id];
     }
     const float sq = warp_sum(o * o);
     if (lane == 0) scratch[64 + warp] = sq;
     __syncthreads();
-    if (part == 0) {
-        const uint32_t warps_per_head = vd / 32, first = m * warps_per_head;
-        float sumsq = 0.f;
-        for (uint32_t w = 0; w < warps_per_head; ++w) sumsq += scratch[64 + first + w];
-        const float scale = rsqrtf(sumsq / (float)vd + p.eps);
-        const float g = p.z[head * vd + j];
-        p.out[head * vd + j] = p.norm_weight[j] * (o * scale) * (g / (1.f + expf(-g)));
+    const bool spans = vd > columns;  // a value head's columns lie in vd / columns CTAs
+    float sumsq = 0.f;
+    {
+        const uint32_t warps_here = (spans ? columns : vd) / 32, first = spans ? 0 : (column_id / vd) * warps_here;
+        for (uint32_t w = 0; w < warps_here; ++w) sumsq += scratch[64 + first + w];
     }
+    if (ranks > 1) {
+        if (tid == 0) head_squares = sumsq;
+        asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+        if (spans) {
+            const uint32_t per_head = vd / columns, first = rank / per_head * per_head;
+            sumsq = 0.f;
+            for (uint32_t c = 0; c < per_head; ++c) {
+                uint32_t at;
+                float other;
+                asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"((uint32_t)__cvta_generic_to_shared(&head_squares)), "r"(first + c));
+                asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(other) : "r"(at) : "memory");
+                sumsq += other;
+            }
+        }
+    }
+    if (rank == 0 && tid < KDIM) {  // every CTA of the cluster has read the old history
+        keep_history(p, key_head * KDIM + tid, qc);
+        keep_history(p, key_dim + key_head * KDIM + tid, kc);
+    }
+    if (part == 0) {
+        const float scale = rsqrtf(sumsq / (float)vd + p.eps);
+        p.out[head * vd + j] = norm_weight * (o * scale) * (gate / (1.f + expf(-gate)));
+    }
+    if (ranks > 1) asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");  // its sums may still be read
 }
 
 // out[t][h][d] *= sigmoid(gate) with the gate read from the interleaved q projection:
@@ -563,10 +615,36 @@ cudaError_t gdn_step(cudaStream_t stream, const float* qkv, const float* taps, f
                      const float* a, const float* dt_bias, float* state, const float* z, const float* norm_weight, float* out,
                      uint32_t n_k_heads, uint32_t n_v_heads, uint32_t k_dim, uint32_t v_dim, uint32_t kernel, float eps) {
     StepParams p{qkv, taps, history, beta, alpha, a, dt_bias, state, z, norm_weight, out, n_k_heads, n_v_heads, k_dim, v_dim, kernel, eps};
-    void* args[] = {&p};
-    const uint32_t threads = kStepParts * (n_v_heads / n_k_heads) * v_dim;
-    const void* kernel_fn = k_dim == 32 ? (const void*)gdn_step_kernel<32> : k_dim == 64 ? (const void*)gdn_step_kernel<64>
-                          : k_dim == 96 ? (const void*)gdn_step_kernel<96> : (const void*)gdn_step_kernel<128>;
+    const uint32_t columns = n_v_heads / n_k_heads * v_dim, share = columns / kStepRanks;
+    // Four CTAs to a key head: whole warps of columns, at most 64 of them, and a value head's either in one CTA or over whole ones.
+    if (columns % (32 * kStepRanks) == 0 && share <= 64 && (share % v_dim == 0 || v_dim % share == 0)) {
+        auto launch = [&](auto kernel) {
+            cudaLaunchConfig_t config = {};
+            config.gridDim = dim3(n_k_heads * kStepRanks);
+            config.blockDim = dim3(share * (k_dim / 8));
+            config.stream = stream;
+            cudaLaunchAttribute attributes[2];
+            attributes[0].id = cudaLaunchAttributeClusterDimension;
+            attributes[0].val.clusterDim.x = kStepRanks;
+            attributes[0].val.clusterDim.y = attributes[0].val.clusterDim.z = 1;
+            attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            attributes[1].val.programmaticStreamSerializationAllowed = 1;
+            config.attrs = attributes;
+            config.numAttrs = pdl_enabled() ? 2 : 1;
+            return cudaLaunchKernelEx(&config, kernel, (const StepParams)p, (uint32_t)kStepRanks);
+        };
+        switch (k_dim) {
+            case 32: return launch(gdn_step_kernel<32, 8, 64>);
+            case 64: return launch(gdn_step_kernel<64, 8, 64>);
+            case 96: return launch(gdn_step_kernel<96, 8, 64>);
+            default: return launch(gdn_step_kernel<128, 8, 64>);
+        }
+    }
+    uint32_t ranks = 1;
+    void* args[] = {&p, &ranks};
+    const uint32_t threads = kStepParts * columns;
+    const void* kernel_fn = k_dim == 32 ? (const void*)gdn_step_kernel<32, 32 / kStepParts, 256> : k_dim == 64 ? (const void*)gdn_step_kernel<64, 64 / kStepParts, 256>
+                          : k_dim == 96 ? (const void*)gdn_step_kernel<96, 96 / kStepParts, 256> : (const void*)gdn_step_kernel<128, 128 / kStepParts, 256>;
     return launch_kernel(kernel_fn, dim3(n_k_heads), dim3(threads), 0, stream, args);
 }
 
