@@ -525,7 +525,7 @@ bc_status bc_op_matmul(bc_backend* b, int32_t format, bc_buffer* weights, size_t
     if (store < BC_STORE_OVERWRITE || store > BC_STORE_SWIGLU) return fail(BC_ERR_ARGUMENT, "unknown store mode %d", store);
     k::Mat w;
     BC_TRY(matrix_view(b, weights, w_off, format, n_rows, n_cols, "matmul", &w));
-    if (n_tokens >= k::kMinHalfTokens) {
+    if (n_tokens >= k::kExpandTokens) {
         BC_TRY(expand_for_many_tokens(b, weights));
         BC_TRY(matrix_view(b, weights, w_off, format, n_rows, n_cols, "matmul", &w));
     }
@@ -534,7 +534,7 @@ bc_status bc_op_matmul(bc_backend* b, int32_t format, bc_buffer* weights, size_t
     BC_TRY(check_aligned("matmul", {x_off, y_off}));
     void* pack = nullptr;
     if (k::matmul_umma_supported(w, n_tokens)) BC_TRY(b->pack_scratch(k::matmul_scratch_bytes(w, n_tokens), &pack));
-    return b->run("matmul", n_rows, n_cols, w.bytes(), pack ? k::matmul_umma_launches(w, n_tokens) : 1, [&] {
+    return b->run("matmul", n_rows, n_cols, w.bytes(), pack ? k::matmul_umma_launches(w, n_tokens, store) : 1, [&] {
         return k::matmul(b->stream, w, reinterpret_cast<const float*>(at(x, x_off)), reinterpret_cast<float*>(at(y, y_off)), n_tokens,
                          n_rows, store, pack);
     });

@@ -351,7 +351,7 @@ bool matmul_umma_supported(const Mat& w, uint32_t n_tokens, uint32_t min_tokens 
 uint64_t matmul_pack_bytes(uint32_t n_tokens, uint32_t n_cols);
 // Packed inputs plus, for shapes that split K, the partial products.
 uint64_t matmul_scratch_bytes(const Mat& w, uint32_t n_tokens);
-int matmul_umma_launches(const Mat& w, uint32_t n_tokens);
+int matmul_umma_launches(const Mat& w, uint32_t n_tokens, int32_t store);
 cudaError_t matmul_pack(cudaStream_t stream, const float* x, uint32_t n_tokens, uint32_t n_cols, void* packed);
 // RMSNorm fused into the packing: packed = fp16(weight * (x * scale)), so a normalised batch that only feeds
 // tensor-core products never exists in f32.
@@ -362,7 +362,7 @@ struct Deferred {
     uint32_t split = 0, n_tokens = 0, n_rows = 0;
 };
 // Bytes of partial products matmul_umma writes for this shape (zero when it does not split K).
-uint64_t matmul_partial_bytes(const Mat& w, uint32_t n_tokens);
+uint64_t matmul_partial_bytes(const Mat& w, uint32_t n_tokens, int32_t store);
 // matmul_pack of x times the sigmoid of its gates (attention_gate), heads of a multiple of 32 elements.
 cudaError_t matmul_pack_gated(cudaStream_t stream, const float* x, const float* q_gate, uint32_t head_dim, uint32_t n_tokens, uint32_t n_cols, void* packed);
 // With `add` (for this x: n_tokens rows of n_cols), x += the deferred partial products first, so
@@ -391,7 +391,9 @@ cudaError_t matmul_umma_swiglu(cudaStream_t stream, const Mat& gate, const Mat& 
 // The same products from expanded weights (kernels_matmul_half.cu), for batches of kMinHalfTokens and more
 // of matrices that carry half_tiles; the functions above hand over to them (BOBCAT_NO_HALF_MATMUL=1: no
 // matrix gets half_tiles).
-constexpr uint32_t kMinHalfTokens = 33;
+constexpr uint32_t kMinHalfTokens = 16;
+// Matrices of single operations are expanded when they first meet this many rows.
+constexpr uint32_t kExpandTokens = 33;
 cudaError_t matmul_half_wait_word(int* word);
 uint64_t half_tiles_bytes(uint32_t n_rows, uint32_t n_cols);
 bool half_tiles_supported(uint32_t n_cols);

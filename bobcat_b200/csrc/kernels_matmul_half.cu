@@ -404,10 +404,10 @@ struct Tiling {
     int kind;
 };
 
-// The tiling with the smallest modelled time, in us, fitted to 33 to 512 tokens of matrices of 2048 to 10752 rows and columns:
+// The tiling with the smallest modelled time, in us, fitted to 16 to 512 tokens of matrices of 2048 to 10752 rows and columns:
 // waves of tiles over the SMs, each chunk of 64 columns bound by the MMA (2 cycles per token and matrix at 1.4 GHz),
 // by the SM's share of L2 or by the ring's round trip; a start and a last epilogue that nothing hides; a split's partial
-// products, written and read once; never less than the weights' time from HBM.
+// products, written and read once; the weights' time from HBM, of which a quarter shows beside the rest.
 Tiling choose_tiling(uint32_t rows, uint32_t n_chunks, uint32_t n_tokens, bool dual, bool may_split) {
     const uint32_t sms = (uint32_t)sm_count();
     Tiling best{};
@@ -426,8 +426,8 @@ Tiling choose_tiling(uint32_t rows, uint32_t n_chunks, uint32_t n_tokens, bool d
                 const uint32_t tiles = row_tiles * needed * split, waves = (tiles + sms - 1) / sms;
                 double us = waves * ((n_chunks + split - 1) / split) * chunk;
                 const double hbm = (double)row_tiles * n_chunks * a_bytes(kind) / 6.2e6;
-                us = (us > hbm ? us : hbm) + 2.8 + 0.0095 * width * (dual ? 2 : 1) + (kind == kWhole ? 2.0 : 0.0);
-                if (split > 1) us += 1.0 + (double)split * n_tokens * rows * 4 / 8e6;
+                us = (us > hbm ? us + 0.25 * hbm : hbm + 0.25 * us) + 2.8 + 0.0095 * width * (dual ? 2 : 1) + (kind == kWhole ? 2.0 : 0.0);
+                if (split > 1) us += 1.0 + 0.15 * split + (double)split * n_tokens * rows * 4 / 8e6;
                 if (us < best_us) best_us = us, best = Tiling{width, split, kind};
             }
         }

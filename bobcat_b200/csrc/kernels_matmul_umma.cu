@@ -35,6 +35,7 @@
 // makes every other wait of the CTA give up, records a code the host reads, skips the stores, and
 // the CTA still frees its tensor memory and returns.
 
+#include <algorithm>
 #include <cstdlib>
 
 #include "async_utils.cuh"
@@ -705,19 +706,41 @@ bool umma_disabled() {
 
 uint64_t matmul_pack_bytes(uint32_t n_tokens, uint32_t n_cols) { return (uint64_t)((n_tokens + 15u) & ~15u) * n_cols * 2; }
 
-uint64_t matmul_partial_bytes(const Mat& w, uint32_t n_tokens) {
-    if (matmul_few_supported(w, n_tokens)) return 0;
+namespace {
+
+// Which kernel takes a product of up to 32 rows of a matrix that is also expanded to fp16. The register-resident kernel
+// (kernels_matmul_few.cu) reads a third of the bytes but is bound by its instructions; the tcgen05 kernel needs many tiles, which
+// a product into the residual stream gets by splitting K (its sums ride on the next normalisation) and
+// others only from many rows. Measured, us, the former then the latter: adding, 24 rows of 2048 x 10752 18.0 / 9.8, of 2048 x
+// 2048 5.0 / 4.5, 16 rows of 2048 x 10752 12.7 / 9.7; storing, 24 rows of 12288 x 4096 28.0 / 19.7, of 3072 x 2048 5.7 / 11;
+// gate and up, 24 rows of 10752 x 2048 16.6 / 18.4, 32 rows 19.1 / 17.8, 24 rows of 12288 x 4096 49.7 / 34.3.
+enum class Use { kAdd, kStore, kDual };
+bool few_serves(const Mat& w, uint32_t rows, uint32_t n_tokens, Use use) {
+    if (!matmul_few_supported(w, n_tokens)) return false;
+    if (!matmul_half_supported(w, n_tokens)) return true;
+    switch (use) {
+        case Use::kAdd: return n_tokens <= 16 && w.n_cols < 4096;
+        case Use::kStore: return n_tokens <= 16 || rows < 64 * (uint32_t)sm_count();
+        default: return n_tokens <= 16 || (n_tokens <= 24 && w.n_cols <= 2048);
+    }
+}
+Use use_of(int32_t store) { return store == BC_STORE_ACCUMULATE ? Use::kAdd : Use::kStore; }
+
+}  // namespace
+
+uint64_t matmul_partial_bytes(const Mat& w, uint32_t n_tokens, int32_t store) {
+    if (few_serves(w, w.n_rows, n_tokens, use_of(store))) return 0;
     const uint32_t split = matmul_half_supported(w, n_tokens) ? matmul_half_split(w, n_tokens) : choose_tiling(w.n_rows, w.n_cols, n_tokens, w.n_rows, 1, true).split;
     return split > 1 ? (uint64_t)split * n_tokens * w.n_rows * 4 : 0;
 }
 
 uint64_t matmul_scratch_bytes(const Mat& w, uint32_t n_tokens) {
     uint64_t pack = (matmul_pack_bytes(n_tokens, w.n_cols) + 255) & ~255ull;
-    return pack + matmul_partial_bytes(w, n_tokens);
+    return pack + std::max(matmul_partial_bytes(w, n_tokens, BC_STORE_ACCUMULATE), matmul_partial_bytes(w, n_tokens, BC_STORE_OVERWRITE));
 }
 
-int matmul_umma_launches(const Mat& w, uint32_t n_tokens) {
-    if (matmul_few_supported(w, n_tokens)) return 2;
+int matmul_umma_launches(const Mat& w, uint32_t n_tokens, int32_t store) {
+    if (few_serves(w, w.n_rows, n_tokens, use_of(store))) return 2;
     if (matmul_half_supported(w, n_tokens)) return matmul_half_split(w, n_tokens) > 1 ? 3 : 2;
     return choose_tiling(w.n_rows, w.n_cols, n_tokens, w.n_rows, 1, true).split > 1 ? 3 : 2;
 }
@@ -768,7 +791,7 @@ cudaError_t matmul_umma(cudaStream_t stream, const Mat& w, const void* scratch, 
                         int32_t store, float* partial_at, Deferred* defer) {
     if (defer) *defer = Deferred{};
     if (n_tokens == 0 || w.n_rows == 0) return cudaSuccess;
-    if (matmul_few_supported(w, n_tokens)) {
+    if (few_serves(w, w.n_rows, n_tokens, use_of(store))) {
         const Mat* ws[1] = {&w};
         float* ys[1] = {y};
         const uint32_t strides[1] = {y_stride};
@@ -824,8 +847,10 @@ cudaError_t matmul_umma(cudaStream_t stream, const Mat& w, const void* scratch, 
 cudaError_t matmul_umma_several(cudaStream_t stream, const Mat* const* ws, float* const* ys, int n, const void* packed, uint32_t n_tokens) {
     if (n < 1 || n > 4) return cudaErrorInvalidValue;
     if (n_tokens == 0) return cudaSuccess;
+    uint32_t all_rows = 0;
+    for (int i = 0; i < n; ++i) all_rows += ws[i]->n_rows;
     bool few = true;
-    for (int i = 0; i < n; ++i) few = few && matmul_few_supported(*ws[i], n_tokens) && ws[i]->n_cols == ws[0]->n_cols;
+    for (int i = 0; i < n; ++i) few = few && few_serves(*ws[i], all_rows, n_tokens, Use::kStore) && ws[i]->n_cols == ws[0]->n_cols;
     if (few) {
         uint32_t strides[4];
         for (int i = 0; i < n; ++i) strides[i] = ws[i]->n_rows;
@@ -883,7 +908,7 @@ cudaError_t matmul_umma_swiglu(cudaStream_t stream, const Mat& gate, const Mat& 
                                uint32_t y_stride, void* packed_out) {
     if (packed_out && (gate.n_rows % kChunkK != 0)) return cudaErrorInvalidValue;
     if (n_tokens == 0 || gate.n_rows == 0) return cudaSuccess;
-    if (matmul_few_supported(gate, n_tokens) && matmul_few_supported(up, n_tokens))
+    if (few_serves(gate, gate.n_rows, n_tokens, Use::kDual) && few_serves(up, up.n_rows, n_tokens, Use::kDual))
         return matmul_few_swiglu(stream, gate, up, packed, y, n_tokens, y_stride, packed_out);
     if (matmul_half_supported(gate, n_tokens) && matmul_half_supported(up, n_tokens))
         return matmul_half_swiglu(stream, gate, up, packed, y, n_tokens, y_stride, packed_out);

@@ -136,7 +136,7 @@ struct Recorder {
     void product_of_packed(const k::Mat& w, const void* packed, float* y, uint32_t n, int store) {
         close_sum();  // the partial scratch is about to be reused (or regrown)
         void* partial = nullptr;
-        const uint64_t partial_bytes = k::matmul_partial_bytes(w, n);
+        const uint64_t partial_bytes = k::matmul_partial_bytes(w, n, store);
         if (status == BC_OK && partial_bytes) status = s.backend->partial_scratch(partial_bytes, &partial);
         k::Deferred left{};
         const bool may_defer = store == BC_STORE_ACCUMULATE;
