@@ -27,6 +27,8 @@ struct bc_engine {
     bc_checkpoint* checkpoint = nullptr;
     uint64_t rng = 0;            // state of the draw generator
     uint32_t last_cached = 0;
+    void* scoring = nullptr;     // device scratch of score: sums, results, label tokens
+    size_t scoring_bytes = 0;
 
     void forget() {
         consumed.clear();
@@ -36,6 +38,7 @@ struct bc_engine {
     }
     ~bc_engine() {
         if (checkpoint) bc_checkpoint_free(checkpoint);
+        if (scoring) cudaFree(scoring);
         if (seq) bc_seq_free(seq);
     }
 };
@@ -195,30 +198,47 @@ bc_status bc_engine_score(bc_engine* e, const uint32_t* prompt_tokens, const siz
         while (same < shared && first[same] == other[same]) ++same;
         shared = same;
     }
+    // The prompts run one after another without the host waiting in between: the log-softmax (f64, :425-433) is taken on the
+    // device and only the labels' values come back.
+    BC_TRY(s->backend->activate());
+    cudaStream_t stream = s->backend->stream;
+    const size_t n_labels = label_offsets[n_prompts] - label_offsets[0], sums = (size_t)k::label_log_probs_scratch(n_vocab);
+    const size_t bytes = (sums + n_labels) * sizeof(double) + n_labels * 4;
+    if (e->scoring_bytes < bytes) {
+        if (e->scoring) BC_CUDA(cudaFree(e->scoring));
+        e->scoring = nullptr;
+        e->scoring_bytes = 0;
+        BC_CUDA(cudaMalloc(&e->scoring, bytes));
+        e->scoring_bytes = bytes;
+    }
+    double* scratch = static_cast<double*>(e->scoring);
+    double* results = scratch + sums;
+    uint32_t* labels = reinterpret_cast<uint32_t*>(results + n_labels);
+    if (n_labels) BC_CUDA(cudaMemcpyAsync(labels, label_tokens + label_offsets[0], n_labels * 4, cudaMemcpyHostToDevice, stream));
     bc_checkpoint* start = nullptr;
-    struct Free {
+    struct Finish {
         bc_checkpoint*& c;
-        ~Free() { if (c) bc_checkpoint_free(c); }
-    } free_start{start};
+        cudaStream_t stream;
+        ~Finish() {
+            cudaStreamSynchronize(stream);
+            if (c) bc_checkpoint_free(c);
+        }
+    } finish{start, stream};
     if (shared > 0) {
-        BC_TRY(bc_seq_prefill(s, first, shared, nullptr, 0, nullptr, 0, nullptr));
+        BC_TRY(prefill_async(s, first, (uint32_t)shared, false));
         BC_TRY(bc_seq_checkpoint(s, &start));
     }
-    std::vector<float> logits(n_vocab);
     for (size_t i = 0; i < n_prompts; ++i) {
         if (start) BC_TRY(bc_seq_restore(s, start));
         else BC_TRY(bc_seq_reset(s));
         const uint32_t* prompt = prompt_tokens + prompt_offsets[i];
-        const size_t len = prompt_offsets[i + 1] - prompt_offsets[i];
-        BC_TRY(bc_seq_prefill(s, prompt + shared, len - shared, logits.data(), logits.size(), nullptr, 0, nullptr));
-        // log-softmax in f64 (:425-433).
-        double top = -INFINITY;
-        for (float v : logits) top = std::max(top, (double)v);
-        double sum = 0.0;
-        for (float v : logits) sum += std::exp((double)v - top);
-        const double log_sum = top + std::log(sum);
-        for (size_t t = label_offsets[i]; t < label_offsets[i + 1]; ++t) scores[t] = (double)logits[label_tokens[t]] - log_sum;
+        const size_t len = prompt_offsets[i + 1] - prompt_offsets[i], at = label_offsets[i] - label_offsets[0], count = label_offsets[i + 1] - label_offsets[i];
+        BC_TRY(prefill_async(s, prompt + shared, (uint32_t)(len - shared), count > 0));
+        BC_CUDA(k::label_log_probs(stream, s->logits, n_vocab, labels + at, (uint32_t)count, scratch, results + at));
     }
+    if (n_labels) BC_CUDA(cudaMemcpyAsync(scores + label_offsets[0], results, n_labels * sizeof(double), cudaMemcpyDeviceToHost, stream));
+    BC_CUDA(cudaStreamSynchronize(stream));
+    BC_TRY(kernel_wait_status());
     return bc_seq_reset(s);
 }
 

@@ -240,6 +240,10 @@ struct Sampling {
 cudaError_t sample(cudaStream_t stream, float* logits, uint32_t n, const uint32_t* recent, uint32_t n_recent, const Sampling& settings,
                    float uniform, uint32_t* out, uint32_t* readback);
 
+// out[i] = the log-softmax (f64) of n logits at labels[i]; scratch of label_log_probs_scratch(n) doubles.
+uint64_t label_log_probs_scratch(uint32_t n);
+cudaError_t label_log_probs(cudaStream_t stream, const float* logits, uint32_t n, const uint32_t* labels, uint32_t n_labels, double* scratch, double* out);
+
 // ---- multi-sequence decode (kernels_batch.cu): one new token of each of n_seqs sequences per pass.
 // What is per sequence is reached through device arrays indexed by the sequence's row.
 struct SeqTable {

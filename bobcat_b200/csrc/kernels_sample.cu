@@ -473,7 +473,74 @@ __global__ void __launch_bounds__(kSampleThreads) sample_kernel(SampleParams p, 
     cluster_sync();
 }
 
+// ---- log-probabilities of label tokens: log-softmax in f64 (engine.rs:425-433)
+
+constexpr uint32_t kLogSumLogits = 512;  // of a CTA
+
+// A CTA's share: its largest logit and the f64 sum of the exponentials relative to it. Bound by f64 arithmetic, about six operations
+// per cycle and SM, so the logits are spread over all of them: 65 536 in 6 us with the kernel below, where reading
+// them back and summing on one host core took 0.4 ms a prompt.
+__global__ void __launch_bounds__(256) log_sum_kernel(const float* __restrict__ logits, uint32_t n, double* __restrict__ partial) {
+    __shared__ float tops[8];
+    __shared__ double sums[8];
+    pdl_launch_dependents();
+    pdl_wait();
+    const uint32_t tid = threadIdx.x, first = blockIdx.x * kLogSumLogits, last = min(n, first + kLogSumLogits);
+    float top = -INFINITY;
+    for (uint32_t i = first + tid; i < last; i += 256) top = fmaxf(top, __ldcg(logits + i));
+    top = warp_max(top);
+    if ((tid & 31) == 0) tops[tid >> 5] = top;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < 8; ++w) top = fmaxf(top, tops[w]);
+    double sum = 0.0;
+    for (uint32_t i = first + tid; i < last; i += 256) sum += exp((double)__ldcg(logits + i) - (double)top);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if ((tid & 31) == 0) sums[tid >> 5] = sum;
+    __syncthreads();
+    if (tid == 0) {
+        for (int w = 1; w < 8; ++w) sum += sums[w];
+        partial[2 * blockIdx.x] = (double)top;
+        partial[2 * blockIdx.x + 1] = sum;
+    }
+}
+
+__global__ void __launch_bounds__(256) label_log_probs_kernel(const float* __restrict__ logits, const double* __restrict__ partial, uint32_t n_partial,
+                                                              const uint32_t* __restrict__ labels, uint32_t n_labels, double* __restrict__ out) {
+    __shared__ double tops[8], sums[8];
+    pdl_launch_dependents();
+    pdl_wait();
+    const uint32_t tid = threadIdx.x;
+    double top = -INFINITY, sum = 0.0;
+    for (uint32_t i = tid; i < n_partial; i += 256) top = fmax(top, __ldcg(partial + 2 * i));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) top = fmax(top, __shfl_xor_sync(0xffffffffu, top, o));
+    if ((tid & 31) == 0) tops[tid >> 5] = top;
+    __syncthreads();
+    for (int w = 0; w < 8; ++w) top = fmax(top, tops[w]);
+    for (uint32_t i = tid; i < n_partial; i += 256) sum += __ldcg(partial + 2 * i + 1) * exp(__ldcg(partial + 2 * i) - top);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if ((tid & 31) == 0) sums[tid >> 5] = sum;
+    __syncthreads();
+    sum = 0.0;
+    for (int w = 0; w < 8; ++w) sum += sums[w];
+    const double log_sum = top + log(sum);
+    for (uint32_t i = tid; i < n_labels; i += 256) out[i] = (double)__ldcg(logits + labels[i]) - log_sum;
+}
+
 }  // namespace
+
+uint64_t label_log_probs_scratch(uint32_t n) { return (uint64_t)((n + kLogSumLogits - 1) / kLogSumLogits) * 2; }
+
+cudaError_t label_log_probs(cudaStream_t stream, const float* logits, uint32_t n, const uint32_t* labels, uint32_t n_labels, double* scratch, double* out) {
+    if (n == 0 || n_labels == 0) return cudaSuccess;
+    const uint32_t parts = (n + kLogSumLogits - 1) / kLogSumLogits;
+    cudaError_t e = launch_dependent(log_sum_kernel, dim3(parts), dim3(256), 0, stream, logits, n, scratch);
+    if (e != cudaSuccess) return e;
+    return launch_dependent(label_log_probs_kernel, dim3(1), dim3(256), 0, stream, logits, static_cast<const double*>(scratch), parts, labels, n_labels, out);
+}
 
 cudaError_t sample(cudaStream_t stream, float* logits, uint32_t n, const uint32_t* recent, uint32_t n_recent, const Sampling& settings,
                    float uniform, uint32_t* out, uint32_t* readback) {

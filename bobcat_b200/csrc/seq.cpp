@@ -478,6 +478,30 @@ bc_status step_impl(bc_seq* s, uint32_t token, float* logits, size_t logits_len,
 
 }  // namespace
 
+namespace bc {
+
+bc_status prefill_async(bc_seq* s, const uint32_t* tokens, uint32_t n, bool want_logits) {
+    if (s->backend->recording) return fail(BC_ERR_ALREADY_RECORDING, "a recording is already open");
+    BC_TRY(s->backend->activate());
+    BC_CUDA(cudaMemcpyAsync(s->tokens + s->n_past, tokens, (size_t)n * 4, cudaMemcpyHostToDevice, s->backend->stream));
+    for (uint32_t done = 0; done < n;) {
+        const uint32_t count = std::min(n - done, s->batch), pos = s->n_past + done;
+        const bool logits = want_logits && done + count == n;
+        Recorder r(*s);
+        if (count == 1) r.step(pos, logits, false);
+        else r.batch(pos, count, logits, false, 0);
+        if (r.status != BC_OK) {
+            cudaStreamSynchronize(s->backend->stream);
+            return r.status;
+        }
+        done += count;
+    }
+    s->n_past += n;
+    return BC_OK;
+}
+
+}  // namespace bc
+
 extern "C" {
 
 bc_status bc_seq_prefill(bc_seq* s, const uint32_t* tokens, size_t n_tokens, float* logits, size_t logits_len, float* final_norm,

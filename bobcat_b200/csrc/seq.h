@@ -143,3 +143,10 @@ struct bc_seq {
     void release();
     ~bc_seq();
 };
+
+namespace bc {
+
+// Prefill of valid tokens that fit the context, without waiting for it; the logits (with `want_logits`) stay in s->logits.
+bc_status prefill_async(bc_seq* s, const uint32_t* tokens, uint32_t n, bool want_logits);
+
+}  // namespace bc
