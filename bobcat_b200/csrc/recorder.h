@@ -303,16 +303,29 @@ struct Recorder {
         run("norm_rope", (hp.n_heads + hp.n_kv_heads) * n, hp.head_dim, 0, 1, [&] { return k::rope_store_batch(stream, rb); });
     }
 
+    // Where a batch's attention leaves its partial sums: the sequence's own scratch, or, when that holds fewer than four parts of the
+    // keys, the backend's. (No sum of a product is open here: the rotation's launch has closed it.)
+    float* attention_scratch(k::AttentionShape& shape) {
+        const uint64_t floats = (uint64_t)4 * shape.n_queries * hp.n_heads * (hp.head_dim + 2);
+        shape.scratch_floats = s.scratch_floats;
+        if (floats <= s.scratch_floats || !k::attention_flash_supported(s.kv_half, shape)) return s.scores;
+        void* parts = nullptr;
+        if (status == BC_OK) status = s.backend->partial_scratch(floats * 4, &parts);
+        shape.scratch_floats = floats;
+        return static_cast<float*>(parts);
+    }
+
     // Norm and rotation of q and k, cache stores, attention over positions [0, pos + n).
     void rotate_and_attend(const DeviceLayer& D, uint32_t cache_index, uint32_t pos, uint32_t n, uint32_t q_stride, uint32_t q_head_stride) {
         size_t slot = layer_base(cache_index) + (size_t)pos * kv_dim();
         rotate_batch(D, slot, pos, n, s.q, q_stride, q_head_stride, q_stride, q_head_stride);
-        k::AttentionShape shape{hp.n_heads, hp.n_kv_heads, hp.head_dim, pos, n, s.n_ctx, q_stride, q_head_stride, nullptr, s.scratch_floats};
+        k::AttentionShape shape{hp.n_heads, hp.n_kv_heads, hp.head_dim, pos, n, s.n_ctx, q_stride, q_head_stride};
+        float* scratch = attention_scratch(shape);
         int kernels = k::attention_launches(s.kv_half, shape);
         uint64_t kv_bytes = (uint64_t)(pos + n) * kv_dim() * kv_element_bytes() * 2;
         run("attention", n, pos + n, kv_bytes, kernels, [&] {
             return k::attention(stream, s.q, cache_at(s.k_cache, layer_base(cache_index)), cache_at(s.v_cache, layer_base(cache_index)), s.kv_half,
-                                s.scores, s.attn, shape);
+                                scratch, s.attn, shape);
         });
     }
 
@@ -641,10 +654,11 @@ struct Recorder {
                 size_t slot = layer_base(S.cache_index) + (size_t)pos * kv_dim();
                 // The rotated queries go to their own compact rows; the gates stay in the projection.
                 rotate_batch(D, slot, pos, n, s.q_rot, 2 * q_dim, 2 * hp.head_dim, q_dim, hp.head_dim);
-                k::AttentionShape shape{hp.n_heads, hp.n_kv_heads, hp.head_dim, pos, n, s.n_ctx, q_dim, hp.head_dim, nullptr, s.scratch_floats};
+                k::AttentionShape shape{hp.n_heads, hp.n_kv_heads, hp.head_dim, pos, n, s.n_ctx, q_dim, hp.head_dim};
+                float* scratch = attention_scratch(shape);
                 run("attention", n, pos + n, (uint64_t)(pos + n) * kv_dim() * kv_element_bytes() * 2, k::attention_launches(s.kv_half, shape), [&] {
                     return k::attention(stream, s.q_rot, cache_at(s.k_cache, layer_base(S.cache_index)), cache_at(s.v_cache, layer_base(S.cache_index)),
-                                        s.kv_half, s.scores, s.attn, shape);
+                                        s.kv_half, scratch, s.attn, shape);
                 });
                 if (tensor_products() && k::matmul_umma_supported(D.output, n, min_tensor_rows) && hp.head_dim % 32 == 0) {
                     // The gates on the way into the packed input of the output projection.

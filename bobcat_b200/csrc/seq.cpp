@@ -306,9 +306,7 @@ bc_status seq_new(bc_model* model, bc_backend* backend, bc_comm* tp, uint32_t n_
     s->conv_floats = qwen ? (size_t)hp.n_delta_layers * conv_dim * (hp.conv_kernel - 1) : (size_t)hp.n_conv_layers * (hp.conv_kernel - 1) * n_embd;
     s->delta_floats = (size_t)hp.n_delta_layers * hp.n_v_heads * hp.k_head_dim * hp.v_head_dim;
     const size_t ffn_width = std::max<size_t>(hp.n_ff, (size_t)hp.n_experts_used * hp.n_ff_expert);
-    // Room for a whole batch's attention with its keys in at least four parts.
-    const size_t scratch_floats = hp.n_attention_layers ? std::max<size_t>(k::attention_scratch_floats(hp.n_heads, hp.head_dim, n_ctx, s->batch),
-                                                                           (size_t)4 * s->batch * hp.n_heads * (hp.head_dim + 2)) : 0;
+    const size_t scratch_floats = hp.n_attention_layers ? k::attention_scratch_floats(hp.n_heads, hp.head_dim, n_ctx, s->batch) : 0;
     s->scratch_floats = scratch_floats;
 
     // Plan the arena: (pointer slot, bytes) pairs, each aligned to 256 bytes.
