@@ -119,18 +119,31 @@ __global__ void __launch_bounds__(flash_threads<HD>(), HD == 64 ? 4 : 1) attenti
     };
     if (first_tile < end_tile) bring(kc, k_tile, first_tile);
 
-    // Stage the scaled queries as hi + lo halves; rows past the batch are zero.
-    for (int i = tid; i < kRows * (kHead / 2); i += kFlashThreads) {
-        const int row = i / (kHead / 2), pair = i % (kHead / 2);
-        float2 v = make_float2(0.f, 0.f);
-        if (row0 + row < n_rows) {
-            const uint32_t query = (row0 + row) / group, head = kv_head * group + (row0 + row) % group;
-            v = *reinterpret_cast<const float2*>(p.q + (uint64_t)query * p.q_stride + (uint64_t)head * p.q_head_stride + 2 * pair);
+    // Stage the scaled queries as hi + lo halves; rows past the batch are zero. Eight loads of a thread are in flight at a time
+    // (one after the other they took 10 us of a CTA with 128 rows of 256).
+    {
+        constexpr int kPairs = kHead / 2, kRowStep = kFlashThreads / kPairs > 0 ? kFlashThreads / kPairs : 1, kAtOnce = 8;
+        static_assert(kFlashThreads % kPairs == 0 && kRows % (kRowStep * kAtOnce) == 0, "whole rounds");
+        const int pair = tid % kPairs;
+        for (int first = tid / kPairs; first < kRows; first += kRowStep * kAtOnce) {
+            float2 v[kAtOnce];
+#pragma unroll
+            for (int n = 0; n < kAtOnce; ++n) {
+                const uint32_t row = row0 + first + n * kRowStep;
+                v[n] = make_float2(0.f, 0.f);
+                if (row < n_rows) {
+                    const uint32_t query = row / group, head = kv_head * group + row % group;
+                    v[n] = *reinterpret_cast<const float2*>(p.q + (uint64_t)query * p.q_stride + (uint64_t)head * p.q_head_stride + 2 * pair);
+                }
+            }
+#pragma unroll
+            for (int n = 0; n < kAtOnce; ++n) {
+                uint32_t hi, lo;
+                split_half2(v[n].x * scale, v[n].y * scale, hi, lo);
+                *reinterpret_cast<uint32_t*>(&q_hi[first + n * kRowStep][2 * pair]) = hi;
+                *reinterpret_cast<uint32_t*>(&q_lo[first + n * kRowStep][2 * pair]) = lo;
+            }
         }
-        uint32_t hi, lo;
-        split_half2(v.x * scale, v.y * scale, hi, lo);
-        *reinterpret_cast<uint32_t*>(&q_hi[row][2 * pair]) = hi;
-        *reinterpret_cast<uint32_t*>(&q_lo[row][2 * pair]) = lo;
     }
 
     // Query fragments: k-steps of 16 elements, hi and lo.
@@ -311,17 +324,24 @@ __global__ void __launch_bounds__(256) attention_join_kernel(const float* __rest
     float2 sum[kQuads];
 #pragma unroll
     for (int i = 0; i < kQuads; ++i) sum[i] = make_float2(0.f, 0.f);
-#pragma unroll 4
-    for (uint32_t z = 0; z < splits; ++z) {
-        const float w = __shfl_sync(0xffffffffu, weight, z);
-        if (w == 0.f) continue;
-        const float2* from = reinterpret_cast<const float2*>(parts + ((uint64_t)z * total + at) * HD) + lane;
+    for (uint32_t z0 = 0; z0 < splits; z0 += 8) {
+        float2 v[8][kQuads];
+        float w[8];
 #pragma unroll
-        for (int i = 0; i < kQuads; ++i) {
-            const float2 v = __ldcg(from + i * 32);
-            sum[i].x += w * v.x;
-            sum[i].y += w * v.y;
+        for (uint32_t k = 0; k < 8; ++k) {
+            const uint32_t z = z0 + k;
+            w[k] = z < splits ? __shfl_sync(0xffffffffu, weight, z & 31) : 0.f;
+            const float2* from = reinterpret_cast<const float2*>(parts + ((uint64_t)z * total + at) * HD) + lane;
+#pragma unroll
+            for (int i = 0; i < kQuads; ++i) v[k][i] = w[k] != 0.f ? __ldcg(from + i * 32) : make_float2(0.f, 0.f);  // unwritten where it weighs nothing
         }
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k)
+#pragma unroll
+            for (int i = 0; i < kQuads; ++i) {
+                sum[i].x += w[k] * v[k][i].x;
+                sum[i].y += w[k] * v[k][i].y;
+            }
     }
 #pragma unroll
     for (int i = 0; i < kQuads; ++i) reinterpret_cast<float2*>(out + (uint64_t)at * HD)[lane + i * 32] = make_float2(sum[i].x * inverse, sum[i].y * inverse);
