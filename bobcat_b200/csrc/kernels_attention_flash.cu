@@ -23,8 +23,8 @@
 // scheduler) for wide heads, by the exponentials' instructions for heads of 64.
 //
 // Measured: 64 queries of 8 heads of 256 behind 0 to 2000 positions 110 us before (four warps, loads and multiplies in
-// turn, a CTA per head), 39 with the join; 512 queries of 16 heads behind 4500 positions 500 us, 284; 512 queries
-// of 32 heads of 64 from position 0 33 us, 29.
+// turn, a CTA per head), 22 with the join; 512 queries of 16 heads behind 4500 positions 500 us, 267; 512 queries
+// of 32 heads of 64 from position 0 33 us, 27.
 
 #include "async_utils.cuh"
 #include "device_utils.cuh"
@@ -89,6 +89,7 @@ __global__ void __launch_bounds__(flash_threads<HD>(), HD == 64 ? 4 : 1) attenti
     __half (*q_lo)[kPitch] = q_hi + kRows;
     __half (*k_tile)[kPitch] = q_lo + kRows;
     __half (*v_tile)[kPitch] = k_tile + kKeys;
+    __shared__ uint64_t row_at[kRows];
 
     pdl_launch_dependents();
     pdl_wait();
@@ -119,8 +120,13 @@ __global__ void __launch_bounds__(flash_threads<HD>(), HD == 64 ? 4 : 1) attenti
     };
     if (first_tile < end_tile) bring(kc, k_tile, first_tile);
 
-    // Stage the scaled queries as hi + lo halves; rows past the batch are zero. Eight loads of a thread are in flight at a time
-    // (one after the other they took 10 us of a CTA with 128 rows of 256).
+    // Stage the scaled queries as hi + lo halves; rows past the batch are zero. Where a row lies is worked out once per row (the
+    // divisions, for every pair of elements, took 18 us of a CTA with 128 rows of 256).
+    if (tid < kRows) {
+        const uint32_t row = row0 + tid;
+        row_at[tid] = row < n_rows ? (uint64_t)(row / group) * p.q_stride + (uint64_t)(kv_head * group + row % group) * p.q_head_stride : ~0ull;
+    }
+    __syncthreads();
     {
         constexpr int kPairs = kHead / 2, kRowStep = kFlashThreads / kPairs > 0 ? kFlashThreads / kPairs : 1, kAtOnce = 8;
         static_assert(kFlashThreads % kPairs == 0 && kRows % (kRowStep * kAtOnce) == 0, "whole rounds");
@@ -129,12 +135,8 @@ __global__ void __launch_bounds__(flash_threads<HD>(), HD == 64 ? 4 : 1) attenti
             float2 v[kAtOnce];
 #pragma unroll
             for (int n = 0; n < kAtOnce; ++n) {
-                const uint32_t row = row0 + first + n * kRowStep;
-                v[n] = make_float2(0.f, 0.f);
-                if (row < n_rows) {
-                    const uint32_t query = row / group, head = kv_head * group + row % group;
-                    v[n] = *reinterpret_cast<const float2*>(p.q + (uint64_t)query * p.q_stride + (uint64_t)head * p.q_head_stride + 2 * pair);
-                }
+                const uint64_t at = row_at[first + n * kRowStep];
+                v[n] = at != ~0ull ? *reinterpret_cast<const float2*>(p.q + at + 2 * pair) : make_float2(0.f, 0.f);
             }
 #pragma unroll
             for (int n = 0; n < kAtOnce; ++n) {
