@@ -23,7 +23,8 @@
 // the next tile is multiplied some of the warps add them up in warp order and store. Wider matrices
 // take a cluster of CTAs, one per range, which meet through distributed shared memory, again in rank order: no partial
 // products in global memory, no second launch, results independent of timing. Rows beyond a launch's group of 8 (exact)
-// or 32 (half) are further groups in blockIdx.y, working at the same time on the same weights out of L2.
+// or 32 (half) are further groups in blockIdx.y, working at the same time on the same weights out of L2; those of experts
+// are cut into equal runs (at the kernel).
 //
 // The weights come through per-lane slots of shared memory filled by cp.async several tiles ahead; a lane reads
 // back only what it copied itself, so the ring needs no barrier. The first tiles are requested before the wait for
@@ -73,10 +74,11 @@ struct FewParams {
     const uint4* packed;           // half: the packed fp16 operand, [pair][token group][8 cores][8 tokens] of 16 bytes
     uint32_t token_groups;
     __half* packed_out;            // half, dual: the result as the packed operand of the product that consumes it
-    // Experts: blockIdx.z is an expert of the stacked matrices (n_jobs tiles each), its rows are the
+    // Experts: expert z has n_jobs tiles of the stacked matrices, its rows are the
     // entries offsets[z] .. offsets[z + 1]; entry e reads x row e / n_used (gather) or e and writes y row e.
     const uint32_t* offsets;
     const uint32_t* entries;
+    uint32_t n_experts;
     uint32_t n_used;
     int gather;
     uint32_t cap_groups;           // half: an expert's rows are packed from token group z * cap_groups on
@@ -136,8 +138,40 @@ __device__ __forceinline__ float remote_float(const float* p, uint32_t rank) {
     return v;
 }
 
+// The expert and the place among its groups (of up to `rows` entries) of group number `group` of all experts; false, with
+// the number of groups in `place`, if there are fewer. The whole warp calls it.
+__device__ __forceinline__ bool find_group(const uint32_t* offsets, uint32_t n_experts, uint32_t rows, uint32_t group, uint32_t& expert, uint32_t& place) {
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t before = 0;
+    for (uint32_t base = 0; base < n_experts; base += 32) {
+        const uint32_t count = base + lane < n_experts ? (offsets[base + lane + 1] - offsets[base + lane] + rows - 1) / rows : 0;
+        uint32_t sum = count;
+#pragma unroll
+        for (int d = 1; d < 32; d *= 2) {
+            const uint32_t lower = __shfl_up_sync(0xffffffffu, sum, d);
+            if (lane >= (uint32_t)d) sum += lower;
+        }
+        const uint32_t holds = __ballot_sync(0xffffffffu, before + sum > group);
+        if (holds) {
+            const int at = __ffs(holds) - 1;
+            expert = base + at;
+            place = group - before - __shfl_sync(0xffffffffu, sum - count, at);
+            return true;
+        }
+        before += __shfl_sync(0xffffffffu, sum, 31);
+    }
+    place = before;
+    return false;
+}
+
 // NT groups of 8 rows (exact: one), W pairs of blocks per warp, DEPTH steps of weights in flight.
-template <bool EXACT, int NT, int W, int DEPTH>
+//
+// Experts: how many rows each has is known on the device alone, so the launch is as wide as the device and every CTA (cluster)
+// takes an equal run of the jobs of all groups of rows, which may end in the next group, whose inputs it then loads. (A share of the CTAs
+// per expert and group, for the likely number of groups, left SMs idle or began a second wave. An expert block of 32 experts of 1792
+// x 2048, us with all its launches: 2 tokens 103 -> 91, 16 tokens 179 -> 151, 64 tokens 222 -> 163, 203 tokens 231 to 352, as the
+// router picks, -> 237 to 251; passes of 15 sequences of such a model 15.6 -> 12.6 ms.)
+template <bool EXACT, bool EXPERTS, int NT, int W, int DEPTH>
 __global__ void __launch_bounds__(kThreads, 1) matmul_few_kernel(const __grid_constant__ FewParams p) {
     static_assert(!EXACT || NT == 1, "the pieces of more rows do not fit the registers");
     constexpr uint32_t kTileSums = 128 * NT, kPieces = EXACT ? 3 : NT, T = tiles_per_step(NT), kStepBytes = T * W * kSlotPair;
@@ -152,19 +186,15 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_few_kernel(const __grid_co
     async::mbar_init_fence();
     __syncthreads();
     pdl_launch_dependents();
-    uint32_t n_tokens = p.n_tokens, first_entry = 0;
     const uint32_t slices = p.slices, slice = blockIdx.x % slices, cta = blockIdx.x / slices, n_ctas = gridDim.x / slices;
-    uint64_t expert_tile = 0;
-    if (p.offsets) {
+    uint64_t run_at = 0, run_end = 0;  // experts: the jobs of this CTA, counted through all groups
+    if constexpr (EXPERTS) {
         pdl_wait();  // the grouping decides the CTA's work
-        first_entry = p.offsets[blockIdx.z];
-        n_tokens = p.offsets[blockIdx.z + 1] - first_entry;
-        expert_tile = (uint64_t)blockIdx.z * p.n_jobs;
+        uint32_t expert, n_groups;
+        find_group(p.offsets, p.n_experts, 8 * NT, ~0u, expert, n_groups);
+        run_at = (uint64_t)n_groups * p.n_jobs * cta / n_ctas;
+        run_end = (uint64_t)n_groups * p.n_jobs * (cta + 1) / n_ctas;
     }
-    const uint32_t token0 = blockIdx.y * (8 * NT);
-    if (token0 >= n_tokens) return;  // a whole cluster leaves together
-    const uint32_t my_jobs = p.n_jobs > cta ? (p.n_jobs - cta + n_ctas - 1) / n_ctas : 0;
-    const uint32_t n_tiles = p.dual ? 2 * my_jobs : my_jobs, n_steps = (n_tiles + T - 1) / T;  // of a pair of matrices the tiles alternate
     // This warp's pairs: [pair0, pair0 + live).
     const uint32_t slice_end = min(p.n_pairs, (slice + 1) * p.slice_pairs), pair0 = slice * p.slice_pairs + warp * W;
     const uint32_t live = pair0 < slice_end ? min((uint32_t)W, slice_end - pair0) : 0;
@@ -179,11 +209,27 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_few_kernel(const __grid_co
         quant_at[i] = chunk * kChunkBytes + in_chunk * kPairQuants + lane * 16;
         scale_at[i] = chunk * kChunkBytes + chunk_pairs * kPairQuants + in_chunk * kPairScales + g * 8;
     }
+    uint32_t steps_before = 0;  // steps of the groups before this one
+    do {  // plain: once; a whole cluster goes round or leaves together
+    uint32_t n_tokens = p.n_tokens, first_entry = 0, expert = 0, group = blockIdx.y;
+    uint32_t first_job = cta, job_step = n_ctas, my_jobs = p.n_jobs > cta ? (p.n_jobs - cta + n_ctas - 1) / n_ctas : 0;
+    if constexpr (EXPERTS) {
+        if (run_at >= run_end || !find_group(p.offsets, p.n_experts, 8 * NT, (uint32_t)(run_at / p.n_jobs), expert, group)) break;
+        first_entry = p.offsets[expert];
+        n_tokens = p.offsets[expert + 1] - first_entry;
+        first_job = (uint32_t)(run_at % p.n_jobs);
+        job_step = 1;
+        my_jobs = (uint32_t)min((uint64_t)(p.n_jobs - first_job), run_end - run_at);
+        run_at += my_jobs;
+    }
+    const uint64_t expert_tile = (uint64_t)expert * p.n_jobs;
+    const uint32_t token0 = group * (8 * NT);
+    const uint32_t n_tiles = p.dual ? 2 * my_jobs : my_jobs, n_steps = (n_tiles + T - 1) / T;  // of a pair of matrices the tiles alternate
     const uint32_t ring = async::smem_u32(smem) + partial_bytes(NT) + warp * (DEPTH * kStepBytes) + lane * 16;
     auto tile_of = [&](uint32_t tile) {
-        if (p.offsets || p.dual || p.n_segments == 1)
-            return p.tiles[p.dual ? tile & 1 : 0] + (expert_tile + cta + n_ctas * (tile >> p.dual)) * tile_bytes;
-        uint32_t job = cta + n_ctas * tile;
+        if (EXPERTS || p.dual || p.n_segments == 1)
+            return p.tiles[p.dual ? tile & 1 : 0] + (expert_tile + first_job + job_step * (tile >> p.dual)) * tile_bytes;
+        uint32_t job = first_job + job_step * tile;
         int seg = 0;
         while (seg + 1 < p.n_segments && job >= p.seg_tiles[seg]) {
             job -= p.seg_tiles[seg];
@@ -230,9 +276,9 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_few_kernel(const __grid_co
                     if (p.norm_weight && (uint32_t)i < live)
                         weight[i][b][h] = __ldg(reinterpret_cast<const float4*>(p.norm_weight + (pair0 + i) * 64 + b * 32 + h * 16 + 4 * t));
                 }
-        if (!p.offsets) pdl_wait();
+        if (!EXPERTS) pdl_wait();
         uint32_t in_row = token;
-        if (p.offsets && has_row) {
+        if (EXPERTS && has_row) {
             const uint32_t entry = p.entries[first_entry + token];
             in_row = p.gather ? entry / p.n_used : entry;
         }
@@ -278,8 +324,8 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_few_kernel(const __grid_co
             if (t == 0) squares[warp][g] = square;
         }
     } else {
-        if (!p.offsets) pdl_wait();
-        const uint32_t group0 = (p.offsets ? blockIdx.z * p.cap_groups : 0) + blockIdx.y * NT;
+        if (!EXPERTS) pdl_wait();
+        const uint32_t group0 = (EXPERTS ? expert * p.cap_groups : 0) + group * NT;
         const uint32_t groups = (n_tokens - token0 + 7) / 8;  // groups past the rows stay zero
 #pragma unroll
         for (int i = 0; i < W; ++i)
@@ -312,7 +358,7 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_few_kernel(const __grid_co
     const uint32_t at = ((((turn >> 2) * 32 + (row_in_tile & 7) * 4 + (tk >> 1)) * 4) + (row_in_tile >> 3) * 2 + (tk & 1)) ^ (row_in_tile & 2);
     auto my_turn = [&](uint32_t step) { return NT == 1 ? (step & 3) == warp >> 2 : NT == 2 ? (step & 1) == warp >> 3 : warp < 4 * NT; };
     auto over_warps = [&](uint32_t step, uint32_t h) {
-        const float* base = reinterpret_cast<const float*>(partial) + ((step & 1) * T + h) * (kWarps * kTileSums) + at;
+        const float* base = reinterpret_cast<const float*>(partial) + (((steps_before + step) & 1) * T + h) * (kWarps * kTileSums) + at;
         float sum = 0.f;
 #pragma unroll
         for (uint32_t w = 0; w < kWarps; ++w) sum += base[w * kTileSums];
@@ -341,9 +387,9 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_few_kernel(const __grid_co
                 gate = total(h) * scale;
                 continue;
             }
-            uint32_t job = cta + n_ctas * (tile >> p.dual);
+            uint32_t job = first_job + job_step * (tile >> p.dual);
             int seg = 0;
-            if (!p.offsets && !p.dual)
+            if (!EXPERTS && !p.dual)
                 while (seg + 1 < p.n_segments && job >= p.seg_tiles[seg]) {
                     job -= p.seg_tiles[seg];
                     ++seg;
@@ -361,7 +407,7 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_few_kernel(const __grid_co
                 continue;
             }
             const bool stores = tok < n_tokens && row < p.seg_rows[seg];
-            float* out = p.y[seg] + (uint64_t)(p.offsets && stores ? p.entries[first_entry + tok] : tok) * p.seg_stride[seg] + row;
+            float* out = p.y[seg] + (uint64_t)(EXPERTS && stores ? p.entries[first_entry + tok] : tok) * p.seg_stride[seg] + row;
             const float old = stores && !p.dual && p.store != BC_STORE_OVERWRITE ? *out : 0.f;
             float sum = total(h) * scale;
             if (p.dual) sum = gate / (1.f + expf(-gate)) * sum;
@@ -441,9 +487,9 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_few_kernel(const __grid_co
             }
         }
         if (u > 0) {
-            const uint32_t before = u - 1;
+            const uint32_t before = u - 1, turns = steps_before + before;  // buffers and barriers alternate through all groups
             // Every warp arrives for every step whatever happens, so the wait ends; it is bounded like all waits.
-            for (uint32_t spin = 0; spin < kSpinLimit && !async::mbar_test(bars + (before & 1) * 8, (before >> 1) & 1); ++spin) {}
+            for (uint32_t spin = 0; spin < kSpinLimit && !async::mbar_test(bars + (turns & 1) * 8, (turns >> 1) & 1); ++spin) {}
             if (slices == 1) {
                 if (my_turn(before)) finish(before, [&](uint32_t h) { return over_warps(before, h); });
             } else {
@@ -461,18 +507,20 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_few_kernel(const __grid_co
                 for (uint32_t h = 0; h < T; ++h)
 #pragma unroll
                     for (int j = 0; j < NT; ++j)
-                        partial[((((u & 1) * T + h) * kWarps + warp) * NT + j) * 32 + lane] =
+                        partial[(((((steps_before + u) & 1) * T + h) * kWarps + warp) * NT + j) * 32 + lane] =
                             g & 2 ? make_float4(acc[h][j][2], acc[h][j][3], acc[h][j][0], acc[h][j][1]) : make_float4(acc[h][j][0], acc[h][j][1], acc[h][j][2], acc[h][j][3]);
             }
             __syncwarp();
-            if (lane == 0) async::mbar_arrive(bars + (u & 1) * 8);
+            if (lane == 0) async::mbar_arrive(bars + ((steps_before + u) & 1) * 8);
         }
     }
     async::cp_async_wait<0>();
     if (slices > 1) {
         if (n_steps) finish_cluster(n_steps - 1);
-        cluster_sync();  // no CTA leaves while another reads its sums
+        cluster_sync();  // no CTA leaves, or goes on, while another reads its sums
     }
+    steps_before += n_steps;
+    } while (EXPERTS);
 }
 
 bool switched_off(const char* name) {
@@ -488,9 +536,9 @@ bool few_disabled() {
     return off;
 }
 
-template <bool EXACT, int NT, int W, int DEPTH>
-cudaError_t launch(cudaStream_t stream, FewParams& p, uint32_t groups, uint32_t experts, uint32_t busy_experts) {
-    const void* kernel = (const void*)matmul_few_kernel<EXACT, NT, W, DEPTH>;
+template <bool EXACT, bool EXPERTS, int NT, int W, int DEPTH>
+cudaError_t launch_as(cudaStream_t stream, FewParams& p, uint32_t groups) {
+    const void* kernel = (const void*)matmul_few_kernel<EXACT, EXPERTS, NT, W, DEPTH>;
     const size_t smem = partial_bytes(NT) + (size_t)kWarps * DEPTH * tiles_per_step(NT) * W * kSlotPair;
     cudaError_t e = ensure_dynamic_smem(kernel, smem);
     if (e != cudaSuccess) return e;
@@ -521,9 +569,12 @@ cudaError_t launch(cudaStream_t stream, FewParams& p, uint32_t groups, uint32_t 
         }
         resident = fit[p.slices];
     }
-    // (Few experts get more than 8 entries: their further groups do not count.)
-    const uint32_t share = (uint32_t)resident / (p.offsets ? busy_experts : groups), most = share > 0 ? share : 1;
-    config.gridDim = dim3(p.slices * (p.n_jobs < most ? p.n_jobs : most), groups, experts);
+    if (EXPERTS) {
+        config.gridDim = dim3(p.slices * (unsigned)resident);
+    } else {
+        const uint32_t share = (uint32_t)resident / groups, most = share > 0 ? share : 1;
+        config.gridDim = dim3(p.slices * (p.n_jobs < most ? p.n_jobs : most), groups);
+    }
     if (pdl_enabled()) {
         attributes[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attributes[n].val.programmaticStreamSerializationAllowed = 1;
@@ -531,7 +582,11 @@ cudaError_t launch(cudaStream_t stream, FewParams& p, uint32_t groups, uint32_t 
     }
     config.attrs = attributes;
     config.numAttrs = n;
-    return cudaLaunchKernelEx(&config, matmul_few_kernel<EXACT, NT, W, DEPTH>, (const FewParams)p);
+    return cudaLaunchKernelEx(&config, matmul_few_kernel<EXACT, EXPERTS, NT, W, DEPTH>, (const FewParams)p);
+}
+template <bool EXACT, int NT, int W, int DEPTH>
+cudaError_t launch(cudaStream_t stream, FewParams& p, uint32_t groups) {
+    return p.offsets ? launch_as<EXACT, true, NT, W, DEPTH>(stream, p, groups) : launch_as<EXACT, false, NT, W, DEPTH>(stream, p, groups);
 }
 
 // Cut K: as few CTAs per cluster as hold the inputs at `most` pairs per warp, evenly.
@@ -542,35 +597,29 @@ uint32_t cut(FewParams& p, uint32_t most) {
     return (p.slice_pairs + kWarps - 1) / kWarps;  // pairs per warp
 }
 
-cudaError_t launch_exact(cudaStream_t stream, FewParams& p, uint32_t experts, uint32_t busy_experts) {
+cudaError_t launch_exact(cudaStream_t stream, FewParams& p) {
     const uint32_t groups = (p.n_tokens + 7) / 8;
     switch (cut(p, kMaxPairsPerWarp)) {
-        case 1: return launch<true, 1, 1, 6>(stream, p, groups, experts, busy_experts);
-        case 2: return launch<true, 1, 2, 3>(stream, p, groups, experts, busy_experts);
-        default: return launch<true, 1, 3, 2>(stream, p, groups, experts, busy_experts);
+        case 1: return launch<true, 1, 1, 6>(stream, p, groups);
+        case 2: return launch<true, 1, 2, 3>(stream, p, groups);
+        default: return launch<true, 1, 3, 2>(stream, p, groups);
     }
 }
 
 // Row groups of 8 a launch's CTA holds: the fewest that cover the rows in as few groups of 32 as possible
 // (33 rows: two groups of 24). `rows`: those of the largest (expert: likely) batch.
-cudaError_t launch_half(cudaStream_t stream, FewParams& p, uint32_t rows, uint32_t experts, uint32_t busy_experts) {
+cudaError_t launch_half(cudaStream_t stream, FewParams& p, uint32_t rows) {
     const uint32_t parts = (rows + kHalfGroup - 1) / kHalfGroup, nt = ((rows + parts - 1) / parts + 7) / 8;
     const uint32_t w = cut(p, nt <= 2 ? 3 : 2), groups = (p.n_tokens + 8 * (nt < 2 ? 2 : nt) - 1) / (8 * (nt < 2 ? 2 : nt));
     if (nt <= 2) {
         switch (w) {
-            case 1: return launch<false, 2, 1, 5>(stream, p, groups, experts, busy_experts);
-            case 2: return launch<false, 2, 2, 3>(stream, p, groups, experts, busy_experts);
-            default: return launch<false, 2, 3, 2>(stream, p, groups, experts, busy_experts);
+            case 1: return launch<false, 2, 1, 5>(stream, p, groups);
+            case 2: return launch<false, 2, 2, 3>(stream, p, groups);
+            default: return launch<false, 2, 3, 2>(stream, p, groups);
         }
     }
-    if (nt == 3) return w == 1 ? launch<false, 3, 1, 8>(stream, p, groups, experts, busy_experts) : launch<false, 3, 2, 6>(stream, p, groups, experts, busy_experts);
-    return w == 1 ? launch<false, 4, 1, 8>(stream, p, groups, experts, busy_experts) : launch<false, 4, 2, 6>(stream, p, groups, experts, busy_experts);
-}
-
-// Experts that probably have entries, if the router spreads its picks: each of the others costs CTAs that leave at once.
-uint32_t likely_busy(uint32_t n_experts, uint32_t entries) {
-    const uint32_t busy = (uint32_t)((uint64_t)n_experts * entries / (n_experts + entries));
-    return busy > 0 ? busy : 1;
+    if (nt == 3) return w == 1 ? launch<false, 3, 1, 8>(stream, p, groups) : launch<false, 3, 2, 6>(stream, p, groups);
+    return w == 1 ? launch<false, 4, 1, 8>(stream, p, groups) : launch<false, 4, 2, 6>(stream, p, groups);
 }
 
 }  // namespace
@@ -603,7 +652,7 @@ cudaError_t matmul_exact(cudaStream_t stream, const Mat* const* ws, float* const
     p.norm_weight = norm.weight;
     p.eps = norm.eps;
     p.store = store;
-    return launch_exact(stream, p, 1, 1);
+    return launch_exact(stream, p);
 }
 
 cudaError_t matmul_exact_swiglu(cudaStream_t stream, const Mat& gate, const Mat& up, const float* x, Norm norm, float* y, uint32_t n_tokens) {
@@ -623,7 +672,7 @@ cudaError_t matmul_exact_swiglu(cudaStream_t stream, const Mat& gate, const Mat&
     p.norm_weight = norm.weight;
     p.eps = norm.eps;
     p.store = BC_STORE_OVERWRITE;
-    return launch_exact(stream, p, 1, 1);
+    return launch_exact(stream, p);
 }
 
 bool matmul_exact_experts_supported(const Mat& w, const Mat* up, uint32_t n_rows, uint32_t n_tokens) {
@@ -647,9 +696,10 @@ cudaError_t matmul_exact_experts(cudaStream_t stream, const Mat& w, const Mat* u
     p.store = BC_STORE_OVERWRITE;
     p.offsets = offsets;
     p.entries = entries;
+    p.n_experts = n_experts;
     p.n_used = n_used;
     p.gather = gather;
-    return launch_exact(stream, p, n_experts, likely_busy(n_experts, n_tokens * n_used));
+    return launch_exact(stream, p);
 }
 
 // ---- half-precision operands
@@ -679,7 +729,7 @@ cudaError_t matmul_few(cudaStream_t stream, const Mat* const* ws, float* const* 
     p.token_groups = ((n_tokens + 15u) & ~15u) / 8;
     p.n_tokens = n_tokens;
     p.store = store;
-    return launch_half(stream, p, n_tokens, 1, 1);
+    return launch_half(stream, p, n_tokens);
 }
 
 cudaError_t matmul_few_swiglu(cudaStream_t stream, const Mat& gate, const Mat& up, const void* packed, float* y, uint32_t n_tokens, uint32_t y_stride,
@@ -701,7 +751,7 @@ cudaError_t matmul_few_swiglu(cudaStream_t stream, const Mat& gate, const Mat& u
     p.n_tokens = n_tokens;
     p.store = BC_STORE_OVERWRITE;
     p.packed_out = static_cast<__half*>(packed_out);
-    return launch_half(stream, p, n_tokens, 1, 1);
+    return launch_half(stream, p, n_tokens);
 }
 
 // Experts: any number of tokens, as long as an expert gets a few of them on average (at most 64).
@@ -729,13 +779,14 @@ cudaError_t matmul_few_experts(cudaStream_t stream, const Mat& w, const Mat* up,
     p.store = BC_STORE_OVERWRITE;
     p.offsets = offsets;
     p.entries = entries;
+    p.n_experts = n_experts;
     p.n_used = 1;
     // Groups of rows as wide as an expert's likely share, with room for the busier ones.
     const uint32_t share = (n_entries + n_experts - 1) / n_experts;
     uint32_t rows = share + 1;
     while ((rows - share) * (rows - share) < share) ++rows;
     rows = rows < n_tokens ? rows : n_tokens;
-    return launch_half(stream, p, rows < kHalfGroup ? rows : kHalfGroup, n_experts, likely_busy(n_experts, n_entries));
+    return launch_half(stream, p, rows < kHalfGroup ? rows : kHalfGroup);
 }
 
 }  // namespace k
