@@ -416,6 +416,8 @@ cudaError_t matmul_half_swiglu(cudaStream_t stream, const Mat& gate, const Mat& 
 // the packed inputs on warp-level MMAs, one launch, no split of K left open. matmul_umma,
 // matmul_umma_several, matmul_umma_swiglu and matmul_experts_umma hand over to these whenever the
 // shape allows (BOBCAT_NO_FEW_MATMUL=1 keeps them on the tcgen05 kernels).
+// Code: 1, a warp on the other warps' sums.
+cudaError_t matmul_few_wait_word(int* word);
 bool matmul_few_supported(const Mat& w, uint32_t n_tokens);
 cudaError_t matmul_few(cudaStream_t stream, const Mat* const* ws, float* const* ys, const uint32_t* strides, int n, const void* packed,
                        uint32_t n_tokens, int32_t store);

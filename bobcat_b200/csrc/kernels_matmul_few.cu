@@ -57,6 +57,17 @@ constexpr uint32_t kSpinLimit = 1u << 22;
 constexpr int tiles_per_step(int nt) { return nt <= 2 ? 2 : 1; }
 constexpr uint32_t partial_bytes(int nt) { return 2 * (uint32_t)tiles_per_step(nt) * kWarps * (uint32_t)nt * 512; }
 
+__device__ int* g_wait_word;  // where a wait that ran out leaves its code (kernels.h), null until set
+
+// The rest of a wait whose first poll failed. One that runs out leaves a code and the warp carries on, because the others and the
+// cluster's barriers need it. A function of its own, out of the way of the steps' code: 11 rows of the 350M shape's prompt take 627 us (626
+// without the report), with the loop and the report inline 629 to 648.
+__device__ __noinline__ void wait_on(uint32_t bar, uint32_t parity) {
+    for (uint32_t spin = 1; spin < kSpinLimit; ++spin)
+        if (async::mbar_test(bar, parity)) return;
+    if (g_wait_word) *reinterpret_cast<volatile int*>(g_wait_word) = 1;
+}
+
 struct FewParams {
     // Plain: up to four matrices that share the inputs, a job per tile of their concatenation.
     // Dual: tiles[0] = gate, tiles[1] = up, a job per tile pair.
@@ -489,7 +500,7 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_few_kernel(const __grid_co
         if (u > 0) {
             const uint32_t before = u - 1, turns = steps_before + before;  // buffers and barriers alternate through all groups
             // Every warp arrives for every step whatever happens, so the wait ends; it is bounded like all waits.
-            for (uint32_t spin = 0; spin < kSpinLimit && !async::mbar_test(bars + (turns & 1) * 8, (turns >> 1) & 1); ++spin) {}
+            if (!async::mbar_test(bars + (turns & 1) * 8, (turns >> 1) & 1)) wait_on(bars + (turns & 1) * 8, (turns >> 1) & 1);
             if (slices == 1) {
                 if (my_turn(before)) finish(before, [&](uint32_t h) { return over_warps(before, h); });
             } else {
@@ -623,6 +634,8 @@ cudaError_t launch_half(cudaStream_t stream, FewParams& p, uint32_t rows) {
 }
 
 }  // namespace
+
+cudaError_t matmul_few_wait_word(int* word) { return cudaMemcpyToSymbol(g_wait_word, &word, sizeof word); }
 
 // Up to 64 rows: every group of 8 rows repeats the weights' unpacking, which stays ahead of the tile
 // kernel at any of these counts. The inputs of a row must fit a cluster's registers (24 576 columns).
