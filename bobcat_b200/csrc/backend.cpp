@@ -103,7 +103,7 @@ bc_status bc_backend::pack_scratch(size_t bytes, void** out) {
         pack = nullptr;
         pack_len = 0;
         size_t want = bytes + bytes / 2;
-        BC_CUDA(cudaMalloc(&pack, want));
+        BC_CUDA(device_malloc(&pack, want));
         pack_len = want;
     }
     *out = pack;
@@ -117,7 +117,7 @@ bc_status bc_backend::partial_scratch(size_t bytes, void** out) {
         partials = nullptr;
         partials_len = 0;
         size_t want = bytes + bytes / 2;
-        BC_CUDA(cudaMalloc(&partials, want));
+        BC_CUDA(device_malloc(&partials, want));
         partials_len = want;
     }
     *out = partials;
@@ -152,21 +152,21 @@ bc_status matrix_view(bc_backend* b, bc_buffer* buffer, size_t offset, int32_t f
     return BC_OK;
 }
 
-// Expand an uploaded matrix for products of many tokens, once. Without room the other kernels serve.
-bc_status expand_for_many_tokens(bc_backend* b, bc_buffer* buffer) {
-    if (buffer->half_tiles_tried) return BC_OK;
-    buffer->half_tiles_tried = true;
-    k::Mat& m = buffer->matrix;
-    const uint64_t bytes = k::half_tiles_bytes(m.n_rows, m.n_cols);
-    if (m.format != BC_Q4_0 || !k::half_tiles_supported(m.n_cols) || !k::half_tiles_fit(bytes)) return BC_OK;
-    if (cudaMalloc(&buffer->half_tiles, bytes) != cudaSuccess) {
-        cudaGetLastError();
-        buffer->half_tiles = nullptr;
-        return BC_OK;
-    }
-    m.half_tiles = buffer->half_tiles;
-    BC_CUDA(k::expand_half_tiles(b->stream, m.data, m.scales, m.n_rows, m.n_cols, buffer->half_tiles));
+// Expand an uploaded matrix for products of many tokens, once. Without room, and while the stream is being captured (which
+// forbids the allocation), the other kernels serve. Inside a LaunchScope.
+bc_status expand_for_many_tokens(bc_backend* b, bc_buffer* buffer, bool capturing) {
+    if (buffer->expanded || capturing) return BC_OK;
+    buffer->expanded.reset(new ExpandedCopies());
+    BC_CUDA(buffer->expanded->expand(b->device, b->stream, {&buffer->matrix}));
+    buffer->expanded->offer();
     return BC_OK;
+}
+
+bool is_capturing(cudaStream_t stream) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &status) == cudaSuccess) return status != cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return true;
 }
 
 // The vectorised kernels read activations 16 bytes at a time: views of activation vectors must
@@ -203,6 +203,7 @@ bc_status bc_backend_open(int32_t device, void* stream, bc_backend** out) {
         BC_CUDA(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
         b->owns_stream = true;
     }
+    backend_opened(b.get());
     *out = b.release();
     return BC_OK;
 }
@@ -214,14 +215,15 @@ void bc_backend_close(bc_backend* b) {
     // Sequences that outlive their backend give up their device state now and stay behind as
     // handles that only bc_seq_free may still be called on.
     while (!b->seqs.empty()) release_seq(*b->seqs.begin());
+    backend_closing(b);
     for (auto& t : b->tickets) cudaEventDestroy(t.second);
     for (auto& t : b->ticket_starts) cudaEventDestroy(t.second);
     if (b->record_start) cudaEventDestroy(b->record_start);
     // Buffers that outlive their backend are orphaned; their frees become no-ops on the pointer.
     for (bc_buffer* buffer : b->buffers) {
         cudaFree(buffer->ptr);
-        cudaFree(buffer->half_tiles);
-        buffer->ptr = buffer->half_tiles = nullptr;
+        buffer->ptr = nullptr;
+        buffer->expanded.reset();
         buffer->backend = nullptr;
     }
     if (b->pack) cudaFree(b->pack);
@@ -239,7 +241,7 @@ bc_status bc_buffer_new(bc_backend* b, size_t len, bc_buffer** out) {
     buffer->backend = b;
     buffer->len = len;
     if (len) {
-        cudaError_t e = cudaMalloc(&buffer->ptr, len);
+        cudaError_t e = device_malloc(&buffer->ptr, len);
         if (e != cudaSuccess) return fail(BC_ERR_ALLOCATION, "cannot allocate a device buffer of %zu bytes: %s", len, cudaGetErrorString(e));
         e = cudaMemsetAsync(buffer->ptr, 0, len, b->stream);
         if (e != cudaSuccess) {
@@ -261,7 +263,6 @@ void bc_buffer_free(bc_buffer* buffer) {
         cudaStreamSynchronize(buffer->backend->stream);
         buffer->backend->buffers.erase(buffer);
         cudaFree(buffer->ptr);
-        cudaFree(buffer->half_tiles);
     }
     delete buffer;
 }
@@ -317,7 +318,7 @@ bc_status bc_matrix_upload(bc_backend* b, int32_t format, const void* data, uint
         uint64_t n_blocks = (uint64_t)n_rows * (n_cols / 32);
         buffer->matrix.scales = reinterpret_cast<const __half*>(static_cast<char*>(buffer->ptr) + n_blocks * 16);
         void* raw = nullptr;
-        cudaError_t e = cudaMalloc(&raw, raw_bytes);
+        cudaError_t e = device_malloc(&raw, raw_bytes);
         if (e != cudaSuccess) status = fail(BC_ERR_ALLOCATION, "cannot allocate %llu staging bytes", (unsigned long long)raw_bytes);
         if (status == BC_OK && (e = cudaMemcpyAsync(raw, data, raw_bytes, cudaMemcpyHostToDevice, b->stream)) != cudaSuccess) status = cuda_fail(e, "upload");
         if (status == BC_OK && (e = k::repack_q4_0(b->stream, static_cast<const uint8_t*>(raw), n_blocks, buffer->ptr,
@@ -526,16 +527,26 @@ bc_status bc_op_matmul(bc_backend* b, int32_t format, bc_buffer* weights, size_t
     BC_TRY(need_recording(b));
     if (store < BC_STORE_OVERWRITE || store > BC_STORE_SWIGLU) return fail(BC_ERR_ARGUMENT, "unknown store mode %d", store);
     k::Mat w;
+    LaunchScope scope(b->device);
     BC_TRY(matrix_view(b, weights, w_off, format, n_rows, n_cols, "matmul", &w));
-    if (n_tokens >= k::kExpandTokens) {
-        BC_TRY(expand_for_many_tokens(b, weights));
+    if (n_tokens >= k::kMinHalfTokens && format == BC_Q4_0) {
+        const bool capturing = is_capturing(b->stream);
+        if (n_tokens >= k::kExpandTokens) BC_TRY(expand_for_many_tokens(b, weights, capturing));
+        if (capturing && weights->expanded) weights->expanded->pin();  // the caller's graph will read the copy
         BC_TRY(matrix_view(b, weights, w_off, format, n_rows, n_cols, "matmul", &w));
     }
     BC_TRY(check_range(b, x, x_off, (size_t)n_tokens * n_cols * 4, "matmul"));
     BC_TRY(check_range(b, y, y_off, (size_t)n_tokens * n_rows * 4, "matmul"));
     BC_TRY(check_aligned("matmul", {x_off, y_off}));
     void* pack = nullptr;
-    if (k::matmul_umma_supported(w, n_tokens)) BC_TRY(b->pack_scratch(k::matmul_scratch_bytes(w, n_tokens), &pack));
+    if (k::matmul_umma_supported(w, n_tokens)) {
+        const void* expanded;
+        do {  // growing the scratch may take the expanded copy, and what the product needs changes with it
+            expanded = w.half_tiles;
+            BC_TRY(b->pack_scratch(k::matmul_scratch_bytes(w, n_tokens), &pack));
+            BC_TRY(matrix_view(b, weights, w_off, format, n_rows, n_cols, "matmul", &w));
+        } while (w.half_tiles != expanded);
+    }
     return b->run("matmul", n_rows, n_cols, w.bytes(), pack ? k::matmul_umma_launches(w, n_tokens, store) : 1, [&] {
         return k::matmul(b->stream, w, reinterpret_cast<const float*>(at(x, x_off)), reinterpret_cast<float*>(at(y, y_off)), n_tokens,
                          n_rows, store, pack);

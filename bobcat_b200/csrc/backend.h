@@ -14,6 +14,7 @@
 #include "common.h"
 #include "gguf.h"
 #include "kernels.h"
+#include "optional_memory.h"
 
 struct bc_seq;
 
@@ -25,9 +26,8 @@ struct bc_buffer {
     bool is_matrix = false;
     bc::k::Mat matrix;
     // The matrix expanded for products of many tokens, made by the first such product (most uploaded
-    // matrices, expert stacks among them, never meet one), unless the device had no room then.
-    void* half_tiles = nullptr;
-    bool half_tiles_tried = false;
+    // matrices, expert stacks among them, never meet one), unless the device had no room then; given back when something else needs it.
+    std::unique_ptr<bc::ExpandedCopies> expanded;
 };
 
 // Token slots in host-mapped memory that argmax launches write and the CPU reads once the

@@ -71,7 +71,7 @@ bc_status bc_batch_new(bc_model* model, bc_backend* backend, uint32_t n_seqs, ui
     }
     const size_t words = (size_t)n_seqs;
     size_t bytes = round_up(words * 4, 256) * 2 + round_up(words * sizeof(void*), 256) * 3 + round_up(words * hp.n_vocab * 4, 256);
-    cudaError_t e = cudaMalloc(&b->arena, bytes);
+    cudaError_t e = device_malloc(&b->arena, bytes);
     if (e != cudaSuccess) return fail(BC_ERR_ALLOCATION, "cannot allocate %zu bytes of batch state: %s", bytes, cudaGetErrorString(e));
     BC_CUDA(cudaMemsetAsync(b->arena, 0, bytes, backend->stream));
     char* p = static_cast<char*>(b->arena);
@@ -159,7 +159,7 @@ bc_status bc_batch_generate(bc_batch* batch, uint32_t* out, size_t n_tokens) {
         cudaFree(batch->generated);
         batch->generated = nullptr;
         batch->generated_cap = 0;
-        cudaError_t e = cudaMalloc(&batch->generated, (size_t)n_seqs * n * 4);
+        cudaError_t e = device_malloc(&batch->generated, (size_t)n_seqs * n * 4);
         if (e != cudaSuccess) return fail(BC_ERR_ALLOCATION, "cannot allocate the generated tokens: %s", cudaGetErrorString(e));
         batch->generated_cap = n;
     }

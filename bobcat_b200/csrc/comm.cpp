@@ -86,7 +86,7 @@ void setup_peer_buffers(bc_comm* c, Nccl* lib) {
     // Every rank takes part in the exchange below whatever happened here, so the collective completes.
     // The zeroed flags and epoch must be in memory before any peer's first store: the exchange
     // below orders every rank's first launch after every rank's synchronize here.
-    bool ok = cudaMalloc(&c->peer_local, bytes) == cudaSuccess && cudaMemset(c->peer_local, 0, bytes) == cudaSuccess &&
+    bool ok = device_malloc(&c->peer_local, bytes) == cudaSuccess && cudaMemset(c->peer_local, 0, bytes) == cudaSuccess &&
               cudaDeviceSynchronize() == cudaSuccess;
     cudaIpcMemHandle_t handle;
     std::memset(&handle, 0, sizeof handle);
@@ -102,7 +102,7 @@ void setup_peer_buffers(bc_comm* c, Nccl* lib) {
     mine.handle = handle;
     mine.ok = ok ? 1 : 0;
     Entry* exchange = nullptr;
-    if (cudaMalloc(&exchange, sizeof(Entry) * c->world) != cudaSuccess) return;
+    if (device_malloc(&exchange, sizeof(Entry) * c->world) != cudaSuccess) return;
     cudaMemcpyAsync(exchange + c->rank, &mine, sizeof mine, cudaMemcpyHostToDevice, stream);
     int rc = lib->AllGather(exchange + c->rank, exchange, sizeof(Entry), /*ncclUint8*/ 1, c->nccl, stream);
     std::vector<Entry> all(c->world);
@@ -123,7 +123,7 @@ void setup_peer_buffers(bc_comm* c, Nccl* lib) {
     }
     // The ranks agree on whether everyone mapped everyone: a sum of successes over ranks.
     float* votes = nullptr;
-    if (cudaMalloc(&votes, 4) != cudaSuccess) return;
+    if (device_malloc(&votes, 4) != cudaSuccess) return;
     const float vote = mapped ? 1.f : 0.f;
     cudaMemcpyAsync(votes, &vote, 4, cudaMemcpyHostToDevice, stream);
     float total = 0.f;
@@ -250,7 +250,7 @@ void bc_comm_free(bc_comm* comm) {
         // No rank unmaps or frees a buffer a peer may still write: meet first (a one-word sum).
         if (comm->peer_ready && lib->AllReduce) {
             float* word = nullptr;
-            if (cudaMalloc(&word, 4) == cudaSuccess) {
+            if (device_malloc(&word, 4) == cudaSuccess) {
                 cudaMemsetAsync(word, 0, 4, comm->backend->stream);
                 lib->AllReduce(word, word, 1, kNcclFloat32, kNcclSum, comm->nccl, comm->backend->stream);
                 cudaStreamSynchronize(comm->backend->stream);

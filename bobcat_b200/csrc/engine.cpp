@@ -208,7 +208,7 @@ bc_status bc_engine_score(bc_engine* e, const uint32_t* prompt_tokens, const siz
         if (e->scoring) BC_CUDA(cudaFree(e->scoring));
         e->scoring = nullptr;
         e->scoring_bytes = 0;
-        BC_CUDA(cudaMalloc(&e->scoring, bytes));
+        BC_CUDA(device_malloc(&e->scoring, bytes));
         e->scoring_bytes = bytes;
     }
     double* scratch = static_cast<double*>(e->scoring);

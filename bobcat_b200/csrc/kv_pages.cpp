@@ -6,6 +6,8 @@
 
 #include <mutex>
 
+#include "optional_memory.h"
+
 using namespace bc;
 
 namespace {
@@ -54,7 +56,9 @@ bc_status new_page(int device, uint64_t bytes, std::shared_ptr<PhysicalPage>* ou
     CUmemAllocationProp prop = device_memory(device);
     auto page = std::make_shared<PhysicalPage>();
     page->device = device;
-    CUresult r = d->Create(&page->handle, bytes, &prop, 0);
+    CUresult r = CUDA_SUCCESS;
+    do r = d->Create(&page->handle, bytes, &prop, 0);
+    while (r == CUDA_ERROR_OUT_OF_MEMORY && give_back_copies(device));
     if (r != CUDA_SUCCESS) {
         page->handle = 0;
         return driver_fail(r, "cuMemCreate");
@@ -100,6 +104,7 @@ bc_status PagedCache::create(int device, const PageGeometry& geometry) {
         BC_TRY(new_page(device, geometry.page_bytes(), &page));
         BC_TRY(map(slot, page));
     }
+    keep_room(reserved_);
     return BC_OK;
 }
 

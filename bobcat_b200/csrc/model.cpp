@@ -285,8 +285,21 @@ uint64_t device_bytes(const HostMatrix& hm) {
 bc::DeviceModel::~DeviceModel() {
     if (arena || !extra.empty()) cudaSetDevice(device);
     if (arena) cudaFree(arena);
-    if (half_arena) cudaFree(half_arena);
     for (void* p : extra) cudaFree(p);
+}
+
+bc_status bc::DeviceModel::expand_dense(cudaStream_t stream, const std::vector<LayerSpec>& specs) {
+    std::vector<k::Mat*> dense;
+    for (size_t il = 0; il < layers.size(); ++il) {
+        DeviceLayer& D = layers[il];
+        for (k::Mat* m : {&D.q, &D.k, &D.v, &D.output, &D.in_proj, &D.out_proj, &D.qkv, &D.z, &D.beta, &D.alpha, &D.ssm_out}) dense.push_back(m);
+        if (specs[il].moe) continue;
+        for (k::Mat* m : {&D.gate, &D.up, &D.down}) dense.push_back(m);
+    }
+    BC_CUDA(expanded.expand(device, stream, dense));
+    BC_CUDA(cudaStreamSynchronize(stream));
+    expanded.offer();
+    return BC_OK;
 }
 
 bc_status bc_model::device_model(bc_backend* backend, std::shared_ptr<DeviceModel>* out) {
@@ -324,12 +337,12 @@ bc_status bc_model::device_model(bc_backend* backend, std::shared_ptr<DeviceMode
         for (const HostVector* hv : {&S.attn_norm, &S.ffn_norm, &S.q_norm, &S.k_norm, &S.taps, &S.conv1d, &S.dt_bias, &S.a, &S.ssm_norm, &S.expert_bias})
             plan_vector(*hv);
     }
-    cudaError_t e = cudaMalloc(&dm->arena, total ? total : 256);
+    cudaError_t e = device_malloc(&dm->arena, total ? total : 256);
     if (e != cudaSuccess) return fail(BC_ERR_ALLOCATION, "cannot allocate %llu bytes of device weights: %s", (unsigned long long)total, cudaGetErrorString(e));
     dm->arena_bytes = total;
     void* staging = nullptr;
     if (largest_raw) {
-        e = cudaMalloc(&staging, largest_raw);
+        e = device_malloc(&staging, largest_raw);
         if (e != cudaSuccess) return fail(BC_ERR_ALLOCATION, "cannot allocate %llu staging bytes: %s", (unsigned long long)largest_raw, cudaGetErrorString(e));
     }
     struct Free {
@@ -411,32 +424,7 @@ bc_status bc_model::device_model(bc_backend* backend, std::shared_ptr<DeviceMode
         BC_TRY(upload_vector(S.ssm_norm, &D.ssm_norm));
         BC_TRY(upload_vector(S.expert_bias, &D.expert_bias));
     }
-    // The expanded copies of the dense matrices (an expert's matrices meet a few tokens at a time).
-    std::vector<k::Mat*> dense;
-    uint64_t half_bytes = 0;
-    for (size_t il = 0; il < layers.size(); ++il) {
-        DeviceLayer& D = dm->layers[il];
-        for (k::Mat* m : {&D.q, &D.k, &D.v, &D.output, &D.in_proj, &D.out_proj, &D.qkv, &D.z, &D.beta, &D.alpha, &D.ssm_out, &D.gate, &D.up, &D.down}) {
-            if (layers[il].moe && (m == &D.gate || m == &D.up || m == &D.down)) continue;
-            if (!m->data || m->format != BC_Q4_0 || !k::half_tiles_supported(m->n_cols)) continue;
-            dense.push_back(m);
-            half_bytes += k::half_tiles_bytes(m->n_rows, m->n_cols);
-        }
-    }
-    if (half_bytes && k::half_tiles_fit(half_bytes)) {
-        if (cudaMalloc(&dm->half_arena, half_bytes) != cudaSuccess) {
-            cudaGetLastError();
-            dm->half_arena = nullptr;
-        } else {
-            char* at = static_cast<char*>(dm->half_arena);
-            for (k::Mat* m : dense) {
-                BC_CUDA(k::expand_half_tiles(backend->stream, m->data, m->scales, m->n_rows, m->n_cols, at));
-                m->half_tiles = at;
-                at += k::half_tiles_bytes(m->n_rows, m->n_cols);
-            }
-        }
-    }
-    BC_CUDA(cudaStreamSynchronize(backend->stream));
+    BC_TRY(dm->expand_dense(backend->stream, layers));
     on_device[backend->device] = dm;
     *out = dm;
     return BC_OK;

@@ -55,7 +55,6 @@ struct DeviceModel {
     int device = 0;
     void* arena = nullptr;
     size_t arena_bytes = 0;
-    void* half_arena = nullptr;  // the dense Q4_0 matrices expanded for products of many tokens; null when they do not fit
     std::vector<DeviceLayer> layers;
     k::Mat token_embd, output;
     const float* output_norm = nullptr;
@@ -63,6 +62,11 @@ struct DeviceModel {
     std::vector<void*> extra;
     // Tensor parallelism: the rows of the output matrix this rank multiplies (all of them otherwise).
     uint32_t first_vocab_row = 0, n_vocab_rows = 0;
+    // The dense Q4_0 matrices expanded for products of many tokens, when they fit. Declared after the matrices, which giving back looks at.
+    ExpandedCopies expanded;
+    // Make the expanded copies, once the uploads are queued on `stream`, and wait for it. Experts' matrices, which
+    // meet a few tokens at a time, stay as they are.
+    bc_status expand_dense(cudaStream_t stream, const std::vector<LayerSpec>& specs);
     ~DeviceModel();
 };
 

@@ -44,7 +44,7 @@ struct Uploader {
 
     bc_status device_alloc(size_t bytes, char** out) {
         void* p = nullptr;
-        cudaError_t e = cudaMalloc(&p, bytes ? bytes : 256);
+        cudaError_t e = device_malloc(&p, bytes ? bytes : 256);
         if (e != cudaSuccess) return fail(BC_ERR_ALLOCATION, "cannot allocate %zu bytes of device weights: %s", bytes, cudaGetErrorString(e));
         dm.extra.push_back(p);
         *out = static_cast<char*>(p);
@@ -69,7 +69,7 @@ struct Uploader {
                 if (staging) cudaFree(staging);
                 staging = nullptr;
                 staging_cap = 0;
-                cudaError_t e = cudaMalloc(&staging, host.size() + host.size() / 4);
+                cudaError_t e = device_malloc(&staging, host.size() + host.size() / 4);
                 if (e != cudaSuccess) return fail(BC_ERR_ALLOCATION, "cannot allocate %zu staging bytes", host.size());
                 staging_cap = host.size() + host.size() / 4;
             }
@@ -80,13 +80,6 @@ struct Uploader {
                 char* tiles = dst + aligned(n_blocks * 16) + aligned(n_blocks * 2);
                 mat->tiles = tiles;
                 BC_CUDA(k::repack_tiles(stream, dst, mat->scales, n_rows, n_cols, tiles));
-            }
-            const uint64_t half_bytes = k::half_tiles_bytes(n_rows, n_cols);
-            if (k::half_tiles_supported(n_cols) && k::half_tiles_fit(half_bytes)) {
-                char* half_tiles = nullptr;
-                BC_TRY(device_alloc(half_bytes, &half_tiles));
-                BC_CUDA(k::expand_half_tiles(stream, dst, mat->scales, n_rows, n_cols, half_tiles));
-                mat->half_tiles = half_tiles;
             }
             BC_CUDA(cudaStreamSynchronize(stream));
             return BC_OK;
@@ -276,6 +269,7 @@ bc_status bc_model::device_model_tp(bc_backend* backend, int rank, int world, st
         BC_TRY(up.rows(S.up, {ff}, &D.up));
         BC_TRY(up.cols(S.down, {ff}, &D.down));
     }
+    BC_TRY(dm->expand_dense(backend->stream, layers));
     on_device_tp[key] = dm;
     *out = dm;
     return BC_OK;

@@ -136,8 +136,14 @@ struct Recorder {
     void product_of_packed(const k::Mat& w, const void* packed, float* y, uint32_t n, int store) {
         close_sum();  // the partial scratch is about to be reused (or regrown)
         void* partial = nullptr;
-        const uint64_t partial_bytes = k::matmul_partial_bytes(w, n, store);
-        if (status == BC_OK && partial_bytes) status = s.backend->partial_scratch(partial_bytes, &partial);
+        uint64_t partial_bytes;
+        const void* expanded;
+        do {  // growing the scratch may take the expanded copies, and what the product needs changes with them
+            expanded = w.half_tiles;
+            partial_bytes = k::matmul_partial_bytes(w, n, store);
+            partial = nullptr;
+            if (status == BC_OK && partial_bytes) status = s.backend->partial_scratch(partial_bytes, &partial);
+        } while (w.half_tiles != expanded);
         k::Deferred left{};
         const bool may_defer = store == BC_STORE_ACCUMULATE;
         run("matmul", w.n_rows, w.n_cols, w.bytes(), 1, [&] {
@@ -692,6 +698,7 @@ struct Recorder {
     // each row computes what lfm2_step computes for its sequence (lfm2_metal.rs:1162-1242).
     // `tokens` holds the n token ids; logits go to `all_logits` ([n][n_vocab]).
     void lfm2_seqs_step(const uint32_t* tokens, uint32_t n, k::SeqTable seqs, float* all_logits, const ExpertParallel* ep = nullptr) {
+        const LaunchScope scope(s.backend->device);
         const DeviceModel& W = *s.weights;
         const uint32_t n_embd = hp.n_embd, q_dim = hp.n_heads * hp.head_dim;
         run("embed", n, n_embd, 0, 1, [&] { return k::embed(stream, W.token_embd, tokens, k::Pos{nullptr, 0}, s.hidden, n); });
@@ -735,6 +742,7 @@ struct Recorder {
     }
 
     void batch(uint32_t pos, uint32_t n, bool want_logits, bool traced, size_t trace_stride) {
+        const LaunchScope scope(s.backend->device);
         if (hp.architecture == BC_ARCH_QWEN35) qwen_batch(pos, n, want_logits, traced, trace_stride);
         else lfm2_batch(pos, n, want_logits, traced, trace_stride);
         close_sum();  // the last layer's product, when no logits were asked for

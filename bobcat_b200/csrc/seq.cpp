@@ -29,8 +29,8 @@ bc_status ensure_trace_rows(bc_seq* s, uint32_t rows) {
     s->trace_rows = 0;
     size_t floats = (size_t)rows * hp.n_embd;
     size_t route_words = std::max<size_t>(1, (size_t)rows * hp.n_layers * 2 * hp.n_experts_used);
-    if (cudaMalloc(&s->trace_embedding, floats * 4) != cudaSuccess || cudaMalloc(&s->trace_layers, floats * 4 * hp.n_layers) != cudaSuccess ||
-        cudaMalloc(&s->trace_final, floats * 4) != cudaSuccess || cudaMalloc(&s->trace_routes, route_words * 4) != cudaSuccess ||
+    if (device_malloc(&s->trace_embedding, floats * 4) != cudaSuccess || device_malloc(&s->trace_layers, floats * 4 * hp.n_layers) != cudaSuccess ||
+        device_malloc(&s->trace_final, floats * 4) != cudaSuccess || device_malloc(&s->trace_routes, route_words * 4) != cudaSuccess ||
         cudaMemset(s->trace_routes, 0, route_words * 4) != cudaSuccess)
         return fail(BC_ERR_ALLOCATION, "cannot allocate trace buffers for %u tokens", rows);
     s->trace_rows = rows;
@@ -83,6 +83,7 @@ bc_status capture_step(bc_seq* s, StepKind kind) {
     cudaStream_t stream = s->backend->stream;
     const uint32_t n_vocab = s->hp.n_vocab;
     uint64_t before = s->launches;
+    std::unique_ptr<LaunchScope> scope(new LaunchScope(s->backend->device));
     BC_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
     Recorder r(*s);
     r.replayed = true;
@@ -101,6 +102,7 @@ bc_status capture_step(bc_seq* s, StepKind kind) {
     }
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamEndCapture(stream, &graph);
+    scope.reset();
     uint64_t kernels = s->launches - before;
     s->launches = before;  // capturing launches nothing
     if (r.status != BC_OK) {
@@ -109,7 +111,7 @@ bc_status capture_step(bc_seq* s, StepKind kind) {
     }
     if (e != cudaSuccess) return cuda_fail(e, "cudaStreamEndCapture");
     cudaGraphExec_t exec = nullptr;
-    e = cudaGraphInstantiate(&exec, graph, 0);
+    while ((e = cudaGraphInstantiate(&exec, graph, 0)) == cudaErrorMemoryAllocation && give_back_copies(s->backend->device)) cudaGetLastError();
     cudaGraphDestroy(graph);
     if (e != cudaSuccess) return cuda_fail(e, "cudaGraphInstantiate");
     if (kind == kStream) {
@@ -358,7 +360,7 @@ bc_status seq_new(bc_model* model, bc_backend* backend, bc_comm* tp, uint32_t n_
     BC_CUDA(k::matvec_prepare(widest));
     size_t total = 0;
     for (Item& it : items) total += round_up(std::max<size_t>(it.bytes, 4), 256);
-    cudaError_t e = cudaMalloc(&s->arena, total);
+    cudaError_t e = device_malloc(&s->arena, total);
     if (e != cudaSuccess) return fail(BC_ERR_ALLOCATION, "cannot allocate %zu bytes of sequence state: %s", total, cudaGetErrorString(e));
     s->arena_bytes = total;
     BC_CUDA(cudaMemsetAsync(s->arena, 0, total, backend->stream));
@@ -802,7 +804,7 @@ bc_status bc_seq_prefix_save(bc_seq* s, bc_prefix** out) {
     p->conv_floats = s->conv_floats;
     p->delta_floats = s->delta_floats;
     const size_t state_floats = s->conv_floats + s->delta_floats + hp.n_vocab;
-    cudaError_t e = cudaMalloc(&p->state, state_floats * 4);
+    cudaError_t e = device_malloc(&p->state, state_floats * 4);
     if (e != cudaSuccess) return fail(BC_ERR_ALLOCATION, "cannot allocate %zu bytes for the prefix state: %s", state_floats * 4, cudaGetErrorString(e));
     if (s->conv_floats) BC_CUDA(cudaMemcpyAsync(p->state, s->conv_state, s->conv_floats * 4, cudaMemcpyDeviceToDevice, stream));
     if (s->delta_floats) BC_CUDA(cudaMemcpyAsync(p->state + s->conv_floats, s->delta_state, s->delta_floats * 4, cudaMemcpyDeviceToDevice, stream));
@@ -826,7 +828,7 @@ bc_status bc_seq_prefix_save(bc_seq* s, bc_prefix** out) {
     p->tail_rows = s->n_past - first_copied;
     if (p->tail_rows && hp.n_attention_layers) {
         const size_t layer_bytes = (size_t)p->tail_rows * kv_dim * element;
-        e = cudaMalloc(&p->tail, 2 * hp.n_attention_layers * layer_bytes);
+        e = device_malloc(&p->tail, 2 * hp.n_attention_layers * layer_bytes);
         if (e != cudaSuccess) return fail(BC_ERR_ALLOCATION, "cannot allocate the prefix's KV rows: %s", cudaGetErrorString(e));
         for (int which = 0; which < 2; ++which)
             for (uint32_t layer = 0; layer < hp.n_attention_layers; ++layer) {
