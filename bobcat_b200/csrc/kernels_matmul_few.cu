@@ -33,6 +33,7 @@
 #include <cstdlib>
 
 #include "async_utils.cuh"
+#include "device_facts.h"
 #include "device_utils.cuh"
 #include "kernels.h"
 #include "../../include/bobcat_cuda.h"
@@ -566,19 +567,20 @@ cudaError_t launch_as(cudaStream_t stream, FewParams& p, uint32_t groups) {
         ++n;
     }
     // Clusters that fit on the device at once: a cluster lives inside one GPC, so a few SMs stay over.
-    static int fit[kMaxSlices + 1] = {};
+    static DeviceFacts<kMaxSlices + 1> fit;
     int resident = sm_count();
     if (p.slices > 1) {
-        if (fit[p.slices] == 0) {
+        int device = 0;
+        cudaGetDevice(&device);
+        const bool known = fit.get(device, (int)p.slices, [&](int* clusters) {
             config.gridDim = dim3(p.slices * (unsigned)sm_count());
             config.attrs = attributes;
             config.numAttrs = n;
-            int clusters = 0;
-            e = cudaOccupancyMaxActiveClusters(&clusters, kernel, &config);
-            if (e != cudaSuccess) return e;
-            fit[p.slices] = clusters > 0 ? clusters : 1;
-        }
-        resident = fit[p.slices];
+            e = cudaOccupancyMaxActiveClusters(clusters, kernel, &config);
+            if (e == cudaSuccess && *clusters < 1) *clusters = 1;
+            return e == cudaSuccess;
+        }, &resident);
+        if (!known) return e;
     }
     if (EXPERTS) {
         config.gridDim = dim3(p.slices * (unsigned)resident);

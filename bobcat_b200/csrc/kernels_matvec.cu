@@ -24,6 +24,7 @@
 #include <mutex>
 #include <utility>
 
+#include "device_facts.h"
 #include "matvec_common.cuh"
 
 namespace bc {
@@ -182,13 +183,13 @@ __global__ void __launch_bounds__(kThreads) matvec_kernel(Params p) {
 }
 
 int sm_count_impl() {
-    static int count = 0;
-    if (count == 0) {
-        int device = 0;
-        cudaGetDevice(&device);
-        cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, device);
-        if (count <= 0) count = 148;
-    }
+    static DeviceFacts<1> sms;
+    int device = 0, count = 0;
+    cudaGetDevice(&device);
+    sms.get(device, 0, [&](int* n) {
+        if (cudaDeviceGetAttribute(n, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || *n <= 0) *n = 148;
+        return true;
+    }, &count);
     return count;
 }
 
