@@ -143,6 +143,7 @@ SIGNATURES = {
     "bc_engine_score": (i32, [vp, vp, vp, sz, vp, vp, vp]),
     "bc_engine_consumed": (u32, [vp]),
     "bc_seq_launches": (u64, [vp]),
+    "bc_test_matmul_swiglu": (i32, [vp, vp, vp, u32, u32, vp, vp, u32, i32, C.POINTER(i32)]),
     "bc_seq_set_skip": (i32, [vp, C.c_char_p, u32, u32]),
 }
 

@@ -553,6 +553,48 @@ bc_status bc_op_matmul(bc_backend* b, int32_t format, bc_buffer* weights, size_t
     });
 }
 
+bc_status bc_test_matmul_swiglu(bc_backend* b, bc_buffer* gate, bc_buffer* up, uint32_t n_rows, uint32_t n_cols, bc_buffer* x, bc_buffer* y,
+                                uint32_t n_tokens, int32_t packed, int32_t* form) {
+    BC_TRY(need_recording(b));
+    if (!form) return fail(BC_ERR_ARGUMENT, "form must be non-null");
+    k::Mat g, u;
+    LaunchScope scope(b->device);
+    auto look = [&]() -> bc_status {
+        BC_TRY(matrix_view(b, gate, 0, BC_Q4_0, n_rows, n_cols, "swiglu", &g));
+        return matrix_view(b, up, 0, BC_Q4_0, n_rows, n_cols, "swiglu", &u);
+    };
+    BC_TRY(look());
+    if (n_tokens >= k::kExpandTokens) {
+        const bool capturing = is_capturing(b->stream);
+        for (bc_buffer* w : {gate, up}) {
+            BC_TRY(expand_for_many_tokens(b, w, capturing));
+            if (capturing && w->expanded) w->expanded->pin();
+        }
+        BC_TRY(look());
+    }
+    const bool tensor = k::matmul_umma_swiglu_supported(g, u, n_tokens);
+    if (!tensor && !k::matmul_exact_supported(g, n_tokens)) return fail(BC_ERR_UNSUPPORTED, "no SwiGLU product in one launch for %u tokens of %u columns", n_tokens, n_cols);
+    if (packed && (!tensor || n_rows % 64 != 0)) return fail(BC_ERR_ARGUMENT, "a packed result needs 16 tokens and a multiple of 64 rows");
+    if (!y) {
+        *form = tensor ? k::matmul_umma_swiglu_form(g, u, n_tokens) : BC_SWIGLU_EXACT;
+        return BC_OK;
+    }
+    BC_TRY(check_range(b, x, 0, (size_t)n_tokens * n_cols * 4, "swiglu"));
+    BC_TRY(check_range(b, y, 0, packed ? k::matmul_pack_bytes(n_tokens, n_rows) : (size_t)n_tokens * n_rows * 4, "swiglu"));
+    const float* xp = reinterpret_cast<const float*>(at(x, 0));
+    float* yp = reinterpret_cast<float*>(at(y, 0));
+    void* pack = nullptr;
+    if (tensor) BC_TRY(b->pack_scratch(k::matmul_pack_bytes(n_tokens, n_cols), &pack));
+    BC_TRY(look());  // the scratch may have taken the expanded copies
+    *form = tensor ? k::matmul_umma_swiglu_form(g, u, n_tokens) : BC_SWIGLU_EXACT;
+    if (!tensor)
+        return b->run("swiglu", n_rows, n_cols, 2 * g.bytes(), 1, [&] { return k::matmul_exact_swiglu(b->stream, g, u, xp, k::Norm{}, yp, n_tokens); });
+    return b->run("swiglu", n_rows, n_cols, 2 * g.bytes(), 2, [&] {
+        const cudaError_t e = k::matmul_pack(b->stream, xp, n_tokens, n_cols, pack);
+        return e != cudaSuccess ? e : k::matmul_umma_swiglu(b->stream, g, u, pack, packed ? nullptr : yp, n_tokens, n_rows, packed ? yp : nullptr);
+    });
+}
+
 bc_status bc_op_expand(bc_backend* b, int32_t format, bc_buffer* weights, size_t w_off, bc_buffer* out, size_t out_off,
                        uint32_t n_rows, uint32_t n_cols, int32_t out_half) {
     BC_TRY(need_recording(b));

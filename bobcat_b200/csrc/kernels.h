@@ -392,6 +392,8 @@ bool matmul_umma_swiglu_supported(const Mat& gate, const Mat& up, uint32_t n_tok
 // is not touched.
 cudaError_t matmul_umma_swiglu(cudaStream_t stream, const Mat& gate, const Mat& up, const void* packed, float* y, uint32_t n_tokens,
                                uint32_t y_stride, void* packed_out = nullptr);
+// Which kernel it runs on (bc_test_matmul_swiglu's codes).
+int matmul_umma_swiglu_form(const Mat& gate, const Mat& up, uint32_t n_tokens);
 // The same products from expanded weights (kernels_matmul_half.cu), for batches of kMinHalfTokens and more
 // of matrices that carry half_tiles; the functions above hand over to them (BOBCAT_NO_HALF_MATMUL=1: no
 // matrix gets half_tiles).
@@ -412,6 +414,7 @@ cudaError_t matmul_half(cudaStream_t stream, const Mat* const* ws, float* const*
                         int32_t store, uint32_t split);
 cudaError_t matmul_half_swiglu(cudaStream_t stream, const Mat& gate, const Mat& up, const void* packed, float* y, uint32_t n_tokens, uint32_t y_stride,
                                void* packed_out);
+bool matmul_half_swiglu_whole(const Mat& gate, uint32_t n_tokens);  // tiles of 128 rows of both matrices, else of 64 rows of either
 // The same products for at most 32 tokens (kernels_matmul_few.cu): the matrices' decode tiles against
 // the packed inputs on warp-level MMAs, one launch, no split of K left open. matmul_umma,
 // matmul_umma_several, matmul_umma_swiglu and matmul_experts_umma hand over to these whenever the

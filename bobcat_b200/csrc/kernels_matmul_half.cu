@@ -524,6 +524,10 @@ cudaError_t matmul_half(cudaStream_t stream, const Mat* const* ws, float* const*
     return launch_half(stream, p, tiling);
 }
 
+bool matmul_half_swiglu_whole(const Mat& gate, uint32_t n_tokens) {
+    return choose_tiling(gate.n_rows, gate.n_cols / kChunkK, n_tokens, true, false).kind == kWhole;
+}
+
 cudaError_t matmul_half_swiglu(cudaStream_t stream, const Mat& gate, const Mat& up, const void* packed, float* y, uint32_t n_tokens, uint32_t y_stride,
                                void* packed_out) {
     if (gate.n_rows != up.n_rows || gate.n_cols != up.n_cols || !gate.half_tiles || !up.half_tiles || (packed_out && gate.n_rows % kChunkK != 0))

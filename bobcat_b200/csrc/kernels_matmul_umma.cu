@@ -42,6 +42,7 @@
 #include "device_utils.cuh"
 #include "kernels.h"
 #include "../../include/bobcat_cuda.h"
+#include "../../include/bobcat_cuda_test.h"
 
 namespace bc {
 namespace k {
@@ -902,6 +903,13 @@ cudaError_t matmul_umma_several(cudaStream_t stream, const Mat* const* ws, float
 bool matmul_umma_swiglu_supported(const Mat& gate, const Mat& up, uint32_t n_tokens, uint32_t min_tokens) {
     return matmul_umma_supported(gate, n_tokens, min_tokens) && matmul_umma_supported(up, n_tokens, min_tokens) && gate.n_rows == up.n_rows &&
            gate.n_cols == up.n_cols;
+}
+
+int matmul_umma_swiglu_form(const Mat& gate, const Mat& up, uint32_t n_tokens) {
+    if (few_serves(gate, gate.n_rows, n_tokens, Use::kDual) && few_serves(up, up.n_rows, n_tokens, Use::kDual)) return BC_SWIGLU_FEW;
+    if (matmul_half_supported(gate, n_tokens) && matmul_half_supported(up, n_tokens))
+        return matmul_half_swiglu_whole(gate, n_tokens) ? BC_SWIGLU_WHOLE : BC_SWIGLU_HALVES;
+    return BC_SWIGLU_DEQUANT;
 }
 
 cudaError_t matmul_umma_swiglu(cudaStream_t stream, const Mat& gate, const Mat& up, const void* packed, float* y, uint32_t n_tokens,

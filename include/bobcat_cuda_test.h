@@ -28,6 +28,15 @@ bc_status bc_seq_read_state(bc_seq* seq, int32_t which, uint32_t layer, float* o
  * decode step is the difference against a full step. The passes then compute garbage; NULL or ""
  * restores them. */
 bc_status bc_seq_set_skip(bc_seq* seq, const char* name, uint32_t n_rows, uint32_t n_cols);
+/* The SwiGLU of a batch as the forward passes run it, y[t][r] = silu(gate[r] . x[t]) * (up[r] . x[t]),
+ * recorded like an op: on the tensor cores with half-precision operands from 16 tokens on, with f32
+ * operands below. With `packed` (16 tokens and more, n_rows a multiple of 64) y takes the result as the
+ * packed fp16 operand of the next product, tokens rounded up to 16, in the layout of
+ * packed_operand_index (device_utils.cuh). `form` says which kernel ran; with a null y only that is
+ * told. */
+enum { BC_SWIGLU_DEQUANT = 0, BC_SWIGLU_FEW = 1, BC_SWIGLU_WHOLE = 2, BC_SWIGLU_HALVES = 3, BC_SWIGLU_EXACT = 4 };
+bc_status bc_test_matmul_swiglu(bc_backend* backend, bc_buffer* gate, bc_buffer* up, uint32_t n_rows, uint32_t n_cols, bc_buffer* x,
+                                bc_buffer* y, uint32_t n_tokens, int32_t packed, int32_t* form);
 /* How many kernels this sequence has launched so far (its own kernels, not library calls). */
 uint64_t bc_seq_launches(const bc_seq* seq);
 
