@@ -145,7 +145,6 @@ struct RopeStore {
     // in place of computing them.
     const float2* table = nullptr;
 };
-// (cos, sin) of every rotation pair at positions [0, n_positions), the values rope_store computes.
 // A batch's queries and keys, normalised and rotated, and its keys and values in the caches, in one launch.
 struct RopeBatch {
     const float* q;   // [token][q_stride], heads q_head_stride apart
@@ -160,6 +159,7 @@ struct RopeBatch {
     const float2* rope_table;  // [position][n_rot / 2] (cos, sin), or null to compute them
 };
 cudaError_t rope_store_batch(cudaStream_t stream, const RopeBatch& p);
+// (cos, sin) of every rotation pair at positions [0, n_positions), the values rope_store computes.
 cudaError_t rope_table(cudaStream_t stream, float2* table, uint32_t n_positions, uint32_t n_rot, float theta);
 cudaError_t rope_store(cudaStream_t stream, const RopeStore& p, Pos pos);
 // One thread: *counter += 1.

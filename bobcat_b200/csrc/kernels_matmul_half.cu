@@ -407,7 +407,10 @@ struct Tiling {
 // The tiling with the smallest modelled time, in us, fitted to 16 to 512 tokens of matrices of 2048 to 10752 rows and columns:
 // waves of tiles over the SMs, each chunk of 64 columns bound by the MMA (2 cycles per token and matrix at 1.4 GHz),
 // by the SM's share of L2 or by the ring's round trip; a start and a last epilogue that nothing hides; a split's partial
-// products, written and read once; the weights' time from HBM, of which a quarter shows beside the rest.
+// products, written and read once; the weights' time from HBM, of which a quarter shows beside the rest. Against the quickest of all tilings, matrices of the
+// 350M shape, which the fit left out, us with the packing and sums' launches for 33, 128 and 512 tokens: 1024 x 4608 10.2, 10.9, 16.3 (quickest 10.0,
+// 10.9, 16.1); gate and up 4608 x 1024 11.3, 11.3, 18.1 (11.1, 11.3, 17.5); 3072 x 1024 14.3, 14.5, 10.6 (11.6, 8.4, 10.6: K in one part, without the
+// sums' launch, which the model takes for cheaper than it is there).
 Tiling choose_tiling(uint32_t rows, uint32_t n_chunks, uint32_t n_tokens, bool dual, bool may_split) {
     const uint32_t sms = (uint32_t)sm_count();
     Tiling best{};

@@ -715,6 +715,10 @@ namespace {
 // others only from many rows. Measured, us, the former then the latter: adding, 24 rows of 2048 x 10752 18.0 / 9.8, of 2048 x
 // 2048 5.0 / 4.5, 16 rows of 2048 x 10752 12.7 / 9.7; storing, 24 rows of 12288 x 4096 28.0 / 19.7, of 3072 x 2048 5.7 / 11;
 // gate and up, 24 rows of 10752 x 2048 16.6 / 18.4, 32 rows 19.1 / 17.8, 24 rows of 12288 x 4096 49.7 / 34.3.
+// More shapes, 24 rows, each with its packing launch and, adding, a launch for the sums: adding, 1024 x 4608 11.1 / 9.3, 2048 x 4096 12.5 / 10.3, 2048 x
+// 6144 16.0 / 11.7, 4096 x 12288 38.1 / 24.0; storing, 3072 x 1024 6.4 / 9.0, 6144 x 2048 10.9 / 10.5, 8256 x 2048 12.3 / 11.9, 6144 x 4096 20.3 / 14.6, 9216 x
+// 4096 25.5 / 18.5 (so at 4096 columns the line of 64 rows per SM lies too high: it holds for up to 2048); gate and up, 4608 x 1024 7.8 /
+// 10.2, 6144 x 2048 14.3 / 15.3, 8192 x 3072 34.6 / 22.3; 28 rows of 4608 x 1024 10.0 / 9.9, of 6144 x 2048 16.4 / 15.0.
 enum class Use { kAdd, kStore, kDual };
 bool few_serves(const Mat& w, uint32_t rows, uint32_t n_tokens, Use use) {
     if (!matmul_few_supported(w, n_tokens)) return false;
