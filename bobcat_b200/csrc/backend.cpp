@@ -527,7 +527,7 @@ bc_status bc_op_matmul(bc_backend* b, int32_t format, bc_buffer* weights, size_t
     BC_TRY(need_recording(b));
     if (store < BC_STORE_OVERWRITE || store > BC_STORE_SWIGLU) return fail(BC_ERR_ARGUMENT, "unknown store mode %d", store);
     k::Mat w;
-    LaunchScope scope(b->device);
+    LaunchScope scope(b);
     BC_TRY(matrix_view(b, weights, w_off, format, n_rows, n_cols, "matmul", &w));
     if (n_tokens >= k::kMinHalfTokens && format == BC_Q4_0) {
         const bool capturing = is_capturing(b->stream);
@@ -558,7 +558,7 @@ bc_status bc_test_matmul_swiglu(bc_backend* b, bc_buffer* gate, bc_buffer* up, u
     BC_TRY(need_recording(b));
     if (!form) return fail(BC_ERR_ARGUMENT, "form must be non-null");
     k::Mat g, u;
-    LaunchScope scope(b->device);
+    LaunchScope scope(b);
     auto look = [&]() -> bc_status {
         BC_TRY(matrix_view(b, gate, 0, BC_Q4_0, n_rows, n_cols, "swiglu", &g));
         return matrix_view(b, up, 0, BC_Q4_0, n_rows, n_cols, "swiglu", &u);

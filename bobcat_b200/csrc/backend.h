@@ -59,6 +59,7 @@ struct bc_backend {
     cudaStream_t stream = nullptr;
     bool owns_stream = false;
     bool recording = false;
+    bool held_launch_scope = false;  // the stream may hold launches that read optional copies (optional_memory.h)
     uint64_t next_ticket = 1;
     cudaEvent_t record_start = nullptr;
     std::map<uint64_t, cudaEvent_t> tickets;  // ticket -> end-of-recording event

@@ -33,10 +33,10 @@ Gate& gate_of(int device) {
 
 thread_local int t_inside = -1;  // the device of this thread's LaunchScope
 
-// Wait for everything the device's backends have queued; false if that cannot be done now.
+// Wait for everything that may read copies; false if that cannot be done now.
 bool drain(Gate& gate, int device) {
     for (bc_backend* b : gate.backends) {
-        if (b->device != device) continue;
+        if (b->device != device || !b->held_launch_scope) continue;
         cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
         if (cudaStreamIsCapturing(b->stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
             cudaGetLastError();
@@ -44,18 +44,19 @@ bool drain(Gate& gate, int device) {
         }
     }
     for (bc_backend* b : gate.backends)
-        if (b->device == device && cudaStreamSynchronize(b->stream) != cudaSuccess) return false;
+        if (b->device == device && b->held_launch_scope && cudaStreamSynchronize(b->stream) != cudaSuccess) return false;
     return true;
 }
 
 }  // namespace
 
-LaunchScope::LaunchScope(int device) : device_(device) {
-    Gate& gate = gate_of(device);
+LaunchScope::LaunchScope(bc_backend* backend) : device_(backend->device) {
+    Gate& gate = gate_of(device_);
     std::unique_lock<std::mutex> lock(gate.mutex);
     gate.changed.wait(lock, [&] { return gate.outer_waiting == 0; });
     ++gate.inside;
-    t_inside = device;
+    t_inside = device_;
+    backend->held_launch_scope = true;
 }
 
 LaunchScope::~LaunchScope() {

@@ -4,8 +4,8 @@
 //
 // Launches read the copies through k::Mat::half_tiles, which host code of several threads looks at (sequences of one
 // model on several backends). So a call that looks at these pointers and launches what they point to holds a LaunchScope for as
-// long as it does, and giving back waits until no other thread is inside one, then for the streams of the device's backends, before it
-// clears the pointers and frees the memory.
+// long as it does, and giving back waits until no other thread is inside one, then for the streams of the device's backends that
+// have held one, before it clears the pointers and frees the memory.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -22,7 +22,7 @@ namespace bc {
 // a step is captured, since a stream that is being captured must not be waited for. Not nested.
 class LaunchScope {
   public:
-    explicit LaunchScope(int device);
+    explicit LaunchScope(bc_backend* backend);
     ~LaunchScope();
     LaunchScope(const LaunchScope&) = delete;
     LaunchScope& operator=(const LaunchScope&) = delete;
@@ -63,7 +63,7 @@ void backend_opened(bc_backend* backend);
 void backend_closing(bc_backend* backend);
 
 // Give the copies of one owner on the device back; false if there are none to be had. Waits for other threads' launch
-// scopes, and for the device's backends, whose streams must not be in capture.
+// scopes, and for the streams of the backends that have held one, none of which may be in capture.
 bool give_back_copies(int device);
 
 // After an allocation of `bytes` on the current device: give copies back while little room is left beside them. Kernels that are

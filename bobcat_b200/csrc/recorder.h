@@ -698,7 +698,7 @@ struct Recorder {
     // each row computes what lfm2_step computes for its sequence (lfm2_metal.rs:1162-1242).
     // `tokens` holds the n token ids; logits go to `all_logits` ([n][n_vocab]).
     void lfm2_seqs_step(const uint32_t* tokens, uint32_t n, k::SeqTable seqs, float* all_logits, const ExpertParallel* ep = nullptr) {
-        const LaunchScope scope(s.backend->device);
+        const LaunchScope scope(s.backend);
         const DeviceModel& W = *s.weights;
         const uint32_t n_embd = hp.n_embd, q_dim = hp.n_heads * hp.head_dim;
         run("embed", n, n_embd, 0, 1, [&] { return k::embed(stream, W.token_embd, tokens, k::Pos{nullptr, 0}, s.hidden, n); });
@@ -742,7 +742,7 @@ struct Recorder {
     }
 
     void batch(uint32_t pos, uint32_t n, bool want_logits, bool traced, size_t trace_stride) {
-        const LaunchScope scope(s.backend->device);
+        const LaunchScope scope(s.backend);
         if (hp.architecture == BC_ARCH_QWEN35) qwen_batch(pos, n, want_logits, traced, trace_stride);
         else lfm2_batch(pos, n, want_logits, traced, trace_stride);
         close_sum();  // the last layer's product, when no logits were asked for

@@ -83,7 +83,7 @@ bc_status capture_step(bc_seq* s, StepKind kind) {
     cudaStream_t stream = s->backend->stream;
     const uint32_t n_vocab = s->hp.n_vocab;
     uint64_t before = s->launches;
-    std::unique_ptr<LaunchScope> scope(new LaunchScope(s->backend->device));
+    std::unique_ptr<LaunchScope> scope(new LaunchScope(s->backend));
     BC_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
     Recorder r(*s);
     r.replayed = true;

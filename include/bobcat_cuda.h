@@ -82,7 +82,8 @@ typedef struct bc_backend bc_backend;
 typedef struct bc_buffer bc_buffer;
 
 /* Metal::open (backend.rs:1083). `stream` may be an existing cudaStream_t the caller owns (work is
- * then ordered with the caller's other work on it) or NULL for a stream the backend creates. */
+ * then ordered with the caller's other work on it) or NULL for a stream the backend creates. A
+ * caller's stream has to live until bc_backend_close: calls on other backends of the device may wait for it. */
 bc_status bc_backend_open(int32_t device, void* stream, bc_backend** out);
 void bc_backend_close(bc_backend* backend);
 /* The cudaStream_t every launch of this backend goes to. */
