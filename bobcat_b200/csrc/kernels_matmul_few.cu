@@ -11,8 +11,9 @@
 // What bounds it. The weights are the decode kernel's tiles (kernels_matvec_mma.cu), unpacked in registers straight into
 // A fragments. A pair of blocks of a 16-row tile is 1024 weights, 576 bytes, 100 cycles per scheduler at the HBM rate. Exact
 // with 8 rows it costs about 75 issue slots and 12 MMAs (one per 8 cycles and scheduler: 96 cycles); half with 32
-// rows about 60 slots and 16 MMAs. So loads, unpacking and multiplies are balanced, and the kernel is a weight
-// stream as long as nothing else is in the loop. That is why the inputs live in registers: a warp owns a fixed range
+// rows about 60 slots and 16 MMAs. Logic, shifts and the packed half and bf16 arithmetic issue every second cycle, so the loop alone, from
+// shared memory and without any waiting, takes 1520 cycles per tile of 2048 columns (0.8 us; its MMAs 768, everything but its MMAs
+// 870), and doubling the warps changes nothing. That is why the inputs live in registers: a warp owns a fixed range
 // of K (one to three pairs of blocks) for the whole launch, loads its inputs' B fragments once, and then walks
 // over the CTA's row tiles, whose weights are all it loads. (The kernels that served these shapes before: f32 tiles
 // through shared memory, 240 us per product whatever its size; a group of warps per tile that read the tokens'
@@ -26,9 +27,12 @@
 // or 32 (half) are further groups in blockIdx.y, working at the same time on the same weights out of L2; those of experts
 // are cut into equal runs (at the kernel).
 //
-// The weights come through per-lane slots of shared memory filled by cp.async several tiles ahead; a lane reads
-// back only what it copied itself, so the ring needs no barrier. The first tiles are requested before the wait for
-// the preceding launch.
+// The weights come through a ring of shared memory, a tile by one bulk copy (a slice of a tile by some more) several steps ahead, which
+// one warp asks for; a step's slot is refilled once every warp has arrived with its sums. The first
+// steps are requested before the wait for the preceding launch. (With per-lane cp.async into slots of a lane's own, 24 requests and their
+// addresses in every warp took 2 us of a launch before its first multiply: 11 rows of the 350M shape's prompt 632 us, now 606, six
+// sequences of the 2.6B shape 12.43 -> 12.16 ms, an expert block of 203 tokens 237 -> 233 us; 24 rows with half operands 11.47 -> 11.52 ms a
+// scoring request.)
 
 #include <cstdlib>
 
@@ -45,13 +49,13 @@ namespace {
 
 constexpr uint32_t kWarps = 16, kThreads = kWarps * 32;
 constexpr uint32_t kChunkPairs = 16;             // pairs of blocks per chunk of the tile layout
-constexpr uint32_t kPairQuants = 512, kPairScales = 64, kBlockBytes = 288;
+constexpr uint32_t kPairQuants = 512, kPairScales = 64;
 constexpr uint32_t kChunkBytes = kChunkPairs * (kPairQuants + kPairScales);
 constexpr uint32_t kMaxPairsPerWarp = 3;
 constexpr uint32_t kMaxSlices = 8;               // CTAs per cluster
 constexpr uint32_t kMaxExactTokens = 64, kHalfGroup = 32;
 constexpr uint32_t kMaxFewTokens = kHalfGroup;   // half: beyond, the tcgen05 kernel on expanded weights is quicker (64 rows of gate and up at 2.6B: 20 us against 33)
-constexpr uint32_t kSlotPair = 768;              // a lane's 16 bytes of quants and 8 of scales, for 32 lanes
+constexpr uint32_t kPairBytes = kPairQuants + kPairScales;
 constexpr uint32_t kSpinLimit = 1u << 22;
 // Tiles per step: two where the registers allow, because what a step costs besides its multiplies (requests, hand-over, sums) is
 // as many instructions as a tile's multiplies.
@@ -135,9 +139,6 @@ __device__ __forceinline__ uint4 quants_bf16(uint32_t w) {
     return make_uint4(v[0], v[1], v[2], v[3]);
 }
 
-__device__ __forceinline__ void cp_async_8(uint32_t dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
-}
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
 }
@@ -183,18 +184,22 @@ __device__ __forceinline__ bool find_group(const uint32_t* offsets, uint32_t n_e
 // per expert and group, for the likely number of groups, left SMs idle or began a second wave. An expert block of 32 experts of 1792
 // x 2048, us with all its launches: 2 tokens 103 -> 91, 16 tokens 179 -> 151, 64 tokens 222 -> 163, 203 tokens 231 to 352, as the
 // router picks, -> 237 to 251; passes of 15 sequences of such a model 15.6 -> 12.6 ms.)
+// Built on the same loop and taken back: four more warps for the sums and stores, so that the others only multiply (12.08 ms
+// against 11.95, and four more sums per tile in flight); with them a tile's loads and its first unpacking ahead of the tile before (13.1 ms: spills).
 template <bool EXACT, bool EXPERTS, int NT, int W, int DEPTH>
 __global__ void __launch_bounds__(kThreads, 1) matmul_few_kernel(const __grid_constant__ FewParams p) {
     static_assert(!EXACT || NT == 1, "the pieces of more rows do not fit the registers");
-    constexpr uint32_t kTileSums = 128 * NT, kPieces = EXACT ? 3 : NT, T = tiles_per_step(NT), kStepBytes = T * W * kSlotPair;
+    constexpr uint32_t kTileSums = 128 * NT, kPieces = EXACT ? 3 : NT, T = tiles_per_step(NT), kTileSlot = W * kWarps * kPairBytes, kStepBytes = T * kTileSlot;
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ float sums[2][T * kTileSums];        // clusters: this CTA's sums of a step
     __shared__ __align__(8) uint64_t arrived[2];    // the warps' sums of a step are there
+    __shared__ __align__(8) uint64_t full[DEPTH];   // the weights of a step are there
     __shared__ float squares[kWarps][8];            // a warp's share of the rows' sums of squares
     float4* partial = reinterpret_cast<float4*>(smem);  // [step % 2][tile][warp][row group][lane]
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
-    const uint32_t bars = async::smem_u32(arrived);
+    const uint32_t bars = async::smem_u32(arrived), full_bars = async::smem_u32(full);
     if (tid < 2) async::mbar_init(bars + tid * 8, kWarps);
+    else if (tid < 2 + DEPTH) async::mbar_init(full_bars + (tid - 2) * 8, 1);
     async::mbar_init_fence();
     __syncthreads();
     pdl_launch_dependents();
@@ -207,21 +212,71 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_few_kernel(const __grid_co
         run_at = (uint64_t)n_groups * p.n_jobs * cta / n_ctas;
         run_end = (uint64_t)n_groups * p.n_jobs * (cta + 1) / n_ctas;
     }
-    // This warp's pairs: [pair0, pair0 + live).
-    const uint32_t slice_end = min(p.n_pairs, (slice + 1) * p.slice_pairs), pair0 = slice * p.slice_pairs + warp * W;
-    const uint32_t live = pair0 < slice_end ? min((uint32_t)W, slice_end - pair0) : 0;
-    const uint64_t tile_bytes = (uint64_t)p.n_pairs * (2 * kBlockBytes);
+    // This CTA's pairs, and of these this warp's: [pair0, pair0 + live).
+    const uint32_t slice_pair0 = slice * p.slice_pairs, slice_pairs = min(p.n_pairs - slice_pair0, p.slice_pairs), pair0 = slice_pair0 + warp * W;
+    const uint32_t live = warp * W < slice_pairs ? min((uint32_t)W, slice_pairs - warp * W) : 0;
+    const uint64_t tile_bytes = (uint64_t)p.n_pairs * kPairBytes;
 
-    // Where the lane's share of each pair lies inside a tile.
+    // Where the lane's share of each pair lies in a slot: a whole tile as it lies in memory, a slice's quants ahead of its scales.
     uint32_t quant_at[W], scale_at[W];
 #pragma unroll
     for (int i = 0; i < W; ++i) {
-        const uint32_t pair = pair0 + i, chunk = pair / kChunkPairs, in_chunk = pair % kChunkPairs;
-        const uint32_t chunk_pairs = min(kChunkPairs, p.n_pairs - chunk * kChunkPairs);
-        quant_at[i] = chunk * kChunkBytes + in_chunk * kPairQuants + lane * 16;
-        scale_at[i] = chunk * kChunkBytes + chunk_pairs * kPairQuants + in_chunk * kPairScales + g * 8;
+        const uint32_t pair = warp * W + i, chunk = pair / kChunkPairs, in_chunk = pair % kChunkPairs;
+        const uint32_t chunk_pairs = min(kChunkPairs, slice_pairs - min(slice_pairs, chunk * kChunkPairs));
+        quant_at[i] = (slices == 1 ? chunk * kChunkBytes + in_chunk * kPairQuants : pair * kPairQuants) + lane * 16;
+        scale_at[i] = (slices == 1 ? chunk * kChunkBytes + chunk_pairs * kPairQuants + in_chunk * kPairScales : kWarps * W * kPairQuants + pair * kPairScales) + g * 8;
     }
+
+    // The stream of weights, in the order in which the steps are multiplied, through all groups. The warps ask for steps in turn (always the
+    // same one made 24 rows of the 2.6B shape 1 % slower); with experts the last one does, which keeps the place. One lane
+    // copies a whole tile; of a slice, each lane the quants or the scales of one chunk. (A lane's copy starts copy_src into the
+    // tile; lanes 16 and up serve the step's second tile.)
+    uint32_t copy_bytes = (lane & 15) == 0 ? (uint32_t)tile_bytes : 0, copy_src = 0, copy_dst = 0;
+    if (slices > 1) {
+        const uint32_t chunk = slice_pair0 / kChunkPairs + (lane >> 1 & 7), unit = lane & 1 ? kPairScales : kPairQuants;
+        const uint32_t from = max(chunk * kChunkPairs, slice_pair0), to = min((chunk + 1) * kChunkPairs, slice_pair0 + slice_pairs);
+        copy_bytes = from < to ? (to - from) * unit : 0;
+        copy_src = chunk * kChunkBytes + (lane & 1 ? min(kChunkPairs, p.n_pairs - min(chunk * kChunkPairs, p.n_pairs)) * kPairQuants : 0) + (from - chunk * kChunkPairs) * unit;
+        copy_dst = (from - slice_pair0) * unit + (lane & 1 ? kWarps * W * kPairQuants : 0);
+    }
+    const uint32_t ring = async::smem_u32(smem) + partial_bytes(NT);
+    uint64_t ask_at = run_at;
+    uint32_t ask_first = cta, ask_step = n_ctas, ask_tile = 0;
+    uint32_t ask_tiles = EXPERTS ? 0 : (p.n_jobs > cta ? (p.n_jobs - cta + n_ctas - 1) / n_ctas : 0) << p.dual;
+    auto tile_of = [&](uint32_t tile) {
+        uint32_t job = ask_first + ask_step * (tile >> p.dual);
+        int seg = p.dual ? tile & 1 : 0;
+        if (!EXPERTS && !p.dual) {
+            while (seg + 1 < p.n_segments && job >= p.seg_tiles[seg]) {
+                job -= p.seg_tiles[seg];
+                ++seg;
+            }
+        }
+        return p.tiles[seg] + (uint64_t)job * tile_bytes;
+    };
+    auto request = [&](uint32_t into) {
+        if (ask_tile >= ask_tiles) {
+            if (!EXPERTS || ask_at >= run_end) return;
+            uint32_t expert = 0, place = 0;
+            if (!find_group(p.offsets, p.n_experts, 8 * NT, (uint32_t)(ask_at / p.n_jobs), expert, place)) return;
+            const uint32_t in_expert = (uint32_t)(ask_at % p.n_jobs), jobs = (uint32_t)min((uint64_t)(p.n_jobs - in_expert), run_end - ask_at);
+            ask_first = expert * p.n_jobs + in_expert;
+            ask_step = 1;
+            ask_tiles = jobs << p.dual;
+            ask_tile = 0;
+            ask_at += jobs;
+        }
+        const uint32_t bar = full_bars + into * 8, tile = ask_tile + (lane >> 4);
+        if (lane == 0) async::mbar_arrive_expect(bar, min(T, ask_tiles - ask_tile) * slice_pairs * kPairBytes);
+        __syncwarp();
+        if (copy_bytes && (lane >> 4) < T && tile < ask_tiles)
+            async::bulk_load(ring + into * kStepBytes + (lane >> 4) * kTileSlot + copy_dst, tile_of(tile) + copy_src, copy_bytes, bar);
+    };
+    for (int d = 0; d < DEPTH; ++d, ask_tile += T)
+        if (warp == kWarps - 1) request(d);
+
     uint32_t steps_before = 0;  // steps of the groups before this one
+    uint32_t slot = 0, slot_parity = 0;
     do {  // plain: once; a whole cluster goes round or leaves together
     uint32_t n_tokens = p.n_tokens, first_entry = 0, expert = 0, group = blockIdx.y;
     uint32_t first_job = cta, job_step = n_ctas, my_jobs = p.n_jobs > cta ? (p.n_jobs - cta + n_ctas - 1) / n_ctas : 0;
@@ -234,42 +289,8 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_few_kernel(const __grid_co
         my_jobs = (uint32_t)min((uint64_t)(p.n_jobs - first_job), run_end - run_at);
         run_at += my_jobs;
     }
-    const uint64_t expert_tile = (uint64_t)expert * p.n_jobs;
     const uint32_t token0 = group * (8 * NT);
     const uint32_t n_tiles = p.dual ? 2 * my_jobs : my_jobs, n_steps = (n_tiles + T - 1) / T;  // of a pair of matrices the tiles alternate
-    const uint32_t ring = async::smem_u32(smem) + partial_bytes(NT) + warp * (DEPTH * kStepBytes) + lane * 16;
-    auto tile_of = [&](uint32_t tile) {
-        if (EXPERTS || p.dual || p.n_segments == 1)
-            return p.tiles[p.dual ? tile & 1 : 0] + (expert_tile + first_job + job_step * (tile >> p.dual)) * tile_bytes;
-        uint32_t job = first_job + job_step * tile;
-        int seg = 0;
-        while (seg + 1 < p.n_segments && job >= p.seg_tiles[seg]) {
-            job -= p.seg_tiles[seg];
-            ++seg;
-        }
-        return p.tiles[seg] + (uint64_t)job * tile_bytes;
-    };
-    uint32_t requested = 0, request_slot = ring;  // steps requested; step u lies in slot u % DEPTH
-    auto request = [&]() {
-#pragma unroll
-        for (uint32_t h = 0; h < T; ++h) {
-            if (requested * T + h < n_tiles) {
-                const uint8_t* tile = tile_of(requested * T + h);
-#pragma unroll
-                for (int i = 0; i < W; ++i) {
-                    if ((uint32_t)i < live) {
-                        async::cp_async_16(request_slot + (h * W + i) * kSlotPair, tile + quant_at[i]);
-                        cp_async_8(request_slot + (h * W + i) * kSlotPair + kPairQuants - lane * 8, tile + scale_at[i]);
-                    }
-                }
-            }
-        }
-        async::cp_async_commit();
-        ++requested;
-        request_slot = request_slot == ring + (DEPTH - 1) * kStepBytes ? ring : request_slot + kStepBytes;
-    };
-#pragma unroll
-    for (int d = 0; d < DEPTH; ++d) request();
 
     // The warp's inputs: for row g of a group, the eight columns of every block that meet this lane's quants, in
     // the order the unpacking emits; exact: as three bf16 pieces of one group, half: one piece per group.
@@ -368,6 +389,7 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_few_kernel(const __grid_co
     // In the accumulator layout [group][lane][4], with the halves of a lane's four values swapped for every other pair of rows, so
     // that the 32 values a warp reads at once lie in different banks.
     const uint32_t at = ((((turn >> 2) * 32 + (row_in_tile & 7) * 4 + (tk >> 1)) * 4) + (row_in_tile >> 3) * 2 + (tk & 1)) ^ (row_in_tile & 2);
+    const uint32_t out_row = EXPERTS && tok < n_tokens ? p.entries[first_entry + tok] : tok;
     auto my_turn = [&](uint32_t step) { return NT == 1 ? (step & 3) == warp >> 2 : NT == 2 ? (step & 1) == warp >> 3 : warp < 4 * NT; };
     auto over_warps = [&](uint32_t step, uint32_t h) {
         const float* base = reinterpret_cast<const float*>(partial) + (((steps_before + step) & 1) * T + h) * (kWarps * kTileSums) + at;
@@ -378,14 +400,39 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_few_kernel(const __grid_co
     };
     float scale = 1.f, gate = 0.f;
     bool scaled = !EXACT || p.norm_weight == nullptr;
+    auto output = [&](uint32_t tile, float*& out) {  // where this thread's output of a tile goes; false: nowhere
+        uint32_t job = first_job + job_step * (tile >> p.dual);
+        int seg = 0;
+        if (!EXPERTS && !p.dual)
+            while (seg + 1 < p.n_segments && job >= p.seg_tiles[seg]) {
+                job -= p.seg_tiles[seg];
+                ++seg;
+            }
+        const uint32_t row = job * 16 + row_in_tile;
+        out = p.y[seg] + (uint64_t)out_row * p.seg_stride[seg] + row;
+        return tok < n_tokens && row < p.seg_rows[seg];
+    };
+    // The outputs' old values of the step that is finished next, read before the multiplies that come in between.
+    float old[T];
+    auto fetch_old = [&](uint32_t step) {
+        if (p.dual || p.store == BC_STORE_OVERWRITE || !my_turn(step) || turn % slices != slice) return;
+#pragma unroll
+        for (uint32_t h = 0; h < T; ++h) {
+            float* out;
+            if (step * T + h < n_tiles && output(step * T + h, out)) old[h] = *out;
+        }
+    };
     // Stores a finished step: `total(h)` gives the sum of this thread's output of its tile h.
     auto finish = [&](uint32_t step, auto&& total) {
         if constexpr (EXACT) {
             if (!scaled) {
-                float squared = 0.f;
+                float squared = 0.f;  // warps without a range of K have left zeros
                 for (uint32_t s = 0; s < slices; ++s) {
-                    const uint32_t pairs = min(p.n_pairs, (s + 1) * p.slice_pairs) - s * p.slice_pairs;
-                    for (uint32_t w = 0; w * W < pairs; ++w) squared += slices == 1 ? squares[w][tk] : remote_float(&squares[w][tk], s);
+                    float part[kWarps];
+#pragma unroll
+                    for (uint32_t w = 0; w < kWarps; ++w) part[w] = slices == 1 ? squares[w][tk] : remote_float(&squares[w][tk], s);
+#pragma unroll
+                    for (uint32_t w = 0; w < kWarps; ++w) squared += part[w];
                 }
                 scale = rsqrtf(squared / (float)(p.n_pairs * 64) + p.eps);
                 scaled = true;
@@ -399,17 +446,10 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_few_kernel(const __grid_co
                 gate = total(h) * scale;
                 continue;
             }
-            uint32_t job = first_job + job_step * (tile >> p.dual);
-            int seg = 0;
-            if (!EXPERTS && !p.dual)
-                while (seg + 1 < p.n_segments && job >= p.seg_tiles[seg]) {
-                    job -= p.seg_tiles[seg];
-                    ++seg;
-                }
-            const uint32_t row = job * 16 + row_in_tile;
             if (!EXACT && p.packed_out) {
                 // The rows are columns of the next product, whose operand wants columns (0, 2), (1, 3) of a group of four
                 // as pairs of halves: the lane of the first row stores the four rows' 8 bytes.
+                const uint32_t row = (first_job + job_step * (tile >> 1)) * 16 + row_in_tile;
                 const float v = gate / (1.f + expf(-gate)) * total(h);
                 const float v1 = __shfl_down_sync(0xffffffffu, v, 1), v2 = __shfl_down_sync(0xffffffffu, v, 2), v3 = __shfl_down_sync(0xffffffffu, v, 3);
                 const __half2 even = __floats2half2_rn(v, v2), odd = __floats2half2_rn(v1, v3);
@@ -418,13 +458,12 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_few_kernel(const __grid_co
                         make_uint2(*reinterpret_cast<const uint32_t*>(&even), *reinterpret_cast<const uint32_t*>(&odd));
                 continue;
             }
-            const bool stores = tok < n_tokens && row < p.seg_rows[seg];
-            float* out = p.y[seg] + (uint64_t)(EXPERTS && stores ? p.entries[first_entry + tok] : tok) * p.seg_stride[seg] + row;
-            const float old = stores && !p.dual && p.store != BC_STORE_OVERWRITE ? *out : 0.f;
+            float* out;
+            const bool stores = output(tile, out);
             float sum = total(h) * scale;
             if (p.dual) sum = gate / (1.f + expf(-gate)) * sum;
-            else if (p.store == BC_STORE_ACCUMULATE) sum += old;
-            else if (p.store == BC_STORE_SWIGLU) sum = old / (1.f + expf(-old)) * sum;
+            else if (p.store == BC_STORE_ACCUMULATE) sum += old[h];
+            else if (p.store == BC_STORE_SWIGLU) sum = old[h] / (1.f + expf(-old[h])) * sum;
             if (stores) *out = sum;
         }
     };
@@ -432,31 +471,38 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_few_kernel(const __grid_co
     // warp's turn falls to.
     auto finish_cluster = [&](uint32_t step) {
         asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
-        if (my_turn(step) && turn % slices == slice)
-            finish(step, [&](uint32_t h) {
-                float sum = 0.f;
-                for (uint32_t s = 0; s < slices; ++s) sum += remote_float(&sums[step & 1][h * kTileSums + turn * 32 + lane], s);
-                return sum;
-            });
+        if (my_turn(step) && turn % slices == slice) {
+            float part[T][kMaxSlices], total[T];  // all on their way before the first is added
+#pragma unroll
+            for (uint32_t h = 0; h < T; ++h)
+#pragma unroll
+                for (uint32_t s = 0; s < kMaxSlices; ++s) part[h][s] = s < slices ? remote_float(&sums[step & 1][h * kTileSums + turn * 32 + lane], s) : 0.f;
+#pragma unroll
+            for (uint32_t h = 0; h < T; ++h) {
+                total[h] = 0.f;
+#pragma unroll
+                for (uint32_t s = 0; s < kMaxSlices; ++s) total[h] += part[h][s];
+            }
+            finish(step, [&](uint32_t h) { return total[h]; });
+        }
     };
 
-    uint32_t slot = ring;
     for (uint32_t u = 0; u <= n_steps; ++u) {
         float acc[T][NT][4];
+        const uint32_t behind = slices == 1 ? 1 : 2;
+        if (u >= behind) fetch_old(u - behind);
         if (u < n_steps && live) {
-            async::cp_async_wait<DEPTH - 1>();
+            if (!async::mbar_test(full_bars + slot * 8, slot_parity)) wait_on(full_bars + slot * 8, slot_parity);
             uint4 q[T][W];
             uint2 d[T][W];
 #pragma unroll
             for (uint32_t h = 0; h < T; ++h)
 #pragma unroll
                 for (int i = 0; i < W; ++i) {
-                    const uint32_t from = slot + (h * W + i) * kSlotPair;
-                    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(q[h][i].x), "=r"(q[h][i].y), "=r"(q[h][i].z), "=r"(q[h][i].w) : "r"(from));
-                    asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(d[h][i].x), "=r"(d[h][i].y) : "r"(from + kPairQuants - lane * 8));
+                    const uint32_t from = ring + slot * kStepBytes + h * kTileSlot;
+                    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(q[h][i].x), "=r"(q[h][i].y), "=r"(q[h][i].z), "=r"(q[h][i].w) : "r"(from + quant_at[i]) : "memory");
+                    asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(d[h][i].x), "=r"(d[h][i].y) : "r"(from + scale_at[i]) : "memory");
                 }
-            slot = slot == ring + (DEPTH - 1) * kStepBytes ? ring : slot + kStepBytes;
-            request();  // refills this slot: the lane has its share in registers
 #pragma unroll
             for (uint32_t h = 0; h < T; ++h) {
 #pragma unroll
@@ -502,6 +548,8 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_few_kernel(const __grid_co
             const uint32_t before = u - 1, turns = steps_before + before;  // buffers and barriers alternate through all groups
             // Every warp arrives for every step whatever happens, so the wait ends; it is bounded like all waits.
             if (!async::mbar_test(bars + (turns & 1) * 8, (turns >> 1) & 1)) wait_on(bars + (turns & 1) * 8, (turns >> 1) & 1);
+            if (warp == (EXPERTS ? kWarps - 1 : before % kWarps)) request(slot == 0 ? DEPTH - 1 : slot - 1);  // every warp has its weights of that step in registers
+            ask_tile += T;
             if (slices == 1) {
                 if (my_turn(before)) finish(before, [&](uint32_t h) { return over_warps(before, h); });
             } else {
@@ -524,11 +572,15 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_few_kernel(const __grid_co
             }
             __syncwarp();
             if (lane == 0) async::mbar_arrive(bars + ((steps_before + u) & 1) * 8);
+            slot = slot == DEPTH - 1 ? 0 : slot + 1;
+            slot_parity ^= slot == 0;
         }
     }
-    async::cp_async_wait<0>();
     if (slices > 1) {
-        if (n_steps) finish_cluster(n_steps - 1);
+        if (n_steps) {
+            fetch_old(n_steps - 1);
+            finish_cluster(n_steps - 1);
+        }
         cluster_sync();  // no CTA leaves, or goes on, while another reads its sums
     }
     steps_before += n_steps;
@@ -551,7 +603,7 @@ bool few_disabled() {
 template <bool EXACT, bool EXPERTS, int NT, int W, int DEPTH>
 cudaError_t launch_as(cudaStream_t stream, FewParams& p, uint32_t groups) {
     const void* kernel = (const void*)matmul_few_kernel<EXACT, EXPERTS, NT, W, DEPTH>;
-    const size_t smem = partial_bytes(NT) + (size_t)kWarps * DEPTH * tiles_per_step(NT) * W * kSlotPair;
+    const size_t smem = partial_bytes(NT) + (size_t)kWarps * DEPTH * tiles_per_step(NT) * W * kPairBytes;
     cudaError_t e = ensure_dynamic_smem(kernel, smem);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t config = {};
@@ -614,8 +666,8 @@ cudaError_t launch_exact(cudaStream_t stream, FewParams& p) {
     const uint32_t groups = (p.n_tokens + 7) / 8;
     switch (cut(p, kMaxPairsPerWarp)) {
         case 1: return launch<true, 1, 1, 6>(stream, p, groups);
-        case 2: return launch<true, 1, 2, 3>(stream, p, groups);
-        default: return launch<true, 1, 3, 2>(stream, p, groups);
+        case 2: return launch<true, 1, 2, 4>(stream, p, groups);
+        default: return launch<true, 1, 3, 3>(stream, p, groups);
     }
 }
 
@@ -626,8 +678,8 @@ cudaError_t launch_half(cudaStream_t stream, FewParams& p, uint32_t rows) {
     const uint32_t w = cut(p, nt <= 2 ? 3 : 2), groups = (p.n_tokens + 8 * (nt < 2 ? 2 : nt) - 1) / (8 * (nt < 2 ? 2 : nt));
     if (nt <= 2) {
         switch (w) {
-            case 1: return launch<false, 2, 1, 5>(stream, p, groups);
-            case 2: return launch<false, 2, 2, 3>(stream, p, groups);
+            case 1: return launch<false, 2, 1, 6>(stream, p, groups);
+            case 2: return launch<false, 2, 2, 4>(stream, p, groups);
             default: return launch<false, 2, 3, 2>(stream, p, groups);
         }
     }
