@@ -190,17 +190,19 @@ struct AttentionShape {
     uint32_t q_stride, q_head_stride;
     const uint32_t* pos_ptr = nullptr;  // when set, first_pos is *pos_ptr + first_pos and the grid covers n_ctx
     uint64_t scratch_floats = 0;  // what the scratch holds; 0: attention_scratch_floats of this shape
+    bool gated = false;  // one query: out *= sigmoid of the values that follow each head's queries
 };
 uint64_t attention_scratch_floats(uint32_t n_heads, uint32_t head_dim, uint32_t n_ctx, uint32_t n_queries);
 cudaError_t attention(cudaStream_t stream, const float* q, const void* k_cache, const void* v_cache, bool kv_half,
                       float* scratch, float* out, const AttentionShape& shape);
 // Kernels `attention` launches for this shape.
 int attention_launches(bool kv_half, const AttentionShape& shape);
-// One decoded token of an attention layer in two launches: the chunk pass normalises and rotates
-// the raw q itself, and the CTA whose chunk ends at the new position prepares that position's key
-// and value rows, stores them in the caches and uses them; then the combine pass. Covers
-// half-precision caches, heads of 64, 128 or 256 elements rotated whole, 16-byte aligned rows.
+// One decoded token of an attention layer: the launch normalises and rotates the raw q itself, and the
+// CTA whose chunk ends at the new position prepares that position's key
+// and value rows, stores them in the caches and uses them. Contexts beyond 2048 positions take a combine
+// pass of its own. Covers heads of 64, 128 or 256 elements rotated whole, 16-byte aligned rows; long contexts: half-precision caches.
 bool attention_step_supported(const RopeStore& r, const AttentionShape& shape);
+int attention_step_launches(const AttentionShape& shape);
 cudaError_t attention_step(cudaStream_t stream, const RopeStore& r, float* scratch, float* out, const AttentionShape& shape);
 // The tensor-core prefill kernel (kernels_attention_flash.cu): heads of 64 elements, f16 cache, at
 // least 32 queries, positions known at launch. `attention` picks it when it applies.

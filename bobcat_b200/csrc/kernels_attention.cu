@@ -1,6 +1,7 @@
 // Causal grouped-query attention over a contiguous KV cache, split over 64-position chunks with a
 // combine pass (the structure of attention_chunk / attention_wide / attention_combine in
-// crates/bobcat-metal/src/attention.metal:26-265, :496-540; host side backend.rs:2150-2320).
+// crates/bobcat-metal/src/attention.metal:26-265, :496-540; host side backend.rs:2150-2320). One query of a short context
+// takes one launch (attention_token_kernel).
 //
 // Chunk pass: one CTA per (KV head, chunk, query). The query heads of the group that shares the KV
 // head are scored together, so each key and value row is read from the cache once per group.
@@ -30,6 +31,7 @@ constexpr int kDecodeQueries = 4;  // up to this many queries use the small chun
 constexpr int kMaxGroup = 8;       // query heads per KV head
 constexpr int kQueryBatch = 64;    // queries per launch, which bounds the scratch
 constexpr int kChunkThreads = 256;
+constexpr int kCombineParts = 4;   // thread groups that share a head's chunks in the combine
 
 template <typename T>
 __device__ __forceinline__ float load_kv(const T* p);
@@ -425,19 +427,354 @@ const void* decode_kernel(bool kv_half, const AttentionShape& s, const float* q,
     }
 }
 
+// ---- One decoded token in one launch: a cluster of eight CTAs per KV head.
+//
+// Bound by latency: 512 positions of 8 KV heads are 1 MB of cache, and as a chunk pass and a combine pass the step took
+// 10 us of which the combine's launch, its trip to L2 and the hand-over were 3, the queries' norm and rotation, once per warp and head, 2. Here a
+// CTA normalises and rotates each query head in one warp; its four teams of four warps take a chunk of 16 positions each, with the
+// arithmetic and the order of attention_decode_kernel; a chunk's partial sums go straight to the shared memory of the CTA
+// that combines the head (one head per CTA, group <= 4), in the order of attention_combine_kernel, so the result is the same to the bit. A
+// cluster covers 32 chunks at a time.
+// Eight CTAs are the portable cluster; contexts beyond kTokenChunks chunks keep the two launches, whose grid covers the device.
+//
+// An f32 cache used to take rope_store_kernel, attention_chunk_kernel and the combine (14 us).
+constexpr uint32_t kTokenCluster = 8, kTokenTeams = 4, kTokenThreads = kTokenTeams * kDecodeThreads, kTokenChunks = 128;
+constexpr uint32_t kTokenGroup = 4;
+
+// The eight elements of a cache row that a lane holds.
+template <typename T>
+struct RowPiece;
+template <>
+struct RowPiece<__half> {
+    uint4 raw;
+    __device__ __forceinline__ void clear() { raw = make_uint4(0, 0, 0, 0); }
+    __device__ __forceinline__ void load(const __half* p) { raw = __ldcg(reinterpret_cast<const uint4*>(p)); }
+    __device__ __forceinline__ void store(__half* p) const { *reinterpret_cast<uint4*>(p) = raw; }
+    __device__ __forceinline__ void get(float (&f)[8]) const { unpack_row(raw, f); }
+    __device__ __forceinline__ void set(const float (&f)[8]) { raw = pack_row(f); }
+};
+template <>
+struct RowPiece<float> {
+    float4 a, b;
+    __device__ __forceinline__ void clear() { a = b = make_float4(0.f, 0.f, 0.f, 0.f); }
+    __device__ __forceinline__ void load(const float* p) {
+        a = __ldcg(reinterpret_cast<const float4*>(p));
+        b = __ldcg(reinterpret_cast<const float4*>(p) + 1);
+    }
+    __device__ __forceinline__ void store(float* p) const {
+        reinterpret_cast<float4*>(p)[0] = a;
+        reinterpret_cast<float4*>(p)[1] = b;
+    }
+    __device__ __forceinline__ void get(float (&f)[8]) const { f[0] = a.x, f[1] = a.y, f[2] = a.z, f[3] = a.w, f[4] = b.x, f[5] = b.y, f[6] = b.z, f[7] = b.w; }
+    __device__ __forceinline__ void set(const float (&f)[8]) {
+        a = make_float4(f[0], f[1], f[2], f[3]);
+        b = make_float4(f[4], f[5], f[6], f[7]);
+    }
+};
+__device__ __forceinline__ void load_eight(const float* p, float (&f)[8]) {
+    const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+    f[0] = a.x, f[1] = a.y, f[2] = a.z, f[3] = a.w, f[4] = b.x, f[5] = b.y, f[6] = b.z, f[7] = b.w;
+}
+__device__ __forceinline__ void team_sync(uint32_t team) { asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "n"(kDecodeThreads) : "memory"); }
+
+template <int HD, int GROUP>
+struct TokenShared {
+    float merged[kTokenTeams][kDecodeThreads / 32][GROUP][HD + 2];
+    float q[GROUP][HD];  // scaled
+    float new_k[HD], new_v[HD];
+    float2 rot[HD / 2];
+    float weights[kTokenChunks], across[2][kTokenThreads / 32], sums[kCombineParts * HD];
+};  // then the head's partial sums, [chunk][HD + 2]
+
+template <typename T, int HD, int GROUP, bool FUSED>
+__global__ void __launch_bounds__(kTokenThreads, 1) attention_token_kernel(ChunkParams p, int gated) {
+    constexpr int kLanesPerRow = HD / 8, kRowsPerLoad = 32 / kLanesPerRow, kWarps = kDecodeThreads / 32;
+    extern __shared__ __align__(16) uint8_t token_smem[];
+    TokenShared<HD, GROUP>& sh = *reinterpret_cast<TokenShared<HD, GROUP>*>(token_smem);
+    float* head_parts = reinterpret_cast<float*>(token_smem + sizeof(TokenShared<HD, GROUP>));
+    pdl_launch_dependents();
+    asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");  // this CTA runs: its shared memory may be written
+    const uint32_t kv_head = blockIdx.x / kTokenCluster, rank = blockIdx.x % kTokenCluster;
+    const uint32_t group = p.n_heads / p.n_kv_heads, kv_dim = p.n_kv_heads * HD;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, cta_warp = tid >> 5, team = cta_warp / kWarps, warp = cta_warp % kWarps, in_team = tid % kDecodeThreads;
+    const uint32_t sub = lane / kLanesPerRow, d0 = (lane % kLanesPerRow) * 8;
+    T* const k_cache = static_cast<T*>(const_cast<void*>(p.k_cache)) + (uint64_t)kv_head * HD + d0;
+    T* const v_cache = static_cast<T*>(const_cast<void*>(p.v_cache)) + (uint64_t)kv_head * HD + d0;
+    auto start_load = [&](RowPiece<T>& k, RowPiece<T>& v, uint32_t position) {
+        k.load(k_cache + (uint64_t)position * kv_dim);
+        v.load(v_cache + (uint64_t)position * kv_dim);
+    };
+
+    // As in attention_decode_kernel: in the fused step the rows of earlier positions were written by earlier tokens' launches, so the
+    // first rows are on their way before the wait; the new position's row is replaced below.
+    uint32_t chunk = rank + kTokenCluster * team, base = warp * kRowsPerLoad;
+    RowPiece<T> k_row, v_row;
+    k_row.clear();
+    v_row.clear();
+    if (FUSED && chunk * kDecodeChunk + base + sub < p.n_ctx) start_load(k_row, v_row, chunk * kDecodeChunk + base + sub);
+    pdl_wait();
+    const uint32_t pos = p.first_pos + (p.pos_ptr ? *p.pos_ptr : 0u);
+    if (!FUSED && chunk * kDecodeChunk + base + sub <= pos) start_load(k_row, v_row, chunk * kDecodeChunk + base + sub);
+
+    // The queries, a head to a warp, and the new position's key and value rows.
+    const float scale = 1.0f / sqrtf((float)HD);
+    const float* raw = cta_warp < group ? p.q + (uint64_t)(kv_head * group + cta_warp) * p.q_head_stride : p.raw_k + (uint64_t)kv_head * HD;
+    float mine[8] = {};
+    if (cta_warp < group || (FUSED && cta_warp == GROUP)) load_eight(raw + d0, mine);
+    if (FUSED) {
+        if (tid < HD / 2) {
+            if (p.rope_table) {
+                sh.rot[tid] = p.rope_table[(uint64_t)pos * (HD / 2) + tid];
+            } else {
+                const float inv_freq = 1.0f / powf(p.theta, (float)(2 * tid) / (float)HD);
+                float sn, cs;
+                sincosf((float)pos * inv_freq, &sn, &cs);
+                sh.rot[tid] = make_float2(cs, sn);
+            }
+        }
+        if (tid >= kTokenThreads - HD) sh.new_v[tid - (kTokenThreads - HD)] = p.raw_v[(uint64_t)kv_head * HD + tid - (kTokenThreads - HD)];
+        __syncthreads();
+        if (cta_warp < group) norm_rotate<HD>(mine, p.q_norm, p.eps, d0, sh.rot);
+        else if (cta_warp == GROUP) norm_rotate<HD>(mine, p.k_norm, p.eps, d0, sh.rot);
+    }
+    if (sub == 0 && cta_warp < group) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) sh.q[cta_warp][d0 + i] = mine[i] * scale;
+    } else if (FUSED && sub == 0 && cta_warp == GROUP) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) sh.new_k[d0 + i] = mine[i];
+    }
+    __syncthreads();
+    float qv[GROUP][8];
+#pragma unroll
+    for (int g = 0; g < GROUP; ++g) {
+        if (g < (int)group) load_eight(sh.q[g] + d0, qv[g]);
+        else
+#pragma unroll
+            for (int i = 0; i < 8; ++i) qv[g][i] = 0.f;
+    }
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+
+    const uint32_t n_chunks = pos / kDecodeChunk + 1;
+    for (; chunk < n_chunks; chunk += kTokenCluster * kTokenTeams) {
+        const uint32_t start = chunk * kDecodeChunk, count = min((uint32_t)kDecodeChunk, pos + 1 - start), new_row = pos - start;
+        const bool holds_new = FUSED && new_row < (uint32_t)kDecodeChunk;
+        RowPiece<T> k_new, v_new;
+        if (holds_new) {
+            float f[8];
+            load_eight(sh.new_k + d0, f);
+            k_new.set(f);
+            load_eight(sh.new_v + d0, f);
+            v_new.set(f);
+            if (warp == 0 && sub == 0) {
+                k_new.store(k_cache + (uint64_t)pos * kv_dim);
+                v_new.store(v_cache + (uint64_t)pos * kv_dim);
+            }
+            if (base + sub == new_row) k_row = k_new, v_row = v_new;
+        }
+        float acc[GROUP][8], top[GROUP], sum[GROUP];
+#pragma unroll
+        for (int g = 0; g < GROUP; ++g) {
+            top[g] = -INFINITY;
+            sum[g] = 0.f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc[g][i] = 0.f;
+        }
+        while (base < count) {
+            float kf[8], vf[8];
+            k_row.get(kf);
+            v_row.get(vf);
+            const bool valid = base + sub < count;
+            const uint32_t next = base + kWarps * kRowsPerLoad;
+            if (holds_new && next + sub == new_row) k_row = k_new, v_row = v_new;  // not in the cache when this launch began
+            else if (next + sub < count) start_load(k_row, v_row, start + next + sub);
+#pragma unroll
+            for (int g = 0; g < GROUP; ++g) {
+                float dot = 0.f;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) dot += kf[i] * qv[g][i];
+#pragma unroll
+                for (int o = 1; o < kLanesPerRow; o <<= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+                if (valid) {
+                    const float m = fmaxf(top[g], dot);
+                    const float keep = expf(top[g] - m), w = expf(dot - m);  // exp(-inf) = 0 on the first row
+                    sum[g] = sum[g] * keep + w;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) acc[g][i] = acc[g][i] * keep + w * vf[i];
+                    top[g] = m;
+                }
+            }
+            base = next;
+        }
+        // The next chunk's first rows.
+        base = warp * kRowsPerLoad;
+        const uint32_t ahead = start + kTokenCluster * kTokenTeams * kDecodeChunk + base + sub;
+        if (ahead < pos || (!FUSED && ahead == pos)) start_load(k_row, v_row, ahead);
+
+        // Merge the rows of the warp, then the warps of the team.
+#pragma unroll
+        for (int g = 0; g < GROUP; ++g) {
+#pragma unroll
+            for (int o = kLanesPerRow; o < 32; o <<= 1) {
+                const float other_top = __shfl_xor_sync(0xffffffffu, top[g], o);
+                const float other_sum = __shfl_xor_sync(0xffffffffu, sum[g], o);
+                const float m = fmaxf(top[g], other_top);
+                const float keep = top[g] == -INFINITY ? 0.f : expf(top[g] - m);
+                const float theirs = other_top == -INFINITY ? 0.f : expf(other_top - m);
+                sum[g] = sum[g] * keep + other_sum * theirs;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const float other = __shfl_xor_sync(0xffffffffu, acc[g][i], o);
+                    acc[g][i] = acc[g][i] * keep + other * theirs;
+                }
+                top[g] = m;
+            }
+            if (sub == 0 && g < (int)group) {
+                float* out = sh.merged[team][warp][g];
+                if (d0 == 0) {
+                    out[0] = top[g];
+                    out[1] = sum[g];
+                }
+#pragma unroll
+                for (int i = 0; i < 8; ++i) out[2 + d0 + i] = acc[g][i];
+            }
+        }
+        team_sync(team);
+        for (uint32_t i = in_team; i < group * HD; i += kDecodeThreads) {
+            const uint32_t g = i / HD, d = i % HD;
+            float m = -INFINITY;
+#pragma unroll
+            for (int w = 0; w < kWarps; ++w) m = fmaxf(m, sh.merged[team][w][g][0]);
+            float total = 0.f, weight = 0.f;
+#pragma unroll
+            for (int w = 0; w < kWarps; ++w) {
+                const float t = sh.merged[team][w][g][0];
+                const float f = t == -INFINITY ? 0.f : expf(t - m);
+                weight += sh.merged[team][w][g][1] * f;
+                total += sh.merged[team][w][g][2 + d] * f;
+            }
+            uint32_t out;  // in the CTA that combines head g
+            asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"((uint32_t)__cvta_generic_to_shared(head_parts + chunk * (HD + 2))), "r"(g));
+            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(out + (2 + d) * 4), "f"(total) : "memory");
+            if (d == 0) {
+                asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(out), "f"(m) : "memory");
+                asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(out + 4), "f"(weight) : "memory");
+            }
+        }
+        team_sync(team);
+    }
+    asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+    if (rank >= group) return;
+
+    // Combine head `rank` of the group.
+    const uint32_t head = kv_head * group + rank;
+    const bool has = tid < n_chunks;
+    const float chunk_top = has ? head_parts[tid * (HD + 2)] : -INFINITY;
+    float m = warp_max(chunk_top);
+    if (lane == 0) sh.across[0][cta_warp] = m;
+    __syncthreads();
+    m = sh.across[0][0];
+#pragma unroll
+    for (uint32_t w = 1; w < kTokenChunks / 32; ++w) m = fmaxf(m, sh.across[0][w]);
+    float sum = 0.f;
+    if (has) {
+        const float w = expf(chunk_top - m);
+        sh.weights[tid] = w;
+        sum += w * head_parts[tid * (HD + 2) + 1];
+    }
+    sum = warp_sum(sum);
+    if (lane == 0) sh.across[1][cta_warp] = sum;
+    __syncthreads();
+    for (uint32_t i = tid; i < kCombineParts * HD; i += kTokenThreads) {
+        const uint32_t part = i / HD, d = i % HD;
+        float acc = 0.f;
+#pragma unroll 8
+        for (uint32_t c = part; c < n_chunks; c += kCombineParts) acc += sh.weights[c] * head_parts[c * (HD + 2) + 2 + d];
+        sh.sums[i] = acc;
+    }
+    __syncthreads();
+    if (tid < HD) {
+        float total = 0.f, all = 0.f;
+#pragma unroll
+        for (uint32_t w = 0; w < kTokenChunks / 32; ++w) total += sh.across[1][w];
+#pragma unroll
+        for (int r = 0; r < kCombineParts; ++r) all += sh.sums[r * HD + tid];
+        float out = all / total;
+        if (gated) out *= 1.f / (1.f + expf(-p.q[(uint64_t)head * p.q_head_stride + HD + tid]));  // gate_factor
+        p.scratch[(uint64_t)head * HD + tid] = out;
+    }
+}
+
+template <typename T, int HD>
+const void* token_kernel_for(uint32_t group, bool fused) {
+    if (fused) return group <= 2 ? (const void*)attention_token_kernel<T, HD, 2, true> : (const void*)attention_token_kernel<T, HD, 4, true>;
+    return group <= 2 ? (const void*)attention_token_kernel<T, HD, 2, false> : (const void*)attention_token_kernel<T, HD, 4, false>;
+}
+template <typename T>
+const void* token_kernel(uint32_t head_dim, uint32_t group, bool fused) {
+    return head_dim == 64 ? token_kernel_for<T, 64>(group, fused) : head_dim == 128 ? token_kernel_for<T, 128>(group, fused) : token_kernel_for<T, 256>(group, fused);
+}
+template <int HD>
+size_t token_shared(uint32_t group) {
+    return group <= 2 ? sizeof(TokenShared<HD, 2>) : sizeof(TokenShared<HD, 4>);
+}
+size_t token_bytes(const AttentionShape& s) {
+    const uint32_t group = s.n_heads / s.n_kv_heads, chunks = (s.n_ctx + kDecodeChunk - 1) / kDecodeChunk;
+    return (s.head_dim == 64 ? token_shared<64>(group) : s.head_dim == 128 ? token_shared<128>(group) : token_shared<256>(group)) +
+           (size_t)chunks * (s.head_dim + 2) * sizeof(float);
+}
+
+// One query over a context of at most four passes of a cluster's warps: a pass covers 32 chunks of heads of 64 elements, 8 of 256. Measured
+// in us per generated token, two launches and one: 350M, f32 cache (8 KV heads of 64) at position 128 358 and 294, 512 354 and 300,
+// 1900 429 and 332, half cache 304 and 286, 365 and 320; 2.6B 128 767 and 741, 1900 878 and 819; two KV heads of 256, 128 842 and
+// 812, but 512 835 and 845, 1000 857 and 878.
+bool token_shape(const AttentionShape& s) {
+    return s.n_queries == 1 && (s.head_dim == 64 || s.head_dim == 128 || s.head_dim == 256) && s.q_stride % 4 == 0 && s.q_head_stride % 4 == 0 &&
+           s.n_heads / s.n_kv_heads <= kTokenGroup && s.n_ctx <= kTokenChunks * kDecodeChunk / (s.head_dim / 64);
+}
+
+// `cp.scratch` is the output.
+cudaError_t launch_token(cudaStream_t stream, ChunkParams cp, const AttentionShape& s, bool kv_half, bool fused, bool gated) {
+    const uint32_t group = s.n_heads / s.n_kv_heads;
+    const void* kernel = kv_half ? token_kernel<__half>(s.head_dim, group, fused) : token_kernel<float>(s.head_dim, group, fused);
+    const size_t smem = token_bytes(s);
+    cudaError_t e = ensure_dynamic_smem(kernel, smem);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(kTokenCluster * s.n_kv_heads);
+    config.blockDim = dim3(kTokenThreads);
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+    cudaLaunchAttribute attributes[2];
+    attributes[0].id = cudaLaunchAttributeClusterDimension;
+    attributes[0].val.clusterDim.x = kTokenCluster;
+    attributes[0].val.clusterDim.y = attributes[0].val.clusterDim.z = 1;
+    attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attributes[1].val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = attributes;
+    config.numAttrs = pdl_enabled() ? 2 : 1;
+    int gate = gated;
+    void* args[] = {&cp, &gate};
+    return cudaLaunchKernelExC(&config, kernel, args);
+}
+
 struct CombineParams {
     const float* scratch;
     float* out;
     uint32_t n_heads, head_dim, first_pos, query0, max_chunks;
     const uint32_t* pos_ptr;
     uint32_t chunk;
+    const float* gates;  // one query, optional: head h's, gate_stride apart
+    uint32_t gate_stride;
 };
+
+// attention_gate_kernel's factor.
+__device__ __forceinline__ float gate_factor(float g) { return 1.f / (1.f + expf(-g)); }
 
 // grid (n_heads, queries in batch), kCombineParts * head_dim threads. The threads first share out
 // the chunks' maxima and sums (so the exponentials are computed once, in parallel); then part r
 // of the threads adds up every kCombineParts-th chunk, each thread one element of the head with
 // independent loads, and the parts are added in order.
-constexpr int kCombineParts = 4;
 constexpr int kCombineSlice = 512;  // chunks whose weights shared memory holds at a time
 
 __global__ void attention_combine_kernel(CombineParams p) {
@@ -502,7 +839,9 @@ __global__ void attention_combine_kernel(CombineParams p) {
         for (uint32_t w = 0; w < n_warps; ++w) total += across[w];
 #pragma unroll
         for (int r = 0; r < kCombineParts; ++r) all += parts[r * hd + d];
-        p.out[(uint64_t)query * p.n_heads * hd + (uint64_t)head * hd + d] = all / total;
+        float out = all / total;
+        if (p.gates) out *= gate_factor(p.gates[(uint64_t)head * p.gate_stride + d]);
+        p.out[(uint64_t)query * p.n_heads * hd + (uint64_t)head * hd + d] = out;
     }
 }
 
@@ -519,6 +858,7 @@ uint64_t attention_scratch_floats(uint32_t n_heads, uint32_t head_dim, uint32_t 
 
 int attention_launches(bool kv_half, const AttentionShape& s) {
     if (attention_flash_supported(kv_half, s)) return attention_flash_launches(s);
+    if (token_shape(s)) return 1;
     return 2 * (int)((s.n_queries + kQueryBatch - 1) / kQueryBatch);
 }
 
@@ -529,6 +869,11 @@ cudaError_t attention(cudaStream_t stream, const float* q, const void* k_cache, 
     // do not start on those boundaries take the chunk kernels, whose loads are scalar.
     const bool flash_aligned = ((uintptr_t)q | (uintptr_t)out) % 8 == 0 && ((uintptr_t)k_cache | (uintptr_t)v_cache) % 16 == 0;
     if (flash_aligned && attention_flash_supported(kv_half, s)) return attention_flash(stream, q, k_cache, v_cache, scratch, out, s);
+    if (token_shape(s) && ((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache) % 16 == 0) {
+        const ChunkParams cp{q, k_cache, v_cache, out, s.n_heads, s.n_kv_heads, s.head_dim, s.first_pos, s.n_ctx,
+                             s.q_stride, s.q_head_stride, 0, 0, s.pos_ptr, (uint32_t)kDecodeChunk, nullptr, nullptr, nullptr, nullptr, 0.f, 0.f, nullptr};
+        return launch_token(stream, cp, s, kv_half, false, s.gated);
+    }
     const uint32_t group = s.n_heads / s.n_kv_heads;
     const uint32_t chunk = s.n_queries <= (uint32_t)kDecodeQueries ? decode_chunk(s.n_ctx) : (uint32_t)kChunk;
     const uint32_t max_chunks = (s.n_ctx + chunk - 1) / chunk;
@@ -553,8 +898,8 @@ cudaError_t attention(cudaStream_t stream, const float* q, const void* k_cache, 
             const void* chunk_kernel = kv_half ? (const void*)attention_chunk_kernel<__half> : (const void*)attention_chunk_kernel<float>;
             if ((e = launch_kernel(chunk_kernel, grid, dim3(kChunkThreads), smem, stream, chunk_args)) != cudaSuccess) return e;
         }
-        CombineParams mp{scratch, out, s.n_heads, s.head_dim, s.first_pos, q0, max_chunks, s.pos_ptr, chunk};
-        void* combine_args[] = {&mp};
+        const CombineParams mp{scratch, out, s.n_heads, s.head_dim, s.first_pos, q0, max_chunks, s.pos_ptr, chunk, s.gated ? q + s.head_dim : nullptr, s.q_head_stride};
+        void* combine_args[] = {const_cast<CombineParams*>(&mp)};
         if ((e = launch_kernel((const void*)attention_combine_kernel, dim3(s.n_heads, nq), dim3(kCombineParts * s.head_dim),
                                (size_t)kCombineParts * s.head_dim * sizeof(float), stream, combine_args)) != cudaSuccess)
             return e;
@@ -563,11 +908,18 @@ cudaError_t attention(cudaStream_t stream, const float* q, const void* k_cache, 
 }
 
 bool attention_step_supported(const RopeStore& r, const AttentionShape& s) {
-    return r.kv_half && s.n_queries == 1 && decode_shape(true, s) && r.n_rot == s.head_dim && r.q_head_stride == s.q_head_stride &&
+    return (token_shape(s) || (r.kv_half && s.n_queries == 1 && decode_shape(true, s))) && r.n_rot == s.head_dim && r.q_head_stride == s.q_head_stride &&
            ((uintptr_t)r.q | (uintptr_t)r.k | (uintptr_t)r.v | (uintptr_t)r.k_cache | (uintptr_t)r.v_cache) % 16 == 0;
 }
 
+int attention_step_launches(const AttentionShape& s) { return token_shape(s) ? 1 : 2; }
+
 cudaError_t attention_step(cudaStream_t stream, const RopeStore& r, float* scratch, float* out, const AttentionShape& s) {
+    if (token_shape(s)) {
+        const ChunkParams cp{r.q, r.k_cache, r.v_cache, out, s.n_heads, s.n_kv_heads, s.head_dim, s.first_pos, s.n_ctx,
+                             s.q_stride, s.q_head_stride, 0, 0, s.pos_ptr, (uint32_t)kDecodeChunk, r.k, r.v, r.q_norm, r.k_norm, r.eps, r.theta, r.table};
+        return launch_token(stream, cp, s, r.kv_half, true, s.gated);
+    }
     const uint32_t chunk = decode_chunk(s.n_ctx), max_chunks = (s.n_ctx + chunk - 1) / chunk;
     ChunkParams cp{r.q, r.k_cache, r.v_cache, scratch, s.n_heads, s.n_kv_heads, s.head_dim, s.first_pos, s.n_ctx,
                    s.q_stride, s.q_head_stride, 0, max_chunks, s.pos_ptr, chunk, r.k, r.v, r.q_norm, r.k_norm, r.eps, r.theta, r.table};
@@ -577,8 +929,8 @@ cudaError_t attention_step(cudaStream_t stream, const RopeStore& r, float* scrat
     if (!kernel) return cudaErrorInvalidValue;
     cudaError_t e = launch_kernel(kernel, grid, dim3(kDecodeThreads), 0, stream, chunk_args);
     if (e != cudaSuccess) return e;
-    CombineParams mp{scratch, out, s.n_heads, s.head_dim, s.first_pos, 0, max_chunks, s.pos_ptr, chunk};
-    void* combine_args[] = {&mp};
+    const CombineParams mp{scratch, out, s.n_heads, s.head_dim, s.first_pos, 0, max_chunks, s.pos_ptr, chunk, s.gated ? r.q + s.head_dim : nullptr, s.q_head_stride};
+    void* combine_args[] = {const_cast<CombineParams*>(&mp)};
     return launch_kernel((const void*)attention_combine_kernel, dim3(s.n_heads, 1), dim3(kCombineParts * s.head_dim),
                          (size_t)kCombineParts * s.head_dim * sizeof(float), stream, combine_args);
 }

@@ -340,16 +340,17 @@ struct Recorder {
         return static_cast<float*>(cache_at(s.v_cache, layer_base(cache_index) + (size_t)pos * kv_dim()));
     }
 
-    // One token: norm and rotation of q and k, the K and V rows of position `pos` into the caches
-    // (one launch), then attention over positions [0, pos].
-    void decode_attend(const DeviceLayer& D, uint32_t cache_index, uint32_t pos, uint32_t q_stride, uint32_t q_head_stride) {
+    // One token: norm and rotation of q and k, the K and V rows of position `pos` into the caches, attention over positions
+    // [0, pos]; `gated`: the outputs times the sigmoid of the values that follow each head's queries.
+    void decode_attend(const DeviceLayer& D, uint32_t cache_index, uint32_t pos, uint32_t q_stride, uint32_t q_head_stride, bool gated = false) {
         k::RopeStore rs{s.q, s.k, s.v, cache_at(s.k_cache, layer_base(cache_index)), cache_at(s.v_cache, layer_base(cache_index)),
                         D.q_norm, D.k_norm, hp.n_heads, hp.n_kv_heads, hp.head_dim, q_head_stride, hp.n_rot, hp.rope_theta, hp.norm_eps, s.kv_half, s.rope_table};
         k::Pos p = at(pos);
         k::AttentionShape shape{hp.n_heads, hp.n_kv_heads, hp.head_dim, p.value, 1, s.n_ctx, q_stride, q_head_stride, p.ptr};
         uint64_t kv_bytes = (uint64_t)(pos + 1) * kv_dim() * kv_element_bytes() * 2;
+        shape.gated = gated;
         if (k::attention_step_supported(rs, shape)) {
-            run("attention_step", 1, pos + 1, kv_bytes, 2, [&] { return k::attention_step(stream, rs, s.scores, s.attn, shape); });
+            run("attention_step", 1, pos + 1, kv_bytes, k::attention_step_launches(shape), [&] { return k::attention_step(stream, rs, s.scores, s.attn, shape); });
             return;
         }
         run("rope_store", hp.n_heads + 2 * hp.n_kv_heads, hp.head_dim, 0, 1, [&] { return k::rope_store(stream, rs, p); });
@@ -626,8 +627,7 @@ struct Recorder {
                 k::MatvecSegment segs[3] = {{D.q, s.q}, {D.k, s.k}, {D.v, s.v}};
                         run("matvec_qkv", D.q.n_rows + D.k.n_rows + D.v.n_rows, D.q.n_cols, D.q.bytes() + D.k.bytes() + D.v.bytes(), 1,
                     [&] { return k::matvec(stream, segs, 3, s.hidden, norm(D.attn_norm), false); });
-                        decode_attend(D, S.cache_index, pos, 2 * q_dim, 2 * hp.head_dim);
-                run("attention_gate", 1, q_dim, 0, 1, [&] { return k::attention_gate(stream, s.attn, s.q, hp.n_heads, hp.head_dim, 1); });
+                        decode_attend(D, S.cache_index, pos, 2 * q_dim, 2 * hp.head_dim, true);
                 matvec_reduced(D.output, s.attn, s.hidden);
             } else {
                 k::MatvecSegment segs[4] = {{D.qkv, s.gdn_qkv}, {D.z, s.gdn_z}, {D.beta, s.gdn_beta}, {D.alpha, s.gdn_alpha}};
