@@ -7,6 +7,7 @@
 // A token's route is 2 * n_used 32-bit words: the picked expert ids, then their weights as float
 // bits (moe.metal:4-6).
 
+#include "device_facts.h"
 #include "matvec_common.cuh"
 
 namespace bc {
@@ -34,6 +35,59 @@ struct RouteParams {
     uint32_t* route;
     uint32_t n_cols, n_experts, n_used, n_tokens;
 };
+
+// A warp picks a token's experts from their scores.
+__device__ __forceinline__ void pick_experts(const RouteParams& p, const float* mine, uint32_t token) {
+    const uint32_t lane = threadIdx.x & 31;
+    // Top n_used by repeated argmax of score + bias, ties to the lower id; the weights are the
+    // unbiased scores over their f32 sum plus 1e-6 (lfm2.rs:698-708). Lane l looks after experts
+    // l, l + 32, l + 64, l + 96; a round is a lane-local scan and a warp-wide compare.
+    float value[kMaxExperts / 32];
+    bool taken[kMaxExperts / 32];
+#pragma unroll
+    for (int k = 0; k < kMaxExperts / 32; ++k) {
+        const uint32_t e = lane + 32 * k;
+        value[k] = e < p.n_experts ? mine[e] + p.bias[e] : 0.f;
+        taken[k] = e >= p.n_experts;
+    }
+    uint32_t picked = 0;   // lane i < n_used ends up holding the i-th pick
+    float picked_score = 0.f, sum = 0.f;
+    for (uint32_t i = 0; i < p.n_used; ++i) {
+        float best_value = 0.f;
+        uint32_t best = 0xffffffffu;
+#pragma unroll
+        for (int k = 0; k < kMaxExperts / 32; ++k) {
+            if (!taken[k] && (best == 0xffffffffu || value[k] > best_value)) {
+                best_value = value[k];
+                best = lane + 32 * k;
+            }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float other_value = __shfl_xor_sync(0xffffffffu, best_value, o);
+            const uint32_t other = __shfl_xor_sync(0xffffffffu, best, o);
+            if (other != 0xffffffffu && (best == 0xffffffffu || other_value > best_value || (other_value == best_value && other < best))) {
+                best_value = other_value;
+                best = other;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < kMaxExperts / 32; ++k)
+            if (best == lane + 32 * k) taken[k] = true;
+        const float score = mine[best];
+        sum += score;  // in pick order, as the scalar code adds them
+        if (lane == i) {
+            picked = best;
+            picked_score = score;
+        }
+    }
+    const float norm = sum + 1e-6f;
+    uint32_t* route = p.route + (uint64_t)token * 2 * p.n_used;
+    if (lane < p.n_used) {
+        route[lane] = picked;
+        route[p.n_used + lane] = __float_as_uint(picked_score / norm);
+    }
+}
 
 constexpr int kRouteThreads = 1024;
 constexpr int kRouteWarps = kRouteThreads / 32;
@@ -206,56 +260,94 @@ __global__ void __launch_bounds__(kRouteThreads) moe_route_kernel(const __grid_c
         __syncthreads();
     }
     if (warp < here) {
-        const float* mine = scores[warp];
-        // Top n_used by repeated argmax of score + bias, ties to the lower id; the weights are the
-        // unbiased scores over their f32 sum plus 1e-6 (lfm2.rs:698-708). Lane l looks after experts
-        // l, l + 32, l + 64, l + 96; a round is a lane-local scan and a warp-wide compare.
-        float value[kMaxExperts / 32];
-        bool taken[kMaxExperts / 32];
+        pick_experts(p, scores[warp], token0 + warp);
+    }
+}
+
+// Few tokens of a router of at most 32 experts and 2048 columns: a cluster of sixteen CTAs per token, two experts to a CTA, the
+// same sums in f64. Bound by the chain from the residual stream to the pick. Eight CTAs of 1024 threads did not
+// fit beside a CTA of the preceding launch, so their weights were on their way only after it, and conversions to f64 (16 per cycle and SM)
+// stood between the norm and the scores: 7.5 us. A CTA of 256 threads and 64 registers does, converts its weights ahead of the
+// wait, and a thread keeps its eight columns in registers through norm and products.
+constexpr uint32_t kTokenCluster = 16, kTokenThreads = 256, kTokenWarps = kTokenThreads / 32, kTokenExperts = 2, kTokenQuads = 2;
+
+__global__ void __launch_bounds__(kTokenThreads, 4) moe_route_token_kernel(const __grid_constant__ RouteParams p) {
+    __shared__ float scores[kTokenCluster * kTokenExperts];
+    __shared__ double reduce[kTokenExperts + 1][kTokenWarps];
+    pdl_launch_dependents();
+    asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");  // this CTA runs: its shared memory may be written
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rank = blockIdx.x % kTokenCluster, token = blockIdx.x / kTokenCluster;
+    const uint32_t quads = p.n_cols / 4;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    double w[kTokenExperts][kTokenQuads][4];
+    float4 nw[kTokenQuads];
 #pragma unroll
-        for (int k = 0; k < kMaxExperts / 32; ++k) {
-            const uint32_t e = lane + 32 * k;
-            value[k] = e < p.n_experts ? mine[e] + p.bias[e] : 0.f;
-            taken[k] = e >= p.n_experts;
-        }
-        uint32_t picked = 0;   // lane i < n_used ends up holding the i-th pick
-        float picked_score = 0.f, sum = 0.f;
-        for (uint32_t i = 0; i < p.n_used; ++i) {
-            float best_value = 0.f;
-            uint32_t best = 0xffffffffu;
+    for (uint32_t q = 0; q < kTokenQuads; ++q) {
+        const uint32_t quad = tid + q * kTokenThreads;
+        nw[q] = p.norm_weight && quad < quads ? __ldg(reinterpret_cast<const float4*>(p.norm_weight) + quad) : zero;
 #pragma unroll
-            for (int k = 0; k < kMaxExperts / 32; ++k) {
-                if (!taken[k] && (best == 0xffffffffu || value[k] > best_value)) {
-                    best_value = value[k];
-                    best = lane + 32 * k;
-                }
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const float other_value = __shfl_xor_sync(0xffffffffu, best_value, o);
-                const uint32_t other = __shfl_xor_sync(0xffffffffu, best, o);
-                if (other != 0xffffffffu && (best == 0xffffffffu || other_value > best_value || (other_value == best_value && other < best))) {
-                    best_value = other_value;
-                    best = other;
-                }
-            }
-#pragma unroll
-            for (int k = 0; k < kMaxExperts / 32; ++k)
-                if (best == lane + 32 * k) taken[k] = true;
-            const float score = mine[best];
-            sum += score;  // in pick order, as the scalar code adds them
-            if (lane == i) {
-                picked = best;
-                picked_score = score;
-            }
-        }
-        const float norm = sum + 1e-6f;
-        uint32_t* route = p.route + (uint64_t)(token0 + warp) * 2 * p.n_used;
-        if (lane < p.n_used) {
-            route[lane] = picked;
-            route[p.n_used + lane] = __float_as_uint(picked_score / norm);
+        for (uint32_t m = 0; m < kTokenExperts; ++m) {
+            const uint32_t e = rank + kTokenCluster * m;
+            const float4 f = e < p.n_experts && quad < quads ? __ldg(reinterpret_cast<const float4*>(p.router + (uint64_t)e * p.n_cols) + quad) : zero;
+            w[m][q][0] = f.x, w[m][q][1] = f.y, w[m][q][2] = f.z, w[m][q][3] = f.w;
         }
     }
+    pdl_wait();
+    float4 x[kTokenQuads];
+#pragma unroll
+    for (uint32_t q = 0; q < kTokenQuads; ++q) {
+        const uint32_t quad = tid + q * kTokenThreads;
+        x[q] = quad < quads ? *(reinterpret_cast<const float4*>(p.x + (uint64_t)token * p.n_cols) + quad) : zero;
+    }
+    if (p.norm_weight) {
+        double square[kTokenQuads];
+#pragma unroll
+        for (uint32_t q = 0; q < kTokenQuads; ++q)
+            square[q] = ((double)x[q].x * x[q].x + (double)x[q].y * x[q].y) + ((double)x[q].z * x[q].z + (double)x[q].w * x[q].w);
+        const double sumsq = warp_sum_f64(square[0] + square[1]);
+        if (lane == 0) reduce[kTokenExperts][warp] = sumsq;
+        __syncthreads();
+        double total = 0.0;
+#pragma unroll
+        for (uint32_t i = 0; i < kTokenWarps; ++i) total += reduce[kTokenExperts][i];
+        const float scale = (float)(1.0 / sqrt(total / (double)p.n_cols + (double)p.eps));
+#pragma unroll
+        for (uint32_t q = 0; q < kTokenQuads; ++q) {
+            x[q] = make_float4(nw[q].x * (x[q].x * scale), nw[q].y * (x[q].y * scale), nw[q].z * (x[q].z * scale), nw[q].w * (x[q].w * scale));
+            const uint32_t quad = tid + q * kTokenThreads;
+            if (rank == 0 && quad < quads) *(reinterpret_cast<float4*>(p.normed + (uint64_t)token * p.n_cols) + quad) = x[q];
+        }
+    }
+    double sum[kTokenExperts];
+#pragma unroll
+    for (uint32_t m = 0; m < kTokenExperts; ++m) sum[m] = 0.0;
+#pragma unroll
+    for (uint32_t q = 0; q < kTokenQuads; ++q) {
+        const double v[4] = {x[q].x, x[q].y, x[q].z, x[q].w};
+#pragma unroll
+        for (uint32_t m = 0; m < kTokenExperts; ++m) sum[m] += (w[m][q][0] * v[0] + w[m][q][1] * v[1]) + (w[m][q][2] * v[2] + w[m][q][3] * v[3]);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (uint32_t m = 0; m < kTokenExperts; ++m) sum[m] += __shfl_xor_sync(0xffffffffu, sum[m], o);
+    if (lane == 0)
+#pragma unroll
+        for (uint32_t m = 0; m < kTokenExperts; ++m) reduce[m][warp] = sum[m];
+    __syncthreads();
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    if (tid < kTokenExperts && rank + kTokenCluster * tid < p.n_experts) {
+        double total = 0.0;
+#pragma unroll
+        for (uint32_t i = 0; i < kTokenWarps; ++i) total += reduce[tid][i];
+        const float score = 1.0f / (1.0f + expf(-(float)total));
+        uint32_t at;
+        asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(at) : "r"((uint32_t)__cvta_generic_to_shared(&scores[rank + kTokenCluster * tid])));
+        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(at), "f"(score) : "memory");
+    }
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+    if (rank == 0 && warp == 0) pick_experts(p, scores, token);
 }
 
 // One CTA: counting sort of the (token, slot) entries by expert. offsets[e] is the first entry of
@@ -501,10 +593,52 @@ cudaError_t launch_experts(Kernel kernel, dim3 grid, size_t smem, cudaStream_t s
 
 }  // namespace
 
+namespace {
+void token_config(cudaLaunchConfig_t& config, cudaLaunchAttribute (&attributes)[2], uint32_t n_tokens) {
+    config.gridDim = dim3(kTokenCluster * n_tokens);
+    config.blockDim = dim3(kTokenThreads);
+    attributes[0].id = cudaLaunchAttributeClusterDimension;
+    attributes[0].val.clusterDim.x = kTokenCluster;
+    attributes[0].val.clusterDim.y = attributes[0].val.clusterDim.z = 1;
+    attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attributes[1].val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = attributes;
+    config.numAttrs = pdl_enabled() ? 2 : 1;
+}
+// Clusters of sixteen are more than every device offers: how many the current one runs at once (0: none).
+int route_clusters() {
+    static DeviceFacts<1> kept;
+    int device = 0, clusters = 0;
+    cudaGetDevice(&device);
+    kept.get(device, 0, [](int* n) {
+        *n = 0;
+        if (cudaFuncSetAttribute((const void*)moe_route_token_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
+            cudaLaunchConfig_t config = {};
+            cudaLaunchAttribute attributes[2];
+            token_config(config, attributes, 1);
+            config.numAttrs = 1;
+            if (cudaOccupancyMaxActiveClusters(n, (const void*)moe_route_token_kernel, &config) != cudaSuccess) *n = 0;
+        }
+        if (*n == 0) cudaGetLastError();  // this device does without
+        *n += 1;                          // kept facts are positive
+        return true;
+    }, &clusters);
+    return clusters - 1;
+}
+}  // namespace
+
 cudaError_t moe_route(cudaStream_t stream, const float* x, Norm norm, float* normed, const float* router, const float* bias,
                       uint32_t* route, uint32_t n_cols, uint32_t n_experts, uint32_t n_used, uint32_t n_tokens) {
     if (n_tokens == 0) return cudaSuccess;
     const RouteParams p{x, norm.weight, norm.eps, normed, router, bias, route, n_cols, n_experts, n_used, n_tokens};
+    if (n_cols % 4 == 0 && n_cols / 4 <= kTokenThreads * kTokenQuads && n_experts <= kTokenCluster * kTokenExperts && n_tokens * kTokenCluster <= (uint32_t)sm_count() &&
+        ((uintptr_t)x | (uintptr_t)norm.weight | (uintptr_t)(norm.weight ? normed : nullptr) | (uintptr_t)router) % 16 == 0 && route_clusters() > 0) {
+        cudaLaunchConfig_t config = {};
+        cudaLaunchAttribute attributes[2];
+        token_config(config, attributes, n_tokens);
+        config.stream = stream;
+        return cudaLaunchKernelEx(&config, moe_route_token_kernel, p);
+    }
     // A cluster per token until they fill the device; rows too wide for f64 in shared memory stay f32 there.
     const bool few = n_tokens * kRouteCluster <= (uint32_t)sm_count();
     const bool wide = (size_t)n_cols * 8 * (few ? 1 : kRouteTokens) <= 200 * 1024;
