@@ -67,6 +67,23 @@ inline cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 b
     config.numAttrs = pdl_enabled() ? 1 : 0;
     return cudaLaunchKernelEx(&config, kernel, std::forward<Args>(args)...);
 }
+// The same in clusters of `cluster` CTAs along x.
+template <typename... Params, typename... Args>
+inline cudaError_t launch_clusters(void (*kernel)(Params...), dim3 grid, dim3 block, unsigned cluster, cudaStream_t stream, Args&&... args) {
+    cudaLaunchConfig_t config = {};
+    config.gridDim = grid;
+    config.blockDim = block;
+    config.stream = stream;
+    cudaLaunchAttribute attributes[2];
+    attributes[0].id = cudaLaunchAttributeClusterDimension;
+    attributes[0].val.clusterDim.x = cluster;
+    attributes[0].val.clusterDim.y = attributes[0].val.clusterDim.z = 1;
+    attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attributes[1].val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = attributes;
+    config.numAttrs = pdl_enabled() ? 2 : 1;
+    return cudaLaunchKernelEx(&config, kernel, std::forward<Args>(args)...);
+}
 // Raise `kernel`'s dynamic shared-memory limit to `smem` bytes on the current device if needed.
 cudaError_t ensure_dynamic_smem(const void* kernel, size_t smem);
 // Number of SMs of the current device.

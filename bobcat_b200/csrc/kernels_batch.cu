@@ -201,56 +201,16 @@ __global__ void short_conv_seqs_kernel(const float* __restrict__ bcx, const floa
     out[(uint64_t)b * n_embd + ch] = c * sum;
 }
 
-// argmax of each row (ties to the lowest index): a CTA per sequence. picked[b] takes the index and,
+// argmax of each row (ties to the lowest index): a cluster per sequence. picked[b] takes the index and,
 // when `record` is non-null, so does record[b * record_stride + record_at].
-__global__ void __launch_bounds__(1024) argmax_rows_kernel(const float* __restrict__ x, uint32_t n, uint32_t* __restrict__ picked,
-                                                           uint32_t* __restrict__ record, uint32_t record_stride, uint32_t record_at) {
-    __shared__ float best_value[32];
-    __shared__ uint32_t best_index[32];
+__global__ void __launch_bounds__(kArgmaxThreads) argmax_rows_kernel(const float* __restrict__ x, uint32_t n, uint32_t* __restrict__ picked,
+                                                                     uint32_t* __restrict__ record, uint32_t record_stride, uint32_t record_at) {
     pdl_launch_dependents();
     pdl_wait();
-    const float* row = x + (uint64_t)blockIdx.x * n;
-    float value = -INFINITY;
-    uint32_t index = 0xffffffffu;
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-        const float v = row[i];
-        if (v > value || index == 0xffffffffu) {
-            value = v;
-            index = i;
-        }
-    }
-    auto better = [](float v, uint32_t i, float bv, uint32_t bi) { return i != 0xffffffffu && (bi == 0xffffffffu || v > bv || (v == bv && i < bi)); };
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        float ov = __shfl_xor_sync(0xffffffffu, value, o);
-        uint32_t oi = __shfl_xor_sync(0xffffffffu, index, o);
-        if (better(ov, oi, value, index)) {
-            value = ov;
-            index = oi;
-        }
-    }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) {
-        best_value[warp] = value;
-        best_index[warp] = index;
-    }
-    __syncthreads();
-    if (warp == 0) {
-        value = best_value[lane];
-        index = best_index[lane];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            float ov = __shfl_xor_sync(0xffffffffu, value, o);
-            uint32_t oi = __shfl_xor_sync(0xffffffffu, index, o);
-            if (better(ov, oi, value, index)) {
-                value = ov;
-                index = oi;
-            }
-        }
-        if (lane == 0) {
-            picked[blockIdx.x] = index;
-            if (record) record[(uint64_t)blockIdx.x * record_stride + record_at] = index;
-        }
+    const uint32_t row = blockIdx.x / kArgmaxCluster, index = argmax_cluster(x + (uint64_t)row * n, n);
+    if (blockIdx.x % kArgmaxCluster == 0 && threadIdx.x == 0) {
+        picked[row] = index;
+        if (record) record[(uint64_t)row * record_stride + record_at] = index;
     }
 }
 
@@ -300,8 +260,7 @@ cudaError_t short_conv_seqs(cudaStream_t stream, const float* bcx, const float* 
 
 cudaError_t argmax_rows(cudaStream_t stream, const float* x, uint32_t n, uint32_t n_rows, uint32_t* picked, uint32_t* record,
                         uint32_t record_stride, uint32_t record_at) {
-    void* args[] = {&x, &n, &picked, &record, &record_stride, &record_at};
-    return launch_kernel((const void*)argmax_rows_kernel, dim3(n_rows), dim3(1024), 0, stream, args);
+    return launch_clusters(argmax_rows_kernel, dim3(kArgmaxCluster * n_rows), dim3(kArgmaxThreads), kArgmaxCluster, stream, x, n, picked, record, record_stride, record_at);
 }
 
 cudaError_t advance_seqs(cudaStream_t stream, uint32_t* pos, uint32_t n_seqs) {

@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(128) short_conv_kernel(const float* __restrict
     }
 }
 
-// One CTA of 1024 threads scans the vocabulary; ties go to the lowest index.
+// One cluster scans the vocabulary; ties go to the lowest index.
 struct ArgmaxOut {
     uint32_t* out;       // direct mode: the word to write
     uint32_t* readback;  // direct mode: optional host-mapped copy
@@ -312,84 +312,22 @@ struct ArgmaxOut {
     uint32_t ring_slots;
 };
 
-__global__ void __launch_bounds__(1024) argmax_kernel(const float* __restrict__ x, uint32_t n, ArgmaxOut o) {
-    __shared__ float best_value[32];
-    __shared__ uint32_t best_index[32];
+__global__ void __launch_bounds__(kArgmaxThreads) argmax_kernel(const float* __restrict__ x, uint32_t n, ArgmaxOut o) {
     pdl_launch_dependents();
     pdl_wait();
-    float value = -INFINITY;
-    uint32_t index = 0xffffffffu;
-    auto consider = [&](float v, uint32_t i) {
-        if (v > value || index == 0xffffffffu) {
-            value = v;
-            index = i;
+    const uint32_t index = argmax_cluster(x, n);
+    if (blockIdx.x != 0 || threadIdx.x != 0) return;
+    if (o.counter) {
+        uint32_t pos = *o.counter;
+        if (o.advance) {
+            pos += 1;
+            *o.counter = pos;
         }
-    };
-    // Eight 16-byte loads in flight per thread, visited in increasing index order so the first
-    // maximum wins; whatever does not fill a float4 goes one by one.
-    const uint32_t n4 = (reinterpret_cast<uintptr_t>(x) & 15) == 0 ? n / 4 : 0;
-    const float4* x4 = reinterpret_cast<const float4*>(x);
-    for (uint32_t base = threadIdx.x; base < n4; base += blockDim.x * 8) {
-        float4 v[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            uint32_t i = base + k * blockDim.x;
-            v[k] = i < n4 ? x4[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            uint32_t i = base + k * blockDim.x;
-            if (i < n4) {
-                consider(v[k].x, 4 * i);
-                consider(v[k].y, 4 * i + 1);
-                consider(v[k].z, 4 * i + 2);
-                consider(v[k].w, 4 * i + 3);
-            }
-        }
-    }
-    for (uint32_t i = 4 * n4 + threadIdx.x; i < n; i += blockDim.x) consider(x[i], i);
-    auto better = [](float v, uint32_t i, float bv, uint32_t bi) { return i != 0xffffffffu && (bi == 0xffffffffu || v > bv || (v == bv && i < bi)); };
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        float ov = __shfl_xor_sync(0xffffffffu, value, o);
-        uint32_t oi = __shfl_xor_sync(0xffffffffu, index, o);
-        if (better(ov, oi, value, index)) {
-            value = ov;
-            index = oi;
-        }
-    }
-    int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) {
-        best_value[warp] = value;
-        best_index[warp] = index;
-    }
-    __syncthreads();
-    if (warp == 0) {
-        value = best_value[lane];
-        index = best_index[lane];
-#pragma unroll
-        for (int step = 16; step > 0; step >>= 1) {
-            float ov = __shfl_xor_sync(0xffffffffu, value, step);
-            uint32_t oi = __shfl_xor_sync(0xffffffffu, index, step);
-            if (better(ov, oi, value, index)) {
-                value = ov;
-                index = oi;
-            }
-        }
-        if (lane == 0) {
-            if (o.counter) {
-                uint32_t pos = *o.counter;
-                if (o.advance) {
-                    pos += 1;
-                    *o.counter = pos;
-                }
-                o.tokens[pos + o.offset] = index;
-                if (o.ring) o.ring[pos % o.ring_slots] = index;
-            } else {
-                *o.out = index;
-                if (o.readback) *o.readback = index;
-            }
-        }
+        o.tokens[pos + o.offset] = index;
+        if (o.ring) o.ring[pos % o.ring_slots] = index;
+    } else {
+        *o.out = index;
+        if (o.readback) *o.readback = index;
     }
 }
 
@@ -660,16 +598,14 @@ cudaError_t short_conv(cudaStream_t stream, const float* bcx, const float* taps,
 }
 
 cudaError_t argmax(cudaStream_t stream, const float* x, uint32_t n, uint32_t* out, uint32_t* readback) {
-    ArgmaxOut o{out, readback, nullptr, 0, nullptr, 0, nullptr, 1};
-    void* args[] = {&x, &n, &o};
-    return launch_kernel((const void*)argmax_kernel, dim3(1), dim3(1024), 0, stream, args);
+    const ArgmaxOut o{out, readback, nullptr, 0, nullptr, 0, nullptr, 1};
+    return launch_clusters(argmax_kernel, dim3(kArgmaxCluster), dim3(kArgmaxThreads), kArgmaxCluster, stream, x, n, o);
 }
 
 cudaError_t argmax_step(cudaStream_t stream, const float* x, uint32_t n, uint32_t* counter, bool advance, uint32_t* tokens,
                         uint32_t offset, uint32_t* ring, uint32_t ring_slots) {
-    ArgmaxOut o{nullptr, nullptr, counter, advance ? 1 : 0, tokens, offset, ring, ring_slots ? ring_slots : 1};
-    void* args[] = {&x, &n, &o};
-    return launch_kernel((const void*)argmax_kernel, dim3(1), dim3(1024), 0, stream, args);
+    const ArgmaxOut o{nullptr, nullptr, counter, advance ? 1 : 0, tokens, offset, ring, ring_slots ? ring_slots : 1};
+    return launch_clusters(argmax_kernel, dim3(kArgmaxCluster), dim3(kArgmaxThreads), kArgmaxCluster, stream, x, n, o);
 }
 
 cudaError_t add_floats(cudaStream_t stream, float* y, const float* x, uint64_t n) {
