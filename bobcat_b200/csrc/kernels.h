@@ -440,14 +440,16 @@ bool matmul_half_swiglu_whole(const Mat& gate, uint32_t n_tokens);  // tiles of 
 // shape allows (BOBCAT_NO_FEW_MATMUL=1 keeps them on the tcgen05 kernels).
 // Code: 1, a warp on the other warps' sums.
 cudaError_t matmul_few_wait_word(int* word);
+// A batch over experts on tcgen05, weights unpacked into tensor memory (kernels_matmul_experts.cu).
+bool matmul_experts_tiles_supported(const Mat& w, const Mat* up, uint32_t n_rows);
+cudaError_t matmul_experts_tiles(cudaStream_t stream, const Mat& w, const Mat* up, uint32_t n_rows, uint32_t n_experts, const float* x, bool gather,
+                                 const uint32_t* offsets, const uint32_t* entries, uint32_t n_used, float* y, uint32_t n_tokens, void* scratch);
+cudaError_t matmul_experts_wait_word(int* word);
 bool matmul_few_supported(const Mat& w, uint32_t n_tokens);
 cudaError_t matmul_few(cudaStream_t stream, const Mat* const* ws, float* const* ys, const uint32_t* strides, int n, const void* packed,
                        uint32_t n_tokens, int32_t store);
 cudaError_t matmul_few_swiglu(cudaStream_t stream, const Mat& gate, const Mat& up, const void* packed, float* y, uint32_t n_tokens, uint32_t y_stride,
                               void* packed_out);
-bool matmul_few_experts_supported(const Mat& w, const Mat* up, uint32_t n_rows, uint32_t n_experts, uint32_t n_tokens, uint32_t n_used);
-cudaError_t matmul_few_experts(cudaStream_t stream, const Mat& w, const Mat* up, uint32_t n_rows, uint32_t n_experts, const void* packed,
-                               const uint32_t* offsets, const uint32_t* entries, float* y, uint32_t n_tokens, uint32_t n_entries);
 // Products of a few rows with f32 operands (the same file): up to four Q4_0 matrices that
 // share the rows, with the rows' RMSNorm when given, in one launch; gate and up of a SwiGLU; the
 // experts of a grouped batch. `matmul` and `matmul_experts` hand over to these when their shape allows

@@ -1,5 +1,5 @@
 // Q4_0 products against few rows (at most 64): passes over several sequences, prompts and prefill chunks of
-// some tokens, the experts of a batch. Two arithmetics, one weight stream.
+// some tokens, the experts of a few rows with f32 operands. Two arithmetics, one weight stream.
 //
 // Exact (the rows stay f32). An f32 input is exactly the sum of three bf16 values (8 significant bits
 // each, and bf16 has the range of f32), a quant minus 8 is exact in bf16, so the products of mma.m16n8k16 are
@@ -31,7 +31,7 @@
 // one warp asks for; a step's slot is refilled once every warp has arrived with its sums. The first
 // steps are requested before the wait for the preceding launch. (With per-lane cp.async into slots of a lane's own, 24 requests and their
 // addresses in every warp took 2 us of a launch before its first multiply: 11 rows of the 350M shape's prompt 632 us, now 606, six
-// sequences of the 2.6B shape 12.43 -> 12.16 ms, an expert block of 203 tokens 237 -> 233 us; 24 rows with half operands 11.47 -> 11.52 ms a
+// sequences of the 2.6B shape 12.43 -> 12.16 ms; 24 rows with half operands 11.47 -> 11.52 ms a
 // scoring request.)
 
 #include <cstdlib>
@@ -97,7 +97,6 @@ struct FewParams {
     uint32_t n_experts;
     uint32_t n_used;
     int gather;
-    uint32_t cap_groups;           // half: an expert's rows are packed from token group z * cap_groups on
 };
 
 __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
@@ -182,13 +181,13 @@ __device__ __forceinline__ bool find_group(const uint32_t* offsets, uint32_t n_e
 // Experts: how many rows each has is known on the device alone, so the launch is as wide as the device and every CTA (cluster)
 // takes an equal run of the jobs of all groups of rows, which may end in the next group, whose inputs it then loads. (A share of the CTAs
 // per expert and group, for the likely number of groups, left SMs idle or began a second wave. An expert block of 32 experts of 1792
-// x 2048, us with all its launches: 2 tokens 103 -> 91, 16 tokens 179 -> 151, 64 tokens 222 -> 163, 203 tokens 231 to 352, as the
-// router picks, -> 237 to 251; passes of 15 sequences of such a model 15.6 -> 12.6 ms.)
+// x 2048, us with all its launches: 2 tokens 103 -> 91; passes of 15 sequences of such a model 15.6 -> 12.6 ms.)
 // Built on the same loop and taken back: four more warps for the sums and stores, so that the others only multiply (12.08 ms
 // against 11.95, and four more sums per tile in flight); with them a tile's loads and its first unpacking ahead of the tile before (13.1 ms: spills).
 template <bool EXACT, bool EXPERTS, int NT, int W, int DEPTH>
 __global__ void __launch_bounds__(kThreads, 1) matmul_few_kernel(const __grid_constant__ FewParams p) {
     static_assert(!EXACT || NT == 1, "the pieces of more rows do not fit the registers");
+    static_assert(EXACT || !EXPERTS, "experts with half operands: kernels_matmul_experts.cu");
     constexpr uint32_t kTileSums = 128 * NT, kPieces = EXACT ? 3 : NT, T = tiles_per_step(NT), kTileSlot = W * kWarps * kPairBytes, kStepBytes = T * kTileSlot;
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ float sums[2][T * kTileSums];        // clusters: this CTA's sums of a step
@@ -357,8 +356,8 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_few_kernel(const __grid_co
             if (t == 0) squares[warp][g] = square;
         }
     } else {
-        if (!EXPERTS) pdl_wait();
-        const uint32_t group0 = (EXPERTS ? expert * p.cap_groups : 0) + group * NT;
+        pdl_wait();
+        const uint32_t group0 = group * NT;
         const uint32_t groups = (n_tokens - token0 + 7) / 8;  // groups past the rows stay zero
 #pragma unroll
         for (int i = 0; i < W; ++i)
@@ -651,7 +650,10 @@ cudaError_t launch_as(cudaStream_t stream, FewParams& p, uint32_t groups) {
 }
 template <bool EXACT, int NT, int W, int DEPTH>
 cudaError_t launch(cudaStream_t stream, FewParams& p, uint32_t groups) {
-    return p.offsets ? launch_as<EXACT, true, NT, W, DEPTH>(stream, p, groups) : launch_as<EXACT, false, NT, W, DEPTH>(stream, p, groups);
+    if constexpr (EXACT) {
+        if (p.offsets) return launch_as<EXACT, true, NT, W, DEPTH>(stream, p, groups);
+    }
+    return launch_as<EXACT, false, NT, W, DEPTH>(stream, p, groups);
 }
 
 // Cut K: as few CTAs per cluster as hold the inputs at `most` pairs per warp, evenly.
@@ -672,9 +674,9 @@ cudaError_t launch_exact(cudaStream_t stream, FewParams& p) {
 }
 
 // Row groups of 8 a launch's CTA holds: the fewest that cover the rows in as few groups of 32 as possible
-// (33 rows: two groups of 24). `rows`: those of the largest (expert: likely) batch.
-cudaError_t launch_half(cudaStream_t stream, FewParams& p, uint32_t rows) {
-    const uint32_t parts = (rows + kHalfGroup - 1) / kHalfGroup, nt = ((rows + parts - 1) / parts + 7) / 8;
+// (33 rows: two groups of 24).
+cudaError_t launch_half(cudaStream_t stream, FewParams& p) {
+    const uint32_t rows = p.n_tokens, parts = (rows + kHalfGroup - 1) / kHalfGroup, nt = ((rows + parts - 1) / parts + 7) / 8;
     const uint32_t w = cut(p, nt <= 2 ? 3 : 2), groups = (p.n_tokens + 8 * (nt < 2 ? 2 : nt) - 1) / (8 * (nt < 2 ? 2 : nt));
     if (nt <= 2) {
         switch (w) {
@@ -796,7 +798,7 @@ cudaError_t matmul_few(cudaStream_t stream, const Mat* const* ws, float* const* 
     p.token_groups = ((n_tokens + 15u) & ~15u) / 8;
     p.n_tokens = n_tokens;
     p.store = store;
-    return launch_half(stream, p, n_tokens);
+    return launch_half(stream, p);
 }
 
 cudaError_t matmul_few_swiglu(cudaStream_t stream, const Mat& gate, const Mat& up, const void* packed, float* y, uint32_t n_tokens, uint32_t y_stride,
@@ -818,42 +820,7 @@ cudaError_t matmul_few_swiglu(cudaStream_t stream, const Mat& gate, const Mat& u
     p.n_tokens = n_tokens;
     p.store = BC_STORE_OVERWRITE;
     p.packed_out = static_cast<__half*>(packed_out);
-    return launch_half(stream, p, n_tokens);
-}
-
-// Experts: any number of tokens, as long as an expert gets a few of them on average (at most 64).
-bool matmul_few_experts_supported(const Mat& w, const Mat* up, uint32_t n_rows, uint32_t n_experts, uint32_t n_tokens, uint32_t n_used) {
-    return !few_disabled() && w.format == BC_Q4_0 && w.tiles != nullptr && n_tokens > 0 && w.n_cols % 64 == 0 && w.n_cols > 0 &&
-           w.n_cols / 64 <= kWarps * 2 * kMaxSlices && (!up || up->tiles != nullptr) && n_rows % 16 == 0 && n_experts <= 65535 &&
-           (uint64_t)n_tokens * n_used <= (uint64_t)64 * n_experts;
-}
-
-cudaError_t matmul_few_experts(cudaStream_t stream, const Mat& w, const Mat* up, uint32_t n_rows, uint32_t n_experts, const void* packed,
-                               const uint32_t* offsets, const uint32_t* entries, float* y, uint32_t n_tokens, uint32_t n_entries) {
-    if (n_rows == 0 || n_experts == 0) return cudaSuccess;
-    FewParams p{};
-    p.n_segments = 1;
-    p.tiles[0] = static_cast<const uint8_t*>(w.tiles);
-    if (up) p.tiles[1] = static_cast<const uint8_t*>(up->tiles), p.dual = 1;
-    p.y[0] = y;
-    p.seg_rows[0] = p.seg_stride[0] = n_rows;
-    p.n_jobs = p.seg_tiles[0] = n_rows / 16;
-    p.n_pairs = w.n_cols / 64;
-    p.packed = static_cast<const uint4*>(packed);
-    p.cap_groups = ((n_tokens + 15u) & ~15u) / 8;
-    p.token_groups = n_experts * p.cap_groups;
-    p.n_tokens = n_tokens;  // an expert gets at most all of them
-    p.store = BC_STORE_OVERWRITE;
-    p.offsets = offsets;
-    p.entries = entries;
-    p.n_experts = n_experts;
-    p.n_used = 1;
-    // Groups of rows as wide as an expert's likely share, with room for the busier ones.
-    const uint32_t share = (n_entries + n_experts - 1) / n_experts;
-    uint32_t rows = share + 1;
-    while ((rows - share) * (rows - share) < share) ++rows;
-    rows = rows < n_tokens ? rows : n_tokens;
-    return launch_half(stream, p, rows < kHalfGroup ? rows : kHalfGroup);
+    return launch_half(stream, p);
 }
 
 }  // namespace k
