@@ -164,16 +164,29 @@ __global__ void __launch_bounds__(256) pack_kernel(const float* __restrict__ x, 
 // in flight together, into shared memory, from where the first warp sums the squares (one warp, so that the order of
 // the sum is that of a warp per row) and all write their part of the operand. The forms before it (8 tokens per CTA with 4 or
 // 8 CTAs repeating the sums; 4 tokens per CTA with the partial sums) read rows twice: 512 tokens of 4096 took 13.0 us
-// plain and 19.0 us with four partial sums, now 8.2 and 10.7; 64 tokens of 2048 with a reduce_kernel before it 7.0, now 4.9.
+// plain and 19.0 us with four partial sums, then 8.2 and 10.7; 64 tokens of 2048 with a reduce_kernel before it 7.0, then 4.9. The norm's
+// weights are on their way before the wait and two of a thread's quads with all their partial sums at once: a scoring
+// request of 24-token suffixes (354 of these launches) 11.52 -> 11.26 ms, 32 chunks of 64 tokens (1504) 72.9 -> 71.8 ms.
 template <bool ADD>
 __global__ void __launch_bounds__(256) pack_norm_kernel(float* __restrict__ x, const float* __restrict__ weight, float eps, __half* __restrict__ packed,
                                                         uint32_t n_tokens, uint32_t n_cols, uint32_t token_groups, const float* __restrict__ partial,
                                                         uint32_t split) {
     constexpr uint32_t kMostParts = 8;
+    constexpr int kAtOnce = 2;
     extern __shared__ float4 norm_row[];
     __shared__ float shared_scale;
     pdl_launch_dependents();
     const uint32_t token = blockIdx.x, tid = threadIdx.x, quads = n_cols / 4;
+    // A 16-byte output: four columns and the four that are 16 further.
+    auto first_quad = [](uint32_t i) { return (i >> 3) * (kChunkK / 4) + ((i >> 2) & 1) * 8 + (i & 3); };
+    const float4* weights = reinterpret_cast<const float4*>(weight);
+    float4 wl[kAtOnce], wu[kAtOnce];
+#pragma unroll
+    for (int k = 0; k < kAtOnce; ++k)
+        if (token < n_tokens && tid + k * 256 < n_cols / 8) {
+            wl[k] = __ldg(weights + first_quad(tid + k * 256));
+            wu[k] = __ldg(weights + first_quad(tid + k * 256) + 4);
+        }
     pdl_wait();
     uint4* out = reinterpret_cast<uint4*>(packed) + (token & 7);
     auto place = [&](uint32_t i) { return (((uint64_t)(i >> 3) * token_groups + (token >> 3)) * kCores + (i & 7)) * 8; };
@@ -184,30 +197,41 @@ __global__ void __launch_bounds__(256) pack_norm_kernel(float* __restrict__ x, c
     float4* row = reinterpret_cast<float4*>(x) + (uint64_t)token * quads;
     const float4* part = reinterpret_cast<const float4*>(partial) + (uint64_t)token * quads;
     const uint64_t total = (uint64_t)n_tokens * quads;
-#pragma unroll ADD ? 1 : 4
-    for (uint32_t i = tid; i < quads; i += 256) {
-        float4 v = __ldcg(row + i);
-        if (ADD) {
-            float4 sum = __ldcg(part + i);
-            float4 o[kMostParts - 1];  // all of them on their way before the first is added
+    for (uint32_t base = tid; base < quads; base += 256 * kAtOnce) {
+        float4 v[kAtOnce], sum[kAtOnce], o[kAtOnce][kMostParts - 1];  // all of them on their way before the first is added
 #pragma unroll
-            for (uint32_t sp = 1; sp < kMostParts; ++sp) o[sp - 1] = sp < split ? __ldcg(part + sp * total + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int k = 0; k < kAtOnce; ++k) {
+            const uint32_t i = base + k * 256;
+            if (i >= quads) break;
+            v[k] = __ldcg(row + i);
+            if (ADD) {
+                sum[k] = __ldcg(part + i);
 #pragma unroll
-            for (uint32_t sp = 1; sp < kMostParts; ++sp)
-                if (sp < split) sum.x += o[sp - 1].x, sum.y += o[sp - 1].y, sum.z += o[sp - 1].z, sum.w += o[sp - 1].w;
-            for (uint32_t sp = kMostParts; sp < split; ++sp) {
-                const float4 more = __ldcg(part + sp * total + i);
-                sum.x += more.x; sum.y += more.y; sum.z += more.z; sum.w += more.w;
+                for (uint32_t sp = 1; sp < kMostParts; ++sp) o[k][sp - 1] = sp < split ? __ldcg(part + sp * total + i) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
-            v.x += sum.x; v.y += sum.y; v.z += sum.z; v.w += sum.w;
-            row[i] = v;
         }
-        norm_row[i] = v;
+#pragma unroll
+        for (int k = 0; k < kAtOnce; ++k) {
+            const uint32_t i = base + k * 256;
+            if (i >= quads) break;
+            if (ADD) {
+#pragma unroll
+                for (uint32_t sp = 1; sp < kMostParts; ++sp)
+                    if (sp < split) sum[k].x += o[k][sp - 1].x, sum[k].y += o[k][sp - 1].y, sum[k].z += o[k][sp - 1].z, sum[k].w += o[k][sp - 1].w;
+                for (uint32_t sp = kMostParts; sp < split; ++sp) {
+                    const float4 more = __ldcg(part + sp * total + i);
+                    sum[k].x += more.x; sum[k].y += more.y; sum[k].z += more.z; sum[k].w += more.w;
+                }
+                v[k].x += sum[k].x; v[k].y += sum[k].y; v[k].z += sum[k].z; v[k].w += sum[k].w;
+                row[i] = v[k];
+            }
+            norm_row[i] = v[k];
+        }
     }
     __syncthreads();
     if (tid < 32) {
         float sumsq = 0.f;
-#pragma unroll 4
+#pragma unroll 16
         for (uint32_t i = tid; i < quads; i += 32) {
             float4 v = norm_row[i];
             sumsq += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
@@ -217,16 +241,18 @@ __global__ void __launch_bounds__(256) pack_norm_kernel(float* __restrict__ x, c
     }
     __syncthreads();
     const float scale = shared_scale;
-#pragma unroll 2
-    for (uint32_t i = tid; i < n_cols / 8; i += 256) {  // a 16-byte output: four columns and the four that are 16 further
-        const uint32_t quad = (i >> 3) * (kChunkK / 4) + ((i >> 2) & 1) * 8 + (i & 3);
+    auto put = [&](uint32_t i, const float4& a, const float4& b) {
+        const uint32_t quad = first_quad(i);
         const float4 l = norm_row[quad], u = norm_row[quad + 4];
-        const float4 a = __ldg(reinterpret_cast<const float4*>(weight) + quad), b = __ldg(reinterpret_cast<const float4*>(weight) + quad + 4);
         const __half2 p0 = __floats2half2_rn(a.x * (l.x * scale), a.z * (l.z * scale)), p1 = __floats2half2_rn(a.y * (l.y * scale), a.w * (l.w * scale));
         const __half2 p2 = __floats2half2_rn(b.x * (u.x * scale), b.z * (u.z * scale)), p3 = __floats2half2_rn(b.y * (u.y * scale), b.w * (u.w * scale));
         out[place(i)] = make_uint4(*reinterpret_cast<const uint32_t*>(&p0), *reinterpret_cast<const uint32_t*>(&p1), *reinterpret_cast<const uint32_t*>(&p2),
                                    *reinterpret_cast<const uint32_t*>(&p3));
-    }
+    };
+#pragma unroll
+    for (int k = 0; k < kAtOnce; ++k)
+        if (tid + k * 256 < n_cols / 8) put(tid + k * 256, wl[k], wu[k]);
+    for (uint32_t i = tid + kAtOnce * 256; i < n_cols / 8; i += 256) put(i, __ldg(weights + first_quad(i)), __ldg(weights + first_quad(i) + 4));
 }
 
 // Packing for grouped mode: sorted entry i of expert e (offsets[e] <= i < offsets[e + 1]) becomes
