@@ -41,7 +41,7 @@ bc_status check_range(const bc_backend* backend, const bc_buffer* buffer, size_t
 namespace {
 
 // Per device: one word of mapped host memory per kernel file with bounded waits, for the life of the process.
-constexpr int kWaitWords = 6, kMaxDevices = 64;
+constexpr int kWaitWords = 7, kMaxDevices = 64;
 std::atomic<volatile int*> g_wait_words[kMaxDevices];
 
 bc_status set_wait_words(int device) {
@@ -58,6 +58,7 @@ bc_status set_wait_words(int device) {
     BC_CUDA(k::peer_wait_word(words + 3));
     BC_CUDA(k::matmul_few_wait_word(words + 4));
     BC_CUDA(k::matmul_experts_wait_word(words + 5));
+    BC_CUDA(k::gdn_chunk_wait_word(words + 6));
     g_wait_words[device].store(words);
     return BC_OK;
 }
@@ -80,6 +81,7 @@ bc_status kernel_wait_status() {
     if (int code = take(1)) return fail(BC_ERR_EXECUTION, "a prefill kernel gave up waiting on its pipeline (code %d)", code);
     if (int code = take(2)) return fail(BC_ERR_EXECUTION, "a prefill kernel gave up waiting on its pipeline (code %d)", code);
     if (int code = take(3)) return fail(BC_ERR_EXECUTION, "a sum over ranks gave up waiting for rank %d", code - 1);
+    if (int code = take(6)) return fail(BC_ERR_EXECUTION, "a delta-rule kernel gave up waiting for its rows (code %d)", code);
     if (int code = take(5)) return fail(BC_ERR_EXECUTION, "a product over experts gave up waiting on its pipeline (code %d)", code);
     if (int code = take(4)) return fail(BC_ERR_EXECUTION, "a product of few rows gave up waiting for its sums (code %d)", code);
     return BC_OK;

@@ -307,6 +307,7 @@ cudaError_t gdn_recurrence(cudaStream_t stream, const float* qkv, const float* b
 // normalised, 16-byte aligned pointers, `scratch` of gdn_chunk_scratch_bytes.
 bool gdn_chunk_supported(uint32_t n_v_heads, uint32_t k_dim, uint32_t v_dim, uint32_t n_tokens);
 uint64_t gdn_chunk_scratch_bytes(uint32_t n_v_heads, uint32_t n_tokens);
+cudaError_t gdn_chunk_wait_word(int* word);
 cudaError_t gdn_chunk(cudaStream_t stream, const float* qkv, const float* beta, const float* decay, float* state, float* out, void* scratch,
                       uint32_t n_k_heads, uint32_t n_v_heads, uint32_t k_dim, uint32_t v_dim, uint32_t n_tokens);
 // One token through the whole mixer after its projections (conv with history shift, gates, L2

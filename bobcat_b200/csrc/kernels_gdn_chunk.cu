@@ -16,9 +16,13 @@
 // (16 rows of L and A, value head, chunk), which also inverts its 16 x 16 diagonal block of I + L (forward
 // substitution; the triangular solve then needs four steps instead of 64). gdn_chunk_kernel carries
 // the state: a CTA per (32 state columns, value head) with its slab of S in shared memory walks over the chunks; columns
-// are independent, so nothing is exchanged. It is bound by its multiply-adds, 0.95 M per chunk and CTA against 128 per
-// cycle (4 us): register tiles of 4 x 4 from shared memory whose rows are padded to keep the reads free of bank
-// conflicts; the next chunk arrives by cp.async while this one is computed.
+// are independent, so nothing is exchanged. Its multiply-adds, 0.95 M per chunk and CTA against 128 per cycle, are 4 us; the reads of their
+// operands from shared memory (128 bytes per cycle into registers, whether lanes share them or not) bound it: register tiles of 4 x 4, from
+// rows padded to keep the reads free of bank conflicts, take as long as the reads. The next chunk arrives by cp.async while this one is
+// computed. After its wait a launch of one chunk takes 12.3 us (17.7 before the outputs' rows went to warps that lie in one
+// block and the loops were unrolled further); a lane per column for the other products too: 16.2.
+
+#include <type_traits>
 
 #include "async_utils.cuh"
 #include "device_utils.cuh"
@@ -44,6 +48,15 @@ struct ChunkParams {
     uint32_t n_k_heads, n_v_heads, v_dim, n_tokens;
 };
 
+__device__ int* g_wait_word;  // where a wait that ran out leaves its code (kernels.h), null until set
+
+// The rows' copies; a wait that runs out leaves a code and the CTA carries on, its results void.
+__device__ __forceinline__ void wait_rows(uint32_t bar) {
+    for (uint32_t spin = 0; spin < 1u << 22; ++spin)
+        if (async::mbar_test(bar, 0)) return;
+    if (g_wait_word) *reinterpret_cast<volatile int*>(g_wait_word) = 1;
+}
+
 // 16 bytes, or zeros.
 __device__ __forceinline__ void cp_async_16_or_zero(uint32_t dst, const void* src, bool live) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(live ? 16 : 0) : "memory");
@@ -54,84 +67,124 @@ __device__ __forceinline__ void fma4(float (&acc)[4], float a, const float4& b) 
     acc[2] = fmaf(a, b.z, acc[2]);
     acc[3] = fmaf(a, b.w, acc[3]);
 }
+__device__ __forceinline__ float along4(const float4& a, const float (&b)[4], float acc) { return fmaf(a.w, b[3], fmaf(a.z, b[2], fmaf(a.y, b[1], fmaf(a.x, b[0], acc)))); }
 __device__ __forceinline__ float dot4(const float4& a, const float4& b, float acc) {
     return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, acc))));
 }
 
-// grid (row block, value head, chunk), 128 threads.
+// grid (row block, value head, chunk), 256 threads. Bound by latency while there are few chunks: with a loop that looked up each decay on
+// the way down to D(t, s) and the rows in pieces of 16 bytes a launch took 10.8 us after its wait (2.8, 1.8, and 5.5 for the products). Now
+// the way down is straight-line code and a row is one copy: 7.3 us.
+constexpr uint32_t kPrepareThreads = 256;
+
 template <int KDIM>
-__global__ void __launch_bounds__(128) gdn_chunk_prepare_kernel(ChunkParams p) {
+__global__ void __launch_bounds__(kPrepareThreads) gdn_chunk_prepare_kernel(ChunkParams p) {
     constexpr uint32_t kPitch = KDIM + 4;  // 16-byte aligned rows, neighbouring rows four banks apart
     extern __shared__ __align__(16) float smem[];
     float* ks = smem;                       // [64][kPitch]
     float* qs = ks + kChunk * kPitch;       // [16][kPitch]
-    __shared__ float decays[kChunk], betas[kBlock], ratio[kBlock][kChunk + 1], low[kBlock][kBlock + 1];
-    pdl_launch_dependents();
-    pdl_wait();
-    const uint32_t block = blockIdx.x, head = blockIdx.y, chunk = blockIdx.z, tid = threadIdx.x;
+    __shared__ __align__(16) float decays[kChunk];
+    __shared__ float betas[kBlock], ratio[kBlock][kChunk + 1], low[kBlock][kBlock + 1];
+    __shared__ __align__(8) uint64_t arrived;
+    const uint32_t block = blockIdx.x, head = blockIdx.y, chunk = blockIdx.z, tid = threadIdx.x, bar = async::smem_u32(&arrived);
     const uint32_t first = chunk * kChunk, live = min(kChunk, p.n_tokens - first), row0 = block * kBlock, n_cols = row0 + kBlock;
     const uint32_t key_dim = p.n_k_heads * KDIM, conv_dim = 2 * key_dim + p.n_v_heads * p.v_dim, key_head = head % p.n_k_heads;
     float* unit = p.scratch + ((uint64_t)chunk * p.n_v_heads + head) * kUnitFloats;
     const bool products = row0 < live;  // a block past the batch only passes the decays on
-    if (products) {
-        for (uint32_t i = tid; i < (n_cols + kBlock) * (KDIM / 4); i += 128) {
-            const uint32_t r = i / (KDIM / 4), c = i % (KDIM / 4);
-            const bool is_q = r >= n_cols;
-            const uint32_t t = is_q ? row0 + r - n_cols : r;
-            const float* src = p.qkv + (uint64_t)(first + (t < live ? t : 0)) * conv_dim + (is_q ? 0 : key_dim) + key_head * KDIM + 4 * c;
-            cp_async_16_or_zero(async::smem_u32((is_q ? qs + (r - n_cols) * kPitch : ks + r * kPitch) + 4 * c), src, t < live);
+    pdl_launch_dependents();
+    if (tid == 0) {
+        async::mbar_init(bar, 1);
+        async::mbar_init_fence();
+    }
+    __syncthreads();
+    pdl_wait();
+    // A row of K or of Q per thread; rows past the batch are zero.
+    if (products && tid < n_cols + kBlock) {
+        const bool is_q = tid >= n_cols;
+        const uint32_t t = is_q ? row0 + tid - n_cols : tid;
+        float* to = is_q ? qs + (tid - n_cols) * kPitch : ks + tid * kPitch;
+        if (tid == 0) async::mbar_arrive_expect(bar, (min(live, n_cols) + min(live - row0, kBlock)) * KDIM * 4);
+        if (t < live) {
+            async::bulk_load(async::smem_u32(to), p.qkv + (uint64_t)(first + t) * conv_dim + (is_q ? 0 : key_dim) + key_head * KDIM, KDIM * 4, bar);
+        } else {
+#pragma unroll 4
+            for (uint32_t c = 0; c < KDIM / 4; ++c) reinterpret_cast<float4*>(to)[c] = make_float4(0.f, 0.f, 0.f, 0.f);
         }
     }
-    async::cp_async_commit();
-    if (tid < kChunk) decays[tid] = tid < live ? p.decay[(uint64_t)(first + tid) * p.n_v_heads + head] : 1.f;
-    else if (tid < kChunk + kBlock) {
-        const uint32_t t = row0 + tid - kChunk;
-        betas[tid - kChunk] = t < live ? p.beta[(uint64_t)(first + t) * p.n_v_heads + head] : 0.f;
+    if (tid >= 3 * kChunk) {
+        const uint32_t t = tid - 3 * kChunk;
+        decays[t] = t < live ? p.decay[(uint64_t)(first + t) * p.n_v_heads + head] : 1.f;
+    } else if (tid >= 2 * kChunk && tid < 2 * kChunk + kBlock) {
+        const uint32_t t = row0 + tid - 2 * kChunk;
+        betas[tid - 2 * kChunk] = t < live ? p.beta[(uint64_t)(first + t) * p.n_v_heads + head] : 0.f;
     }
     __syncthreads();
     // D(t, s) for the block's rows: a thread per s multiplies its way down.
     if (tid < n_cols) {
         float d = 1.f;
-        for (uint32_t t = tid; t < n_cols; ++t) {
-            if (t > tid) d *= decays[t];
-            if (t >= row0) ratio[t - row0][tid] = d;
+        for (uint32_t b = 0; b < block; ++b) {
+            float a[kBlock];
+#pragma unroll
+            for (uint32_t i = 0; i < kBlock; ++i) a[i] = decays[b * kBlock + i];
+#pragma unroll
+            for (uint32_t i = 0; i < kBlock; ++i)
+                if (b * kBlock + i > tid) d *= a[i];
+        }
+        float a[kBlock];
+#pragma unroll
+        for (uint32_t i = 0; i < kBlock; ++i) a[i] = decays[row0 + i];
+#pragma unroll
+        for (uint32_t i = 0; i < kBlock; ++i) {
+            if (row0 + i > tid) d *= a[i];
+            if (row0 + i >= tid) ratio[i][tid] = d;
         }
     }
-    async::cp_async_wait<0>();
+    if (products) wait_rows(bar);
     __syncthreads();
     if (tid < kBlock) unit[kGAt + row0 + tid] = decays[0] * ratio[tid][0];
     if (block == kBlocks - 1 && tid < kChunk) unit[kLastAt + tid] = ratio[kBlock - 1][tid];
     if (!products) return;
-    // Two rows of K and of Q against up to four interleaved columns per thread.
-    const uint32_t rg = tid >> 4, cg = tid & 15;
-    float kk[2][kBlocks] = {}, qk[2][kBlocks] = {};
-    const float4* k_rows[2] = {reinterpret_cast<const float4*>(ks + (row0 + rg) * kPitch), reinterpret_cast<const float4*>(ks + (row0 + rg + 8) * kPitch)};
-    const float4* q_rows[2] = {reinterpret_cast<const float4*>(qs + rg * kPitch), reinterpret_cast<const float4*>(qs + (rg + 8) * kPitch)};
-#pragma unroll 2
-    for (int c = 0; c < KDIM / 4; ++c) {
-        const float4 a0 = k_rows[0][c], a1 = k_rows[1][c], b0 = q_rows[0][c], b1 = q_rows[1][c];
+    // Two rows of K and of Q against up to four interleaved columns per thread of the first half. (One half K, the other Q: 9 us instead of
+    // 5.5, the columns' reads from shared memory twice.)
+    auto multiply = [&](auto columns) {
+        constexpr uint32_t kColumns = decltype(columns)::value;  // per thread: the blocks up to this one
+        const uint32_t rg = tid >> 4, cg = tid & 15;
+        float kk[2][kColumns] = {}, qk[2][kColumns] = {};
+        const float4* k_rows[2] = {reinterpret_cast<const float4*>(ks + (row0 + rg) * kPitch), reinterpret_cast<const float4*>(ks + (row0 + rg + 8) * kPitch)};
+        const float4* q_rows[2] = {reinterpret_cast<const float4*>(qs + rg * kPitch), reinterpret_cast<const float4*>(qs + (rg + 8) * kPitch)};
+#pragma unroll 4
+        for (int c = 0; c < KDIM / 4; ++c) {
+            const float4 a0 = k_rows[0][c], a1 = k_rows[1][c], b0 = q_rows[0][c], b1 = q_rows[1][c];
 #pragma unroll
-        for (uint32_t j = 0; j < kBlocks; ++j) {
-            if (j > block) break;
-            const float4 col = *reinterpret_cast<const float4*>(ks + (cg + kBlock * j) * kPitch + 4 * c);
-            kk[0][j] = dot4(a0, col, kk[0][j]);
-            kk[1][j] = dot4(a1, col, kk[1][j]);
-            qk[0][j] = dot4(b0, col, qk[0][j]);
-            qk[1][j] = dot4(b1, col, qk[1][j]);
+            for (uint32_t j = 0; j < kColumns; ++j) {
+                const float4 col = *reinterpret_cast<const float4*>(ks + (cg + kBlock * j) * kPitch + 4 * c);
+                kk[0][j] = dot4(a0, col, kk[0][j]);
+                kk[1][j] = dot4(a1, col, kk[1][j]);
+                qk[0][j] = dot4(b0, col, qk[0][j]);
+                qk[1][j] = dot4(b1, col, qk[1][j]);
+            }
+        }
+#pragma unroll
+        for (uint32_t i = 0; i < 2; ++i)
+#pragma unroll
+            for (uint32_t j = 0; j < kColumns; ++j) {
+                const uint32_t r = rg + 8 * i, t = row0 + r, s = cg + kBlock * j;
+                const float d = s <= t ? ratio[r][s] : 0.f;
+                const float l = s < t ? betas[r] * d * kk[i][j] : 0.f;
+                unit[kLAt + t * kChunk + s] = l;
+                unit[kAAt + t * kChunk + s] = s <= t ? d * qk[i][j] : 0.f;
+                if (j + 1 == kColumns) low[r][cg] = l;
+            }
+    };
+    if (tid < 128) {
+        static_assert(kBlocks == 4, "a chunk is four blocks");
+        switch (block) {
+            case 0: multiply(std::integral_constant<uint32_t, 1>()); break;
+            case 1: multiply(std::integral_constant<uint32_t, 2>()); break;
+            case 2: multiply(std::integral_constant<uint32_t, 3>()); break;
+            default: multiply(std::integral_constant<uint32_t, 4>()); break;
         }
     }
-#pragma unroll
-    for (uint32_t i = 0; i < 2; ++i)
-#pragma unroll
-        for (uint32_t j = 0; j < kBlocks; ++j) {
-            if (j > block) break;
-            const uint32_t r = rg + 8 * i, t = row0 + r, s = cg + kBlock * j;
-            const float d = s <= t ? ratio[r][s] : 0.f;
-            const float l = s < t ? betas[r] * d * kk[i][j] : 0.f;
-            unit[kLAt + t * kChunk + s] = l;
-            unit[kAAt + t * kChunk + s] = s <= t ? d * qk[i][j] : 0.f;
-            if (j == block) low[r][cg] = l;
-        }
     __syncthreads();
     // The inverse of the diagonal block: a thread per column of the identity.
     if (tid < kBlock) {
@@ -148,7 +201,7 @@ __global__ void __launch_bounds__(128) gdn_chunk_prepare_kernel(ChunkParams p) {
     }
 }
 
-constexpr uint32_t kSlab = 32, kThreads = 256;
+constexpr uint32_t kSlab = 32, kThreads = 256, kWarps = kThreads / 32;
 
 template <int KDIM>
 struct Slots {
@@ -227,6 +280,8 @@ __global__ void __launch_bounds__(kThreads, 1) gdn_chunk_kernel(ChunkParams p) {
     async::cp_async_commit();
 
     const uint32_t rg = tid >> 3, cg = tid & 7;  // 32 row groups x 8 groups of 4 columns
+    const uint32_t lane = tid & 31, t0 = (tid >> 5) * (kChunk / kWarps);  // the outputs: a lane owns a column, a warp eight tokens
+    constexpr uint32_t kTokens = kChunk / kWarps;
     for (uint32_t chunk = 0; chunk < n_chunks; ++chunk) {
         const uint32_t slot = chunk & 1, live = min(kChunk, p.n_tokens - chunk * kChunk), blocks = (live + kBlock - 1) / kBlock;
         async::cp_async_wait<0>();
@@ -239,7 +294,7 @@ __global__ void __launch_bounds__(kThreads, 1) gdn_chunk_kernel(ChunkParams p) {
             const float4* rows[4] = {reinterpret_cast<const float4*>(sh.k[slot] + rg * S::kPitch), reinterpret_cast<const float4*>(sh.q + rg * S::kPitch),
                                      reinterpret_cast<const float4*>(sh.k[slot] + (rg + 32) * S::kPitch), reinterpret_cast<const float4*>(sh.q + (rg + 32) * S::kPitch)};
             const int n_rows = live > 32 ? 4 : 2;
-#pragma unroll 2
+#pragma unroll 4
             for (uint32_t c = 0; c < kRowVec; ++c) {
                 float4 s[4];
 #pragma unroll
@@ -276,7 +331,8 @@ __global__ void __launch_bounds__(kThreads, 1) gdn_chunk_kernel(ChunkParams p) {
                 const uint32_t t = b * kBlock + r;
                 float2 y = *reinterpret_cast<const float2*>(x + t * S::kSlabPitch + c2);
                 const float4* l = reinterpret_cast<const float4*>(sh.l[slot] + t * S::kTriPitch);
-                for (uint32_t s4 = 0; s4 < b * kBlock / 4; ++s4) {
+#pragma unroll 4
+                for (uint32_t s4 = 0; s4 < b * (kBlock / 4); ++s4) {
                     const float4 w = l[s4];
                     const float* d = x + 4 * s4 * S::kSlabPitch + c2;
 #pragma unroll
@@ -306,35 +362,31 @@ __global__ void __launch_bounds__(kThreads, 1) gdn_chunk_kernel(ChunkParams p) {
                 __syncthreads();
             }
         }
-        // ---- the outputs: rows rg and rg + 32 of A delta on top of the state's share.
-        {
+        // ---- the outputs of the warp's tokens, A delta on top of the state's share.
+        if (t0 < live) {
+            float acc[kTokens];
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const uint32_t t = rg + 32 * h;
-                if (t >= live) continue;
-                float acc[4];
-                const float4 before = *reinterpret_cast<const float4*>(sh.past + t * S::kSlabPitch + 4 * cg);
-                acc[0] = before.x, acc[1] = before.y, acc[2] = before.z, acc[3] = before.w;
-                const float4* a = reinterpret_cast<const float4*>(sh.a[slot] + t * S::kTriPitch);
-                const uint32_t vectors = (t / kBlock + 1) * (kBlock / 4);
-                for (uint32_t s4 = 0; s4 < vectors; ++s4) {
-                    const float4 w = a[s4];
-                    const float* d = x + 4 * s4 * S::kSlabPitch + 4 * cg;
-                    fma4(acc, w.x, *reinterpret_cast<const float4*>(d));
-                    fma4(acc, w.y, *reinterpret_cast<const float4*>(d + S::kSlabPitch));
-                    fma4(acc, w.z, *reinterpret_cast<const float4*>(d + 2 * S::kSlabPitch));
-                    fma4(acc, w.w, *reinterpret_cast<const float4*>(d + 3 * S::kSlabPitch));
-                }
-                *reinterpret_cast<float4*>(p.out + (uint64_t)(chunk * kChunk + t) * p.n_v_heads * vd + head * vd + col0 + 4 * cg) =
-                    make_float4(acc[0], acc[1], acc[2], acc[3]);
+            for (uint32_t i = 0; i < kTokens; ++i) acc[i] = sh.past[(t0 + i) * S::kSlabPitch + lane];
+            const float4* a4 = reinterpret_cast<const float4*>(sh.a[slot] + t0 * S::kTriPitch);
+            const uint32_t vectors = (t0 / kBlock + 1) * (kBlock / 4);  // the tokens lie in one block
+#pragma unroll 2
+            for (uint32_t s4 = 0; s4 < vectors; ++s4) {
+                float delta[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) delta[e] = x[(4 * s4 + e) * S::kSlabPitch + lane];
+#pragma unroll
+                for (uint32_t i = 0; i < kTokens; ++i) acc[i] = along4(a4[i * (S::kTriPitch / 4) + s4], delta, acc[i]);
             }
+#pragma unroll
+            for (uint32_t i = 0; i < kTokens; ++i)
+                if (t0 + i < live) p.out[(uint64_t)(chunk * kChunk + t0 + i) * p.n_v_heads * vd + head * vd + col0 + lane] = acc[i];
         }
         // ---- the state: a thread owns KDIM / 32 rows of S x 4 columns.
         {
             constexpr int kOwn = KDIM / 32;  // rows rg * kOwn ..
             float acc[kOwn][4] = {};
             const float* kr = sh.k[slot] + rg * kOwn;
-#pragma unroll 4
+#pragma unroll 8
             for (uint32_t s = 0; s < blocks * kBlock; ++s) {
                 const float w = sh.last[slot][s];
                 float4 d = *reinterpret_cast<const float4*>(x + s * S::kSlabPitch + 4 * cg);
@@ -374,12 +426,14 @@ cudaError_t launch_chunks(cudaStream_t stream, const ChunkParams& p) {
     cudaError_t e = ensure_dynamic_smem((const void*)gdn_chunk_prepare_kernel<KDIM>, prepare_smem);
     if (e == cudaSuccess) e = ensure_dynamic_smem((const void*)gdn_chunk_kernel<KDIM>, sizeof(Slots<KDIM>));
     if (e != cudaSuccess) return e;
-    e = launch_dependent(gdn_chunk_prepare_kernel<KDIM>, dim3(kBlocks, p.n_v_heads, n_chunks), dim3(128), prepare_smem, stream, p);
+    e = launch_dependent(gdn_chunk_prepare_kernel<KDIM>, dim3(kBlocks, p.n_v_heads, n_chunks), dim3(kPrepareThreads), prepare_smem, stream, p);
     if (e != cudaSuccess) return e;
     return launch_dependent(gdn_chunk_kernel<KDIM>, dim3(p.v_dim / kSlab, p.n_v_heads), dim3(kThreads), sizeof(Slots<KDIM>), stream, p);
 }
 
 }  // namespace
+
+cudaError_t gdn_chunk_wait_word(int* word) { return cudaMemcpyToSymbol(g_wait_word, &word, sizeof word); }
 
 uint64_t gdn_chunk_scratch_bytes(uint32_t n_v_heads, uint32_t n_tokens) {
     return (uint64_t)((n_tokens + kChunk - 1) / kChunk) * n_v_heads * kUnitFloats * sizeof(float);
