@@ -112,44 +112,69 @@ __global__ void __launch_bounds__(256) gdn_conv_kernel(const __grid_constant__ C
             else if (src < (int64_t)p.n_tokens) window[e][i] = p.x[(uint64_t)src * p.conv_dim + c];
         }
     }
+    // The history after the batch: slot i holds the input of token n_tokens - (kernel - 1) + i, or an older slot when the
+    // batch is shorter than the history. Read here, beside the window, and written at the end by the first run's threads.
+    float kept[PER][K - 1];
+    if (t0 == 0) {
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-        if (t0 + r >= p.n_tokens) break;
-        float v[PER];
+        for (int e = 0; e < PER; ++e) {
+            const uint32_t c = c0 + e * 32;
+#pragma unroll
+            for (int i = 0; i < K - 1; ++i) {
+                if (c >= p.conv_dim || i < (int)skip) continue;
+                const int64_t src = (int64_t)p.n_tokens - (K - 1) + i;
+                kept[e][i] = src >= 0 ? p.x[(uint64_t)src * p.conv_dim + c] : p.history[(uint64_t)c * (p.kernel - 1) + src + (K - 1) - skip];
+            }
+        }
+    }
+    // All tokens of the run at once: their sums over the warp are independent. (Rows past the batch are zeros and not stored.)
+    float v[R][PER];
+#pragma unroll
+    for (int r = 0; r < R; ++r)
 #pragma unroll
         for (int e = 0; e < PER; ++e) {
             float sum = tap[e][K - 1] * window[e][K - 1 + r];
 #pragma unroll
             for (int i = 0; i < K - 1; ++i)
                 if (i >= (int)skip) sum += tap[e][i] * window[e][i + r];
-            v[e] = sum / (1.f + expf(-sum));
+            v[r][e] = sum / (1.f + expf(-sum));
         }
-        if (group < p.n_norm) {
-            float factor = l2_factor<PER>(v);
+    if (group < p.n_norm) {
+        float squares[R][PER];
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+            for (int e = 0; e < PER; ++e) squares[r][e] = v[r][e] * v[r][e];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+#pragma unroll
+                for (int e = 0; e < PER; ++e) squares[r][e] += __shfl_xor_sync(0xffffffffu, squares[r][e], o);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            float sum = 0.f;  // l2_factor's sum
+#pragma unroll
+            for (int e = 0; e < PER; ++e) sum += squares[r][e];
+            float factor = 1.0f / sqrtf(sum + 1e-6f);
             if (group < p.n_norm / 2) factor = (1.0f / sqrtf((float)(32 * PER))) * factor;
 #pragma unroll
-            for (int e = 0; e < PER; ++e) v[e] *= factor;
+            for (int e = 0; e < PER; ++e) v[r][e] *= factor;
         }
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        if (t0 + r >= p.n_tokens) break;
 #pragma unroll
         for (int e = 0; e < PER; ++e)
-            if (c0 + e * 32 < p.conv_dim) p.out[(uint64_t)(t0 + r) * p.conv_dim + c0 + e * 32] = v[e];
+            if (c0 + e * 32 < p.conv_dim) p.out[(uint64_t)(t0 + r) * p.conv_dim + c0 + e * 32] = v[r][e];
     }
     if (t0 != 0) return;
-    // The history after the batch: slot i holds the input of token n_tokens - (kernel - 1) + i, or an older slot when the
-    // batch is shorter than the history.
 #pragma unroll
-    for (int e = 0; e < PER; ++e) {
-        const uint32_t c = c0 + e * 32;
-        if (c >= p.conv_dim) continue;
+    for (int e = 0; e < PER; ++e)
 #pragma unroll
-        for (int i = 0; i < K - 1; ++i) {
-            if (i < (int)skip) continue;
-            // Slots are rewritten oldest first, so an older slot that moves down is still there to be read.
-            const int64_t src = (int64_t)p.n_tokens - (K - 1) + i;
-            const float next = src >= 0 ? p.x[(uint64_t)src * p.conv_dim + c] : p.history[(uint64_t)c * (p.kernel - 1) + src + (K - 1) - skip];
-            p.history[(uint64_t)c * (p.kernel - 1) + i - skip] = next;
-        }
-    }
+        for (int i = 0; i < K - 1; ++i)
+            if (c0 + e * 32 < p.conv_dim && i >= (int)skip) p.history[(uint64_t)(c0 + e * 32) * (p.kernel - 1) + i - skip] = kept[e][i];
 }
 
 // The delta rule over a run of tokens. One warp (a CTA of its own) per 8 state columns of a value
