@@ -156,13 +156,14 @@ bc_status bc_engine_generate(bc_engine* e, const uint32_t* tokens, size_t n_toke
     while (remaining > 0) {
         uint32_t token = 0;
         if ((st = bc_seq_sample(s, sampling, next_uniform(&e->rng), e->consumed.data(), e->consumed.size(), &token)) != BC_OK) return failed(st);
+        if ((st = kernel_wait_status()) != BC_OK) return failed(st);  // of the step before
         remaining -= 1;
         if (produced < out_cap) out[produced] = token;
         produced += 1;
         const bool go_on = emit ? emit(token, user) != 0 : true;
         if (!go_on || remaining == 0) break;
-        // The step's logits stay on the device, where the next pick reads them.
-        if ((st = bc_seq_step_on_device(s, token)) != BC_OK) return failed(st);
+        // The step's logits stay on the device, where the next pick reads them; its token is what is waited for.
+        if ((st = step_unwaited(s, token)) != BC_OK) return failed(st);
         e->consumed.push_back(token);
     }
     *n_out = std::min(produced, out_cap);

@@ -412,7 +412,7 @@ uint64_t bc_seq_launches(const bc_seq* seq) { return seq ? seq->launches : 0; }
 }  // extern "C"
 
 namespace {
-bc_status step_impl(bc_seq* s, uint32_t token, float* logits, size_t logits_len, bc_trace* trace, bool device_logits);
+bc_status step_impl(bc_seq* s, uint32_t token, float* logits, size_t logits_len, bc_trace* trace, bool device_logits, bool wait = true);
 }
 
 extern "C" {
@@ -427,7 +427,9 @@ bc_status bc_seq_step_on_device(bc_seq* s, uint32_t token) { return step_impl(s,
 
 namespace {
 
-bc_status step_impl(bc_seq* s, uint32_t token, float* logits, size_t logits_len, bc_trace* trace, bool device_logits) {
+// Without `wait` (device_logits only) the step is left to run: the caller waits for the stream before the next one, whose position and
+// token go through host memory that the device reads.
+bc_status step_impl(bc_seq* s, uint32_t token, float* logits, size_t logits_len, bc_trace* trace, bool device_logits, bool wait) {
     if (!s || !s->backend) return fail(BC_ERR_ARGUMENT, "seq must be non-null and its backend open");
     const bc_hparams& hp = s->hp;
     uint32_t pos = s->n_past;
@@ -460,6 +462,11 @@ bc_status step_impl(bc_seq* s, uint32_t token, float* logits, size_t logits_len,
     }
     double encode = since(encode_start);
     double gpu = 0;
+    if (!wait && r.status == BC_OK) {
+        s->n_past += 1;
+        s->last_encode_seconds = encode;
+        return BC_OK;
+    }
     bc_status finish = timing_end(s, &gpu);
     if (r.status != BC_OK) return r.status;
     BC_TRY(finish);
@@ -479,6 +486,8 @@ bc_status step_impl(bc_seq* s, uint32_t token, float* logits, size_t logits_len,
 }  // namespace
 
 namespace bc {
+
+bc_status step_unwaited(bc_seq* s, uint32_t token) { return step_impl(s, token, nullptr, 0, nullptr, true, false); }
 
 bc_status prefill_async(bc_seq* s, const uint32_t* tokens, uint32_t n, bool want_logits) {
     if (s->backend->recording) return fail(BC_ERR_ALREADY_RECORDING, "a recording is already open");

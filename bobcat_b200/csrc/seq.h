@@ -148,5 +148,7 @@ namespace bc {
 
 // Prefill of valid tokens that fit the context, without waiting for it; the logits (with `want_logits`) stay in s->logits.
 bc_status prefill_async(bc_seq* s, const uint32_t* tokens, uint32_t n, bool want_logits);
+// bc_seq_step_on_device without its wait: the caller waits for the stream before the next step, and reports kernel_wait_status.
+bc_status step_unwaited(bc_seq* s, uint32_t token);
 
 }  // namespace bc
