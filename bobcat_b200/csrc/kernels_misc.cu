@@ -261,6 +261,18 @@ __global__ void __launch_bounds__(128) short_conv_kernel(const float* __restrict
                 load(bcx + (uint64_t)(t0 + r) * 3 * n_embd + n_embd + ch, c[r]);
             }
         }
+        // The history after the batch: slot kk holds the product of token n_tokens - (kernel - 1) + kk, or an older slot when the batch is
+        // shorter than the history. Read beside the rest, written at the end: one after the other behind the outputs they were two trips to L2.
+        float kept[K - 1][V];
+        if (t0 == 0) {
+#pragma unroll
+            for (int kk = 0; kk < K - 1; ++kk) {
+                if (kk < (int)skip) continue;
+                const int64_t src = (int64_t)n_tokens - (K - 1) + kk;
+                if (src >= 0) products((uint32_t)src, kept[kk]);
+                else load(history + (uint64_t)(src + K - 1 - skip) * n_embd + ch, kept[kk]);
+            }
+        }
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             float y[V];
@@ -284,18 +296,11 @@ __global__ void __launch_bounds__(128) short_conv_kernel(const float* __restrict
             }
         }
         if (t0 != 0) continue;
-        // The history after the batch: slot kk holds the product of token n_tokens - (kernel - 1) + kk, or an older
-        // slot when the batch is shorter than the history.
 #pragma unroll
         for (int kk = 0; kk < K - 1; ++kk) {
             if (kk < (int)skip) continue;
-            const int64_t src = (int64_t)n_tokens - (K - 1) + kk;
-            float next[V];
-            // Slots are rewritten oldest first, so an older slot that moves down is still there to be read.
-            if (src >= 0) products((uint32_t)src, next);
-            else load(history + (uint64_t)(src + K - 1 - skip) * n_embd + ch, next);
 #pragma unroll
-            for (int v = 0; v < V; ++v) history[(uint64_t)(kk - skip) * n_embd + ch + v] = next[v];
+            for (int v = 0; v < V; ++v) history[(uint64_t)(kk - skip) * n_embd + ch + v] = kept[kk][v];
         }
     }
 }
