@@ -330,8 +330,10 @@ cudaError_t attention_gate(cudaStream_t stream, float* out, const float* q_gate,
 // weights as float bits.
 // Router: optional RMSNorm (normalised tokens also go to `normed`), F32 router logits in f64,
 // sigmoid, top n_used of score + bias with ties to the lower id, weights = score / (sum + 1e-6).
+// `constant`: no launch that may still run writes the norm or the router (a model's weights), so they are read ahead of
+// the wait for the preceding launch. An op call's are buffers that its recording may write: read after the wait.
 cudaError_t moe_route(cudaStream_t stream, const float* x, Norm norm, float* normed, const float* router, const float* bias,
-                      uint32_t* route, uint32_t n_cols, uint32_t n_experts, uint32_t n_used, uint32_t n_tokens);
+                      uint32_t* route, uint32_t n_cols, uint32_t n_experts, uint32_t n_used, uint32_t n_tokens, bool constant = false);
 // Counting sort of the (token, slot) entries by expert: offsets[n_experts + 1], entries[n_tokens * n_used].
 // With first_expert > 0 (or fewer experts than the router has) only the entries of experts
 // [first_expert, first_expert + n_experts) are kept, numbered from zero: offsets[n_experts] is then

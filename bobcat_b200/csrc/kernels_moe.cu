@@ -34,6 +34,7 @@ struct RouteParams {
     const float* bias;
     uint32_t* route;
     uint32_t n_cols, n_experts, n_used, n_tokens;
+    bool constant;             // no launch of the recording writes the norm or the router: they may be read ahead of the wait
 };
 
 // A warp picks a token's experts from their scores.
@@ -125,9 +126,10 @@ __global__ void __launch_bounds__(kRouteThreads) moe_route_kernel(const __grid_c
             const uint32_t e = rank + ranks * (local + m);
             const float4* row = reinterpret_cast<const float4*>(p.router + (uint64_t)e * n_cols);
 #pragma unroll
-            for (int k = 0; k < kHeld; ++k) held[m][k] = e < p.n_experts && at + k * stride < quads ? __ldg(row + at + k * stride) : make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int k = 0; k < kHeld; ++k) held[m][k] = e < p.n_experts && at + k * stride < quads ? row[at + k * stride] : make_float4(0.f, 0.f, 0.f, 0.f);
         }
     };
+    if (!p.constant) pdl_wait();
     if (wide) load(EXPERTS * group, first);
     if (ranks > 1) asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");  // this CTA runs: its shared memory may be written
     pdl_wait();
@@ -281,14 +283,16 @@ __global__ void __launch_bounds__(kTokenThreads, 4) moe_route_token_kernel(const
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
     double w[kTokenExperts][kTokenQuads][4];
     float4 nw[kTokenQuads];
+    // Plain loads: a load through the read-only path may move ahead of a wait.
+    if (!p.constant) pdl_wait();
 #pragma unroll
     for (uint32_t q = 0; q < kTokenQuads; ++q) {
         const uint32_t quad = tid + q * kTokenThreads;
-        nw[q] = p.norm_weight && quad < quads ? __ldg(reinterpret_cast<const float4*>(p.norm_weight) + quad) : zero;
+        nw[q] = p.norm_weight && quad < quads ? *(reinterpret_cast<const float4*>(p.norm_weight) + quad) : zero;
 #pragma unroll
         for (uint32_t m = 0; m < kTokenExperts; ++m) {
             const uint32_t e = rank + kTokenCluster * m;
-            const float4 f = e < p.n_experts && quad < quads ? __ldg(reinterpret_cast<const float4*>(p.router + (uint64_t)e * p.n_cols) + quad) : zero;
+            const float4 f = e < p.n_experts && quad < quads ? *(reinterpret_cast<const float4*>(p.router + (uint64_t)e * p.n_cols) + quad) : zero;
             w[m][q][0] = f.x, w[m][q][1] = f.y, w[m][q][2] = f.z, w[m][q][3] = f.w;
         }
     }
@@ -628,9 +632,9 @@ int route_clusters() {
 }  // namespace
 
 cudaError_t moe_route(cudaStream_t stream, const float* x, Norm norm, float* normed, const float* router, const float* bias,
-                      uint32_t* route, uint32_t n_cols, uint32_t n_experts, uint32_t n_used, uint32_t n_tokens) {
+                      uint32_t* route, uint32_t n_cols, uint32_t n_experts, uint32_t n_used, uint32_t n_tokens, bool constant) {
     if (n_tokens == 0) return cudaSuccess;
-    const RouteParams p{x, norm.weight, norm.eps, normed, router, bias, route, n_cols, n_experts, n_used, n_tokens};
+    const RouteParams p{x, norm.weight, norm.eps, normed, router, bias, route, n_cols, n_experts, n_used, n_tokens, constant};
     if (n_cols % 4 == 0 && n_cols / 4 <= kTokenThreads * kTokenQuads && n_experts <= kTokenCluster * kTokenExperts && n_tokens * kTokenCluster <= (uint32_t)sm_count() &&
         ((uintptr_t)x | (uintptr_t)norm.weight | (uintptr_t)(norm.weight ? normed : nullptr) | (uintptr_t)router) % 16 == 0 && route_clusters() > 0) {
         cudaLaunchConfig_t config = {};

@@ -394,7 +394,7 @@ struct Recorder {
         k::Norm nm = fused_norm ? norm(D.ffn_norm) : k::Norm{};
         run("moe_route", hp.n_experts, n_embd, D.router.bytes(), 1, [&] {
             return k::moe_route(stream, input, nm, s.normed, static_cast<const float*>(D.router.data), D.expert_bias, s.route, n_embd, hp.n_experts,
-                                n_used, n);
+                                n_used, n, true);
         });
         if (route_trace) run("copy", 1, n * 2 * n_used, 0, 0, [&] {
             return k::copy_floats(stream, reinterpret_cast<const float*>(s.route), reinterpret_cast<float*>(route_trace), (uint64_t)n * 2 * n_used);
@@ -449,7 +449,7 @@ struct Recorder {
         run_status([&] { return comm_all_gather(ep.comm, mine, s.normed, (size_t)n_local * n_embd); });
         run("moe_route", hp.n_experts, n_embd, D.router.bytes(), 1, [&] {
             return k::moe_route(stream, s.normed, k::Norm{}, s.normed, static_cast<const float*>(D.router.data), D.expert_bias, s.route, n_embd, hp.n_experts,
-                                n_used, n);
+                                n_used, n, true);
         });
         run("moe_group", n, ep.n_local_experts, 0, 1,
             [&] { return k::moe_group(stream, s.route, s.expert_offsets, s.expert_entries, ep.n_local_experts, n_used, n, ep.first_expert); });

@@ -45,6 +45,40 @@ def test_route_ids_are_bit_exact(cuda, n_tokens, fused_norm):
         assert rel_error(normed, want) < 1e-6
 
 
+@pytest.mark.parametrize("n_tokens,n_cols,n_experts", [(1, 2048, 32), (9, 260, 31), (10, 2048, 32), (3, 2048, 64), (37, 256, 32)])
+def test_route_reads_what_its_recording_wrote(cuda, n_tokens, n_cols, n_experts):
+    """The norm and the router of an op call are the caller's buffers: written by launches of the same recording they give the
+    bits that they give when written beforehand, on each kernel of the router."""
+    rng = np.random.default_rng(n_cols + n_tokens)
+    n_used, rows = 4, 300
+    x = rng.standard_normal((n_tokens, n_cols)).astype(np.float32)
+    source = rng.standard_normal((rows, n_cols)).astype(np.float32)  # its last row, normalised, is the norm
+    router = (rng.standard_normal((n_experts, n_cols)) * 0.05).astype(np.float32)
+    xb, sb, ones = cuda.buffer_from(x), cuda.buffer_from(source), cuda.buffer_from(np.ones(n_cols, dtype=np.float32))
+    fresh, bb = cuda.buffer_from(router), cuda.buffer_from(np.zeros(n_experts, dtype=np.float32))
+
+    def route(norms, router_b, write_first):
+        normed, out = cuda.new_buffer(x.nbytes), cuda.new_buffer(cuda.route_bytes(n_used, n_tokens))
+
+        def write():
+            cuda.copy(fresh, router_b, n_experts * n_cols)
+            cuda.rms_norm(sb, ones, norms, n_cols, rows, 1e-5)
+
+        cuda.begin()
+        write()
+        if write_first:
+            cuda.end()
+            cuda.begin()
+        cuda.moe_route(xb, (Norm(norms.floats((rows - 1) * n_cols), 1e-5), normed.at(0)), router_b, bb, out, n_cols, n_experts, n_used, n_tokens)
+        cuda.end()
+        return cuda.read(normed, np.zeros_like(x)), cuda.read(out, np.zeros((n_tokens, 2 * n_used), dtype=np.uint32))
+
+    want = route(cuda.new_buffer(source.nbytes), cuda.new_buffer(router.nbytes), True)
+    got = route(cuda.new_buffer(source.nbytes), cuda.new_buffer(router.nbytes), False)
+    assert np.abs(want[0]).max() > 0
+    assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+
+
 def test_route_ties_go_to_the_lower_expert_and_limits(cuda):
     n_cols, n_experts, n_used = 32, 8, 3
     x = np.ones((1, n_cols), dtype=np.float32)
