@@ -522,7 +522,7 @@ bc_status bc_op_short_conv(bc_backend* b, bc_buffer* bcx, size_t bcx_off, bc_buf
     return b->run("short_conv", n_tokens, n_embd, 0, 1, [&] {
         return k::short_conv(b->stream, reinterpret_cast<const float*>(at(bcx, bcx_off)), reinterpret_cast<const float*>(at(taps, taps_off)),
                              reinterpret_cast<float*>(at(history, hist_off)), reinterpret_cast<float*>(at(out, out_off)), n_embd, kernel,
-                             n_tokens);
+                             n_tokens, false);
     });
 }
 

@@ -132,9 +132,10 @@ cudaError_t matvec_swiglu(cudaStream_t stream, const Mat& gate, const Mat& up, c
 cudaError_t matvec_conv(cudaStream_t stream, const Mat& in_proj, const float* x, Norm norm, const float* taps,
                         float* history, float* out, uint32_t n_embd, uint32_t kernel);
 // With `packed` (matmul_pack_bytes(n_tokens, n_embd) bytes; n_embd a multiple of 64) the results go
-// out as the packed fp16 input of the product that consumes them, and `out` is not written.
+// out as the packed fp16 input of the product that consumes them, and `out` is not written. `constant_taps`: a model's, which no
+// launch writes, so they are read ahead of the wait for the preceding one.
 cudaError_t short_conv(cudaStream_t stream, const float* bcx, const float* taps, float* history, float* out,
-                       uint32_t n_embd, uint32_t kernel, uint32_t n_tokens, void* packed = nullptr);
+                       uint32_t n_embd, uint32_t kernel, uint32_t n_tokens, bool constant_taps, void* packed = nullptr);
 cudaError_t expand(cudaStream_t stream, const Mat& w, void* out, bool out_half);
 // A position that is either immediate or read from device memory at run time (`*ptr + value`), so
 // one captured launch sequence can be replayed at every position of a decode.

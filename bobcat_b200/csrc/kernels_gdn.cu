@@ -75,6 +75,7 @@ struct ConvParams {
     float *beta, *alpha;  // gates: with n_gates
     const float *a, *dt_bias;
     uint32_t n_v_heads, n_gates;
+    bool constant_taps;  // a model's: read ahead of the wait. An op call's are read after it: its recording may write them
 };
 
 template <int PER, int K, int R>
@@ -92,6 +93,7 @@ __global__ void __launch_bounds__(256) gdn_conv_kernel(const __grid_constant__ C
     const uint32_t group = (uint32_t)(item % n_groups), t0 = (uint32_t)(item / n_groups) * R;
     if (t0 >= p.n_tokens) return;
     const uint32_t c0 = group * 32 * PER + lane;
+    if (!p.constant_taps) pdl_wait();
     float tap[PER][K], window[PER][K - 1 + R];  // inputs of tokens t0 - (K - 1) .. t0 + R - 1
 #pragma unroll
     for (int e = 0; e < PER; ++e) {
@@ -592,7 +594,7 @@ cudaError_t launch_conv(cudaStream_t stream, ConvParams& p) {
 cudaError_t gdn_conv(cudaStream_t stream, const float* x, const float* taps, float* history, float* out, uint32_t conv_dim,
                      uint32_t kernel, uint32_t n_tokens) {
     if (n_tokens == 0) return cudaSuccess;
-    ConvParams p{x, taps, history, out, conv_dim, kernel, n_tokens, 0, 0, nullptr, nullptr, nullptr, nullptr, 1, 0};
+    ConvParams p{x, taps, history, out, conv_dim, kernel, n_tokens, 0, 0, nullptr, nullptr, nullptr, nullptr, 1, 0, false};
     return launch_conv<4>(stream, p);
 }
 
@@ -600,7 +602,7 @@ cudaError_t gdn_conv_gates(cudaStream_t stream, const float* x, const float* tap
                            const float* dt_bias, uint32_t n_k_heads, uint32_t n_v_heads, uint32_t k_dim, uint32_t v_dim, uint32_t kernel, uint32_t n_tokens) {
     if (n_tokens == 0) return cudaSuccess;
     ConvParams p{x, taps, history, out, 2 * n_k_heads * k_dim + n_v_heads * v_dim, kernel, n_tokens, 2 * n_k_heads, 0, beta, alpha, a, dt_bias, n_v_heads,
-                 n_v_heads * n_tokens};
+                 n_v_heads * n_tokens, true};
     switch (k_dim) {
         case 32: return launch_conv<1>(stream, p);
         case 64: return launch_conv<2>(stream, p);

@@ -210,14 +210,15 @@ __global__ void norm_rope_kernel(NormRopeParams p) {
 // reads them K times, took 9.1 us at 512 tokens of 2048 channels and 1.9 more for the history in a second launch, now
 // 5.2 together. Only the first run of tokens reads the history (R >= K - 1), and the same threads rewrite it.
 template <int K, int V>
-__global__ void __launch_bounds__(128) short_conv_kernel(const float* __restrict__ bcx, const float* __restrict__ taps, float* history,
+__global__ void __launch_bounds__(128) short_conv_kernel(const float* __restrict__ bcx, const float* taps, float* history,
                                                          float* __restrict__ out, __half* __restrict__ packed, uint32_t n_embd, uint32_t kernel,
-                                                         uint32_t n_tokens) {
+                                                         uint32_t n_tokens, bool constant_taps) {
     constexpr int R = K <= 4 ? 4 : 8;
     static_assert(R >= K - 1, "only the first run may read the history");
     pdl_launch_dependents();  // the output projection that reads the packed results may set itself up meanwhile
     const uint32_t ch = (blockIdx.x * blockDim.x + threadIdx.x) * V, skip = K - kernel;  // taps and window are aligned to the newest
     if (ch >= n_embd) return;
+    if (!constant_taps) pdl_wait();  // the recording may have written them
     float tap[K][V];
 #pragma unroll
     for (int kk = 0; kk < K; ++kk)
@@ -586,7 +587,7 @@ cudaError_t silu_mul(cudaStream_t stream, float* x, const float* gate, uint64_t 
 }
 
 cudaError_t short_conv(cudaStream_t stream, const float* bcx, const float* taps, float* history, float* out, uint32_t n_embd,
-                       uint32_t kernel, uint32_t n_tokens, void* packed) {
+                       uint32_t kernel, uint32_t n_tokens, bool constant_taps, void* packed) {
     if (n_tokens == 0) return cudaSuccess;
     if (packed && n_embd % 64 != 0) return cudaErrorInvalidValue;
     if (kernel < 2 || kernel > 9) return cudaErrorInvalidValue;
@@ -596,7 +597,7 @@ cudaError_t short_conv(cudaStream_t stream, const float* bcx, const float* taps,
     auto launch = [&](auto conv, uint32_t per_thread, uint32_t run) {
         const uint32_t runs = (rows + run - 1) / run;
         return launch_dependent(conv, dim3((n_embd / per_thread + 127) / 128, runs < 65535u ? runs : 65535u), dim3(128), 0, stream, bcx, taps, history, out,
-                                static_cast<__half*>(packed), n_embd, kernel, n_tokens);
+                                static_cast<__half*>(packed), n_embd, kernel, n_tokens, constant_taps);
     };
     if (kernel <= 4) return wide ? launch(short_conv_kernel<4, 4>, 4, 4) : launch(short_conv_kernel<4, 1>, 1, 4);
     return wide ? launch(short_conv_kernel<9, 4>, 4, 8) : launch(short_conv_kernel<9, 1>, 1, 8);

@@ -532,11 +532,11 @@ struct Recorder {
                     void* pack = nullptr;
                     if (status == BC_OK) status = s.backend->pack_scratch(k::matmul_pack_bytes(n, n_embd), &pack);
                     run("short_conv", n, n_embd, 0, 1,
-                        [&] { return k::short_conv(stream, s.bcx, D.taps, history, nullptr, n_embd, hp.conv_kernel, n, pack); });
+                        [&] { return k::short_conv(stream, s.bcx, D.taps, history, nullptr, n_embd, hp.conv_kernel, n, true, pack); });
                     product_of_packed(D.out_proj, pack, s.hidden, n, BC_STORE_ACCUMULATE);
                 } else {
                     run("short_conv", n, n_embd, 0, 1,
-                        [&] { return k::short_conv(stream, s.bcx, D.taps, history, s.conv_out, n_embd, hp.conv_kernel, n); });
+                        [&] { return k::short_conv(stream, s.bcx, D.taps, history, s.conv_out, n_embd, hp.conv_kernel, n, true); });
                     matmul(D.out_proj, s.conv_out, s.hidden, n, BC_STORE_ACCUMULATE);
                 }
             }

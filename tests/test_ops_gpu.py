@@ -271,6 +271,44 @@ def test_short_conv_batches_carry_history(cuda, kernel):
         assert np.abs(cuda.read(hb, np.zeros_like(hist)) - ref_hist).max() < 1e-6
 
 
+def written_and_read(cuda, values, run):
+    """``run(view)``'s result when `values` stand at the view beforehand, and when the last elements of a long copy in the recording of
+    the op that reads them put them there."""
+    padded = np.concatenate([np.zeros(1 << 20, dtype=np.float32), values.reshape(-1).astype(np.float32)])
+    source = cuda.buffer_from(padded)
+    results = []
+    for beforehand in (True, False):
+        target = cuda.new_buffer(padded.nbytes)
+        cuda.begin()
+        cuda.copy(source, target, padded.size)
+        if beforehand:
+            cuda.end()
+            cuda.begin()
+        read = run(target.floats(1 << 20))
+        cuda.end()
+        results.append(read())
+    return results
+
+
+@pytest.mark.parametrize("channels,kernel", [(96, 3), (96, 9), (2050, 4), (2048, 3), (6144, 8)])
+def test_convolutions_read_the_taps_their_recording_wrote(cuda, channels, kernel):
+    rng = np.random.default_rng(channels + kernel)
+    taps = rng.uniform(-1, 1, (channels, kernel)).astype(np.float32)
+    for n in (1, 37):
+        for op, width in ((cuda.short_conv, 3 * channels), (cuda.gdn_conv, channels)):
+            if op == cuda.gdn_conv and kernel > 8:
+                continue
+            xb = cuda.buffer_from(rng.uniform(-1, 1, (n, width)).astype(np.float32))
+
+            def run(tb):
+                hb, ob = cuda.new_buffer(channels * (kernel - 1) * 4), cuda.new_buffer(n * channels * 4)
+                op(xb, tb, hb, ob, channels, kernel, n)
+                return lambda: cuda.read(ob, np.zeros((n, channels), dtype=np.float32))
+
+            want, got = written_and_read(cuda, taps, run)
+            assert np.abs(want).max() > 0 and np.array_equal(got, want), op.__name__
+
+
 def test_matvec_conv_equals_projection_then_conv(cuda):
     rng = np.random.default_rng(4)
     n_embd, kernel = 128, 3
