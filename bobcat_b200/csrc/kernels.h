@@ -37,6 +37,7 @@ struct Mat {
 struct Norm {
     const float* weight = nullptr;  // null: no normalisation
     float eps = 0.f;
+    bool constant = false;  // no launch that may still run writes the weights (a model's): they may be read ahead of the wait
 };
 
 // Up to four matrices that share an input vector, multiplied in one launch.

@@ -85,7 +85,7 @@ struct FewParams {
     uint32_t slices;               // CTAs per cluster
     uint32_t n_tokens;
     const float* x;                // exact: [n_tokens][n_pairs * 64]
-    const float* norm_weight;
+    const float* norm_weight;      // constant: read ahead of the wait
     float eps;
     const uint4* packed;           // half: the packed fp16 operand, [pair][token group][8 cores][8 tokens] of 16 bytes
     uint32_t token_groups;
@@ -702,7 +702,7 @@ bool matmul_exact_supported(const Mat& w, uint32_t n_tokens) {
 
 cudaError_t matmul_exact(cudaStream_t stream, const Mat* const* ws, float* const* ys, const uint32_t* strides, int n, const float* x, Norm norm,
                          uint32_t n_tokens, int32_t store) {
-    if (n < 1 || n > 4 || !matmul_exact_supported(*ws[0], n_tokens)) return cudaErrorInvalidValue;
+    if (n < 1 || n > 4 || !matmul_exact_supported(*ws[0], n_tokens) || (norm.weight && !norm.constant)) return cudaErrorInvalidValue;
     FewParams p{};
     p.n_segments = n;
     for (int i = 0; i < n; ++i) {
@@ -725,7 +725,7 @@ cudaError_t matmul_exact(cudaStream_t stream, const Mat* const* ws, float* const
 }
 
 cudaError_t matmul_exact_swiglu(cudaStream_t stream, const Mat& gate, const Mat& up, const float* x, Norm norm, float* y, uint32_t n_tokens) {
-    if (gate.n_rows != up.n_rows || gate.n_cols != up.n_cols || !matmul_exact_supported(gate, n_tokens) || !up.tiles) return cudaErrorInvalidValue;
+    if (gate.n_rows != up.n_rows || gate.n_cols != up.n_cols || !matmul_exact_supported(gate, n_tokens) || !up.tiles || (norm.weight && !norm.constant)) return cudaErrorInvalidValue;
     FewParams p{};
     p.n_segments = 1;
     p.dual = 1;

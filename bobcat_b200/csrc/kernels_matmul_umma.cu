@@ -799,6 +799,7 @@ cudaError_t matmul_pack_gated(cudaStream_t stream, const float* x, const float* 
 cudaError_t matmul_pack_norm(cudaStream_t stream, float* x, Norm norm, uint32_t n_tokens, uint32_t n_cols, void* packed, const Deferred* add) {
     uint32_t token_groups = ((n_tokens + 15u) & ~15u) / 8;
     if (token_groups == 0 || n_cols == 0) return cudaSuccess;
+    if (!norm.constant) return cudaErrorInvalidValue;  // read ahead of the wait
     const bool adding = add && add->partial;
     if (adding && (add->n_tokens != n_tokens || add->n_rows != n_cols || n_cols % 4 != 0)) return cudaErrorInvalidValue;
     const size_t smem = (size_t)n_cols * 4;

@@ -128,6 +128,7 @@ struct Params {
     const float* x;
     const float* norm_weight;
     float eps;
+    bool norm_constant;
     int accumulate;
     const float* taps;
     float* history;
@@ -240,11 +241,13 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) matvec_mma_kernel(Params
 
     // Everything above touched only weights; the input vector (and y, the conv history) belong
     // to earlier launches.
-    // The norm's weights are the model's, not a predecessor's: a thread's share of them is on its
+    // A model's norm weights are nobody's output: a thread's share of them is on its
     // way before the wait, so the input's loads after the wait are the only trip to L2 the
-    // staging waits for (inputs of up to one item per thread; longer inputs load them in the loop).
+    // staging waits for (inputs of up to one item per thread; longer inputs load them in the loop,
+    // as do op calls, whose recording may have written them; plain loads there, since one through the
+    // read-only path may move ahead of the wait).
     float4 early_wl = make_float4(1.f, 1.f, 1.f, 1.f), early_wh = early_wl;
-    const bool norm_early = p.norm_weight != nullptr && p.n_blocks * 4 <= (uint32_t)kThreads;
+    const bool norm_early = p.norm_weight != nullptr && p.norm_constant && p.n_blocks * 4 <= (uint32_t)kThreads;
     if (norm_early && (uint32_t)threadIdx.x < p.n_blocks * 4) {
         const float4* w4e = reinterpret_cast<const float4*>(p.norm_weight);
         early_wl = __ldg(w4e + (threadIdx.x >> 2) * 8 + (threadIdx.x & 3));
@@ -276,8 +279,8 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) matvec_mma_kernel(Params
             if (p.norm_weight) {
                 float4 wl = early_wl, wh = early_wh;
                 if (!norm_early) {
-                    wl = __ldg(w4 + b * 8 + t);
-                    wh = __ldg(w4 + b * 8 + 4 + t);
+                    wl = w4[b * 8 + t];
+                    wh = w4[b * 8 + 4 + t];
                 }
                 lo4.x *= wl.x; lo4.y *= wl.y; lo4.z *= wl.z; lo4.w *= wl.w;
                 hi4.x *= wh.x; hi4.y *= wh.y; hi4.z *= wh.z; hi4.w *= wh.w;
@@ -621,6 +624,7 @@ cudaError_t matvec_mma(cudaStream_t stream, const MatvecSegment* segments, int n
     p.x = x;
     p.norm_weight = norm.weight;
     p.eps = norm.eps;
+    p.norm_constant = norm.constant;
     p.accumulate = accumulate;
     return launch<kPlain>(stream, p);
 }
@@ -638,6 +642,7 @@ cudaError_t matvec_swiglu_mma(cudaStream_t stream, const Mat& gate, const Mat& u
     p.x = x;
     p.norm_weight = norm.weight;
     p.eps = norm.eps;
+    p.norm_constant = norm.constant;
     return launch<kSwiglu>(stream, p);
 }
 
@@ -693,6 +698,7 @@ cudaError_t matvec_conv_mma(cudaStream_t stream, const Mat& in_proj, const float
     p.x = x;
     p.norm_weight = norm.weight;
     p.eps = norm.eps;
+    p.norm_constant = norm.constant;
     p.taps = taps;
     p.history = history;
     p.n_embd = n_embd;

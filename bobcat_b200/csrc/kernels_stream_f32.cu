@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(kThreads, 1) stream_f32_kernel(const __grid_co
         float4 v = T == 1 || i < p.n_tokens * quads ? x4[i] : make_float4(0.f, 0.f, 0.f, 0.f);
         if (T == 1 && p.norm_weight) {
             sumsq += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
-            const float4 w = __ldg(reinterpret_cast<const float4*>(p.norm_weight) + i);
+            const float4 w = reinterpret_cast<const float4*>(p.norm_weight)[i];
             v.x *= w.x; v.y *= w.y; v.z *= w.z; v.w *= w.w;
         }
         xs[i] = v;

@@ -56,7 +56,7 @@ __device__ __forceinline__ void prefetch_row(const RowPtr& r, uint32_t n_cols) {
 
 // Stage x into shared memory in the rotated chunk layout, times the norm weight when given.
 // Returns the factor the finished row sums are multiplied by (1 without a norm).
-__device__ inline float stage_input(const float* __restrict__ x, const float* __restrict__ norm_weight, float eps,
+__device__ inline float stage_input(const float* __restrict__ x, const float* norm_weight, float eps,
                              uint32_t n_cols, float4* xs, float* reduce_scratch) {
     const float4* x4 = reinterpret_cast<const float4*>(x);
     const float4* w4 = reinterpret_cast<const float4*>(norm_weight);
@@ -65,7 +65,7 @@ __device__ inline float stage_input(const float* __restrict__ x, const float* __
         float4 v = x4[ci];
         if (norm_weight) {
             sumsq += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
-            float4 w = __ldg(w4 + ci);
+            float4 w = w4[ci];  // plain: one through the read-only path may move ahead of the caller's wait
             v.x *= w.x; v.y *= w.y; v.z *= w.z; v.w *= w.w;
         }
         xs[x_slot(ci >> 3, ci & 7)] = v;

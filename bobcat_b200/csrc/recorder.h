@@ -72,7 +72,7 @@ struct Recorder {
         status = f();
     }
 
-    k::Norm norm(const float* weight) const { return k::Norm{weight, hp.norm_eps}; }
+    k::Norm norm(const float* weight) const { return k::Norm{weight, hp.norm_eps, true}; }
 
     // Batched products run on the tensor cores with half-precision operands (as the reference's
     // Q4_0 prefill does, matmul.metal:519-521) unless the sequence asks for f32 operands, which

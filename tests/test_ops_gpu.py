@@ -271,22 +271,22 @@ def test_short_conv_batches_carry_history(cuda, kernel):
         assert np.abs(cuda.read(hb, np.zeros_like(hist)) - ref_hist).max() < 1e-6
 
 
-def written_and_read(cuda, values, run):
-    """``run(view)``'s result when `values` stand at the view beforehand, and when the last elements of a long copy in the recording of
-    the op that reads them put them there."""
+def written_and_read(cuda, values, floats, op):
+    """What ``op(view, *buffers)`` leaves in the first of new buffers of `floats` floats each: with `values` at the view beforehand, and with the last
+    elements of a long copy in the op's own recording putting them there."""
     padded = np.concatenate([np.zeros(1 << 20, dtype=np.float32), values.reshape(-1).astype(np.float32)])
     source = cuda.buffer_from(padded)
     results = []
     for beforehand in (True, False):
-        target = cuda.new_buffer(padded.nbytes)
+        target, buffers = cuda.new_buffer(padded.nbytes), [cuda.new_buffer(4 * n) for n in floats]
         cuda.begin()
         cuda.copy(source, target, padded.size)
         if beforehand:
             cuda.end()
             cuda.begin()
-        read = run(target.floats(1 << 20))
+        op(target.floats(1 << 20), *buffers)
         cuda.end()
-        results.append(read())
+        results.append(cuda.read(buffers[0], np.zeros(floats[0], dtype=np.float32)))
     return results
 
 
@@ -296,17 +296,29 @@ def test_convolutions_read_the_taps_their_recording_wrote(cuda, channels, kernel
     taps = rng.uniform(-1, 1, (channels, kernel)).astype(np.float32)
     for n in (1, 37):
         for op, width in ((cuda.short_conv, 3 * channels), (cuda.gdn_conv, channels)):
-            if op == cuda.gdn_conv and kernel > 8:
-                continue
+            if width == channels and kernel > 8:
+                continue  # beyond the DeltaNet convolution's limit
             xb = cuda.buffer_from(rng.uniform(-1, 1, (n, width)).astype(np.float32))
+            want, got = written_and_read(cuda, taps, (n * channels, channels * (kernel - 1)), lambda tb, ob, hb: op(xb, tb, hb, ob, channels, kernel, n))
+            assert np.abs(want).max() > 0 and np.array_equal(got, want), (n, width)
 
-            def run(tb):
-                hb, ob = cuda.new_buffer(channels * (kernel - 1) * 4), cuda.new_buffer(n * channels * 4)
-                op(xb, tb, hb, ob, channels, kernel, n)
-                return lambda: cuda.read(ob, np.zeros((n, channels), dtype=np.float32))
 
-            want, got = written_and_read(cuda, taps, run)
-            assert np.abs(want).max() > 0 and np.array_equal(got, want), op.__name__
+@pytest.mark.parametrize("fmt,n_rows,n_cols", [(Q4_0, 96, 64), (Q4_0, 6144, 2048), (Q4_0, 512, 10752), (F32, 1000, 96), (F32, 6000, 1024), (F16, 1000, 1024)])
+def test_matvecs_read_the_norm_their_recording_wrote(cuda, fmt, n_rows, n_cols):
+    """On every kernel of a matrix times a row: inputs of one item a thread and longer ones, f32 rows streamed or not."""
+    rng = np.random.default_rng(n_rows + n_cols)
+    raw, _ = make_matrix(rng, fmt, n_rows, n_cols)
+    wb, xb = cuda.upload_matrix(fmt, raw, n_rows, n_cols), cuda.buffer_from(rng.uniform(-1, 1, n_cols).astype(np.float32))
+    channels = n_rows // 3
+    tb = cuda.buffer_from(rng.uniform(-1, 1, (channels, 3)).astype(np.float32))
+    ops = {
+        "matvec": ((n_rows,), lambda nb, yb: cuda.matvec(fmt, wb, n_rows, n_cols, xb, yb, norm=Norm(nb, 1e-5))),
+        "swiglu": ((n_rows,), lambda nb, yb: cuda.matvec_swiglu(fmt, wb, wb, n_rows, n_cols, xb, Norm(nb, 1e-5), yb)),
+        "conv": ((channels, 2 * channels), lambda nb, yb, hb: cuda.matvec_conv(fmt, wb, n_cols, xb, Norm(nb, 1e-5), tb, hb, yb, channels, 3)),
+    }
+    for name, (floats, op) in ops.items():
+        want, got = written_and_read(cuda, rng.uniform(0.5, 1.5, n_cols).astype(np.float32), floats, op)
+        assert np.abs(want).max() > 0 and np.array_equal(got, want), name
 
 
 def test_matvec_conv_equals_projection_then_conv(cuda):
