@@ -153,6 +153,7 @@ bc_status matrix_view(bc_backend* b, bc_buffer* buffer, size_t offset, int32_t f
         return fail(BC_ERR_OUT_OF_BOUNDS, "the %s launch needs %llu bytes at offset %zu of a %llu-byte matrix", op,
                     (unsigned long long)(n_rows * row_bytes), offset, (unsigned long long)(m.n_rows * row_bytes));
     *out = m.rows((uint32_t)first, n_rows);
+    out->constant = false;  // the caller's buffer: an op of the recording may have written f32 values
     return BC_OK;
 }
 

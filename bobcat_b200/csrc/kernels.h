@@ -29,6 +29,8 @@ struct Mat {
     // (kernels_matmul_half.cu), for products of many tokens.
     const void* half_tiles = nullptr;
     uint32_t n_rows = 0, n_cols = 0;
+    // No launch that may still run writes the matrix: f32 values may be read ahead of the wait. (The copies above exist only of constant ones.)
+    bool constant = true;
     // Rows [first, first + rows) of this matrix.
     Mat rows(uint32_t first, uint32_t count) const;
     uint64_t bytes() const;  // bytes a full pass over the matrix reads

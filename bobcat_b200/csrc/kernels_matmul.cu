@@ -130,7 +130,7 @@ constexpr size_t few_smem_bytes() { return (size_t)kStages * (kFewRows + 32) * (
 
 template <int kFewStep, int kStages>
 __global__ void __launch_bounds__(kFewThreads) matmul_f32_few_kernel(const float* __restrict__ w, const float* __restrict__ x, float* __restrict__ y,
-                                                                     uint32_t n_rows, uint32_t n_cols, uint32_t n_tokens, uint32_t y_stride) {
+                                                                     uint32_t n_rows, uint32_t n_cols, uint32_t n_tokens, uint32_t y_stride, bool constant) {
     constexpr int kFewPitch = kFewStep + 4;
     extern __shared__ __align__(16) float few_smem[];
     float (*ws)[kFewRows][kFewPitch] = reinterpret_cast<float (*)[kFewRows][kFewPitch]>(few_smem);
@@ -161,7 +161,8 @@ __global__ void __launch_bounds__(kFewThreads) matmul_f32_few_kernel(const float
         }
     };
     const uint32_t steps = n_cols / kFewStep;
-    bring_w(0, 0);  // the weights are nobody's output
+    if (!constant) pdl_wait();
+    bring_w(0, 0);  // constant weights are nobody's output
     pdl_wait();
     bring_x(0, 0);
     async::cp_async_commit();
@@ -231,7 +232,7 @@ cudaError_t matmul(cudaStream_t stream, const Mat& w, const float* x, float* y, 
         cudaError_t e = ensure_dynamic_smem((const void*)matmul_f32_few_kernel<32, 2>, bytes);
         if (e != cudaSuccess) return e;
         return launch_dependent(matmul_f32_few_kernel<32, 2>, dim3((w.n_rows + kFewRows - 1) / kFewRows), dim3(kFewThreads), bytes, stream,
-                                static_cast<const float*>(w.data), x, y, w.n_rows, w.n_cols, n_tokens, y_stride);
+                                static_cast<const float*>(w.data), x, y, w.n_rows, w.n_cols, n_tokens, y_stride, w.constant);
     }
     if (pack && matmul_umma_supported(w, n_tokens)) {
         cudaError_t e = matmul_pack(stream, x, n_tokens, w.n_cols, pack);

@@ -37,6 +37,7 @@ struct StreamParams {
     float* y;        // [n_tokens][y_stride]
     uint32_t n_rows, n_cols, n_tokens, y_stride;
     float eps;
+    bool constant;   // w: its first rows are on their way before the wait
 };
 
 template <int R, int T>
@@ -75,6 +76,7 @@ __global__ void __launch_bounds__(kThreads, 1) stream_f32_kernel(const __grid_co
         ahead_slot = ahead_slot + 1 == kStages ? 0 : ahead_slot + 1;
         async::cp_async_commit();  // a group per step, empty past the end
     };
+    if (!p.constant) pdl_wait();
 #pragma unroll
     for (int i = 0; i < kStages - 1; ++i) copy_next();
     pdl_wait();
@@ -170,7 +172,7 @@ bool stream_f32_supported(const Mat& w, const float* x) {
 }
 
 cudaError_t stream_f32(cudaStream_t stream, const Mat& w, const float* x, Norm norm, float* y) {
-    return launch_stream<4, 1>(stream, StreamParams{static_cast<const float*>(w.data), x, norm.weight, y, w.n_rows, w.n_cols, 1, w.n_rows, norm.eps});
+    return launch_stream<4, 1>(stream, StreamParams{static_cast<const float*>(w.data), x, norm.weight, y, w.n_rows, w.n_cols, 1, w.n_rows, norm.eps, w.constant});
 }
 
 // Several rows: as many as sixteen, when they fit beside the ring at once (a second pass would read the matrix again).
@@ -180,7 +182,7 @@ bool stream_f32_rows_supported(const Mat& w, const float* x, uint32_t n_tokens) 
 }
 
 cudaError_t stream_f32_rows(cudaStream_t stream, const Mat& w, const float* x, float* y, uint32_t n_tokens, uint32_t y_stride) {
-    const StreamParams p{static_cast<const float*>(w.data), x, nullptr, y, w.n_rows, w.n_cols, n_tokens, y_stride, 0.f};
+    const StreamParams p{static_cast<const float*>(w.data), x, nullptr, y, w.n_rows, w.n_cols, n_tokens, y_stride, 0.f, w.constant};
     if (n_tokens <= 4) return launch_stream<8, 4>(stream, p);
     if (n_tokens <= 8) return launch_stream<8, 8>(stream, p);
     return launch_stream<8, 16>(stream, p);

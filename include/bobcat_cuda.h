@@ -15,9 +15,8 @@
  *  - Views of activation vectors (x, y, norm weights, q, out) must start on a 16-byte boundary; the
  *    kernels read them with 128-bit loads. Ops with a scalar variant fall back to it; the others
  *    reject the offset with BC_ERR_ARGUMENT before launching anything.
- *  - A recorded op sees what the ops recorded before it wrote, in every buffer it names. Matrices of
- *    bc_matrix_upload are constants: they are held in more than one layout and read ahead of the
- *    launches before, so no op may write them.
+ *  - A recorded op sees what the ops recorded before it wrote, in every buffer it names. (Writing into a
+ *    Q4_0 matrix was never an update: bc_matrix_upload holds it in layouts of its own.)
  *  - There is no CPU fallback. Opening a backend without a CUDA device fails with BC_ERR_NO_DEVICE.
  */
 #ifndef BOBCAT_CUDA_H

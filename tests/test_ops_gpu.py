@@ -321,6 +321,30 @@ def test_matvecs_read_the_norm_their_recording_wrote(cuda, fmt, n_rows, n_cols):
         assert np.abs(want).max() > 0 and np.array_equal(got, want), name
 
 
+@pytest.mark.parametrize("n_rows,n_tokens", [(6000, 1), (6000, 5), (200, 32), (200, 1)])
+def test_f32_products_read_the_matrix_their_recording_wrote(cuda, n_rows, n_tokens):
+    """The streaming kernel with one row and with several, the tiles of 17 to 32, the general kernel."""
+    rng = np.random.default_rng(n_rows + n_tokens)
+    n_cols = 512
+    raw, w = make_matrix(rng, F32, n_rows, n_cols)
+    fresh, xb = cuda.buffer_from(w), cuda.buffer_from(rng.uniform(-1, 1, (n_tokens, n_cols)).astype(np.float32))
+    results = []
+    for beforehand in (True, False):
+        wb, yb = cuda.upload_matrix(F32, np.zeros_like(raw), n_rows, n_cols), cuda.new_buffer(n_tokens * n_rows * 4)
+        cuda.begin()
+        cuda.copy(fresh, wb, n_rows * n_cols)
+        if beforehand:
+            cuda.end()
+            cuda.begin()
+        if n_tokens == 1:
+            cuda.matvec(F32, wb, n_rows, n_cols, xb, yb)
+        else:
+            cuda.matmul(F32, wb, n_rows, n_cols, xb, yb, n_tokens, OVERWRITE)
+        cuda.end()
+        results.append(cuda.read(yb, np.zeros(n_tokens * n_rows, dtype=np.float32)))
+    assert np.abs(results[0]).max() > 0 and np.array_equal(results[0], results[1])
+
+
 def test_matvec_conv_equals_projection_then_conv(cuda):
     rng = np.random.default_rng(4)
     n_embd, kernel = 128, 3
