@@ -693,11 +693,11 @@ bc_status bc_op_attention(bc_backend* b, bc_buffer* q, size_t q_off, bc_buffer* 
     BC_TRY(check_range(b, scratch, s_off, bc_attention_scratch_floats(n_heads, head_dim, n_ctx, n_queries) * 4, "attention"));
     BC_TRY(check_range(b, out, out_off, (size_t)n_queries * n_heads * head_dim * 4, "attention"));
     k::AttentionShape shape{n_heads, n_kv_heads, head_dim, first_pos, n_queries, n_ctx, n_heads * head_dim, head_dim};
-    int launches = k::attention_launches(kv_half != 0, shape);
-    return b->run("attention", n_queries, first_pos + n_queries, kv_bytes * 2, launches, [&] {
-        return k::attention(b->stream, reinterpret_cast<const float*>(at(q, q_off)), at(k_cache, k_off), at(v_cache, v_off), kv_half != 0,
-                            reinterpret_cast<float*>(at(scratch, s_off)), reinterpret_cast<float*>(at(out, out_off)), shape);
-    });
+    const float* qp = reinterpret_cast<const float*>(at(q, q_off));
+    const void *kp = at(k_cache, k_off), *vp = at(v_cache, v_off);
+    float *sp = reinterpret_cast<float*>(at(scratch, s_off)), *op = reinterpret_cast<float*>(at(out, out_off));
+    return b->run("attention", n_queries, first_pos + n_queries, kv_bytes * 2, k::attention_launches(qp, kp, vp, kv_half != 0, sp, op, shape),
+                  [&] { return k::attention(b->stream, qp, kp, vp, kv_half != 0, sp, op, shape); });
 }
 
 bc_status bc_op_argmax(bc_backend* b, bc_buffer* x, size_t x_off, bc_buffer* out, size_t out_off, uint32_t n) {

@@ -216,8 +216,8 @@ struct AttentionShape {
 uint64_t attention_scratch_floats(uint32_t n_heads, uint32_t head_dim, uint32_t n_ctx, uint32_t n_queries);
 cudaError_t attention(cudaStream_t stream, const float* q, const void* k_cache, const void* v_cache, bool kv_half,
                       float* scratch, float* out, const AttentionShape& shape);
-// Kernels `attention` launches for this shape.
-int attention_launches(bool kv_half, const AttentionShape& shape);
+// Kernels `attention` launches for these arguments.
+int attention_launches(const float* q, const void* k_cache, const void* v_cache, bool kv_half, const float* scratch, const float* out, const AttentionShape& shape);
 // One decoded token of an attention layer: the launch normalises and rotates the raw q itself, and the
 // CTA whose chunk ends at the new position prepares that position's key
 // and value rows, stores them in the caches and uses them. Contexts beyond 2048 positions take a combine
@@ -228,7 +228,7 @@ cudaError_t attention_step(cudaStream_t stream, const RopeStore& r, float* scrat
 // The tensor-core prefill kernel (kernels_attention_flash.cu): heads of 64 elements, f16 cache, at
 // least 32 queries, positions known at launch. `attention` picks it when it applies.
 bool attention_flash_supported(bool kv_half, const AttentionShape& shape);
-int attention_flash_launches(const AttentionShape& s);
+int attention_flash_launches(const float* scratch, const AttentionShape& s);
 cudaError_t attention_flash(cudaStream_t stream, const float* q, const void* k_cache, const void* v_cache, float* scratch, float* out,
                             const AttentionShape& shape);
 

@@ -856,20 +856,29 @@ uint64_t attention_scratch_floats(uint32_t n_heads, uint32_t head_dim, uint32_t 
     return (batch > decode ? batch : decode) * n_heads * (head_dim + 2);
 }
 
-int attention_launches(bool kv_half, const AttentionShape& s) {
-    if (attention_flash_supported(kv_half, s)) return attention_flash_launches(s);
-    if (token_shape(s)) return 1;
+namespace {
+// The tensor-core kernel reads q and out 8 bytes and the caches 16 bytes at a time, the kernel of one token q and the caches 16; views that
+// do not start on those boundaries take the chunk kernels, whose loads are scalar.
+bool flash_route(const float* q, const void* k_cache, const void* v_cache, bool kv_half, const float* out, const AttentionShape& s) {
+    return ((uintptr_t)q | (uintptr_t)out) % 8 == 0 && ((uintptr_t)k_cache | (uintptr_t)v_cache) % 16 == 0 && attention_flash_supported(kv_half, s);
+}
+bool token_route(const float* q, const void* k_cache, const void* v_cache, const AttentionShape& s) {
+    return token_shape(s) && ((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache) % 16 == 0;
+}
+}  // namespace
+
+int attention_launches(const float* q, const void* k_cache, const void* v_cache, bool kv_half, const float* scratch, const float* out, const AttentionShape& s) {
+    if (s.n_queries == 0) return 0;
+    if (flash_route(q, k_cache, v_cache, kv_half, out, s)) return attention_flash_launches(scratch, s);
+    if (token_route(q, k_cache, v_cache, s)) return 1;
     return 2 * (int)((s.n_queries + kQueryBatch - 1) / kQueryBatch);
 }
 
 cudaError_t attention(cudaStream_t stream, const float* q, const void* k_cache, const void* v_cache, bool kv_half,
                       float* scratch, float* out, const AttentionShape& s) {
     if (s.n_queries == 0) return cudaSuccess;
-    // The tensor-core kernel reads q and out 8 bytes and the caches 16 bytes at a time; views that
-    // do not start on those boundaries take the chunk kernels, whose loads are scalar.
-    const bool flash_aligned = ((uintptr_t)q | (uintptr_t)out) % 8 == 0 && ((uintptr_t)k_cache | (uintptr_t)v_cache) % 16 == 0;
-    if (flash_aligned && attention_flash_supported(kv_half, s)) return attention_flash(stream, q, k_cache, v_cache, scratch, out, s);
-    if (token_shape(s) && ((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache) % 16 == 0) {
+    if (flash_route(q, k_cache, v_cache, kv_half, out, s)) return attention_flash(stream, q, k_cache, v_cache, scratch, out, s);
+    if (token_route(q, k_cache, v_cache, s)) {
         const ChunkParams cp{q, k_cache, v_cache, out, s.n_heads, s.n_kv_heads, s.head_dim, s.first_pos, s.n_ctx,
                              s.q_stride, s.q_head_stride, 0, 0, s.pos_ptr, (uint32_t)kDecodeChunk, nullptr, nullptr, nullptr, nullptr, 0.f, 0.f, nullptr};
         return launch_token(stream, cp, s, kv_half, false, s.gated);

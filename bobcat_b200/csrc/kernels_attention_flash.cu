@@ -372,6 +372,9 @@ uint32_t choose_splits(const AttentionShape& s) {
     return best;
 }
 
+// The parts are stored 8 bytes at a time.
+uint32_t splits_for(const float* scratch, const AttentionShape& s) { return (uintptr_t)scratch % 8 == 0 ? choose_splits(s) : 1; }
+
 template <int HD>
 cudaError_t launch_flash(cudaStream_t stream, const FlashParams& p) {
     const uint32_t group = p.n_heads / p.n_kv_heads, total = p.n_queries * p.n_heads;
@@ -390,11 +393,11 @@ bool attention_flash_supported(bool kv_half, const AttentionShape& s) {
            s.n_kv_heads > 0 && s.n_heads % s.n_kv_heads == 0 && s.q_stride % 2 == 0 && s.q_head_stride % 2 == 0;
 }
 
-int attention_flash_launches(const AttentionShape& s) { return choose_splits(s) > 1 ? 2 : 1; }
+int attention_flash_launches(const float* scratch, const AttentionShape& s) { return splits_for(scratch, s) > 1 ? 2 : 1; }
 
 cudaError_t attention_flash(cudaStream_t stream, const float* q, const void* k_cache, const void* v_cache, float* scratch, float* out,
                             const AttentionShape& s) {
-    const uint32_t splits = (uintptr_t)scratch % 8 == 0 ? choose_splits(s) : 1;
+    const uint32_t splits = splits_for(scratch, s);
     const FlashParams p{q, static_cast<const __half*>(k_cache), static_cast<const __half*>(v_cache), out, s.n_heads, s.n_kv_heads,
                         s.first_pos, s.n_queries, s.q_stride, s.q_head_stride, splits, scratch};
     switch (s.head_dim) {

@@ -321,18 +321,22 @@ struct Recorder {
         return static_cast<float*>(parts);
     }
 
+    // Attention of the shape's queries over positions [0, pos + n) of a layer's caches.
+    void attend(const float* q, uint32_t cache_index, uint32_t pos, float* scratch, const k::AttentionShape& shape) {
+        const void *k_rows = cache_at(s.k_cache, layer_base(cache_index)), *v_rows = cache_at(s.v_cache, layer_base(cache_index));
+        const uint32_t n = shape.n_queries;
+        const int kernels = k::attention_launches(q, k_rows, v_rows, s.kv_half, scratch, s.attn, shape);
+        run("attention", n, pos + n, (uint64_t)(pos + n) * kv_dim() * kv_element_bytes() * 2, kernels,
+            [&] { return k::attention(stream, q, k_rows, v_rows, s.kv_half, scratch, s.attn, shape); });
+    }
+
     // Norm and rotation of q and k, cache stores, attention over positions [0, pos + n).
     void rotate_and_attend(const DeviceLayer& D, uint32_t cache_index, uint32_t pos, uint32_t n, uint32_t q_stride, uint32_t q_head_stride) {
         size_t slot = layer_base(cache_index) + (size_t)pos * kv_dim();
         rotate_batch(D, slot, pos, n, s.q, q_stride, q_head_stride, q_stride, q_head_stride);
         k::AttentionShape shape{hp.n_heads, hp.n_kv_heads, hp.head_dim, pos, n, s.n_ctx, q_stride, q_head_stride};
         float* scratch = attention_scratch(shape);
-        int kernels = k::attention_launches(s.kv_half, shape);
-        uint64_t kv_bytes = (uint64_t)(pos + n) * kv_dim() * kv_element_bytes() * 2;
-        run("attention", n, pos + n, kv_bytes, kernels, [&] {
-            return k::attention(stream, s.q, cache_at(s.k_cache, layer_base(cache_index)), cache_at(s.v_cache, layer_base(cache_index)), s.kv_half,
-                                scratch, s.attn, shape);
-        });
+        attend(s.q, cache_index, pos, scratch, shape);
     }
 
     float* value_target(uint32_t cache_index, uint32_t pos) {
@@ -354,10 +358,7 @@ struct Recorder {
             return;
         }
         run("rope_store", hp.n_heads + 2 * hp.n_kv_heads, hp.head_dim, 0, 1, [&] { return k::rope_store(stream, rs, p); });
-        run("attention", 1, pos + 1, kv_bytes, k::attention_launches(s.kv_half, shape), [&] {
-            return k::attention(stream, s.q, cache_at(s.k_cache, layer_base(cache_index)), cache_at(s.v_cache, layer_base(cache_index)), s.kv_half,
-                                s.scores, s.attn, shape);
-        });
+        attend(s.q, cache_index, pos, s.scores, shape);
     }
 
     void lfm2_attention(const DeviceLayer& D, uint32_t cache_index, uint32_t pos) {
@@ -662,10 +663,7 @@ struct Recorder {
                 rotate_batch(D, slot, pos, n, s.q_rot, 2 * q_dim, 2 * hp.head_dim, q_dim, hp.head_dim);
                 k::AttentionShape shape{hp.n_heads, hp.n_kv_heads, hp.head_dim, pos, n, s.n_ctx, q_dim, hp.head_dim};
                 float* scratch = attention_scratch(shape);
-                run("attention", n, pos + n, (uint64_t)(pos + n) * kv_dim() * kv_element_bytes() * 2, k::attention_launches(s.kv_half, shape), [&] {
-                    return k::attention(stream, s.q_rot, cache_at(s.k_cache, layer_base(S.cache_index)), cache_at(s.v_cache, layer_base(S.cache_index)),
-                                        s.kv_half, scratch, s.attn, shape);
-                });
+                attend(s.q_rot, S.cache_index, pos, scratch, shape);
                 if (tensor_products() && k::matmul_umma_supported(D.output, n, min_tensor_rows) && hp.head_dim % 32 == 0) {
                     // The gates on the way into the packed input of the output projection.
                     void* pack = nullptr;
