@@ -4,23 +4,33 @@
 // Arithmetic: that of the other half-precision products (kernels_matmul_umma.cu): weights (q - 8) * d rounded to
 // fp16 once, inputs rounded to fp16, products accumulated in f32 (crates/bobcat-metal/src/matmul.metal:473-506).
 //
+// Sums. An instruction cuts its sum off instead of rounding it, so what one accumulator loses grows with its K: against float64 of the same
+// rounded operands (2-norm), 1.1e-7 for 64 columns, 1.8e-7 for 128, 6.4e-7 for 512, 2.1e-6 for 1792. Up to 64 rows an expert on the average, tensor
+// memory therefore sums 128 columns (of up to 1024 columns, 64), and the storing warps add the parts up in registers, rounding: 2.0e-7 for 1792 and more (stretches
+// of 2048 columns are added up by themselves), what sums on mma.sync over 16 warps have. Experts of more rows sum all of K in tensor memory, as
+// matmul_umma_kernel does.
+//
 // What bounds it. Every expert's weights are read and unpacked once for a few dozen rows, so unpacking is the work: a stage (128 rows x
 // 256 columns) is 32 pairs of blocks, each 104 packed-half and logic instructions of a warp, which issue every second cycle: 512 cycles on four
 // schedulers. On mma.sync (matmul_few_kernel) the multiplies took the same issue slots (8 cycles each, 32 rows in four groups),
 // and every 16-row tile's sums met over 16 warps: 1.9 us per tile of 2048 columns, 0.8 of them multiplies. Here one instruction multiplies
-// 128 rows by all of an expert's, K accumulates in tensor memory and is read once. The unpacked
+// 128 rows by all of an expert's. The unpacked
 // weights go to tensor memory, not to shared memory, whose 128 bytes per cycle writing and reading them back (1024 cycles a stage) would
 // take instead: tcgen05.st 16x128b takes the registers as they are unpacked, because the decode tiles
 // are in mma fragment order (lane (g, t): rows g and g + 8, word t of a block), so a row's columns lie in the order (pair of halves j,
-// word t); the rows' operand is packed in the same order. What a stage takes is 900 cycles, the unpacking and the hand-over between warps:
-// with stages of 64 columns gate and up of the block below took 82 us, of 128 67, of 256 52.
+// word t); the rows' operand is packed in the same order. What a stage takes beyond that is the hand-over between warps:
+// with stages of 64 columns (and one accumulator) gate and up of the block below took 82 us, of 128 67, of 256 52.
 //
 // Shape. Persistent CTAs, one per SM, equal runs of the jobs (128 weight rows, of a SwiGLU 64 of either matrix) of all experts' groups of
 // up to `tile_tokens` rows. 16 unpacking warps: a warp owns 16 of the tile's rows (its lanes of tensor memory) in every other stage.
 // One warp brings the weights' bytes (a lane per tile, eight pairs of blocks at a time), one the rows' operand, one issues the
-// multiplies, four store, from one of two accumulators while the other fills. Every wait is bounded.
+// multiplies, eight (two a quarter of the lanes, half of the rows each) sum and store, from one of two sets of accumulators while the other fills. A set is
+// two parts, a stage's: handed over one by one, with the wait for a free accumulator behind the stage's, parts cost 24 us more than the 9 they cost. Eight warps, since
+// four would need 64 registers a thread for the sums and 27 warps leave 72. Every wait is bounded.
 //
-// Measured: 203 tokens, 4 of 32 experts: gate and up 1792 x 2048 52 us, down 2048 x 1792 29 (matmul_few_kernel 91 and 58; HBM time 20 and 10).
+// Measured with the packing of the rows, 4 of 32 experts, gate and up 1792 x 2048 and down 2048 x 1792, us: 203 tokens 68.6 and 39.2 (one accumulator 60.0 and
+// 37.5, matmul_few_kernel 102 and 65.5; HBM time 20 and 10); 16 tokens 55.9 and 35.9 (46.6 and 29.7; 57.0 and 35.3); 512 tokens 101 and 57.6 (81.8
+// and 47.6 with groups of 128 rows, whose sums do not fit the registers; 220 and 137).
 
 #include "async_utils.cuh"
 #include "device_utils.cuh"
@@ -35,13 +45,15 @@ namespace {
 using namespace async;
 
 constexpr uint32_t kMaxStages = 3, kStageColumns = 128, kStagePairs = 4;  // columns of tensor memory: 256 fp16 weights
-constexpr uint32_t kTmemColumns = 512;                                    // two accumulators, then the stages' weights: 3 beside up to 64 rows, else 2
-constexpr uint32_t kUnpackWarps = 16, kMmaWarp = 20, kRowsWarp = 21, kTilesWarp = 22, kThreads = 23 * 32;  // in between, four that store
+constexpr uint32_t kTmemColumns = 512;                                    // the accumulators, then the stages' weights: 3 beside up to 32 rows, else 2
+constexpr uint32_t kUnpackWarps = 16, kStoreWarps = 8, kMmaWarp = 24, kRowsWarp = 25, kTilesWarp = 26, kThreads = 27 * 32;
+constexpr uint32_t kSegmentRows = 64;                                     // rows whose parts of K are added up in registers: half of them per storing warp
 constexpr uint32_t kChunkPairs = 16, kPairQuants = 512, kPairScales = 64, kChunkBytes = kChunkPairs * (kPairQuants + kPairScales);  // decode tiles
 constexpr uint32_t kTiles = 8, kMaxRawSlots = 3, kRawPairs = 8, kRawSlot = kRawPairs * (kPairQuants + kPairScales);  // of a tile of 16 rows: quants, then scales
 constexpr uint32_t kRawStages = kRawPairs / kStagePairs;
 constexpr uint32_t kGroupBytes = 1024;                                  // 8 rows x 64 columns of the rows' operand
 constexpr uint32_t kSwapFloats = 2 * 16 * 32;                           // per pair of storing warps: 16 rows x 32 outputs, two in turn
+constexpr uint32_t kKeepPairs = 32;                                     // pairs of blocks summed in one go
 constexpr uint32_t kSpinLimit = 1u << 22;
 
 __device__ int* g_wait_word;  // where a wait that ran out leaves its code (kernels.h), null until set
@@ -97,22 +109,28 @@ __device__ __forceinline__ bool find_group(const ExpertsUmmaParams& p, uint32_t 
     return false;
 }
 
-// A CTA's run of jobs, counted through all groups; each role walks it by itself.
+// A CTA's run of jobs through all groups; each role walks it by itself.
 struct Run {
-    uint64_t at, end;
-    uint32_t expert = 0, place = 0, job = 0, left = 0;
+    uint32_t left, group, job, expert, place;
+    // The CTA's share of the jobs of n_groups groups.
+    __device__ __forceinline__ void start(const ExpertsUmmaParams& p, uint32_t n_groups) {
+        const uint64_t jobs = (uint64_t)n_groups * p.n_jobs, at = jobs * blockIdx.x / gridDim.x;
+        left = (uint32_t)(jobs * (blockIdx.x + 1) / gridDim.x - at);
+        group = (uint32_t)(at / p.n_jobs) - 1;  // the first step goes on to its group
+        job = p.n_jobs - 1;
+        first = (uint32_t)(at % p.n_jobs);
+    }
     __device__ __forceinline__ bool next(const ExpertsUmmaParams& p) {
-        if (left == 0) {
-            if (at >= end || !find_group(p, (uint32_t)(at / p.n_jobs), expert, place)) return false;
-            job = (uint32_t)(at % p.n_jobs);
-            left = (uint32_t)min((uint64_t)(p.n_jobs - job), end - at);
-            at += left;
-        } else {
-            ++job;
-        }
+        if (left == 0) return false;
         --left;
+        if (++job == p.n_jobs) {
+            job = first;
+            first = 0;
+            find_group(p, ++group, expert, place);
+        }
         return true;
     }
+    uint32_t first;
 };
 
 // One thread: D[tmem] (+)= A[tmem] * B^T over K = 16.
@@ -133,7 +151,23 @@ __device__ __forceinline__ void tmem_store_16x32(uint32_t taddr, const uint32_t 
                  : "memory");
 }
 
-template <bool DUAL>
+// a += b, both pairs of lanes rounded to nearest.
+__device__ __forceinline__ void add_two(float& a0, float& a1, float b0, float b1) {
+    asm("{\n\t.reg .b64 a, b;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 b, {%2, %3};\n\tadd.rn.f32x2 a, a, b;\n\tmov.b64 {%0, %1}, a;\n\t}" : "+f"(a0), "+f"(a1) : "f"(b0), "f"(b1));
+}
+
+// Whole warp: 8 accumulator columns of its 32 lanes (tmem_load_16).
+__device__ __forceinline__ void tmem_load_8(uint32_t taddr, float (&v)[8]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+        : "r"(taddr)
+        : "memory");
+}
+
+// SEGMENT: pairs of blocks (64 columns each) that tensor memory sums, the sums being added up in registers, two at a time; 0: it sums all of K.
+template <bool DUAL, uint32_t SEGMENT>
 __global__ void __launch_bounds__(kThreads, 1) experts_umma_kernel(const __grid_constant__ ExpertsUmmaParams p) {
     extern __shared__ __align__(1024) uint8_t smem[];  // the rows' stages, the raw slots, the swap buffers
     __shared__ __align__(8) uint64_t bars[2 * kMaxStages + 4], raw_bars[2 * kTiles * kMaxRawSlots];
@@ -143,7 +177,7 @@ __global__ void __launch_bounds__(kThreads, 1) experts_umma_kernel(const __grid_
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t full = smem_u32(bars), free = full + kMaxStages * 8, acc_full = free + kMaxStages * 8, acc_empty = acc_full + 16;
     const uint32_t pair_bytes = p.tile_tokens / 8 * kGroupBytes, stage_bytes = kStagePairs * pair_bytes, job_stages = (p.n_pairs + kStagePairs - 1) / kStagePairs;
-    const uint32_t n_stages = p.stages, a_at = 2 * p.tile_tokens, raw_slots = p.raw_slots;
+    const uint32_t set_columns = (SEGMENT ? 2 : 1) * p.tile_tokens, n_stages = p.stages, a_at = 2 * set_columns, raw_slots = p.raw_slots;
     const uint32_t raw_full = smem_u32(raw_bars), raw_free = raw_full + kTiles * kMaxRawSlots * 8, raw = smem_u32(smem) + n_stages * stage_bytes;
     pdl_launch_dependents();
     if (tid == 0) {
@@ -153,7 +187,7 @@ __global__ void __launch_bounds__(kThreads, 1) experts_umma_kernel(const __grid_
         }
         for (uint32_t a = 0; a < 2; ++a) {
             mbar_init(acc_full + 8 * a, 1);
-            mbar_init(acc_empty + 8 * a, 4);
+            mbar_init(acc_empty + 8 * a, kStoreWarps);
         }
         for (uint32_t i = 0; i < kTiles * kMaxRawSlots; ++i) {
             mbar_init(raw_full + 8 * i, 1);
@@ -172,8 +206,7 @@ __global__ void __launch_bounds__(kThreads, 1) experts_umma_kernel(const __grid_
     {
         uint32_t expert, n_groups;
         find_group(p, ~0u, expert, n_groups);
-        run.at = (uint64_t)n_groups * p.n_jobs * blockIdx.x / gridDim.x;
-        run.end = (uint64_t)n_groups * p.n_jobs * (blockIdx.x + 1) / gridDim.x;
+        run.start(p, n_groups);
     }
 
     if (warp < kUnpackWarps) {
@@ -181,7 +214,7 @@ __global__ void __launch_bounds__(kThreads, 1) experts_umma_kernel(const __grid_
         const uint32_t tile = 2 * (warp & 3) + (warp >> 2 & 1), g = lane >> 2, weights_at = tmem + ((tile * 16) << 16) + a_at;
         uint32_t slot = 0, slot_phase = 0, stage = 0, phase = 1, turn = warp >> 3;  // turn 0: the warp's stage
         bool alive = true;
-        for (uint32_t jobs = (uint32_t)(run.end - run.at); jobs > 0 && alive; --jobs) {
+        for (uint32_t jobs = run.left; jobs > 0 && alive; --jobs) {
             for (uint32_t first = 0; first < job_stages && alive; first += kRawStages) {
                 const uint32_t bar = (tile * kMaxRawSlots + slot) * 8, from = raw + (tile * raw_slots + slot) * kRawSlot, here = min(kRawStages, job_stages - first);
                 alive = await(raw_full + bar, slot_phase, dead, 6);
@@ -288,81 +321,149 @@ __global__ void __launch_bounds__(kThreads, 1) experts_umma_kernel(const __grid_
         const uint64_t desc0 = umma_desc(smem_u32(smem), 128, kGroupBytes);
         const uint32_t idesc = umma_idesc_f16(128, p.tile_tokens);
         // Every loop ends by a vote: the compiler then keeps the descriptors in uniform registers, where the instruction wants them.
-        const uint32_t jobs = (uint32_t)(run.end - run.at);
+        const uint32_t jobs = run.left;
         bool alive = true;
-        for (uint32_t job = 0; __all_sync(0xffffffffu, job < jobs && alive); ++job) {
+        // A set of accumulators (of two segments, or of all of K): free, filled, handed to the storing warps.
+        auto begin = [&]() {
             alive = await(acc_empty + 8 * acc, acc_phase, dead, 3);
-            if (__any_sync(0xffffffffu, !alive)) break;
             tc_fence_after_sync();
+            return __all_sync(0xffffffffu, alive);
+        };
+        auto finish = [&]() {
+            if (elect_one()) umma_commit(acc_full + 8 * acc);
+            __syncwarp();
+            if (++acc == 2) acc = 0, acc_phase ^= 1;
+        };
+        constexpr uint32_t kPart = SEGMENT ? 2 * SEGMENT : kStagePairs;
+        for (uint32_t job = 0; __all_sync(0xffffffffu, job < jobs && alive); ++job) {
+            if (SEGMENT == 0 && !begin()) break;
             for (uint32_t c = 0; c < job_stages; ++c) {
+                if (SEGMENT && !begin()) break;  // ahead of the stage, which takes longer
                 alive = await(full + 8 * stage, phase, dead, 4);
                 if (__any_sync(0xffffffffu, !alive)) break;
                 tc_fence_after_sync();
                 const uint64_t b_desc = desc0 + ((stage * stage_bytes) >> 4);
                 const uint32_t pairs = min(kStagePairs, p.n_pairs - c * kStagePairs);
-                if (elect_one()) {
 #pragma unroll
-                    for (uint32_t i = 0; i < kStagePairs; ++i) {
-                        if (i >= pairs) break;
+                for (uint32_t part = 0; part < kStagePairs; part += kPart) {
+                    if (part >= pairs || (part > 0 && !begin())) break;
+                    if (elect_one()) {
 #pragma unroll
-                        for (uint32_t j = 0; j < 4; ++j)
-                            umma_f16_a_tmem(tmem + acc * p.tile_tokens, tmem + a_at + stage * kStageColumns + i * 32 + j * 8,
-                                            b_desc + ((i * pair_bytes + j * 256) >> 4), idesc, (c | i | j) != 0);
+                        for (uint32_t i = part; i < part + kPart; ++i) {
+                            if (i >= pairs) break;
+                            const uint32_t segment = SEGMENT ? (i - part) / SEGMENT : 0, first = SEGMENT ? (i - part) % SEGMENT : c | i;
+#pragma unroll
+                            for (uint32_t j = 0; j < 4; ++j)
+                                umma_f16_a_tmem(tmem + acc * set_columns + segment * p.tile_tokens, tmem + a_at + stage * kStageColumns + i * 32 + j * 8,
+                                                b_desc + ((i * pair_bytes + j * 256) >> 4), idesc, (first | j) != 0);
+                        }
                     }
-                    umma_commit(free + 8 * stage);
+                    __syncwarp();
+                    if (SEGMENT) finish();
                 }
+                if (__any_sync(0xffffffffu, !alive)) break;
+                if (elect_one()) umma_commit(free + 8 * stage);
                 __syncwarp();
                 if (++stage == n_stages) stage = 0, phase ^= 1;
             }
-            if (alive && elect_one()) umma_commit(acc_full + 8 * acc);
-            __syncwarp();
-            if (++acc == 2) acc = 0, acc_phase ^= 1;
+            if (SEGMENT == 0 && alive) finish();
         }
     } else {
-        // ---- the stores: a warp reads lanes 32 * (warp % 4).. of tensor memory, 16 rows of x at a time. Of a SwiGLU lanes 0 to 63 are rows of
-        // gate, the other 64 the same rows of up: of 16 rows of x either warp takes eight, and they swap what the other one needs.
-        const uint32_t quarter = warp & 3, block = DUAL ? quarter & 1 : quarter;
+        // ---- the sums and stores: a warp reads lanes 32 * (warp % 4).. of tensor memory and has one half of the rows of x, 16 at a time. Of a
+        // SwiGLU lanes 0 to 63 are rows of gate, the other 64 the same rows of up: of 16 rows of x either warp takes eight, and
+        // they swap what the other one needs.
+        const uint32_t quarter = warp & 3, half = (warp - kUnpackWarps) >> 2, block = DUAL ? quarter & 1 : quarter;
         const bool has_gate = quarter < 2;
-        float* swap = reinterpret_cast<float*>(smem + n_stages * stage_bytes + kTiles * raw_slots * kRawSlot) + (quarter & 1) * kSwapFloats;
+        const uint32_t couple = half * 2 + (quarter & 1);
+        float* swap = reinterpret_cast<float*>(smem + n_stages * stage_bytes + kTiles * raw_slots * kRawSlot) + couple * kSwapFloats;
         uint32_t acc = 0, acc_phase = 0, turn = 0;
         while (run.next(p)) {
-            const uint32_t first = p.offsets[run.expert] + run.place * p.tile_tokens, rows = min(p.tile_tokens, p.offsets[run.expert + 1] - first);
-            const uint32_t out = run.job * (DUAL ? 64 : 128) + block * 32 + lane;
-            const bool ok = lane != 0 || mbar_wait(acc_full + 8 * acc, acc_phase, kSpinLimit, dead);
-            // A wait that ran out voids the results; the warp walks on (further waits end at once), because another meets it below.
-            if (!__all_sync(0xffffffffu, ok) && lane == 0) give_up(dead, 5);
-            tc_fence_after_sync();
-            const uint32_t from = tmem + ((quarter * 32) << 16) + acc * p.tile_tokens;
-            for (uint32_t r = 0; r < rows; r += 16) {
-                const uint32_t entry = r + (lane & 15) < rows ? p.entries[first + r + (lane & 15)] : 0;
-                float v[16];
+            auto begin = [&]() {
+                const bool ok = lane != 0 || mbar_wait(acc_full + 8 * acc, acc_phase, kSpinLimit, dead);
+                // A wait that ran out voids the results; the warp walks on (further waits end at once), because another meets it below.
+                if (!__all_sync(0xffffffffu, ok) && lane == 0) give_up(dead, 5);
+                tc_fence_after_sync();
+                return tmem + ((quarter * 32) << 16) + acc * set_columns;
+            };
+            auto finish = [&]() {  // the accumulator is read: the MMA thread may overwrite it
+                tc_fence_before_sync();
                 __syncwarp();
-                tmem_load_16(from + r, v);
+                if (lane == 0) mbar_arrive(acc_empty + 8 * acc);
+                if (++acc == 2) acc = 0, acc_phase ^= 1;
+            };
+            // The warp's share of the rows.
+            const uint32_t first = p.offsets[run.expert] + run.place * p.tile_tokens, rows = min(p.tile_tokens, p.offsets[run.expert + 1] - first);
+            const uint32_t each = (rows + 31) / 32 * 16, row0 = half * each, row_end = min(rows, row0 + each);
+            auto entry_of = [&](uint32_t r) { return r + (lane & 15) < row_end ? p.entries[first + r + (lane & 15)] : 0; };
+            auto store = [&](uint32_t r, uint32_t entry, const float (&v)[16]) {  // rows r .. r + 15
+                const uint32_t out = run.job * (DUAL ? 64 : 128) + block * 32 + lane;
+                __syncwarp();
                 if constexpr (DUAL) {
                     float* buffer = swap + (turn++ & 1) * (16 * 32);
 #pragma unroll
                     for (int j = 0; j < 8; ++j) buffer[(has_gate ? 8 + j : j) * 32 + lane] = has_gate ? v[8 + j] : v[j];
-                    asm volatile("bar.sync %0, 64;" ::"r"(1 + (quarter & 1)) : "memory");
+                    asm volatile("bar.sync %0, 64;" ::"r"(1 + couple) : "memory");
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
                         const float other = buffer[(has_gate ? j : 8 + j) * 32 + lane], mine = has_gate ? v[j] : v[8 + j];
                         const float gate = has_gate ? mine : other, up = has_gate ? other : mine;
                         const uint32_t at = (has_gate ? 0 : 8) + j, row = __shfl_sync(0xffffffffu, entry, at);
-                        if (r + at < rows && out < p.n_rows) p.y[(uint64_t)row * p.n_rows + out] = gate / (1.f + expf(-gate)) * up;
+                        if (r + at < row_end && out < p.n_rows) p.y[(uint64_t)row * p.n_rows + out] = gate / (1.f + expf(-gate)) * up;
                     }
                 } else {
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
                         const uint32_t row = __shfl_sync(0xffffffffu, entry, j);
-                        if (r + j < rows && out < p.n_rows) p.y[(uint64_t)row * p.n_rows + out] = v[j];
+                        if (r + j < row_end && out < p.n_rows) p.y[(uint64_t)row * p.n_rows + out] = v[j];
                     }
                 }
+            };
+            if constexpr (SEGMENT != 0) {
+                // Looked up here: behind the sums, the trips to memory would keep the accumulators of the next job waiting.
+                const uint32_t entry0 = entry_of(row0), entry1 = entry_of(row0 + 16);
+                const uint32_t blocks = row_end <= row0 ? 0 : row_end <= row0 + 16 ? 2 : 4;  // of eight rows
+                float sum[32], *kept = reinterpret_cast<float*>(smem + n_stages * stage_bytes + kTiles * raw_slots * kRawSlot) + kStoreWarps / 2 * kSwapFloats + (warp - kUnpackWarps) * (32 * 32) + lane;
+#pragma unroll
+                for (int i = 0; i < 32; ++i) sum[i] = -0.f;  // leaves the first part as it is
+                for (uint32_t pair = 0; pair < p.n_pairs; pair += 2 * SEGMENT) {
+                    const uint32_t from = begin() + row0;
+#pragma unroll
+                    for (uint32_t g = 0; g < 2; ++g) {
+                        if (g > 0 && pair + SEGMENT >= p.n_pairs) break;
+#pragma unroll
+                        for (uint32_t b = 0; b < 4; ++b) {
+                            if (b >= blocks) break;
+                            float v[8];
+                            tmem_load_8(from + g * p.tile_tokens + 8 * b, v);
+#pragma unroll
+                            for (int i = 0; i < 8; i += 2) add_two(sum[8 * b + i], sum[8 * b + i + 1], v[i], v[i + 1]);
+                        }
+                    }
+                    finish();
+                    const uint32_t done = pair + 2 * SEGMENT;
+                    if (done % kKeepPairs == 0 && done < p.n_pairs) {  // a long sum would lose more: its stretches are added up by themselves
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) {
+                            kept[i * 32] = done == kKeepPairs ? sum[i] : kept[i * 32] + sum[i];
+                            sum[i] = -0.f;
+                        }
+                    }
+                }
+                if (p.n_pairs > kKeepPairs)
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) sum[i] += kept[i * 32];
+                if (blocks > 0) store(row0, entry0, *reinterpret_cast<const float(*)[16]>(sum));
+                if (blocks > 2) store(row0 + 16, entry1, *reinterpret_cast<const float(*)[16]>(sum + 16));
+            } else {
+                const uint32_t from = begin();
+                for (uint32_t r = row0; r < row_end; r += 16) {
+                    float v[16];
+                    const uint32_t entry = entry_of(r);
+                    tmem_load_16(from + r, v);
+                    store(r, entry, v);
+                }
+                finish();
             }
-            // The accumulator is read: the MMA thread may overwrite it.
-            tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(acc_empty + 8 * acc);
-            if (++acc == 2) acc = 0, acc_phase ^= 1;
         }
     }
 
@@ -447,11 +548,15 @@ cudaError_t matmul_experts_tiles(cudaStream_t stream, const Mat& w, const Mat* u
     p.n_pairs = w.n_cols / 64;
     p.n_jobs = (n_rows + (up ? 63 : 127)) / (up ? 64 : 128);
     p.cap_groups = cap_groups;
-    p.tile_tokens = likely <= 32 ? 32 : likely <= 64 ? 64 : 128;
-    p.stages = p.tile_tokens <= 64 ? 3 : 2;
-    p.raw_slots = p.tile_tokens <= 64 ? kMaxRawSlots : 2;
-    const size_t smem = (size_t)p.stages * kStagePairs * (p.tile_tokens / 8) * kGroupBytes + kTiles * p.raw_slots * kRawSlot + 2 * kSwapFloats * sizeof(float);
-    const void* kernel = up ? (const void*)experts_umma_kernel<true> : (const void*)experts_umma_kernel<false>;
+    const uint32_t segment = share > kSegmentRows ? 0 : p.n_pairs <= 16 ? 1 : 2;
+    p.tile_tokens = segment == 0 ? 128 : likely <= 32 ? 32 : 64;
+    p.stages = p.tile_tokens == 32 ? kMaxStages : 2;
+    p.raw_slots = segment == 0 ? 2 : kMaxRawSlots;
+    const size_t smem = (size_t)p.stages * kStagePairs * (p.tile_tokens / 8) * kGroupBytes + kTiles * p.raw_slots * kRawSlot + kStoreWarps / 2 * kSwapFloats * sizeof(float) +
+                        (segment != 0 && p.n_pairs > kKeepPairs ? kStoreWarps * 32 * 32 * sizeof(float) : 0);
+    const void* kernel = segment == 0   ? up ? (const void*)experts_umma_kernel<true, 0> : (const void*)experts_umma_kernel<false, 0>
+                         : segment == 1 ? up ? (const void*)experts_umma_kernel<true, 1> : (const void*)experts_umma_kernel<false, 1>
+                                        : up ? (const void*)experts_umma_kernel<true, 2> : (const void*)experts_umma_kernel<false, 2>;
     if ((e = ensure_dynamic_smem(kernel, smem)) != cudaSuccess) return e;
     void* args[] = {&p};
     return launch_kernel(kernel, dim3((unsigned)sm_count()), dim3(kThreads), smem, stream, args);

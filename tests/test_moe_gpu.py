@@ -106,6 +106,39 @@ def make_routes(rng, n_tokens, n_experts, n_used):
     return route
 
 
+@pytest.mark.parametrize("n_tokens,n_used,n_experts,n_ff,n_embd", [(16, 1, 4, 64, 2048), (60, 2, 8, 128, 1792), (33, 3, 4, 80, 4160), (100, 2, 4, 96, 1088),
+                                                                   (200, 1, 4, 64, 640)])
+def test_expert_sums_lose_no_more_than_rounded_parts(cuda, n_tokens, n_used, n_experts, n_ff, n_embd):
+    """Against float64 of the same fp16 operands, in the 2-norm. Measured: 2.0e-7 and, for the SwiGLU of two such sums, 3.7e-7, from 128 columns on whatever
+    the width, since parts of at most 128 columns are cut off by the tensor core and added up rounding. One accumulator over all of K loses
+    1.2e-9 and 2.4e-9 a column: 2.1e-6 and 4.8e-6 for 1792 and 2048. The bounds are half as much again as measured. Few and ragged rows, experts of several
+    groups of rows, parts of 64 columns, K beyond one stretch and no multiple of a stage."""
+    rng = np.random.default_rng(n_embd)
+    gate_raw, up_raw, down_raw = (random_q4_0(rng, n_experts * r, c) for r, c in ((n_ff, n_embd), (n_ff, n_embd), (n_ff, n_embd)))
+
+    def halves(raw, n_cols):
+        return oracle.dequantize(2, raw, raw.shape[0] * n_cols).reshape(n_experts, -1, n_cols).astype(np.float16).astype(np.float64)
+
+    gate, up, down = (halves(raw, n_embd) for raw in (gate_raw, up_raw, down_raw))
+    x = rng.standard_normal((n_tokens, n_embd)).astype(np.float32)
+    route = make_routes(rng, n_tokens, n_experts, n_used)
+    xb, rb = cuda.buffer_from(x), cuda.buffer_from(route)
+    ob, eb = cuda.new_buffer((n_experts + 1) * 4), cuda.new_buffer(n_tokens * n_used * 4)
+    pair_b, plain_b = cuda.new_buffer(n_tokens * n_used * n_ff * 4), cuda.new_buffer(n_tokens * n_used * n_ff * 4)
+    gb, ub, db = (cuda.upload_matrix(Q4_0, raw, n_experts * n_ff, n_embd) for raw in (gate_raw, up_raw, down_raw))
+    cuda.begin()
+    cuda.moe_group(rb, ob, eb, n_experts, n_used, n_tokens)
+    cuda.matmul_experts(Q4_0, gb, ub, n_ff, n_embd, n_experts, xb, True, ob, eb, n_used, pair_b, n_tokens)
+    cuda.matmul_experts(Q4_0, db, None, n_ff, n_embd, n_experts, xb, True, ob, eb, n_used, plain_b, n_tokens)
+    cuda.end()
+    experts, rows = route[:, :n_used].reshape(-1), np.repeat(x.astype(np.float16).astype(np.float64), n_used, axis=0)
+    want_pair = np.stack([silu(gate[e] @ r) * (up[e] @ r) for e, r in zip(experts, rows)])
+    want_plain = np.stack([down[e] @ r for e, r in zip(experts, rows)])
+    for buffer, want, bound in ((pair_b, want_pair, 5.6e-7), (plain_b, want_plain, 3e-7)):
+        got = cuda.read(buffer, np.zeros(want.shape, dtype=np.float32)).astype(np.float64)
+        assert np.linalg.norm(got - want) / np.linalg.norm(want) < bound
+
+
 def test_group_is_a_stable_counting_sort(cuda):
     rng = np.random.default_rng(5)
     n_tokens, n_experts, n_used = 77, 16, 4
