@@ -83,7 +83,7 @@ bc_status kernel_wait_status() {
     if (int code = take(3)) return fail(BC_ERR_EXECUTION, "a sum over ranks gave up waiting for rank %d", code - 1);
     if (int code = take(6)) return fail(BC_ERR_EXECUTION, "a delta-rule kernel gave up waiting for its rows (code %d)", code);
     if (int code = take(5)) return fail(BC_ERR_EXECUTION, "a product over experts gave up waiting on its pipeline (code %d)", code);
-    if (int code = take(4)) return fail(BC_ERR_EXECUTION, "a product of few rows gave up waiting for its sums (code %d)", code);
+    if (int code = take(4)) return fail(BC_ERR_EXECUTION, "a product of few rows gave up waiting for its %s (code %d)", code == 2 ? "weights" : "sums", code);
     return BC_OK;
 }
 

@@ -445,7 +445,7 @@ bool matmul_half_swiglu_whole(const Mat& gate, uint32_t n_tokens);  // tiles of 
 // the packed inputs on warp-level MMAs, one launch, no split of K left open. matmul_umma,
 // matmul_umma_several, matmul_umma_swiglu and matmul_experts_umma hand over to these whenever the
 // shape allows (BOBCAT_NO_FEW_MATMUL=1 keeps them on the tcgen05 kernels).
-// Code: 1, a warp on the other warps' sums.
+// Codes: 1, a warp on the other warps' sums; 2, on the copies of a step's weights.
 cudaError_t matmul_few_wait_word(int* word);
 // A batch over experts on tcgen05, weights unpacked into tensor memory (kernels_matmul_experts.cu).
 bool matmul_experts_tiles_supported(const Mat& w, const Mat* up, uint32_t n_rows);

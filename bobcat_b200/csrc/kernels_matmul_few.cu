@@ -67,10 +67,10 @@ __device__ int* g_wait_word;  // where a wait that ran out leaves its code (kern
 // The rest of a wait whose first poll failed. One that runs out leaves a code and the warp carries on, because the others and the
 // cluster's barriers need it. A function of its own, out of the way of the steps' code: 11 rows of the 350M shape's prompt take 627 us (626
 // without the report), with the loop and the report inline 629 to 648.
-__device__ __noinline__ void wait_on(uint32_t bar, uint32_t parity) {
+__device__ __noinline__ void wait_on(uint32_t bar, uint32_t parity, int code) {
     for (uint32_t spin = 1; spin < kSpinLimit; ++spin)
         if (async::mbar_test(bar, parity)) return;
-    if (g_wait_word) *reinterpret_cast<volatile int*>(g_wait_word) = 1;
+    if (g_wait_word) *reinterpret_cast<volatile int*>(g_wait_word) = code;
 }
 
 struct FewParams {
@@ -491,7 +491,7 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_few_kernel(const __grid_co
         const uint32_t behind = slices == 1 ? 1 : 2;
         if (u >= behind) fetch_old(u - behind);
         if (u < n_steps && live) {
-            if (!async::mbar_test(full_bars + slot * 8, slot_parity)) wait_on(full_bars + slot * 8, slot_parity);
+            if (!async::mbar_test(full_bars + slot * 8, slot_parity)) wait_on(full_bars + slot * 8, slot_parity, 2);
             uint4 q[T][W];
             uint2 d[T][W];
 #pragma unroll
@@ -546,7 +546,7 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_few_kernel(const __grid_co
         if (u > 0) {
             const uint32_t before = u - 1, turns = steps_before + before;  // buffers and barriers alternate through all groups
             // Every warp arrives for every step whatever happens, so the wait ends; it is bounded like all waits.
-            if (!async::mbar_test(bars + (turns & 1) * 8, (turns >> 1) & 1)) wait_on(bars + (turns & 1) * 8, (turns >> 1) & 1);
+            if (!async::mbar_test(bars + (turns & 1) * 8, (turns >> 1) & 1)) wait_on(bars + (turns & 1) * 8, (turns >> 1) & 1, 1);
             if (warp == (EXPERTS ? kWarps - 1 : before % kWarps)) request(slot == 0 ? DEPTH - 1 : slot - 1);  // every warp has its weights of that step in registers
             ask_tile += T;
             if (slices == 1) {

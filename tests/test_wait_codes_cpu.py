@@ -37,3 +37,10 @@ def test_every_word_is_read():
     read = re.findall(r"= take\((\d+)\)", backend)
     words = int(re.search(r"kWaitWords = (\d+)", backend).group(1))
     assert sorted(int(i or 0) for i in handed) == sorted(int(i) for i in read) == list(range(words))
+
+
+def test_the_few_row_kernel_tells_its_waits_apart():
+    """On the copies of the weights and on the other warps' sums: the report names which one ran out."""
+    calls = re.findall(r"wait_on\((\w+) [^;]*, (\d+)\);", source("kernels_matmul_few.cu"))
+    assert sorted(calls) == [("bars", "1"), ("full_bars", "2")]
+    assert re.search(r'gave up waiting for its %s \(code %d\)", code == 2 \? "weights" : "sums", code', source("backend.cpp"))
