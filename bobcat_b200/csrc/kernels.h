@@ -355,8 +355,9 @@ cudaError_t matvec_experts_down(cudaStream_t stream, const Mat& down, uint32_t n
 int matvec_experts_down_launches(const Mat& down, uint32_t n_rows, uint32_t n_used, uint32_t n_tokens, bool has_scratch);
 // Prefill: for each expert, its entries times its rows; with `up` the store is silu(gate) * up.
 // Input rows are the tokens' (gather) or the entries' own; output rows are the entries'.
-// With `scratch` (matmul_experts_scratch_bytes) and Q4_0 experts the tcgen05 kernel runs in its
-// grouped mode (two launches: gather-pack, then the product); otherwise the SIMT tile kernel.
+// With `scratch` (matmul_experts_scratch_bytes) and Q4_0 experts two launches run: gather-pack, then the product on fp16 operands
+// (matmul_experts_umma: the kernel with weights in tensor memory, the few-row kernel or the dequantising kernel's grouped mode, by size);
+// otherwise the few-row kernel with f32 operands or the SIMT tile kernel.
 cudaError_t matmul_experts(cudaStream_t stream, const Mat& w, const Mat* up, uint32_t n_rows, uint32_t n_experts, const float* x,
                            bool gather, const uint32_t* offsets, const uint32_t* entries, uint32_t n_used, float* y, uint32_t n_tokens,
                            void* scratch);
@@ -443,12 +444,12 @@ cudaError_t matmul_half_swiglu(cudaStream_t stream, const Mat& gate, const Mat& 
 bool matmul_half_swiglu_whole(const Mat& gate, uint32_t n_tokens);  // tiles of 128 rows of both matrices, else of 64 rows of either
 // The same products for at most 32 tokens (kernels_matmul_few.cu): the matrices' decode tiles against
 // the packed inputs on warp-level MMAs, one launch, no split of K left open. matmul_umma,
-// matmul_umma_several, matmul_umma_swiglu and matmul_experts_umma hand over to these whenever the
-// shape allows (BOBCAT_NO_FEW_MATMUL=1 keeps them on the tcgen05 kernels).
+// matmul_umma_several and matmul_umma_swiglu hand over to these whenever the shape allows, matmul_experts_umma
+// where the experts' jobs do not fill the device (BOBCAT_NO_FEW_MATMUL=1 keeps them on the tcgen05 kernels).
 // Codes: 1, a warp on the other warps' sums; 2, on the copies of a step's weights.
 cudaError_t matmul_few_wait_word(int* word);
 // A batch over experts on tcgen05, weights unpacked into tensor memory (kernels_matmul_experts.cu).
-bool matmul_experts_tiles_supported(const Mat& w, const Mat* up, uint32_t n_rows);
+bool matmul_experts_tiles_supported(const Mat& w, const Mat* up, uint32_t n_rows, uint32_t n_experts, uint32_t n_tokens, uint32_t n_used);
 cudaError_t matmul_experts_tiles(cudaStream_t stream, const Mat& w, const Mat* up, uint32_t n_rows, uint32_t n_experts, const float* x, bool gather,
                                  const uint32_t* offsets, const uint32_t* entries, uint32_t n_used, float* y, uint32_t n_tokens, void* scratch);
 cudaError_t matmul_experts_wait_word(int* word);
@@ -457,6 +458,9 @@ cudaError_t matmul_few(cudaStream_t stream, const Mat* const* ws, float* const* 
                        uint32_t n_tokens, int32_t store);
 cudaError_t matmul_few_swiglu(cudaStream_t stream, const Mat& gate, const Mat& up, const void* packed, float* y, uint32_t n_tokens, uint32_t y_stride,
                               void* packed_out);
+bool matmul_few_experts_supported(const Mat& w, const Mat* up, uint32_t n_rows, uint32_t n_experts, uint32_t n_tokens, uint32_t n_used);
+cudaError_t matmul_few_experts(cudaStream_t stream, const Mat& w, const Mat* up, uint32_t n_rows, uint32_t n_experts, const void* packed,
+                               const uint32_t* offsets, const uint32_t* entries, float* y, uint32_t n_tokens, uint32_t n_entries);
 // Products of a few rows with f32 operands (the same file): up to four Q4_0 matrices that
 // share the rows, with the rows' RMSNorm when given, in one launch; gate and up of a SwiGLU; the
 // experts of a grouped batch. `matmul` and `matmul_experts` hand over to these when their shape allows

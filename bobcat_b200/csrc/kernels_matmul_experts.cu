@@ -515,11 +515,19 @@ __global__ void __launch_bounds__(256) pack_experts_kernel(const float* __restri
 
 cudaError_t matmul_experts_wait_word(int* word) { return cudaMemcpyToSymbol(g_wait_word, &word, sizeof word); }
 
-// Any number of rows, where the matrices have decode tiles. An expert block of op calls (32 experts of 1792 x 2048, 4 to a token), us before and
-// now: 16 tokens 154 and 135, 64 162 and 149, 203 251 and 158, 512 455 and 220 (all matmul_few_kernel before), 600 358 and 251, 1024 413 and 356, 2048
-// 669 and 577 (matmul_umma_kernel's grouped mode, which the others keep).
-bool matmul_experts_tiles_supported(const Mat& w, const Mat* up, uint32_t n_rows) {
-    return w.format == BC_Q4_0 && w.tiles != nullptr && w.n_cols % 64 == 0 && w.n_cols > 0 && (!up || up->tiles != nullptr) && n_rows % 16 == 0;
+// Where the matrices have decode tiles and the jobs fill the device. Up to 64 rows an expert on the average, fewer than three jobs an SM of
+// which an SM's have fewer than 16 rows together leave a batch to matmul_few_kernel, whose jobs are tiles of 16 rows: us, this kernel and that one, both with
+// their packing: 4 experts of 512 x 512, 40 tokens of 2 14 and 8, of 256 x 4096, 64 tokens of 1 25 and 13; 8 of 1792 x 2048 with up (224 jobs), 40 tokens of
+// 2 28 and 25, 64 tokens 28 and 32; 8 of 2048 x 1792 (128 jobs), 40 tokens 18.9 and 18.4, 96 tokens 20 and 26; 16 of 1408 x 2048 with up (352 jobs), 16 tokens of 4 35 and 32;
+// 32 of 1792 x 2048 with up (896 jobs), 16 tokens of 4 50 and 53, 203 tokens 72 and 106. With more rows, narrow matrices
+// of few jobs go to matmul_umma_kernel's grouped mode, whose start is shorter: 8 of 128 x 128, 300 tokens of 2 14 and 10, 4 of 512 x 512 16.5 and 15 (700 tokens 16.9 and
+// 17.5), with up 8 of 96 x 128 16 and 14 (700 tokens 17 and 20); wider ones 2 of 1024 x 2816, 300 tokens of 1 25 and 31, 32 of 1792 x 2048 with up, 2048 tokens of
+// 4 203 and 292. (2 of 1024 x 2816 with 2048 rows each, where this kernel's 256 jobs are a second round on some SMs: 63 and 52.)
+bool matmul_experts_tiles_supported(const Mat& w, const Mat* up, uint32_t n_rows, uint32_t n_experts, uint32_t n_tokens, uint32_t n_used) {
+    if (w.format != BC_Q4_0 || w.tiles == nullptr || w.n_cols % 64 != 0 || w.n_cols == 0 || (up && up->tiles == nullptr) || n_rows % 16 != 0) return false;
+    const uint64_t share = ((uint64_t)n_tokens * n_used + n_experts - 1) / n_experts, jobs = (uint64_t)n_experts * ((n_rows + (up ? 63 : 127)) / (up ? 64 : 128)), sms = (uint64_t)sm_count();
+    if (matmul_few_experts_supported(w, up, n_rows, n_experts, n_tokens, n_used)) return jobs >= 3 * sms || jobs * share >= 16 * sms;
+    return w.n_cols > 512 || jobs * ((share + 127) / 128) >= (up ? 20u : 40u);
 }
 
 cudaError_t matmul_experts_tiles(cudaStream_t stream, const Mat& w, const Mat* up, uint32_t n_rows, uint32_t n_experts, const float* x, bool gather,

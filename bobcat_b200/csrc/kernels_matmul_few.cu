@@ -1,5 +1,5 @@
 // Q4_0 products against few rows (at most 64): passes over several sequences, prompts and prefill chunks of
-// some tokens, the experts of a few rows with f32 operands. Two arithmetics, one weight stream.
+// some tokens, the experts of a batch. Two arithmetics, one weight stream.
 //
 // Exact (the rows stay f32). An f32 input is exactly the sum of three bf16 values (8 significant bits
 // each, and bf16 has the range of f32), a quant minus 8 is exact in bf16, so the products of mma.m16n8k16 are
@@ -97,6 +97,7 @@ struct FewParams {
     uint32_t n_experts;
     uint32_t n_used;
     int gather;
+    uint32_t cap_groups;           // half: an expert's rows are packed from token group z * cap_groups on
 };
 
 __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
@@ -187,7 +188,6 @@ __device__ __forceinline__ bool find_group(const uint32_t* offsets, uint32_t n_e
 template <bool EXACT, bool EXPERTS, int NT, int W, int DEPTH>
 __global__ void __launch_bounds__(kThreads, 1) matmul_few_kernel(const __grid_constant__ FewParams p) {
     static_assert(!EXACT || NT == 1, "the pieces of more rows do not fit the registers");
-    static_assert(EXACT || !EXPERTS, "experts with half operands: kernels_matmul_experts.cu");
     constexpr uint32_t kTileSums = 128 * NT, kPieces = EXACT ? 3 : NT, T = tiles_per_step(NT), kTileSlot = W * kWarps * kPairBytes, kStepBytes = T * kTileSlot;
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ float sums[2][T * kTileSums];        // clusters: this CTA's sums of a step
@@ -356,8 +356,8 @@ __global__ void __launch_bounds__(kThreads, 1) matmul_few_kernel(const __grid_co
             if (t == 0) squares[warp][g] = square;
         }
     } else {
-        pdl_wait();
-        const uint32_t group0 = group * NT;
+        if (!EXPERTS) pdl_wait();
+        const uint32_t group0 = (EXPERTS ? expert * p.cap_groups : 0) + group * NT;
         const uint32_t groups = (n_tokens - token0 + 7) / 8;  // groups past the rows stay zero
 #pragma unroll
         for (int i = 0; i < W; ++i)
@@ -650,10 +650,7 @@ cudaError_t launch_as(cudaStream_t stream, FewParams& p, uint32_t groups) {
 }
 template <bool EXACT, int NT, int W, int DEPTH>
 cudaError_t launch(cudaStream_t stream, FewParams& p, uint32_t groups) {
-    if constexpr (EXACT) {
-        if (p.offsets) return launch_as<EXACT, true, NT, W, DEPTH>(stream, p, groups);
-    }
-    return launch_as<EXACT, false, NT, W, DEPTH>(stream, p, groups);
+    return p.offsets ? launch_as<EXACT, true, NT, W, DEPTH>(stream, p, groups) : launch_as<EXACT, false, NT, W, DEPTH>(stream, p, groups);
 }
 
 // Cut K: as few CTAs per cluster as hold the inputs at `most` pairs per warp, evenly.
@@ -674,9 +671,9 @@ cudaError_t launch_exact(cudaStream_t stream, FewParams& p) {
 }
 
 // Row groups of 8 a launch's CTA holds: the fewest that cover the rows in as few groups of 32 as possible
-// (33 rows: two groups of 24).
-cudaError_t launch_half(cudaStream_t stream, FewParams& p) {
-    const uint32_t rows = p.n_tokens, parts = (rows + kHalfGroup - 1) / kHalfGroup, nt = ((rows + parts - 1) / parts + 7) / 8;
+// (33 rows: two groups of 24). `rows`: those of the largest (expert: likely) batch.
+cudaError_t launch_half(cudaStream_t stream, FewParams& p, uint32_t rows) {
+    const uint32_t parts = (rows + kHalfGroup - 1) / kHalfGroup, nt = ((rows + parts - 1) / parts + 7) / 8;
     const uint32_t w = cut(p, nt <= 2 ? 3 : 2), groups = (p.n_tokens + 8 * (nt < 2 ? 2 : nt) - 1) / (8 * (nt < 2 ? 2 : nt));
     if (nt <= 2) {
         switch (w) {
@@ -798,7 +795,7 @@ cudaError_t matmul_few(cudaStream_t stream, const Mat* const* ws, float* const* 
     p.token_groups = ((n_tokens + 15u) & ~15u) / 8;
     p.n_tokens = n_tokens;
     p.store = store;
-    return launch_half(stream, p);
+    return launch_half(stream, p, n_tokens);
 }
 
 cudaError_t matmul_few_swiglu(cudaStream_t stream, const Mat& gate, const Mat& up, const void* packed, float* y, uint32_t n_tokens, uint32_t y_stride,
@@ -820,7 +817,43 @@ cudaError_t matmul_few_swiglu(cudaStream_t stream, const Mat& gate, const Mat& u
     p.n_tokens = n_tokens;
     p.store = BC_STORE_OVERWRITE;
     p.packed_out = static_cast<__half*>(packed_out);
-    return launch_half(stream, p);
+    return launch_half(stream, p, n_tokens);
+}
+
+// Experts: any number of tokens, as long as an expert gets a few of them on average (at most 64). Batches whose jobs fill the device
+// go to kernels_matmul_experts.cu first.
+bool matmul_few_experts_supported(const Mat& w, const Mat* up, uint32_t n_rows, uint32_t n_experts, uint32_t n_tokens, uint32_t n_used) {
+    return !few_disabled() && w.format == BC_Q4_0 && w.tiles != nullptr && n_tokens > 0 && w.n_cols % 64 == 0 && w.n_cols > 0 &&
+           w.n_cols / 64 <= kWarps * 2 * kMaxSlices && (!up || up->tiles != nullptr) && n_rows % 16 == 0 &&
+           (uint64_t)n_tokens * n_used <= (uint64_t)64 * n_experts;
+}
+
+cudaError_t matmul_few_experts(cudaStream_t stream, const Mat& w, const Mat* up, uint32_t n_rows, uint32_t n_experts, const void* packed,
+                               const uint32_t* offsets, const uint32_t* entries, float* y, uint32_t n_tokens, uint32_t n_entries) {
+    if (n_rows == 0 || n_experts == 0) return cudaSuccess;
+    FewParams p{};
+    p.n_segments = 1;
+    p.tiles[0] = static_cast<const uint8_t*>(w.tiles);
+    if (up) p.tiles[1] = static_cast<const uint8_t*>(up->tiles), p.dual = 1;
+    p.y[0] = y;
+    p.seg_rows[0] = p.seg_stride[0] = n_rows;
+    p.n_jobs = p.seg_tiles[0] = n_rows / 16;
+    p.n_pairs = w.n_cols / 64;
+    p.packed = static_cast<const uint4*>(packed);
+    p.cap_groups = ((n_tokens + 15u) & ~15u) / 8;
+    p.token_groups = n_experts * p.cap_groups;
+    p.n_tokens = n_tokens;  // an expert gets at most all of them
+    p.store = BC_STORE_OVERWRITE;
+    p.offsets = offsets;
+    p.entries = entries;
+    p.n_experts = n_experts;
+    p.n_used = 1;
+    // Groups of rows as wide as an expert's likely share, with room for the busier ones.
+    const uint32_t share = (n_entries + n_experts - 1) / n_experts;
+    uint32_t rows = share + 1;
+    while ((rows - share) * (rows - share) < share) ++rows;
+    rows = rows < n_tokens ? rows : n_tokens;
+    return launch_half(stream, p, rows < kHalfGroup ? rows : kHalfGroup);
 }
 
 }  // namespace k

@@ -993,14 +993,16 @@ uint64_t matmul_experts_scratch_bytes(uint32_t n_experts, uint32_t n_tokens, uin
 
 cudaError_t matmul_experts_umma(cudaStream_t stream, const Mat& w, const Mat* up, uint32_t n_rows, uint32_t n_experts, const float* x, bool gather,
                                 const uint32_t* offsets, const uint32_t* entries, uint32_t n_used, float* y, uint32_t n_tokens, void* scratch) {
-    if (n_tokens == 0 || n_rows == 0) return cudaSuccess;
-    if (matmul_experts_tiles_supported(w, up, n_rows))
+    if (n_tokens == 0 || n_rows == 0 || n_experts == 0) return cudaSuccess;
+    if (matmul_experts_tiles_supported(w, up, n_rows, n_experts, n_tokens, n_used))
         return matmul_experts_tiles(stream, w, up, n_rows, n_experts, x, gather, offsets, entries, n_used, y, n_tokens, scratch);
     const uint32_t cap_groups = ((n_tokens + 15u) & ~15u) / 8, total = n_tokens * n_used;
     const uint64_t outputs = (uint64_t)total * (w.n_cols / kChunkK) * kCores;
     cudaError_t err = launch_dependent(pack_grouped_kernel, dim3((unsigned)((outputs + 255) / 256)), dim3(256), 0, stream, x, static_cast<__half*>(scratch),
                                        offsets, entries, n_experts, n_used, gather ? 1 : 0, w.n_cols, cap_groups, total);
     if (err != cudaSuccess) return err;
+    if (matmul_few_experts_supported(w, up, n_rows, n_experts, n_tokens, n_used))
+        return matmul_few_experts(stream, w, up, n_rows, n_experts, scratch, offsets, entries, y, n_tokens, total);
     UmmaParams p{};
     p.quants[0] = static_cast<const uint4*>(w.data);
     p.scales[0] = w.scales;

@@ -410,7 +410,7 @@ struct Recorder {
             return;
         }
         run("moe_group", n, hp.n_experts, 0, 1, [&] { return k::moe_group(stream, s.route, s.expert_offsets, s.expert_entries, hp.n_experts, n_used, n); });
-        // Q4_0 experts run on the tensor-core kernel in its grouped mode, from a gathered fp16 packing.
+        // Q4_0 experts run on the tensor cores from a gathered fp16 packing.
         void* up_scratch = nullptr;
         void* down_scratch = nullptr;
         const bool tensor_up = tensor_products() && k::matmul_experts_umma_supported(D.gate, &D.up, n);
