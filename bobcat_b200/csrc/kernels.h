@@ -220,10 +220,11 @@ cudaError_t attention(cudaStream_t stream, const float* q, const void* k_cache, 
 int attention_launches(const float* q, const void* k_cache, const void* v_cache, bool kv_half, const float* scratch, const float* out, const AttentionShape& shape);
 // One decoded token of an attention layer: the launch normalises and rotates the raw q itself, and the
 // CTA whose chunk ends at the new position prepares that position's key
-// and value rows, stores them in the caches and uses them. Contexts beyond 2048 positions take a combine
-// pass of its own. Covers heads of 64, 128 or 256 elements rotated whole, 16-byte aligned rows; long contexts: half-precision caches.
+// and value rows, stores them in the caches and uses them. Sequences opened for more than 2048 positions of heads of 64 elements (1024 of
+// 128, 512 of 256) and models of many KV heads take a combine pass of its own. Covers heads of 64, 128 or 256 elements rotated whole, 16-byte aligned
+// rows; with the combine pass half-precision caches.
 bool attention_step_supported(const RopeStore& r, const AttentionShape& shape);
-int attention_step_launches(const AttentionShape& shape);
+int attention_step_launches(const RopeStore& r, const AttentionShape& shape);
 cudaError_t attention_step(cudaStream_t stream, const RopeStore& r, float* scratch, float* out, const AttentionShape& shape);
 // The tensor-core prefill kernel (kernels_attention_flash.cu): heads of 64 elements, f16 cache, at
 // least 32 queries, positions known at launch. `attention` picks it when it applies.

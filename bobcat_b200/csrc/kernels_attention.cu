@@ -435,7 +435,8 @@ const void* decode_kernel(bool kv_half, const AttentionShape& s, const float* q,
 // arithmetic and the order of attention_decode_kernel; a chunk's partial sums go straight to the shared memory of the CTA
 // that combines the head (one head per CTA, group <= 4), in the order of attention_combine_kernel, so the result is the same to the bit. A
 // cluster covers 32 chunks at a time.
-// Eight CTAs are the portable cluster; contexts beyond kTokenChunks chunks keep the two launches, whose grid covers the device.
+// Eight CTAs are the portable cluster; contexts beyond kTokenChunks chunks and more KV heads than clusters that run at once keep the two launches, whose
+// grid covers the device (token_shape).
 //
 // An f32 cache used to take rope_store_kernel, attention_chunk_kernel and the combine (14 us).
 constexpr uint32_t kTokenCluster = 8, kTokenTeams = 4, kTokenThreads = kTokenTeams * kDecodeThreads, kTokenChunks = 128;
@@ -724,13 +725,22 @@ size_t token_bytes(const AttentionShape& s) {
            (size_t)chunks * (s.head_dim + 2) * sizeof(float);
 }
 
-// One query over a context of at most four passes of a cluster's warps: a pass covers 32 chunks of heads of 64 elements, 8 of 256. Measured
-// in us per generated token, two launches and one: 350M, f32 cache (8 KV heads of 64) at position 128 358 and 294, 512 354 and 300,
-// 1900 429 and 332, half cache 304 and 286, 365 and 320; 2.6B 128 767 and 741, 1900 878 and 819; two KV heads of 256, 128 842 and
-// 812, but 512 835 and 845, 1000 857 and 878.
-bool token_shape(const AttentionShape& s) {
-    return s.n_queries == 1 && (s.head_dim == 64 || s.head_dim == 128 || s.head_dim == 256) && s.q_stride % 4 == 0 && s.q_head_stride % 4 == 0 &&
-           s.n_heads / s.n_kv_heads <= kTokenGroup && s.n_ctx <= kTokenChunks * kDecodeChunk / (s.head_dim / 64);
+// One query over a context (what the sequence holds, not where it stands) of at most four passes of a cluster's warps: a pass covers 32 chunks of heads of 64
+// elements, 8 of 256. `fused`: a decoded step with its norms, rotation and cache rows.
+// Measured, us a layer, two launches (f32 caches: three) and one. Fused, contexts just beyond the position: 8 KV heads of 64, two query heads each, position 127
+// 18.9 and 16.3, 1980 29.7 and 22.3, f32 24.7 and 16.6, 37.9 and 23.6; four query heads each 22.8 and 18.4, at 800 the least, 0.97 of the time. Clusters of eight lie
+// inside a GPC, so sixteen do not run at once: 16 KV heads of 64 18.3 and 19.3, 32 20.3 and 24.1, of 128 21.6 and 22.1; over an f32 cache 24.4 and 19.4, 27.4 and
+// 24.9, because a launch more is saved. Not fused, a half cache: up to 32 chunks 0.7 to 0.95 of the time, from 33 to 64 up to 1.3 (two rounds of a
+// cluster's chunks against one of the device's), beyond 64 (whose combine pass takes longer) 0.6 to 0.9, with four query heads each on two or four KV heads up to 1.15; 16 KV heads and more
+// up to 1.8. An f32 cache: 0.3 to 1.0 with up to 12 KV heads, 0.5 to 1.0 with up to two query heads each on up to 24, else up to 1.4.
+bool token_shape(const AttentionShape& s, bool kv_half, bool fused) {
+    if (s.n_queries != 1 || (s.head_dim != 64 && s.head_dim != 128 && s.head_dim != 256) || s.q_stride % 4 != 0 || s.q_head_stride % 4 != 0) return false;
+    const uint32_t group = s.n_heads / s.n_kv_heads;
+    if (group > kTokenGroup || s.n_ctx > kTokenChunks * kDecodeChunk / (s.head_dim / 64)) return false;
+    const bool at_once = s.n_kv_heads * kTokenCluster * 5 <= (uint32_t)sm_count() * 4;  // 14 KV heads on 148 SMs
+    if (!kv_half) return at_once || (group <= 2 && (fused || s.n_kv_heads <= 24));
+    if (!at_once || fused) return at_once;
+    return s.n_ctx <= 32 * kDecodeChunk || (s.n_ctx > 64 * kDecodeChunk && (group <= 2 || s.n_kv_heads >= 8));
 }
 
 // `cp.scratch` is the output.
@@ -862,15 +872,15 @@ namespace {
 bool flash_route(const float* q, const void* k_cache, const void* v_cache, bool kv_half, const float* out, const AttentionShape& s) {
     return ((uintptr_t)q | (uintptr_t)out) % 8 == 0 && ((uintptr_t)k_cache | (uintptr_t)v_cache) % 16 == 0 && attention_flash_supported(kv_half, s);
 }
-bool token_route(const float* q, const void* k_cache, const void* v_cache, const AttentionShape& s) {
-    return token_shape(s) && ((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache) % 16 == 0;
+bool token_route(const float* q, const void* k_cache, const void* v_cache, bool kv_half, const AttentionShape& s) {
+    return token_shape(s, kv_half, false) && ((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache) % 16 == 0;
 }
 }  // namespace
 
 int attention_launches(const float* q, const void* k_cache, const void* v_cache, bool kv_half, const float* scratch, const float* out, const AttentionShape& s) {
     if (s.n_queries == 0) return 0;
     if (flash_route(q, k_cache, v_cache, kv_half, out, s)) return attention_flash_launches(scratch, s);
-    if (token_route(q, k_cache, v_cache, s)) return 1;
+    if (token_route(q, k_cache, v_cache, kv_half, s)) return 1;
     return 2 * (int)((s.n_queries + kQueryBatch - 1) / kQueryBatch);
 }
 
@@ -878,7 +888,7 @@ cudaError_t attention(cudaStream_t stream, const float* q, const void* k_cache, 
                       float* scratch, float* out, const AttentionShape& s) {
     if (s.n_queries == 0) return cudaSuccess;
     if (flash_route(q, k_cache, v_cache, kv_half, out, s)) return attention_flash(stream, q, k_cache, v_cache, scratch, out, s);
-    if (token_route(q, k_cache, v_cache, s)) {
+    if (token_route(q, k_cache, v_cache, kv_half, s)) {
         const ChunkParams cp{q, k_cache, v_cache, out, s.n_heads, s.n_kv_heads, s.head_dim, s.first_pos, s.n_ctx,
                              s.q_stride, s.q_head_stride, 0, 0, s.pos_ptr, (uint32_t)kDecodeChunk, nullptr, nullptr, nullptr, nullptr, 0.f, 0.f, nullptr};
         return launch_token(stream, cp, s, kv_half, false, s.gated);
@@ -917,14 +927,14 @@ cudaError_t attention(cudaStream_t stream, const float* q, const void* k_cache, 
 }
 
 bool attention_step_supported(const RopeStore& r, const AttentionShape& s) {
-    return (token_shape(s) || (r.kv_half && s.n_queries == 1 && decode_shape(true, s))) && r.n_rot == s.head_dim && r.q_head_stride == s.q_head_stride &&
+    return (token_shape(s, r.kv_half, true) || (r.kv_half && s.n_queries == 1 && decode_shape(true, s))) && r.n_rot == s.head_dim && r.q_head_stride == s.q_head_stride &&
            ((uintptr_t)r.q | (uintptr_t)r.k | (uintptr_t)r.v | (uintptr_t)r.k_cache | (uintptr_t)r.v_cache) % 16 == 0;
 }
 
-int attention_step_launches(const AttentionShape& s) { return token_shape(s) ? 1 : 2; }
+int attention_step_launches(const RopeStore& r, const AttentionShape& s) { return token_shape(s, r.kv_half, true) ? 1 : 2; }
 
 cudaError_t attention_step(cudaStream_t stream, const RopeStore& r, float* scratch, float* out, const AttentionShape& s) {
-    if (token_shape(s)) {
+    if (token_shape(s, r.kv_half, true)) {
         const ChunkParams cp{r.q, r.k_cache, r.v_cache, out, s.n_heads, s.n_kv_heads, s.head_dim, s.first_pos, s.n_ctx,
                              s.q_stride, s.q_head_stride, 0, 0, s.pos_ptr, (uint32_t)kDecodeChunk, r.k, r.v, r.q_norm, r.k_norm, r.eps, r.theta, r.table};
         return launch_token(stream, cp, s, r.kv_half, true, s.gated);

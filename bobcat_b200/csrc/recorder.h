@@ -354,7 +354,7 @@ struct Recorder {
         uint64_t kv_bytes = (uint64_t)(pos + 1) * kv_dim() * kv_element_bytes() * 2;
         shape.gated = gated;
         if (k::attention_step_supported(rs, shape)) {
-            run("attention_step", 1, pos + 1, kv_bytes, k::attention_step_launches(shape), [&] { return k::attention_step(stream, rs, s.scores, s.attn, shape); });
+            run("attention_step", 1, pos + 1, kv_bytes, k::attention_step_launches(rs, shape), [&] { return k::attention_step(stream, rs, s.scores, s.attn, shape); });
             return;
         }
         run("rope_store", hp.n_heads + 2 * hp.n_kv_heads, hp.head_dim, 0, 1, [&] { return k::rope_store(stream, rs, p); });

@@ -38,3 +38,11 @@ def test_one_query(kv_half, heads, kv_heads, hd, pos, n_ctx):
     # The bound of the other float32 attention kernels on inputs of this size (test_ops_gpu.py).
     assert np.abs(got - want).max() < 2e-6
     cuda.close()
+
+
+@pytest.mark.parametrize("kv_half", [True, False])
+@pytest.mark.parametrize("heads, kv_heads, hd", [(14, 14, 64), (30, 15, 64), (64, 16, 64), (24, 24, 128), (32, 32, 64), (8, 2, 64)])
+@pytest.mark.parametrize("pos, n_ctx", [(100, 512), (512, 513), (1000, 1024), (1000, 1025)])
+def test_either_side_of_the_lines(kv_half, heads, kv_heads, hd, pos, n_ctx):
+    """Many KV heads, whose clusters do not run at once, and contexts of 33 to 64 chunks of a half cache take two launches."""
+    test_one_query(kv_half, heads, kv_heads, hd, pos, n_ctx)
