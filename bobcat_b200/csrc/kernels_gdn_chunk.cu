@@ -19,8 +19,9 @@
 // are independent, so nothing is exchanged. Its multiply-adds, 0.95 M per chunk and CTA against 128 per cycle, are 4 us; the reads of their
 // operands from shared memory (128 bytes per cycle into registers, whether lanes share them or not) bound it: register tiles of 4 x 4, from
 // rows padded to keep the reads free of bank conflicts, take as long as the reads. The next chunk arrives by cp.async while this one is
-// computed. After its wait a launch of one chunk takes 12.3 us (17.7 before the outputs' rows went to warps that lie in one
-// block and the loops were unrolled further); a lane per column for the other products too: 16.2.
+// computed. One chunk of 64 tokens takes 21.5 us of both launches in a chain of them, 512 tokens 111 (26.4 and 117 before the outputs' rows went to warps that lie in
+// one block, the loops were unrolled further and the preparation below got its copies and straight-line decays). By the device's timer after the wait this
+// kernel's part is 12.3 us, with a lane per column for the other products too 16.2; with cold caches under ncu a launch of it is no quicker than before (17.5 and 18.0).
 
 #include <type_traits>
 

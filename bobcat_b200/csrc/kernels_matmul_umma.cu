@@ -166,7 +166,8 @@ __global__ void __launch_bounds__(256) pack_kernel(const float* __restrict__ x, 
 // 8 CTAs repeating the sums; 4 tokens per CTA with the partial sums) read rows twice: 512 tokens of 4096 took 13.0 us
 // plain and 19.0 us with four partial sums, then 8.2 and 10.7; 64 tokens of 2048 with a reduce_kernel before it 7.0, then 4.9. The norm's
 // weights are on their way before the wait and two of a thread's quads with all their partial sums at once: a scoring
-// request of 24-token suffixes (354 of these launches) 11.52 -> 11.26 ms, 32 chunks of 64 tokens (1504) 72.9 -> 71.8 ms.
+// request of 24-token suffixes (354 of these launches) 11.52 -> 11.26 ms, 32 chunks of 64 tokens (1504) 72.9 -> 71.8 ms; 512 tokens of 2048 gain nothing (under ncu, with
+// cold caches, 7.5 -> 7.8 us with partial sums, 6.0 -> 5.6 without; the prompt of 60 such launches takes the same time).
 template <bool ADD>
 __global__ void __launch_bounds__(256) pack_norm_kernel(float* __restrict__ x, const float* __restrict__ weight, float eps, __half* __restrict__ packed,
                                                         uint32_t n_tokens, uint32_t n_cols, uint32_t token_groups, const float* __restrict__ partial,
