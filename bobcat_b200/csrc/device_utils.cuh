@@ -43,10 +43,12 @@ __device__ __forceinline__ float block_sum(float v, float* scratch) {
     return warp_sum(total);
 }
 
-// The index of the first maximum of x[0 .. n), by a cluster of kArgmaxCluster CTAs of kArgmaxThreads threads that all call
+// The index of the first maximum of x[0 .. n), by a cluster of CTAS CTAs (or one CTA, not launched as a cluster) of kArgmaxThreads threads that all call
 // this; thread 0 of the first CTA receives it. One SM reads 65536 floats out of L2 in 5 us and a row of 65536 one float at a time in 28:
-// each CTA takes an eighth, in 16-byte loads that are all on their way at once.
+// each CTA of eight takes an eighth, in 16-byte loads that are all on their way at once. Up to kArgmaxAlone values the cluster's barriers cost more than
+// they save (512 values 2.5 us, by one CTA 1.6; 4096 2.6 and 1.8; 16384 2.6, by one CTA of 1024 threads 2.7).
 constexpr unsigned kArgmaxCluster = 8, kArgmaxThreads = 512;
+constexpr uint32_t kArgmaxAlone = 8192;
 __device__ __forceinline__ bool argmax_better(float v, uint32_t i, float bv, uint32_t bi) {
     return i != 0xffffffffu && (bi == 0xffffffffu || v > bv || (v == bv && i < bi));
 }
@@ -61,14 +63,15 @@ __device__ __forceinline__ void argmax_lanes(float& value, uint32_t& index) {
         }
     }
 }
+template <unsigned CTAS>
 __device__ __forceinline__ uint32_t argmax_cluster(const float* __restrict__ x, uint32_t n) {
     constexpr uint32_t kLoads = 4, kWarps = kArgmaxThreads / 32;
-    __shared__ float best_value[kWarps], cta_value[kArgmaxCluster];
-    __shared__ uint32_t best_index[kWarps], cta_index[kArgmaxCluster];
-    asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");  // this CTA runs: its shared memory may be written
+    __shared__ float best_value[kWarps], cta_value[CTAS];
+    __shared__ uint32_t best_index[kWarps], cta_index[CTAS];
+    if constexpr (CTAS > 1) asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");  // this CTA runs: its shared memory may be written
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    uint32_t rank;
-    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    uint32_t rank = 0;
+    if constexpr (CTAS > 1) asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
     float value = -INFINITY;
     uint32_t index = 0xffffffffu;
     auto consider = [&](float v, uint32_t i) {  // in increasing index order, so the first maximum wins
@@ -77,7 +80,7 @@ __device__ __forceinline__ uint32_t argmax_cluster(const float* __restrict__ x, 
             index = i;
         }
     };
-    const uint32_t n4 = (reinterpret_cast<uintptr_t>(x) & 15) == 0 ? n / 4 : 0, share = (n4 + kArgmaxCluster - 1) / kArgmaxCluster;
+    const uint32_t n4 = (reinterpret_cast<uintptr_t>(x) & 15) == 0 ? n / 4 : 0, share = (n4 + CTAS - 1) / CTAS;
     const uint32_t from = min(rank * share, n4), to = min(from + share, n4);
     const float4* x4 = reinterpret_cast<const float4*>(x);
     for (uint32_t base = from + tid; base < to; base += kArgmaxThreads * kLoads) {
@@ -94,32 +97,36 @@ __device__ __forceinline__ uint32_t argmax_cluster(const float* __restrict__ x, 
             consider(v[k].w, 4 * i + 3);
         }
     }
-    for (uint32_t i = 4 * n4 + rank * kArgmaxThreads + tid; i < n; i += kArgmaxCluster * kArgmaxThreads) consider(x[i], i);
+    for (uint32_t i = 4 * n4 + rank * kArgmaxThreads + tid; i < n; i += CTAS * kArgmaxThreads) consider(x[i], i);
     argmax_lanes(value, index);
     if (lane == 0) {
         best_value[warp] = value;
         best_index[warp] = index;
     }
     __syncthreads();
-    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    if constexpr (CTAS > 1) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
     if (warp == 0) {
         value = lane < kWarps ? best_value[lane] : -INFINITY;
         index = lane < kWarps ? best_index[lane] : 0xffffffffu;
         argmax_lanes(value, index);
-        if (lane == 0) {
-            uint32_t value_at, index_at;
-            asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(value_at) : "r"((uint32_t)__cvta_generic_to_shared(&cta_value[rank])));
-            asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(index_at) : "r"((uint32_t)__cvta_generic_to_shared(&cta_index[rank])));
-            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(value_at), "f"(value) : "memory");
-            asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(index_at), "r"(index) : "memory");
+        if constexpr (CTAS > 1) {
+            if (lane == 0) {
+                uint32_t value_at, index_at;
+                asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(value_at) : "r"((uint32_t)__cvta_generic_to_shared(&cta_value[rank])));
+                asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(index_at) : "r"((uint32_t)__cvta_generic_to_shared(&cta_index[rank])));
+                asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(value_at), "f"(value) : "memory");
+                asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(index_at), "r"(index) : "memory");
+            }
+            __syncwarp();
         }
-        __syncwarp();
     }
-    asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
-    if (rank == 0 && warp == 0) {
-        value = lane < kArgmaxCluster ? cta_value[lane] : -INFINITY;
-        index = lane < kArgmaxCluster ? cta_index[lane] : 0xffffffffu;
-        argmax_lanes(value, index);
+    if constexpr (CTAS > 1) {
+        asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+        if (rank == 0 && warp == 0) {
+            value = lane < CTAS ? cta_value[lane] : -INFINITY;
+            index = lane < CTAS ? cta_index[lane] : 0xffffffffu;
+            argmax_lanes(value, index);
+        }
     }
     return index;
 }

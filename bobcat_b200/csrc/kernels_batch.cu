@@ -201,14 +201,15 @@ __global__ void short_conv_seqs_kernel(const float* __restrict__ bcx, const floa
     out[(uint64_t)b * n_embd + ch] = c * sum;
 }
 
-// argmax of each row (ties to the lowest index): a cluster per sequence. picked[b] takes the index and,
+// argmax of each row (ties to the lowest index): a cluster (or a CTA) per sequence. picked[b] takes the index and,
 // when `record` is non-null, so does record[b * record_stride + record_at].
+template <unsigned CTAS>
 __global__ void __launch_bounds__(kArgmaxThreads) argmax_rows_kernel(const float* __restrict__ x, uint32_t n, uint32_t* __restrict__ picked,
                                                                      uint32_t* __restrict__ record, uint32_t record_stride, uint32_t record_at) {
     pdl_launch_dependents();
     pdl_wait();
-    const uint32_t row = blockIdx.x / kArgmaxCluster, index = argmax_cluster(x + (uint64_t)row * n, n);
-    if (blockIdx.x % kArgmaxCluster == 0 && threadIdx.x == 0) {
+    const uint32_t row = blockIdx.x / CTAS, index = argmax_cluster<CTAS>(x + (uint64_t)row * n, n);
+    if (blockIdx.x % CTAS == 0 && threadIdx.x == 0) {
         picked[row] = index;
         if (record) record[(uint64_t)row * record_stride + record_at] = index;
     }
@@ -260,7 +261,9 @@ cudaError_t short_conv_seqs(cudaStream_t stream, const float* bcx, const float* 
 
 cudaError_t argmax_rows(cudaStream_t stream, const float* x, uint32_t n, uint32_t n_rows, uint32_t* picked, uint32_t* record,
                         uint32_t record_stride, uint32_t record_at) {
-    return launch_clusters(argmax_rows_kernel, dim3(kArgmaxCluster * n_rows), dim3(kArgmaxThreads), kArgmaxCluster, stream, x, n, picked, record, record_stride, record_at);
+    if (n <= kArgmaxAlone)
+        return launch_dependent(argmax_rows_kernel<1>, dim3(n_rows), dim3(kArgmaxThreads), 0, stream, x, n, picked, record, record_stride, record_at);
+    return launch_clusters(argmax_rows_kernel<kArgmaxCluster>, dim3(kArgmaxCluster * n_rows), dim3(kArgmaxThreads), kArgmaxCluster, stream, x, n, picked, record, record_stride, record_at);
 }
 
 cudaError_t advance_seqs(cudaStream_t stream, uint32_t* pos, uint32_t n_seqs) {

@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(128) short_conv_kernel(const float* __restrict
     }
 }
 
-// One cluster scans the vocabulary; ties go to the lowest index.
+// One cluster (or a CTA) scans the vocabulary; ties go to the lowest index.
 struct ArgmaxOut {
     uint32_t* out;       // direct mode: the word to write
     uint32_t* readback;  // direct mode: optional host-mapped copy
@@ -318,10 +318,11 @@ struct ArgmaxOut {
     uint32_t ring_slots;
 };
 
+template <unsigned CTAS>
 __global__ void __launch_bounds__(kArgmaxThreads) argmax_kernel(const float* __restrict__ x, uint32_t n, ArgmaxOut o) {
     pdl_launch_dependents();
     pdl_wait();
-    const uint32_t index = argmax_cluster(x, n);
+    const uint32_t index = argmax_cluster<CTAS>(x, n);
     if (blockIdx.x != 0 || threadIdx.x != 0) return;
     if (o.counter) {
         uint32_t pos = *o.counter;
@@ -603,15 +604,22 @@ cudaError_t short_conv(cudaStream_t stream, const float* bcx, const float* taps,
     return wide ? launch(short_conv_kernel<9, 4>, 4, 8) : launch(short_conv_kernel<9, 1>, 1, 8);
 }
 
+namespace {
+cudaError_t launch_argmax(cudaStream_t stream, const float* x, uint32_t n, const ArgmaxOut& o) {
+    if (n <= kArgmaxAlone) return launch_dependent(argmax_kernel<1>, dim3(1), dim3(kArgmaxThreads), 0, stream, x, n, o);
+    return launch_clusters(argmax_kernel<kArgmaxCluster>, dim3(kArgmaxCluster), dim3(kArgmaxThreads), kArgmaxCluster, stream, x, n, o);
+}
+}  // namespace
+
 cudaError_t argmax(cudaStream_t stream, const float* x, uint32_t n, uint32_t* out, uint32_t* readback) {
     const ArgmaxOut o{out, readback, nullptr, 0, nullptr, 0, nullptr, 1};
-    return launch_clusters(argmax_kernel, dim3(kArgmaxCluster), dim3(kArgmaxThreads), kArgmaxCluster, stream, x, n, o);
+    return launch_argmax(stream, x, n, o);
 }
 
 cudaError_t argmax_step(cudaStream_t stream, const float* x, uint32_t n, uint32_t* counter, bool advance, uint32_t* tokens,
                         uint32_t offset, uint32_t* ring, uint32_t ring_slots) {
     const ArgmaxOut o{nullptr, nullptr, counter, advance ? 1 : 0, tokens, offset, ring, ring_slots ? ring_slots : 1};
-    return launch_clusters(argmax_kernel, dim3(kArgmaxCluster), dim3(kArgmaxThreads), kArgmaxCluster, stream, x, n, o);
+    return launch_argmax(stream, x, n, o);
 }
 
 cudaError_t add_floats(cudaStream_t stream, float* y, const float* x, uint64_t n) {

@@ -1,4 +1,4 @@
-"""The vocabulary's argmax, cut over a cluster's CTAs: every place a share or a 16-byte load ends, rows that do not
+"""The vocabulary's argmax, by one CTA up to 8192 values and cut over a cluster's CTAs beyond: every place a share or a 16-byte load ends, rows that do not
 start on 16 bytes, ties in different shares, -inf everywhere."""
 
 import numpy as np
@@ -9,7 +9,7 @@ from bobcat_b200 import Cuda
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [1, 3, 4, 31, 33, 4096, 65536, 65539, 100003])
+@pytest.mark.parametrize("n", [1, 3, 4, 31, 33, 4096, 8191, 8192, 8193, 65536, 65539, 100003])
 @pytest.mark.parametrize("shift", [0, 1])
 def test_argmax(n, shift):
     cuda = Cuda.open(0)
